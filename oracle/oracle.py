@@ -25,7 +25,7 @@ def build(ref: bool = False) -> None:
     """Builds liboracle.so (and the reference binary if `ref` and its
     sources are present)."""
     subprocess.run(["make", "-s", "-C", str(HERE), "liboracle.so"], check=True)
-    if ref and Path(os.environ.get("FAP_REFERENCE_DIR", "/root/reference")).exists():
+    if ref and Path(os.environ.get("FAP_REFERENCE_DIR", "/root/reference"), "fap", "fap.cpp").exists():
         subprocess.run(["make", "-s", "-C", str(HERE), "ref",
                         "REF=" + os.environ.get("FAP_REFERENCE_DIR", "/root/reference")], check=True)
 
