@@ -529,60 +529,56 @@ void fw_segments(void *D, int32_t *P, int64_t ld, int size, int r, MpSegment &ro
   t_rest = pairs * pairs;
 }
 
-// CTAs of an FW segment in the strip form (tiles_y row tiles).
-int fw_strips_of(const MpSegment &s, int tiles_y) {
-  const int T = fapk::fw_strip_tiles();
-  return tiles_y * ((s.tiles_x + T - 1) / T);
+// Numbers the CTAs of one launch's FW segments in the strip form, with the
+// strip length that suits the launch; returns their count.
+int fw_number_strips(std::vector<MpSegment> &segs, int sm_count) {
+  const int T = fapk::fw_strip_tiles(segs.data(), (int)segs.size(), sm_count);
+  int strips = 0;
+  for (MpSegment &s : segs) {
+    s.strip_tiles = T;
+    s.strip_begin = strips;
+    strips += fapk::fw_strips_of(s, T);
+  }
+  return strips;
 }
 
 // FP32 form: fw_segments' two panels of pivot block r of nb as strip-form
-// segments, appended to `out` from CTA `strips` on.  Each reads and writes
+// segments, appended to `out`.  Each reads and writes
 // the same entries (the row panel is B and C, the column panel A and C); a
 // CTA reads the entries it writes into shared memory before its epilogue,
 // and no two CTAs write the same entries.
-void fw_panel_strips(const MpSegment &rowp, const MpSegment &colp, int nb, std::vector<MpSegment> &out,
-                     int &strips) {
-  MpSegment a = rowp, c = colp;
-  a.strip_begin = strips;
-  strips += fw_strips_of(rowp, 1);
-  out.push_back(a);
-  c.strip_begin = strips;
-  strips += fw_strips_of(colp, nb / 2);  // (nb - 1) row blocks in pairs
-  out.push_back(c);
+void fw_panel_strips(const MpSegment &rowp, const MpSegment &colp, std::vector<MpSegment> &out) {
+  out.push_back(rowp);
+  out.push_back(colp);
 }
 
 // Lookahead form of fw_segments' `rest` for pivot block r of nb: the rows and
 // columns other than r and r + 1 (block row and column r + 1 get round r's
-// update inside pivot step r + 1).  Returns its CTAs in the strip form.
-int fw_rest_lookahead(MpSegment &rest, int nb, int r) {
+// update inside pivot step r + 1).
+void fw_rest_lookahead(MpSegment &rest, int nb, int r) {
   const int pairs = (nb - 2 + 1) / 2;
   rest.row_skip2 = r + 1;
   rest.col_skip2 = r + 1;
   rest.tiles_x = pairs;
-  return fw_strips_of(rest, pairs);
 }
 
 // FP32 form with lookahead: round r - 1's update of block row and column r
 // of nb (r >= 1; the tiles that fw_rest_lookahead leaves out of round
-// r - 1) as strip-form segments appended to `out` from CTA `strips` on:
+// r - 1) as strip-form segments appended to `out`:
 // block row r over the columns other than r - 1 (the pivot block (r, r)
 // with them), and block column r over the rows other than r - 1 and r.  The
 // two write disjoint blocks and read block row and column r - 1 only, which
 // neither writes; no tile reads entries it or another tile writes.
 void fw_look_strips(void *D, int32_t *P, int64_t ld, int size, int r, int nb, int32_t tmap1,
-                    std::vector<MpSegment> &out, int &strips) {
+                    std::vector<MpSegment> &out) {
   MpSegment rowp, colp, rest;
   int t1, t2, t3;
   fw_segments(D, P, ld, size, r - 1, rowp, colp, rest, t1, t2, t3, true, tmap1);
   rowp.row_fix = r;  // (the row panel of pivot r - 1, moved to block row r)
-  rowp.strip_begin = strips;
-  strips += fw_strips_of(rowp, 1);
   out.push_back(rowp);
   if (nb > 2) {
     colp.col_fix = r;  // (the column panel, moved to block column r, without row r)
     colp.row_skip2 = r;
-    colp.strip_begin = strips;
-    strips += fw_strips_of(colp, (nb - 1) / 2);  // (nb - 2) row blocks in pairs
     out.push_back(colp);
   }
 }
@@ -864,7 +860,7 @@ int build_plan(fap_engine *e, Plan &pl) {
     for (int r = 0; r < maxnb; r++) {
       std::vector<FwDiagJob> dj;
       std::vector<MpSegment> ps, rs, r2s, pss, ls;
-      int pt = 0, rt = 0, r2strips = 0, psstrips = 0, lstrips = 0;
+      int pt = 0, rt = 0;
       for (size_t pi = 0; pi < pdesc.size(); pi++) {
         const PartDesc &d = pdesc[pi];
         int nb = d.ld / B;
@@ -888,7 +884,7 @@ int build_plan(fap_engine *e, Plan &pl) {
           MpSegment rp, cp, rest;
           int a1, a2, a3;
           fw_segments(D, P, d.ld, d.ld, r, rp, cp, rest, a1, a2, a3, e->f32(), tmap1[pi]);
-          if (e->f32() && r > 0) fw_look_strips(D, P, d.ld, d.ld, r, nb, tmap1[pi], ls, lstrips);
+          if (e->f32() && r > 0) fw_look_strips(D, P, d.ld, d.ld, r, nb, tmap1[pi], ls);
           rp.tile_begin = pt;
           pt += a1;
           ps.push_back(rp);
@@ -898,16 +894,14 @@ int build_plan(fap_engine *e, Plan &pl) {
           rest.tile_begin = rt;
           rt += a3;
           rs.push_back(rest);
-          fw_panel_strips(rp, cp, nb, pss, psstrips);
-          MpSegment rest2 = rest;
-          const int s2 = r + 1 < nb ? fw_rest_lookahead(rest2, nb, r) : fw_strips_of(rest, rest.tiles_x);
-          if (s2 > 0) {
-            rest2.strip_begin = r2strips;
-            r2strips += s2;
-            r2s.push_back(rest2);
-          }
+          fw_panel_strips(rp, cp, pss);
+          if (r + 1 < nb) fw_rest_lookahead(rest, nb, r);
+          if (rest.tiles_x > 0) r2s.push_back(rest);
         }
       }
+      const int r2strips = fw_number_strips(r2s, e->sm_count);
+      const int psstrips = fw_number_strips(pss, e->sm_count);
+      const int lstrips = fw_number_strips(ls, e->sm_count);
       G.diag_cnt[r] = (int)dj.size();
       O.diag[r] = tb.add(dj.data(), dj.size());
       G.panel_nseg[r] = (int)ps.size();
@@ -2333,7 +2327,7 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
   for (int r = 0; r < maxnb; r++) {
     std::vector<FwDiagJob> dj;
     std::vector<MpSegment> ps, rs, r2s, pss, ls;
-    int pt = 0, rt = 0, r2strips = 0, psstrips = 0, lstrips = 0;
+    int pt = 0, rt = 0;
     for (int32_t b = 0; b < count; b++) {
       int nb = (sizes[b] + Bk - 1) / Bk;
       if (r >= nb) continue;
@@ -2351,7 +2345,7 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
         fw_segments(D[b], pred ? P[b] : nullptr, ld[b], sizes[b], r, a, c, rest, t1, t2, t3,
                     dtype == FAP_DTYPE_F32, tmap1[b]);
         if (dtype == FAP_DTYPE_F32 && r > 0)
-          fw_look_strips(D[b], pred ? P[b] : nullptr, ld[b], sizes[b], r, nb, tmap1[b], ls, lstrips);
+          fw_look_strips(D[b], pred ? P[b] : nullptr, ld[b], sizes[b], r, nb, tmap1[b], ls);
         a.tile_begin = pt;
         pt += t1;
         ps.push_back(a);
@@ -2361,16 +2355,14 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
         rest.tile_begin = rt;
         rt += t3;
         rs.push_back(rest);
-        fw_panel_strips(a, c, nb, pss, psstrips);
-        MpSegment rest2 = rest;
-        const int s2 = r + 1 < nb ? fw_rest_lookahead(rest2, nb, r) : fw_strips_of(rest, rest.tiles_x);
-        if (s2 > 0) {
-          rest2.strip_begin = r2strips;
-          r2strips += s2;
-          r2s.push_back(rest2);
-        }
+        fw_panel_strips(a, c, pss);
+        if (r + 1 < nb) fw_rest_lookahead(rest, nb, r);
+        if (rest.tiles_x > 0) r2s.push_back(rest);
       }
     }
+    const int r2strips = fw_number_strips(r2s, e->sm_count);
+    const int psstrips = fw_number_strips(pss, e->sm_count);
+    const int lstrips = fw_number_strips(ls, e->sm_count);
     nr2[r] = (int)r2s.size();
     sr2[r] = r2strips;
     or2[r] = tb.add(r2s.data(), r2s.size());

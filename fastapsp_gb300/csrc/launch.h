@@ -37,7 +37,7 @@ int minplus_strip_class_cols(int c);
 int minplus_strip_tiles();
 // Strip form of the FW remaining-tile phase (packed int32, or FP32 with
 // f32; init_from_c = 1, K <= 64): CTAs numbered by MpSegment::strip_begin,
-// tiles_y x ceil(tiles_x / fw_strip_tiles()) strips per segment.  tmaps:
+// fw_strips_of(segment, strip_tiles) per segment.  tmaps:
 // device array of CUtensorMap pairs (distances, predecessors) indexed by
 // MpSegment::tmap1 - 1 (64-byte aligned; null: no segment uses one).
 cudaError_t launch_fw_strips(bool pred, const MpSegment *d_segs, int nseg, int strips,
@@ -51,7 +51,8 @@ cudaError_t tma_status(unsigned *out, bool reset);
 // the copy unit's alignment rules (16-byte base and row stride) or the
 // driver has no encoder.
 bool encode_fw_tmaps(void *out, const void *d, const void *p, int64_t ld, int rows, int cols);
-int fw_strip_tiles();
+int fw_strips_of(const MpSegment &s, int tiles);  // CTAs of a segment with that many column tiles each
+int fw_strip_tiles(const MpSegment *segs, int nseg, int sm_count);  // column tiles per CTA for a launch of these
 int minplus_strip_max_k();   // largest K of the strip form
 // Segments go to the strip form in classes of K (one launch per class, each
 // with its own CTAs per SM): class c takes K <= minplus_strip_class_k(c)

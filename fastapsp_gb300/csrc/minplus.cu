@@ -138,7 +138,7 @@ __device__ __forceinline__ int list_block(int g, int skip, int skip2, int fix, i
 }
 
 // Length of such a list.
-__device__ __forceinline__ int list_len(int skip, int skip2, int fix, int nblocks) {
+__host__ __device__ __forceinline__ int list_len(int skip, int skip2, int fix, int nblocks) {
   if (fix >= 0) return 1;
   int len = nblocks;
   if (skip >= 0 && skip < nblocks) {
@@ -1431,13 +1431,12 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
 // Strip form of the accumulating packed product of the Floyd-Warshall
 // remaining-tile phase: D_ij = min(D_ij, D_ir (x) D_rj) with K <= 64 (one
 // pivot block), ties keeping D_ij.  A CTA owns a strip: one 128-row tile of
-// the segment's row list (A = D_ir resident) and the column tiles of up to
-// kFwStripTiles block pairs of its column list.  Everything a tile needs is
+// the segment's row list (A = D_ir resident) and strip_tiles consecutive
+// column tiles of its column list (chosen per launch, fw_strip_tiles).  Everything a tile needs is
 // in flight before it is needed: B (= D_rj) double-buffered, the current
 // tile's C and B's predecessors staged behind its DPX loop.  The product starts from "unreached" and C joins in the
 // epilogue with index 0, which gives the same minimum and tie rule as
 // starting from C.
-constexpr int kFwStripTiles = 4;  // block pairs (128 columns) per strip
 // Column tile of the form used: one 64-column block (128 x 64 tiles, 8 x 4
 // outputs a thread, 112 KB of shared memory, two CTAs per SM, so that one
 // CTA's epilogue overlaps the other's add-mins).  TN = 128 (block pairs,
@@ -1451,10 +1450,6 @@ struct FwStripSmem {
   int32_t Bp[kBlk][TN];        // B's predecessors of the current tile
   unsigned C[kTile][TN];       // C of the current tile
 };
-
-__device__ __forceinline__ int fw_strips_x(const MpSegment &s) {
-  return (s.tiles_x + kFwStripTiles - 1) / kFwStripTiles;
-}
 
 // Copies rows [0, 64) of B-like data (row k at src + k * ld, columns of the
 // tile's 64-column blocks starting at cbase.x / cbase.y, -1 for none) into
@@ -1543,14 +1538,14 @@ __global__ void __launch_bounds__(kThreads, TN == 128 ? 1 : 2)
     tmap_acquire(tmap_d);
     if (PRED) tmap_acquire(tmap_d + 1);
   }
-  const int sx = fw_strips_x(s);
   const int local = blockIdx.x - s.strip_begin;
-  const int tyt = local / sx;
   const int nbr = (s.M + kBlk - 1) / kBlk, nbc = (s.N + kBlk - 1) / kBlk;
-  // column list length, in blocks, and this strip's column tiles of CH blocks
-  const int ncb = list_len(s.col_skip, s.col_skip2, s.col_fix, nbc);
-  const int jt0 = (local - tyt * sx) * kFwStripTiles * (2 / CH);
-  const int jt1 = min(jt0 + kFwStripTiles * (2 / CH), (ncb + CH - 1) / CH);
+  // column list length, in tiles of CH blocks, and this strip's column tiles
+  const int nct = (list_len(s.col_skip, s.col_skip2, s.col_fix, nbc) + CH - 1) / CH;
+  const int per = s.strip_tiles, sx = (nct + per - 1) / per;
+  const int tyt = local / sx;
+  const int jt0 = (local - tyt * sx) * per;
+  const int jt1 = min(jt0 + per, nct);
   const int rl0 = list_block(2 * tyt, s.row_skip, s.row_skip2, s.row_fix, nbr);
   const int rl1 = list_block(2 * tyt + 1, s.row_skip, s.row_skip2, s.row_fix, nbr);
   const int rbase0 = rl0 >= 0 ? rl0 * kBlk : -1, rbase1 = rl1 >= 0 ? rl1 * kBlk : -1;
@@ -2411,7 +2406,24 @@ cudaError_t tma_status(unsigned *out, bool reset) {
   }
   return e;
 }
-int fw_strip_tiles() { return kFwStripTiles; }
+int fw_strips_of(const MpSegment &s, int tiles) {
+  const int rows = list_len(s.row_skip, s.row_skip2, s.row_fix, (s.M + kBlk - 1) / kBlk);
+  const int cols = list_len(s.col_skip, s.col_skip2, s.col_fix, (s.N + kBlk - 1) / kBlk);
+  return (rows + 1) / 2 * ((cols + tiles - 1) / tiles);
+}
+// The column tiles a CTA takes: the most (up to 8, which amortise the staging
+// of A, about two tiles' time) that still give the launch one CTA for every
+// slot of the GPU (two per SM).  A single 910-vertex matrix then runs its
+// remaining tiles in 98 CTAs of one tile instead of 14 of eight: its 14
+// rounds took 2.33 ms in strips of 8 and take 1.15 ms.
+int fw_strip_tiles(const MpSegment *segs, int nseg, int sm_count) {
+  for (int tiles = 8; tiles > 1; tiles /= 2) {
+    long long strips = 0;
+    for (int i = 0; i < nseg; i++) strips += fw_strips_of(segs[i], tiles);
+    if (strips >= 2LL * sm_count) return tiles;
+  }
+  return 1;
+}
 int minplus_strip_max_k() { return kStripMaxK; }
 int minplus_strip_classes() { return kStripClasses; }
 int minplus_strip_class_k(int c) { return c >= 0 && c < kStripClasses ? kStripClassK[c] : -1; }

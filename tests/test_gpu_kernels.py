@@ -260,3 +260,34 @@ def test_addmin_peak_probe_modes(ctx):
     from fastapsp_gb300._lib import FapError
     with pytest.raises(FapError):
         ctx.addmin_peak(13)
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("size", [129, 513, 530])
+def test_floyd_strip_lengths_agree(ctx, oracle_lib, f32, size):
+    """A launch's strips are 1, 2, 4 or 8 column tiles long, by how many
+    matrices it holds; every copy of a matrix in a batch of any size comes
+    out as the same bits, and as the distances of naive Floyd-Warshall."""
+    rng = np.random.default_rng(size)
+    inf = np.float32(1e8) if f32 else np.int32(1 << 30)
+    a = np.full((size, size), inf)
+    edge = rng.random((size, size)) < 0.02
+    a[edge] = rng.uniform(0.5, 10, edge.sum()).astype(np.float32) if f32 else rng.integers(1, 50, edge.sum())
+    np.fill_diagonal(a, 0)
+    p = np.where(a < inf, np.arange(size, dtype=np.int32)[:, None], -1).astype(np.int32)
+    first = None
+    for count in (1, 24, 48, 90):
+        ds = [torch.from_numpy(a).cuda() for _ in range(count)]
+        ps = [torch.from_numpy(p).cuda() for _ in range(count)]
+        ctx.floyd_batched(0 if f32 else 1, ds, ps)
+        torch.cuda.synchronize()
+        first = first or (ds[0], ps[0])
+        for d, q in zip(ds, ps):
+            assert torch.equal(d, first[0]) and torch.equal(q, first[1])
+    w = torch.from_numpy(np.where(a < inf, a, np.inf).astype(np.float64)).cuda()
+    for k in range(size):
+        w = torch.minimum(w, w[:, k:k + 1] + w[k:k + 1, :])
+    w = torch.where(torch.isinf(w), float(inf), w)
+    # FP32: at most size - 1 sums, each rounded once (relative 2^-24)
+    tol = size * 2.0 ** -24 * w if f32 else torch.zeros_like(w)
+    assert bool(((first[0].double() - w).abs() <= tol).all())
