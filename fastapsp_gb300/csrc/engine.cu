@@ -180,6 +180,8 @@ struct Plan {
   int pack = -1;        // packed int32 form: -1 undecided, 0 no, 1 yes
   int sssp_lanes = 32;  // sources per SSSP batch
   int sssp_lanes_alt = 0;  // the other width the autotuner tries (0: none)
+  bool sssp_row = false;   // the whole-graph search runs one CTA per source (sssp_row.cu)
+  int row_ctas = 0;        // CTAs that the scratch holds frontiers of
   int bsssp = 0;        // boundary SSSP through the boundary graph (bgraph.cu) instead of the search
   bool method_trial = false;  // first run times both SSSP methods (automatic choice)
   // FW add-mins of one run outside the remaining-tile strips: the pivot
@@ -226,6 +228,7 @@ struct fap_engine {
   std::vector<float> w;
   uint32_t wmax = 0;  // largest weight (int32 mode)
   double wmean = 1.0; // mean weight (sets the SSSP near-far step)
+  int32_t max_deg = 0; // largest out- or in-degree
   // SSSP options (fap_set_option)
   int sssp_fp64 = 0;       // FP32 engines: search in FP64
   double sssp_delta = 0;   // near-far threshold step; 0 = auto (tuned on first solve)
@@ -269,6 +272,7 @@ struct fap_engine {
   // work buffers
   DevBuf fw_d, fw_p;           // FW matrices arena
   DevBuf sssp_scratch, sssp_bits;
+  DevBuf row_edges;             // the graph's edge records for the search with one CTA per source
   int sssp_slots_alloc = 0;
   bool sssp_wide = false;       // the scratch holds FP64 32-lane slots
   DevBuf res_d, res_p;         // device results when the caller passes host memory
@@ -285,11 +289,23 @@ struct fap_engine {
 
 namespace {
 
+// Whether the whole-graph search runs one CTA per source: 4-byte distances
+// and the batch width left automatic, on graphs whose tables fit.
+bool sssp_row_form(const fap_engine *e) {
+  return !(e->f32() && e->sssp_fp64) && e->sssp_lanes == 0 && fapk::sssp_row_fits(e->n, e->max_deg);
+}
+
+// Near-far step of that search in mean edge weights.  Measured on road graphs
+// of 4,801 to 114,599 vertices, a grid and a nearest-neighbour graph, with 16
+// to 2,448 sources: 64 is within 5 % of the best of 2 to 512 on each (8, the
+// batched search's, 5 to 30 % slower), so no trial runs choose it.
+constexpr double kRowDelta = 64.0;
+
 double sssp_delta_of(const fap_engine *e) {
   if (e->delta_try > 0) return e->delta_try;
   if (e->sssp_delta > 0) return e->sssp_delta;
   // a few mean edge weights per near-far step (at least one unit for int32)
-  double d = 8.0 * e->wmean;
+  double d = (sssp_row_form(e) ? kRowDelta : 8.0) * e->wmean;
   return e->f32() ? std::max(d, 1e-30) : std::max(1.0, std::floor(d));
 }
 
@@ -320,6 +336,21 @@ int ensure_sssp_scratch(fap_engine *e, int slots, bool wide = false) {
     return st;
   e->sssp_slots_alloc = slots;
   return FAP_OK;
+}
+
+// CTAs of that search for `jobs` sources, within a 4 GiB scratch budget; the
+// scratch is the batched search's buffer.  The edge records are made on
+// first use, on the calling stream (calls end with a synchronize).
+int ensure_row_scratch(fap_engine *e, int64_t jobs, int *ctas, cudaStream_t st) {
+  if (!e->row_edges.p) {
+    int rc = e->row_edges.ensure(std::max<size_t>((size_t)e->m * 16, 16));
+    if (rc != FAP_OK) return rc;
+    FAP_CUDA(fapk::launch_row_edges(e->m, e->d_ro, e->d_col, e->d_w, e->row_edges.p, st));
+  }
+  const size_t per = std::max<size_t>(fapk::sssp_row_scratch_bytes(e->n), 4);
+  const int64_t fit = std::max<int64_t>(1, (int64_t)(((size_t)4 << 30) / per));
+  *ctas = (int)std::min<int64_t>(fapk::sssp_row_ctas(e->n, jobs, e->sm_count), fit);
+  return e->sssp_scratch.ensure(per * (size_t)*ctas);
 }
 
 // Host tables of the boundary graph for the current partition (bgraph.cu):
@@ -1017,6 +1048,7 @@ struct Issuer {
     sa.lanes = pl.sssp_lanes;
     sa.acc64 = e->f32() && e->sssp_fp64;
     sa.delta = sssp_delta_of(e);
+    sa.row_edges = e->row_edges.p;
     sa.stats = e->d_stats;
     if (g == 0) FAP_CUDA(cudaMemsetAsync(e->d_stats, 0, 8 * sizeof(unsigned long long), st));
     if (pl.bsssp) {
@@ -1048,6 +1080,11 @@ struct Issuer {
         sa.fix_scale = std::ldexp(1.0, -e->fix_shift);
       }
       FAP_CUDA(fapk::launch_sssp_output(e->f32(), sa, st));
+      return FAP_OK;
+    }
+    if (pl.sssp_row) {
+      sa.slots = std::min(fapk::sssp_row_ctas(e->n, (int64_t)G.nbatches * sa.lanes, e->sm_count), pl.row_ctas);
+      FAP_CUDA(fapk::launch_sssp_rows(e->f32(), sa, e->sm_count, st));
       return FAP_OK;
     }
     FAP_CUDA(fapk::launch_sssp(e->f32(), sa, st));
@@ -1515,7 +1552,8 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
   // The SSSP autotuner also tries a second batch width (8 -> 16, 16 -> 32,
   // 32 -> 16; not for the FP64 search, whose 32-source slots have another
   // layout); scratch for the larger batch count of the two.
-  const bool tune_lanes = e->autotune && e->sssp_delta <= 0 && e->sssp_lanes == 0 && !acc64 && !bs;
+  const bool row = sssp_row_form(e);
+  const bool tune_lanes = e->autotune && e->sssp_delta <= 0 && e->sssp_lanes == 0 && !acc64 && !bs && !row;
   const int alt_lanes = lanes == 16 ? 32 : 16;
   const bool wide = acc64 && lanes == 32;
   const int count_lanes = tune_lanes ? std::min(lanes, alt_lanes) : lanes;
@@ -1523,8 +1561,13 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
   for (int p : parts) max_batches += (e->bdy_num[p] + count_lanes - 1) / count_lanes;
   if ((rc = e->fw_d.ensure(std::max<size_t>(fw_elems, 1) * 4)) != FAP_OK) return rc;
   if (pred && (rc = e->fw_p.ensure(std::max<size_t>(fw_elems, 1) * 4)) != FAP_OK) return rc;
-  int slots = std::min(std::max(max_batches, 1), max_sssp_slots(e, wide));
-  if ((rc = ensure_sssp_scratch(e, slots, wide)) != FAP_OK) return rc;
+  int row_ctas = 0;
+  if (!row || bs) {  // tables of the batched search, or of the boundary graph's rows
+    int slots = std::min(std::max(max_batches, 1), max_sssp_slots(e, wide));
+    if ((rc = ensure_sssp_scratch(e, slots, wide)) != FAP_OK) return rc;
+  }
+  if (row && (!bs || trial) && (rc = ensure_row_scratch(e, (int64_t)max_batches * lanes, &row_ctas, st)) != FAP_OK)
+    return rc;
 
   Plan *pl = find_plan(e, mode, dist, pred, parts, offs, bdist, bpred, hdist, hpred, ring_elems);
   if (!pl) {
@@ -1544,6 +1587,8 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
     np->sig = buffer_signature(e);
     np->sssp_lanes = lanes;
     np->sssp_lanes_alt = tune_lanes ? alt_lanes : 0;
+    np->sssp_row = row;
+    np->row_ctas = row_ctas;
     np->bsssp = bs ? 1 : 0;
     np->method_trial = trial;
     if ((rc = build_plan(e, *np)) != FAP_OK) return rc;
@@ -1553,8 +1598,14 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
   if (pl->pack < 0) {  // first run: trials and tuners, then the plan without a graph
     const int c0 = fapk::launch_count();
     if (pl->method_trial && (rc = trial_sssp_method(e, *pl, st)) != FAP_OK) return rc;
-    if (e->autotune && e->sssp_delta <= 0 && !pl->bsssp && (rc = autotune_sssp(e, *pl, st)) != FAP_OK)
-      return rc;
+    if (e->autotune && e->sssp_delta <= 0 && !pl->bsssp) {
+      if (pl->sssp_row) {  // nothing to try: the step as it is, and the width of its tables
+        e->sssp_delta = sssp_delta_of(e);
+        e->sssp_lanes_tuned = pl->sssp_lanes;
+      } else if ((rc = autotune_sssp(e, *pl, st)) != FAP_OK) {
+        return rc;
+      }
+    }
     if ((rc = first_run(e, *pl, st)) != FAP_OK) return rc;
     e->fw_host_work += pl->pack == 1 ? pl->fw_pivot_work : pl->fw_tile_work;
     if (e->autotune && e->tile_cols == 0 && (rc = autotune_tiles(e, *pl, st)) != FAP_OK) return rc;
@@ -1656,6 +1707,7 @@ int init_device(fap_engine *e, int device) {
   FAP_CUDA(cudaMemset(e->d_stats, 0, 8 * sizeof(unsigned long long)));
   FAP_CUDA(fapk::init_minplus_kernels());
   FAP_CUDA(fapk::init_sssp_kernels());
+  FAP_CUDA(fapk::init_sssp_row_kernels());
   FAP_CUDA(fapk::init_bg_kernels());
   return FAP_OK;
 }
@@ -1881,6 +1933,8 @@ int fap_create(int32_t n, int64_t m, const int32_t *row_offset, const int32_t *c
     for (int64_t j = 0; j < m; j++) sum += weight[j];
     E->wmean = m > 0 ? std::max(sum / (double)m, 1e-30) : 1.0;
   }
+  for (int32_t i = 0; i < n; i++)
+    E->max_deg = std::max({E->max_deg, row_offset[i + 1] - row_offset[i], iro[i + 1] - iro[i]});
   E->has_graph = true;
   *out = e.release();
   return FAP_OK;
@@ -1896,6 +1950,7 @@ int fap_destroy(fap_engine *e) {
     e->fw_p.release();
     e->sssp_scratch.release();
     e->sssp_bits.release();
+    e->row_edges.release();
     e->res_d.release();
     e->res_p.release();
     e->bnd_d.release();
@@ -2475,7 +2530,10 @@ int fap_sssp(fap_engine *e, const int32_t *sources, int32_t num_sources, void *d
   }
   int rc;
   int slots = std::min((int)batches.size(), max_sssp_slots(e, wide));
-  if ((rc = ensure_sssp_scratch(e, slots, wide)) != FAP_OK) return rc;
+  const bool row = sssp_row_form(e) && is_device_ptr(dist);
+  if (row) rc = ensure_row_scratch(e, (int64_t)batches.size() * lanes, &slots, st);
+  else rc = ensure_sssp_scratch(e, slots, wide);
+  if (rc != FAP_OK) return rc;
   if ((rc = e->small.ensure(batches.size() * sizeof(SsspBatch))) != FAP_OK) return rc;
   FAP_CUDA(cudaMemcpyAsync(e->small.p, batches.data(), batches.size() * sizeof(SsspBatch),
                            cudaMemcpyHostToDevice, st));
@@ -2492,7 +2550,7 @@ int fap_sssp(fap_engine *e, const int32_t *sources, int32_t num_sources, void *d
   sa.dist = dist;
   sa.pred = pred;
   sa.scratch = e->sssp_scratch.p;
-  sa.slots = std::min(sa.nbatches, e->sssp_slots_alloc);
+  sa.slots = row ? slots : std::min(sa.nbatches, e->sssp_slots_alloc);
   sa.bits = e->sssp_bits.p;
   sa.status = e->d_status;
   sa.maxd = nullptr;
@@ -2500,7 +2558,9 @@ int fap_sssp(fap_engine *e, const int32_t *sources, int32_t num_sources, void *d
   sa.lanes = lanes;
   sa.acc64 = acc64;
   sa.delta = sssp_delta_of(e);
-  FAP_CUDA(fapk::launch_sssp(e->f32(), sa, st));
+  sa.row_edges = e->row_edges.p;
+  if (row) FAP_CUDA(fapk::launch_sssp_rows(e->f32(), sa, e->sm_count, st));
+  else FAP_CUDA(fapk::launch_sssp(e->f32(), sa, st));
   FAP_CUDA(cudaStreamSynchronize(st));
   return check_status(e);
 }

@@ -104,6 +104,7 @@ struct SsspArgs {
   unsigned long long *stats;  // may be null: [near steps, far splits, frontier
                               // vertices relaxed, far entries scanned, batches]
   int32_t defer_output;       // set by launch_sssp: output pass in its own launch
+  const void *row_edges;      // launch_sssp_rows: the edge records (launch_row_edges)
   // launch_sssp_output on tables of exact 64-bit fixed point (FP32 graphs):
   int32_t fix;                        // 1: tables hold fixed-point values, not FP64
   const unsigned long long *iwfix;    // in-edge weights in the same units
@@ -119,6 +120,19 @@ size_t sssp_bits_bytes(int32_t n);  // per slot; 0 when the bitmaps fit in share
 int sssp_lanes_for(int64_t batches8, int64_t batches32, int sm_count, bool acc64);
 int sssp_threads();
 cudaError_t launch_sssp(bool f32, const SsspArgs &a, cudaStream_t st);
+
+// sssp_row.cu: the same search and rows with one CTA per source (4-byte
+// distances; the batch width plays no part).  slots = CTAs
+// (sssp_row_ctas), scratch = slots * sssp_row_scratch_bytes(n), dist in device
+// memory.
+bool sssp_row_fits(int32_t n, int32_t max_deg);  // bitmaps fit in shared memory, no vertex has too many edges
+// Edge records of the graph for it (m * 16 bytes; SsspArgs::row_edges).
+cudaError_t launch_row_edges(int64_t m, const int32_t *ro, const int32_t *col, const void *w, void *edges,
+                             cudaStream_t st);
+size_t sssp_row_scratch_bytes(int32_t n);
+int sssp_row_ctas(int32_t n, int64_t jobs, int sm_count);
+cudaError_t init_sssp_row_kernels();
+cudaError_t launch_sssp_rows(bool f32, const SsspArgs &a, int sm_count, cudaStream_t st);
 
 // Output pass of the whole-graph search alone, over per-batch vertex-major
 // tables that something else filled (batch b's table in scratch slot b,

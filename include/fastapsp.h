@@ -189,14 +189,20 @@ int fap_precondition(fap_engine *e);
  *                      Dijkstra.
  *   FAP_OPT_SSSP_DELTA near-far threshold step of the SSSP in distance units
  *                      (0 = automatic).  Changes speed only, never results.
+ *                      Automatic is 64 x the mean weight where the search
+ *                      runs one CTA per source (4-byte distances, automatic
+ *                      batch width, no vertex of more than 64 edges), else
+ *                      8 x, or what FAP_OPT_AUTOTUNE finds.
  *   FAP_OPT_AUTOTUNE   1 (default) = while the step is automatic, the first
- *                      run of a solve times the SSSP phase with a few steps
- *                      (multiples of the mean edge weight, and plain
- *                      Bellman-Ford) and keeps the fastest; fap_get_option
- *                      then reports the chosen step.  0 = 8 x the mean weight.
+ *                      run of a solve with the batched search times the SSSP
+ *                      phase with a few steps (multiples of the mean edge
+ *                      weight, and plain Bellman-Ford) and keeps the fastest;
+ *                      fap_get_option then reports the chosen step.
  *   FAP_OPT_SSSP_LANES sources per SSSP batch (one CTA each; 8 = four lane
- *                      groups a warp, 16 = two, 32 = one): 8, 16 or 32, or 0
- *                      (default) = automatic: chosen from the batch count,
+ *                      groups a warp, 16 = two, 32 = one): 8, 16 or 32, which
+ *                      also selects the batched search, or 0 (default) =
+ *                      automatic: one CTA per source where that search
+ *                      applies, else chosen from the batch count,
  *                      and while the step is tuned (above), the first run
  *                      also times a second width at the chosen step and
  *                      keeps the faster, which fap_get_option then reports

@@ -291,3 +291,34 @@ def test_floyd_strip_lengths_agree(ctx, oracle_lib, f32, size):
     # FP32: at most size - 1 sums, each rounded once (relative 2^-24)
     tol = size * 2.0 ** -24 * w if f32 else torch.zeros_like(w)
     assert bool(((first[0].double() - w).abs() <= tol).all())
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("n,sources", [(33, 1), (1025, 33), (4097, 152), (4097, 153), (60000, 5)])
+def test_sssp_one_cta_per_source_matches_batches(gpu, f32, n, sources):
+    """Few sources (distances in shared memory, or past its size in the rows)
+    and more than one per SM give the batched search's rows bit for bit, on
+    graphs with unreached vertices, parallel edges, self loops, degrees past
+    one lane group's four edges and frontiers past the shared-memory list; a
+    vertex of more than 64 edges keeps the batched search."""
+    rng = np.random.default_rng(n + sources)
+    hubs = [graphs.small_random_graph(n, 3 * n, True, True, seed=n, integer=not f32)]
+    star = np.r_[np.zeros(min(n - 1, 200), np.int64), rng.integers(0, n, 2 * n)]
+    ends = np.r_[1 + np.arange(min(n - 1, 200)), rng.integers(0, n, 2 * n)]
+    hubs.append(graphs.csr_from_lines(n, star, ends, rng.integers(1, 9, star.shape[0]).astype(np.float32), True, True))
+    for g in hubs:
+        src = rng.permutation(n)[:sources].astype(np.int32)
+        with gpu.Engine(n, g.row_offset, g.col_val, g.weight, 1, graph_id=np.ones(n, np.int32),
+                        dtype=gpu.DTYPE_F32 if f32 else gpu.DTYPE_I32) as eng:
+            out = []
+            for lanes, delta, pred in ((8, 0.0, True), (0, 0.0, True), (0, 2.0, True), (0, 0.0, False)):
+                eng.set_option(gpu._lib.OPT_SSSP_LANES, lanes)
+                eng.set_option(gpu._lib.OPT_SSSP_DELTA, delta)
+                d = torch.full((sources, n + 3), 7, dtype=torch.float32 if f32 else torch.int32, device="cuda")
+                p = torch.full((sources, n + 3), 7, dtype=torch.int32, device="cuda")
+                eng.sssp(src, d, p if pred else None, ld=n + 3)
+                torch.cuda.synchronize()
+                out.append((d, p))
+            for d, p in out[1:3]:
+                assert torch.equal(d, out[0][0]) and torch.equal(p, out[0][1])
+            assert torch.equal(out[3][0], out[0][0]) and bool((out[3][1] == 7).all())
