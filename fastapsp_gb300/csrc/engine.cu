@@ -134,7 +134,7 @@ struct Plan {
     int64_t dec_rows = 0;
     // FW: per round r, diag jobs [diag_off[r], +diag_cnt[r]) and segments
     std::vector<const FwDiagJob *> diag;
-    std::vector<int> diag_cnt;
+    std::vector<int> diag_cnt, diag_blocks;  // jobs, and their panel blocks
     std::vector<const MpSegment *> panel;
     std::vector<int> panel_nseg, panel_tiles;
     std::vector<const MpSegment *> rest;
@@ -144,14 +144,7 @@ struct Plan {
     // round r + 1 updates itself), strip form
     std::vector<const MpSegment *> rest2;
     std::vector<int> rest2_nseg, rest2_strips;
-    // FP32 form: round r's row and column panels, strip form
-    std::vector<const MpSegment *> pstrips;
-    // FP32 form with lookahead: round r - 1's update of block row and column
-    // r (the tiles `rest2` of round r - 1 leaves out), strip form
-    std::vector<const MpSegment *> look;
-    std::vector<int> look_nseg, look_strips;
     const void *tmaps = nullptr;  // tensor-map pairs of the FW matrices (null: none)
-    std::vector<int> pstrips_nseg, pstrips_strips;
     // boundary rows in their own buffer (host results): per part {element
     // offset in the results, element offset in the buffer, elements}, copied
     // out as soon as the SSSP has written them
@@ -271,6 +264,7 @@ struct fap_engine {
   cudaEvent_t ev_slot[2] = {};    // staged host results in two slots: slot s's last copy-out done
   // work buffers
   DevBuf fw_d, fw_p;           // FW matrices arena
+  DevBuf fw_look;              // the pivot chain's copies, per matrix (fapk::fw_look_bytes)
   DevBuf sssp_scratch, sssp_bits;
   DevBuf row_edges;             // the graph's edge records for the search with one CTA per source
   int sssp_slots_alloc = 0;
@@ -573,16 +567,6 @@ int fw_number_strips(std::vector<MpSegment> &segs, int sm_count) {
   return strips;
 }
 
-// FP32 form: fw_segments' two panels of pivot block r of nb as strip-form
-// segments, appended to `out`.  Each reads and writes
-// the same entries (the row panel is B and C, the column panel A and C); a
-// CTA reads the entries it writes into shared memory before its epilogue,
-// and no two CTAs write the same entries.
-void fw_panel_strips(const MpSegment &rowp, const MpSegment &colp, std::vector<MpSegment> &out) {
-  out.push_back(rowp);
-  out.push_back(colp);
-}
-
 // Lookahead form of fw_segments' `rest` for pivot block r of nb: the rows and
 // columns other than r and r + 1 (block row and column r + 1 get round r's
 // update inside pivot step r + 1).
@@ -591,27 +575,6 @@ void fw_rest_lookahead(MpSegment &rest, int nb, int r) {
   rest.row_skip2 = r + 1;
   rest.col_skip2 = r + 1;
   rest.tiles_x = pairs;
-}
-
-// FP32 form with lookahead: round r - 1's update of block row and column r
-// of nb (r >= 1; the tiles that fw_rest_lookahead leaves out of round
-// r - 1) as strip-form segments appended to `out`:
-// block row r over the columns other than r - 1 (the pivot block (r, r)
-// with them), and block column r over the rows other than r - 1 and r.  The
-// two write disjoint blocks and read block row and column r - 1 only, which
-// neither writes; no tile reads entries it or another tile writes.
-void fw_look_strips(void *D, int32_t *P, int64_t ld, int size, int r, int nb, int32_t tmap1,
-                    std::vector<MpSegment> &out) {
-  MpSegment rowp, colp, rest;
-  int t1, t2, t3;
-  fw_segments(D, P, ld, size, r - 1, rowp, colp, rest, t1, t2, t3, true, tmap1);
-  rowp.row_fix = r;  // (the row panel of pivot r - 1, moved to block row r)
-  out.push_back(rowp);
-  if (nb > 2) {
-    colp.col_fix = r;  // (the column panel, moved to block column r, without row r)
-    colp.row_skip2 = r;
-    out.push_back(colp);
-  }
 }
 
 // Min-plus segment C = A (x) B (fresh C), tiled in 128x128.
@@ -720,7 +683,7 @@ int build_plan(fap_engine *e, Plan &pl) {
   TableBuilder tb;
   struct GroupOffs {
     size_t batches, batches_alt, pdesc, row_begin, dec_begin, mp, bjobs, bsrc;
-    std::vector<size_t> diag, panel, rest, rest2, pstrips, look;
+    std::vector<size_t> diag, panel, rest, rest2;
     size_t tmaps = 0;
     bool has_tmaps = false;
   };
@@ -732,6 +695,7 @@ int build_plan(fap_engine *e, Plan &pl) {
     // SSSP batches: per part, its boundary vertices in mapping order.
     std::vector<SsspBatch> batches, batches_alt;
     std::vector<PartDesc> pdesc;
+    std::vector<int> mat_index;  // pdesc entry -> index in pl.parts
     std::vector<int64_t> row_begin(1, 0), dec_begin(1, 0);
     // min-plus segments: the strip form's classes of K in order, then those
     // above its limit; tiles are numbered over all of them
@@ -772,6 +736,7 @@ int build_plan(fap_engine *e, Plan &pl) {
       d.row_off = boff;
       d.dec_off = roff;  // the decode writes the result rows themselves
       pdesc.push_back(d);
+      mat_index.push_back(idx);
       if (pl.bdist && bdy > 0) G.bnd_copies.push_back({roff, boff, (int64_t)bdy * n});
       row_begin.push_back(row_begin.back() + d.ld);
       dec_begin.push_back(dec_begin.back() + bdy);
@@ -857,12 +822,7 @@ int build_plan(fap_engine *e, Plan &pl) {
     G.rest_tiles.assign(maxnb, 0);
     G.rest2_nseg.assign(maxnb, 0);
     G.rest2_strips.assign(maxnb, 0);
-    G.pstrips_nseg.assign(maxnb, 0);
-    G.pstrips_strips.assign(maxnb, 0);
-    O.pstrips.assign(maxnb, 0);
-    G.look_nseg.assign(maxnb, 0);
-    G.look_strips.assign(maxnb, 0);
-    O.look.assign(maxnb, 0);
+    G.diag_blocks.assign(maxnb, 0);
     O.diag.assign(maxnb, 0);
     O.panel.assign(maxnb, 0);
     O.rest.assign(maxnb, 0);
@@ -890,8 +850,8 @@ int build_plan(fap_engine *e, Plan &pl) {
     }
     for (int r = 0; r < maxnb; r++) {
       std::vector<FwDiagJob> dj;
-      std::vector<MpSegment> ps, rs, r2s, pss, ls;
-      int pt = 0, rt = 0;
+      std::vector<MpSegment> ps, rs, r2s;
+      int pt = 0, rt = 0, blocks = 0;
       for (size_t pi = 0; pi < pdesc.size(); pi++) {
         const PartDesc &d = pdesc[pi];
         int nb = d.ld / B;
@@ -904,36 +864,38 @@ int build_plan(fap_engine *e, Plan &pl) {
         j.ld = d.ld;
         j.size = d.ld;
         j.block = r;
-        j.prev = r - 1;  // used by the packed form's pivot step (lookahead) only
+        j.prev = r - 1;
+        j.panel_begin = blocks;
+        j.look = static_cast<char *>(e->fw_look.p) + (size_t)mat_index[pi] * fapk::fw_look_bytes();
+        blocks += 2 * (nb - 1);
         dj.push_back(j);
         {  // 64^3 block products: pivot step (lookahead update, closure, panels); tile form (all blocks)
           const unsigned long long blk = (unsigned long long)B * B * B;
           pl.fw_pivot_work += blk * ((r > 0 ? 2ull * (nb - 2) + 1 : 0ull) + 1ull + 2ull * (nb - 1));
-          pl.fw_tile_work += blk * (e->f32() ? 1ull : (unsigned long long)nb * nb);
+          pl.fw_tile_work += blk * (unsigned long long)nb * nb;
         }
         if (nb > 1) {
           MpSegment rp, cp, rest;
           int a1, a2, a3;
           fw_segments(D, P, d.ld, d.ld, r, rp, cp, rest, a1, a2, a3, e->f32(), tmap1[pi]);
-          if (e->f32() && r > 0) fw_look_strips(D, P, d.ld, d.ld, r, nb, tmap1[pi], ls);
-          rp.tile_begin = pt;
-          pt += a1;
-          ps.push_back(rp);
-          cp.tile_begin = pt;
-          pt += a2;
-          ps.push_back(cp);
-          rest.tile_begin = rt;
-          rt += a3;
-          rs.push_back(rest);
-          fw_panel_strips(rp, cp, pss);
+          if (!e->f32()) {  // the wide int32 form's tiles
+            rp.tile_begin = pt;
+            pt += a1;
+            ps.push_back(rp);
+            cp.tile_begin = pt;
+            pt += a2;
+            ps.push_back(cp);
+            rest.tile_begin = rt;
+            rt += a3;
+            rs.push_back(rest);
+          }
           if (r + 1 < nb) fw_rest_lookahead(rest, nb, r);
           if (rest.tiles_x > 0) r2s.push_back(rest);
         }
       }
       const int r2strips = fw_number_strips(r2s, e->sm_count);
-      const int psstrips = fw_number_strips(pss, e->sm_count);
-      const int lstrips = fw_number_strips(ls, e->sm_count);
       G.diag_cnt[r] = (int)dj.size();
+      G.diag_blocks[r] = blocks;
       O.diag[r] = tb.add(dj.data(), dj.size());
       G.panel_nseg[r] = (int)ps.size();
       G.panel_tiles[r] = pt;
@@ -944,12 +906,6 @@ int build_plan(fap_engine *e, Plan &pl) {
       G.rest2_nseg[r] = (int)r2s.size();
       G.rest2_strips[r] = r2strips;
       O.rest2[r] = tb.add(r2s.data(), r2s.size());
-      G.pstrips_nseg[r] = (int)pss.size();
-      G.pstrips_strips[r] = psstrips;
-      O.pstrips[r] = tb.add(pss.data(), pss.size());
-      G.look_nseg[r] = (int)ls.size();
-      G.look_strips[r] = lstrips;
-      O.look[r] = tb.add(ls.data(), ls.size());
     }
   }
   int st = pl.tables.ensure(std::max<size_t>(tb.bytes.size(), 64));
@@ -975,15 +931,11 @@ int build_plan(fap_engine *e, Plan &pl) {
     G.panel.resize(R);
     G.rest.resize(R);
     G.rest2.resize(R);
-    G.pstrips.resize(R);
-    G.look.resize(R);
     for (size_t r = 0; r < R; r++) {
       G.diag[r] = reinterpret_cast<const FwDiagJob *>(base + O.diag[r]);
       G.panel[r] = reinterpret_cast<const MpSegment *>(base + O.panel[r]);
       G.rest[r] = reinterpret_cast<const MpSegment *>(base + O.rest[r]);
       G.rest2[r] = reinterpret_cast<const MpSegment *>(base + O.rest2[r]);
-      G.pstrips[r] = reinterpret_cast<const MpSegment *>(base + O.pstrips[r]);
-      G.look[r] = reinterpret_cast<const MpSegment *>(base + O.look[r]);
     }
   }
   return FAP_OK;
@@ -1118,46 +1070,27 @@ struct Issuer {
     if (last) FAP_CUDA(rec(2));
     const int rounds = (int)G.diag.size();
     for (int r = 0; r < rounds; r++) {
-      if (packed) {
-        // Lookahead.  Pivot step r (one launch: round r - 1's update of block
-        // row and column r, the closure, both panels) runs on the issuing
-        // stream; round r's remaining tiles other than block row and column
-        // r + 1 (`rest2`) on the side stream, where they overlap pivot step
-        // r + 1.  Pivot step r waits for `rest2` of round r - 2 (the last
-        // launch that wrote block row and column r); `rest2` of round r waits
-        // for pivot step r.  Pivot step r + 1 and `rest2` of round r touch
-        // disjoint entries: the pivot step reads block rows and columns r and
-        // r + 1 and writes r + 1; `rest2` reads block row and column r outside
+      if (packed || f32) {
+        // Lookahead.  The pivot chain of round r (round r - 1's update of
+        // block row and column r, the closure, both panels) runs on the
+        // issuing stream; round r's remaining tiles other than block row and
+        // column r + 1 (`rest2`) on the side stream, where they overlap the
+        // chain of round r + 1.  Chain r waits for `rest2` of round r - 2 (the
+        // last launch that wrote block row and column r); `rest2` of round r
+        // waits for chain r.  Chain r + 1 and `rest2` of round r touch
+        // disjoint entries: the chain reads block rows and columns r and r + 1
+        // and writes r + 1; `rest2` reads block row and column r outside
         // blocks r and r + 1 and writes neither.
         if (r >= 2) FAP_CUDA(cudaStreamWaitEvent(st, e->ev_fw[1 + r % 2], 0));
-        FAP_CUDA(fapk::launch_fw_pivot(pred, G.diag[r], G.diag_cnt[r], st));
-        FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
-        FAP_CUDA(cudaStreamWaitEvent(e->side, e->ev_fw[0], 0));
-        FAP_CUDA(fapk::launch_fw_strips(pred, G.rest2[r], G.rest2_nseg[r], G.rest2_strips[r], e->side, false,
-                                        G.tmaps));
-        FAP_CUDA(cudaEventRecord(e->ev_fw[1 + r % 2], e->side));
-      } else if (f32) {
-        // FP32 lookahead, in strip launches: the pivot chain of round r
-        // (round r - 1's update of block row and column r, the closure of
-        // pivot block r, both panels) on the issuing stream, round r's
-        // remaining tiles other than block row and column r + 1 (`rest2`) on
-        // the side stream, beside the pivot chain of round r + 1.  The events
-        // and the entries each side touches are those of the packed form.
-        if (r >= 2) FAP_CUDA(cudaStreamWaitEvent(st, e->ev_fw[1 + r % 2], 0));
-        if (G.look_nseg[r] > 0)
-          FAP_CUDA(fapk::launch_fw_strips(pred, G.look[r], G.look_nseg[r], G.look_strips[r], st, true, G.tmaps));
-        FAP_CUDA(fapk::launch_fw_diag(f32, pred, G.diag[r], G.diag_cnt[r], st));
-        if (G.pstrips_nseg[r] > 0)
-          FAP_CUDA(fapk::launch_fw_strips(pred, G.pstrips[r], G.pstrips_nseg[r], G.pstrips_strips[r], st, true,
-                                          G.tmaps));
+        FAP_CUDA(fapk::launch_fw_chain(f32, pred, G.diag[r], G.diag_cnt[r], G.diag_blocks[r], st));
         FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
         FAP_CUDA(cudaStreamWaitEvent(e->side, e->ev_fw[0], 0));
         if (G.rest2_nseg[r] > 0)
-          FAP_CUDA(fapk::launch_fw_strips(pred, G.rest2[r], G.rest2_nseg[r], G.rest2_strips[r], e->side, true,
+          FAP_CUDA(fapk::launch_fw_strips(pred, G.rest2[r], G.rest2_nseg[r], G.rest2_strips[r], e->side, f32,
                                           G.tmaps));
         FAP_CUDA(cudaEventRecord(e->ev_fw[1 + r % 2], e->side));
       } else {
-        FAP_CUDA(fapk::launch_fw_diag(f32, pred, G.diag[r], G.diag_cnt[r], st));
+        FAP_CUDA(fapk::launch_fw_diag(pred, G.diag[r], G.diag_cnt[r], st));
         {
           FAP_CUDA(fapk::launch_minplus_tiles(f32, pred, G.panel[r], G.panel_nseg[r], G.panel_tiles[r], packed, st));
           FAP_CUDA(fapk::launch_minplus_tiles(f32, pred, G.rest[r], G.rest_nseg[r], G.rest_tiles[r], packed, st));
@@ -1486,7 +1419,7 @@ std::vector<const void *> buffer_signature(const fap_engine *e) {
   double d = sssp_delta_of(e);
   intptr_t dbits;
   std::memcpy(&dbits, &d, sizeof(dbits));
-  return {e->fw_d.p, e->fw_p.p, e->sssp_scratch.p, e->sssp_bits.p,
+  return {e->fw_d.p, e->fw_p.p, e->fw_look.p, e->sssp_scratch.p, e->sssp_bits.p,
           reinterpret_cast<const void *>((intptr_t)e->sssp_slots_alloc),
           reinterpret_cast<const void *>((intptr_t)e->sssp_fp64),
           reinterpret_cast<const void *>((intptr_t)e->sssp_lanes),
@@ -1561,6 +1494,7 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
   for (int p : parts) max_batches += (e->bdy_num[p] + count_lanes - 1) / count_lanes;
   if ((rc = e->fw_d.ensure(std::max<size_t>(fw_elems, 1) * 4)) != FAP_OK) return rc;
   if (pred && (rc = e->fw_p.ensure(std::max<size_t>(fw_elems, 1) * 4)) != FAP_OK) return rc;
+  if ((rc = e->fw_look.ensure(parts.size() * fapk::fw_look_bytes())) != FAP_OK) return rc;
   int row_ctas = 0;
   if (!row || bs) {  // tables of the batched search, or of the boundary graph's rows
     int slots = std::min(std::max(max_batches, 1), max_sssp_slots(e, wide));
@@ -1607,7 +1541,7 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
       }
     }
     if ((rc = first_run(e, *pl, st)) != FAP_OK) return rc;
-    e->fw_host_work += pl->pack == 1 ? pl->fw_pivot_work : pl->fw_tile_work;
+    e->fw_host_work += pl->pack == 1 || e->f32() ? pl->fw_pivot_work : pl->fw_tile_work;
     if (e->autotune && e->tile_cols == 0 && (rc = autotune_tiles(e, *pl, st)) != FAP_OK) return rc;
     e->last_launches = fapk::launch_count() - c0;  // every kernel of this call, trials included
     return FAP_OK;
@@ -1646,7 +1580,7 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
     Issuer is{e, *pl, st, false};
     if ((rc = is.all()) != FAP_OK) return rc;
   }
-  e->fw_host_work += pl->pack == 1 ? pl->fw_pivot_work : pl->fw_tile_work;
+  e->fw_host_work += pl->pack == 1 || e->f32() ? pl->fw_pivot_work : pl->fw_tile_work;
   e->last_launches = pl->launches;
   return FAP_OK;
 }
@@ -1706,6 +1640,7 @@ int init_device(fap_engine *e, int device) {
   FAP_CUDA(cudaMalloc(&e->d_stats, 8 * sizeof(unsigned long long)));
   FAP_CUDA(cudaMemset(e->d_stats, 0, 8 * sizeof(unsigned long long)));
   FAP_CUDA(fapk::init_minplus_kernels());
+  FAP_CUDA(fapk::init_fw_pivot_kernels());
   FAP_CUDA(fapk::init_sssp_kernels());
   FAP_CUDA(fapk::init_sssp_row_kernels());
   FAP_CUDA(fapk::init_bg_kernels());
@@ -1948,6 +1883,7 @@ int fap_destroy(fap_engine *e) {
     e->plans.clear();
     e->fw_d.release();
     e->fw_p.release();
+    e->fw_look.release();
     e->sssp_scratch.release();
     e->sssp_bits.release();
     e->row_edges.release();
@@ -2356,9 +2292,10 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
   DeviceGuard g(e->device);
   cudaStream_t st = pick_stream(e, stream);
   TableBuilder tb;
-  std::vector<size_t> od(maxnb), op(maxnb), orr(maxnb), or2(maxnb), ops(maxnb), ols(maxnb);
-  std::vector<int> nd(maxnb), np(maxnb), tp(maxnb), nr(maxnb), tr(maxnb), nr2(maxnb), sr2(maxnb), nps(maxnb),
-      sps(maxnb), nls(maxnb), sls(maxnb);
+  std::vector<size_t> od(maxnb), op(maxnb), orr(maxnb), or2(maxnb);
+  std::vector<int> nd(maxnb), bd(maxnb), np(maxnb), tp(maxnb), nr(maxnb), tr(maxnb), nr2(maxnb), sr2(maxnb);
+  int rc;
+  if ((rc = e->fw_look.ensure((size_t)count * fapk::fw_look_bytes())) != FAP_OK) return rc;
   // tensor-map pairs of the matrices that meet the copy unit's alignment
   // rules (16-byte base and row stride); the others keep per-thread copies
   std::vector<int32_t> tmap1(count, 0);
@@ -2381,8 +2318,8 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
   }
   for (int r = 0; r < maxnb; r++) {
     std::vector<FwDiagJob> dj;
-    std::vector<MpSegment> ps, rs, r2s, pss, ls;
-    int pt = 0, rt = 0;
+    std::vector<MpSegment> ps, rs, r2s;
+    int pt = 0, rt = 0, blocks = 0;
     for (int32_t b = 0; b < count; b++) {
       int nb = (sizes[b] + Bk - 1) / Bk;
       if (r >= nb) continue;
@@ -2392,42 +2329,37 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
       j.ld = ld[b];
       j.size = sizes[b];
       j.block = r;
-      j.prev = r - 1;  // used by the packed form's pivot step (lookahead) only
+      j.prev = r - 1;
+      j.panel_begin = blocks;
+      j.look = static_cast<char *>(e->fw_look.p) + (size_t)b * fapk::fw_look_bytes();
+      blocks += 2 * (nb - 1);
       dj.push_back(j);
       if (nb > 1) {
         MpSegment a, c, rest;
         int t1, t2, t3;
         fw_segments(D[b], pred ? P[b] : nullptr, ld[b], sizes[b], r, a, c, rest, t1, t2, t3,
                     dtype == FAP_DTYPE_F32, tmap1[b]);
-        if (dtype == FAP_DTYPE_F32 && r > 0)
-          fw_look_strips(D[b], pred ? P[b] : nullptr, ld[b], sizes[b], r, nb, tmap1[b], ls);
-        a.tile_begin = pt;
-        pt += t1;
-        ps.push_back(a);
-        c.tile_begin = pt;
-        pt += t2;
-        ps.push_back(c);
-        rest.tile_begin = rt;
-        rt += t3;
-        rs.push_back(rest);
-        fw_panel_strips(a, c, pss);
+        if (dtype != FAP_DTYPE_F32) {  // the wide int32 form's tiles
+          a.tile_begin = pt;
+          pt += t1;
+          ps.push_back(a);
+          c.tile_begin = pt;
+          pt += t2;
+          ps.push_back(c);
+          rest.tile_begin = rt;
+          rt += t3;
+          rs.push_back(rest);
+        }
         if (r + 1 < nb) fw_rest_lookahead(rest, nb, r);
         if (rest.tiles_x > 0) r2s.push_back(rest);
       }
     }
     const int r2strips = fw_number_strips(r2s, e->sm_count);
-    const int psstrips = fw_number_strips(pss, e->sm_count);
-    const int lstrips = fw_number_strips(ls, e->sm_count);
     nr2[r] = (int)r2s.size();
     sr2[r] = r2strips;
     or2[r] = tb.add(r2s.data(), r2s.size());
-    nps[r] = (int)pss.size();
-    sps[r] = psstrips;
-    ops[r] = tb.add(pss.data(), pss.size());
-    nls[r] = (int)ls.size();
-    sls[r] = lstrips;
-    ols[r] = tb.add(ls.data(), ls.size());
     nd[r] = (int)dj.size();
+    bd[r] = blocks;
     od[r] = tb.add(dj.data(), dj.size());
     np[r] = (int)ps.size();
     tp[r] = pt;
@@ -2445,7 +2377,6 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
       max_size = std::max(max_size, sizes[b]);
     }
   size_t o_ref = tb.add(refs.data(), refs.size());
-  int rc;
   if ((rc = e->small.ensure(std::max<size_t>(tb.bytes.size(), 64))) != FAP_OK) return rc;
   FAP_CUDA(cudaMemcpyAsync(e->small.p, tb.bytes.data(), tb.bytes.size(), cudaMemcpyHostToDevice, st));
   unsigned char *base = static_cast<unsigned char *>(e->small.p);
@@ -2463,31 +2394,17 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
   }
   for (int r = 0; r < maxnb; r++) {
     const FwDiagJob *djobs = reinterpret_cast<const FwDiagJob *>(base + od[r]);
-    if (packed) {  // lookahead, as in the solve's issue order
+    if (packed || f32) {  // lookahead, as in the solve's issue order
       if (r >= 2) FAP_CUDA(cudaStreamWaitEvent(st, e->ev_fw[1 + r % 2], 0));
-      FAP_CUDA(fapk::launch_fw_pivot(pred, djobs, nd[r], st));
-      FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
-      FAP_CUDA(cudaStreamWaitEvent(e->side, e->ev_fw[0], 0));
-      FAP_CUDA(fapk::launch_fw_strips(pred, reinterpret_cast<const MpSegment *>(base + or2[r]), nr2[r],
-                                      sr2[r], e->side, false, tmaps));
-      FAP_CUDA(cudaEventRecord(e->ev_fw[1 + r % 2], e->side));
-    } else if (f32) {  // FP32 lookahead, as in the solve's issue order
-      if (r >= 2) FAP_CUDA(cudaStreamWaitEvent(st, e->ev_fw[1 + r % 2], 0));
-      if (nls[r] > 0)
-        FAP_CUDA(fapk::launch_fw_strips(pred, reinterpret_cast<const MpSegment *>(base + ols[r]), nls[r],
-                                        sls[r], st, true, tmaps));
-      FAP_CUDA(fapk::launch_fw_diag(f32, pred, djobs, nd[r], st));
-      if (nps[r] > 0)
-        FAP_CUDA(fapk::launch_fw_strips(pred, reinterpret_cast<const MpSegment *>(base + ops[r]), nps[r],
-                                        sps[r], st, true, tmaps));
+      FAP_CUDA(fapk::launch_fw_chain(f32, pred, djobs, nd[r], bd[r], st));
       FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
       FAP_CUDA(cudaStreamWaitEvent(e->side, e->ev_fw[0], 0));
       if (nr2[r] > 0)
-        FAP_CUDA(fapk::launch_fw_strips(pred, reinterpret_cast<const MpSegment *>(base + or2[r]), nr2[r],
-                                        sr2[r], e->side, true, tmaps));
+        FAP_CUDA(fapk::launch_fw_strips(pred, reinterpret_cast<const MpSegment *>(base + or2[r]), nr2[r], sr2[r],
+                                        e->side, f32, tmaps));
       FAP_CUDA(cudaEventRecord(e->ev_fw[1 + r % 2], e->side));
     } else {
-      FAP_CUDA(fapk::launch_fw_diag(f32, pred, djobs, nd[r], st));
+      FAP_CUDA(fapk::launch_fw_diag(pred, djobs, nd[r], st));
       {
         FAP_CUDA(fapk::launch_minplus_tiles(f32, pred, reinterpret_cast<const MpSegment *>(base + op[r]), np[r],
                                             tp[r], packed, st));

@@ -80,7 +80,8 @@ struct MpSegment {
   int32_t b_row0;
 };
 
-// FW diagonal-block job: close the 64x64 pivot block of one matrix.
+// FW pivot job: close the 64x64 pivot block of one matrix and update its
+// block row and column.
 struct FwDiagJob {
   void *D;
   int32_t *P;
@@ -90,6 +91,8 @@ struct FwDiagJob {
   int32_t prev;  // >= 0: the update of round `prev` (pivot block prev) to this
                  // block row and column is applied first (lookahead: the
                  // remaining-tile launch of round prev left them out); -1: none
+  int32_t panel_begin;  // first CTA of its panel blocks in the launch's numbering
+  void *look;           // the matrix's scratch of fw_look_bytes() (used when prev >= 0)
 };
 
 // A strided row-major matrix of 4-byte values.

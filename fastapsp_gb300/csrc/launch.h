@@ -69,12 +69,15 @@ int max_packed_k();
 // Add-mins executed by the FW remaining-tile strips on the current device
 // since the last reset; optionally reset.
 cudaError_t fw_strip_counter(unsigned long long *out, bool reset);
-cudaError_t launch_fw_diag(bool f32, bool pred, const FwDiagJob *d_jobs, int njobs,
-                           cudaStream_t st);
-// Packed int32 form: closes each job's pivot block and updates its row and
-// column panels (a cluster of CTAs per job); replaces launch_fw_diag and the
-// panel launch.
-cudaError_t launch_fw_pivot(bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st);
+// Wide int32 form: closes each job's pivot block.
+cudaError_t launch_fw_diag(bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st);
+// fw_pivot.cu (packed int32 and FP32 forms): round job.prev's update of each
+// job's block row and column job.block, the closure of the pivot block and the
+// panels: two launches.  blocks = the jobs' panel blocks, 2 (blocks a side - 1)
+// each, numbered by FwDiagJob::panel_begin.
+cudaError_t launch_fw_chain(bool f32, bool pred, const FwDiagJob *d_jobs, int njobs, int blocks, cudaStream_t st);
+size_t fw_look_bytes();  // device scratch per matrix
+cudaError_t init_fw_pivot_kernels();
 int minplus_tile_rows();  // CTA output tile edge (128)
 int fw_block();           // FW pivot block edge (64)
 cudaError_t init_minplus_kernels();

@@ -15,7 +15,7 @@
 //    B-predecessor tile after each chunk.  A batch of segments (one per
 //    matrix or FW panel) is one launch; each CTA finds its segment by binary
 //    search over the segments' first tile.
-//  - mp_tile_packed_kernel, mp_strip_kernel, mp_fwstrip_kernel, fw_pivot_kernel
+//  - mp_tile_packed_kernel, mp_strip_kernel, mp_fwstrip_kernel
 //    (int32 whose finite results stay below 2^24 - 1): packed keys
 //    (d << 7) | idx, one DPX __viaddmin_u32 per add-min, which gives the
 //    minimum and, on ties, the smallest idx -- the current value (idx 0)
@@ -29,7 +29,6 @@
 // min(D_ij, D_ir (x) D_rj).  Ties keep the current value, so predecessors
 // follow P[i][j] = P[k][j] on strict improvement as in the reference.
 
-#include <cooperative_groups.h>
 #include <cuda.h>  // CUtensorMap (the type only; maps are encoded on the host)
 #include <cudaTypedefs.h>
 #include <cuda_runtime.h>
@@ -37,6 +36,7 @@
 
 #include <type_traits>
 
+#include "fw_tile.cuh"
 #include "kernels.cuh"
 #include "launch.h"
 
@@ -45,7 +45,6 @@ namespace fapk {
 namespace {
 
 constexpr int kTile = 128;   // CTA tile (rows and columns)
-constexpr int kBlk = 64;     // 64-row / 64-column blocks of a tile
 constexpr int kBK = 32;      // k chunk staged in shared memory
 constexpr int kThreads = 256;
 constexpr int kApad = kBK + 1;  // A rows padded against bank conflicts
@@ -440,21 +439,6 @@ __device__ __forceinline__ void tile_wide(MpSmem<T> &sm, const MpSegment &s, con
   }
 }
 
-// Packed int32 form.  Keys are (min(d, kPackH) << 7) | idx: idx 0 marks the
-// value the output held before the product, idx = k+1 the candidate k.  One
-// DPX __viaddmin_u32 per add-min then yields the minimum and, on equal
-// distances, the smallest idx -- the current value first, then the first k
-// -- which is the strict-improvement, ascending-k rule of the reference.  Two
-// keys sum to at most (2 * kPackH) << 7 | 127 < 2^32, so nothing wraps, and
-// saturation at kPackH commutes with + and min, so the results are exact when
-// every finite result stays below kPackH (checked by the caller).  With
-// predecessors K <= 127, so the final idx names k* directly and the
-// predecessor is read once, in the epilogue, from B's predecessor row k*.
-constexpr unsigned kPackH = (1u << 24) - 1;
-constexpr unsigned kIdxBits = 7;
-constexpr unsigned kIdxMask = (1u << kIdxBits) - 1;
-constexpr int kMaxPackedK = 127;
-
 constexpr int kStagedBpRows = 64;  // B-predecessor rows kept in shared memory
 
 struct KeySmem {
@@ -715,19 +699,6 @@ __device__ __forceinline__ const MpSegment &find_strip_segment(const MpSegment *
   return segs[lo];
 }
 
-// Layout of the FP32 strip kernels' operands in shared memory: entry (k, m)
-// of A^T and entry (k, col) of B sit at row k, position m ^ swz(k) and
-// col ^ swz(k) -- the 4-entry chunks of step group k / 4 permuted by XOR with
-// its low three bits.  Within a group the permutation is the same, so a
-// thread's four consecutive rows or columns stay one aligned 16-byte chunk;
-// after the add-mins, threads that look up entries of different step groups
-// of the same rows or columns hit different banks.  The packed form keeps
-// the plain layout (SWZ false).
-template <bool SWZ>
-__device__ __forceinline__ int swz(int k) {
-  return SWZ ? ((k >> 2) & 7) << 2 : 0;
-}
-
 // Copies a ks x TN tile of a row-major 4-byte matrix (rows < K, columns
 // [col0, col0 + TN) < N) into dst[ks][TN] (SWZ: chunks permuted by swz);
 // each thread moves 4 consecutive columns of a row per pass (one 16-byte
@@ -819,49 +790,6 @@ __device__ __forceinline__ void strip_addmin(unsigned &acc, int &arg, unsigned a
   }
 }
 
-// Four add-mins of the FP32 strip kernels, steps k0 .. k0 + 3: the current
-// value replaced by the minimum of the four sums when that is below it (a
-// strict improvement), and then the group tag (k0 + 1) too.  That leaves the
-// step of the last strict improvement in the tagged group: its first step
-// whose sum equals the final value, since every earlier step's sum is above
-// it (strip_resolve_f32 finds it after the loop).  Four FP32 adds, then
-// (MIN3ACC, both strip kernels) two 3-input minimums with the current value
-// as an input, a compare and one select, or a 3-input and a 2-input minimum,
-// a compare and two selects: one ALU instruction more, but the old and the
-// new value are not live together (the min-plus took that form while its
-// epilogue still spilled at 128 registers a thread).
-template <bool MIN3ACC>
-__device__ __forceinline__ void strip_addmin4_f32(unsigned &acc, int &tag, const unsigned a[4],
-                                                  const unsigned b[4], int grp) {
-  const unsigned v0 = __float_as_uint(__fadd_rn(__uint_as_float(a[0]), __uint_as_float(b[0])));
-  const unsigned v1 = __float_as_uint(__fadd_rn(__uint_as_float(a[1]), __uint_as_float(b[1])));
-  const unsigned v2 = __float_as_uint(__fadd_rn(__uint_as_float(a[2]), __uint_as_float(b[2])));
-  const unsigned v3 = __float_as_uint(__fadd_rn(__uint_as_float(a[3]), __uint_as_float(b[3])));
-  if constexpr (MIN3ACC) {
-    const unsigned nacc = __vimin3_u32(acc, __vimin3_u32(v0, v1, v2), v3);
-    tag = nacc != acc ? grp : tag;
-    acc = nacc;
-  } else {
-    const unsigned t = min(__vimin3_u32(v0, v1, v2), v3);
-    const bool imp = t < acc;
-    acc = imp ? t : acc;
-    tag = imp ? grp : tag;
-  }
-}
-
-// The step idx (k + 1) of an output whose last strict improvement fell in the
-// group tagged `tag` (0: none): the group's first step whose sum has the
-// final value's bits.  ap / bp point at the output's A and B entries of the
-// group's first step (strides sa, sb between steps).
-__device__ __forceinline__ int strip_resolve_f32(unsigned acc, int tag, const unsigned *ap, int sa,
-                                                 const unsigned *bp, int sb) {
-  const unsigned v0 = __float_as_uint(__fadd_rn(__uint_as_float(ap[0]), __uint_as_float(bp[0])));
-  const unsigned v1 = __float_as_uint(__fadd_rn(__uint_as_float(ap[sa]), __uint_as_float(bp[sb])));
-  const unsigned v2 = __float_as_uint(__fadd_rn(__uint_as_float(ap[2 * sa]), __uint_as_float(bp[2 * sb])));
-  const int j = v0 == acc ? 0 : v1 == acc ? 1 : v2 == acc ? 2 : 3;
-  return tag > 0 ? tag + j : 0;
-}
-
 // FP32 add-mins of a thread's 8 x 4 outputs over steps [0, kseg) (kseg a
 // multiple of 4) in groups of four, then, with PRED, each output's group
 // resolved to the step idx (k + 1) of its last strict improvement -- the
@@ -909,7 +837,7 @@ __device__ __forceinline__ void addmin_groups_f32(unsigned (&acc)[8][4], int (&a
         for (int r = 0; r < 4; r++)
 #pragma unroll
           for (int c = ch * 2; c < ch * 2 + 2; c++)
-            strip_addmin4_f32<true>(acc[h * 4 + r][c], arg[h * 4 + r][c], a[r], b[c], kk + 1);
+            strip_addmin4_f32(acc[h * 4 + r][c], arg[h * 4 + r][c], a[r], b[c], kk + 1);
       }
     }
   }
@@ -968,7 +896,7 @@ __device__ __forceinline__ void addmin_groups_rows_f32(unsigned (&acc)[8][4], in
         for (int r = 0; r < 4; r++)
 #pragma unroll
           for (int c = 0; c < 2; c++)
-            strip_addmin4_f32<true>(acc[h * 4 + r][ch * 2 + c], arg[h * 4 + r][ch * 2 + c], a[r], b[c], kk + 1);
+            strip_addmin4_f32(acc[h * 4 + r][ch * 2 + c], arg[h * 4 + r][ch * 2 + c], a[r], b[c], kk + 1);
       }
     }
   }
@@ -1975,300 +1903,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Pivot step of one FW round in the packed int32 form, for every matrix of
-// the batch: a cluster of kPivotCtas CTAs per matrix (two CTAs per SM).  CTA
-// 0 closes the pivot block (as fw_diag_kernel) and writes it back; after a
-// cluster barrier the others copy the closed block out of CTA 0's shared
-// memory (no second closure, and no read of the block while it is being
-// written).  Then CTAs of the first half update the row panel
-// D_rb = min(D_rb, D_rr (x) D_rb) and those of the second half the column
-// panel D_br = min(D_br, D_br (x) D_rr), each taking every (kPivotCtas/2)-th
-// block: 64x64 outputs, 4x4 per thread, packed keys, the block's own values
-// joining with index 0.  The panel blocks are a pipeline: the first one's
-// copy is issued before the closure (it lands while CTA 0 closes and the
-// others wait), each next block's values are copied behind the current
-// block's add-mins, and (row panel) its predecessors behind the current
-// block's epilogue.  One launch replaces the diagonal launch and the panel
-// launch of the tile kernel (whose 128x128 tiles were half empty for 64-wide
-// panels).
-constexpr int kPivotCtas = 4;
-
-struct PivotSmem {
-  unsigned D[kBlk][kBlk + 1];  // pivot block values (closure)
-  int32_t P[kBlk][kBlk + 1];   // and predecessors
-  unsigned Kp[kBlk][kBlk];     // pivot keys: A^T (row panel) or B (column panel)
-  unsigned Xv[kBlk][kBlk];     // the next panel block's values (copy in flight)
-  int32_t Xp[kBlk][kBlk];      // the current block's predecessors (row panel)
-  unsigned Kx[kBlk][kBlk];     // the current block's keys: B (row panel) or A^T (column panel)
-};
-
-// Copies the 64x64 block (rb, cb) of a job's matrix (values, or predecessors
-// when P) into dst[64][64], "unreached" / -1 outside the matrix.
-template <bool P>
-__device__ __forceinline__ void pivot_load_block(unsigned *dst, const FwDiagJob &job, int rb, int cb) {
-  const unsigned *src = P ? reinterpret_cast<const unsigned *>(job.P) : static_cast<const unsigned *>(job.D);
-  for (int idx = threadIdx.x; idx < kBlk * kBlk; idx += kThreads) {
-    const int i = idx >> 6, j = idx & 63;
-    const int gi = rb * kBlk + i, gj = cb * kBlk + j;
-    if (gi < job.size && gj < job.size) cp_async4(&dst[idx], src + (int64_t)gi * job.ld + gj);
-    else dst[idx] = P ? 0xffffffffu : Dist<uint32_t>::inf();
-  }
-}
-
-// Lookahead part of round `r` of the blocked FW for the 64x64 block (cr, cc)
-// of a job's matrix (a block of the next pivot's row or column, or the next
-// pivot block itself), which the remaining-tile launch of round r left out:
-// C = min(C, A (x) B) with A = block (cr, r), B = block (r, cc), ties keeping
-// C, a strict improvement taking B's predecessor -- the same update that
-// launch applies to every other tile.  C comes from and goes back to the
-// closure buffer sm.D / sm.P (TO_SMEM) or global memory.  Kp, Kx and Xp are
-// scratch; ends with a barrier.
-template <bool PRED, bool TO_SMEM>
-__device__ void pivot_prev_block(PivotSmem &sm, const FwDiagJob &job, int cr, int cc, int r) {
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  unsigned *Dg = static_cast<unsigned *>(job.D);
-  const unsigned INF = Dist<uint32_t>::inf();
-  auto inside = [&](int gi, int gj) { return gi < job.size && gj < job.size; };
-  unsigned av[4][4], cv[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int li = ty * 4 + i;
-    unsigned bv[4];
-    int32_t bp[4];
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int lj = tx * 4 + c;
-      const int ai = cr * kBlk + li, aj = r * kBlk + lj;
-      const int bi = r * kBlk + li, bj = cc * kBlk + lj;
-      const int ci = cr * kBlk + li, cj = cc * kBlk + lj;
-      av[i][c] = inside(ai, aj) ? Dg[(int64_t)ai * job.ld + aj] : INF;
-      bv[c] = inside(bi, bj) ? Dg[(int64_t)bi * job.ld + bj] : INF;
-      bp[c] = PRED && inside(bi, bj) ? job.P[(int64_t)bi * job.ld + bj] : -1;
-      if (TO_SMEM) cv[i][c] = sm.D[li][lj];
-      else cv[i][c] = inside(ci, cj) ? Dg[(int64_t)ci * job.ld + cj] : INF;
-    }
-    const unsigned id = (unsigned)(li + 1);  // B row k = li
-    *reinterpret_cast<uint4 *>(&sm.Kx[li][tx * 4]) =
-        make_uint4((min(bv[0], kPackH) << kIdxBits) | id, (min(bv[1], kPackH) << kIdxBits) | id,
-                   (min(bv[2], kPackH) << kIdxBits) | id, (min(bv[3], kPackH) << kIdxBits) | id);
-    if (PRED) *reinterpret_cast<int4 *>(&sm.Xp[li][tx * 4]) = make_int4(bp[0], bp[1], bp[2], bp[3]);
-  }
-#pragma unroll
-  for (int c = 0; c < 4; c++)  // A^T: k = column of A
-    *reinterpret_cast<uint4 *>(&sm.Kp[tx * 4 + c][ty * 4]) =
-        make_uint4(min(av[0][c], kPackH) << kIdxBits, min(av[1][c], kPackH) << kIdxBits,
-                   min(av[2][c], kPackH) << kIdxBits, min(av[3][c], kPackH) << kIdxBits);
-  __syncthreads();
-  unsigned acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int c = 0; c < 4; c++) acc[i][c] = kPackH << kIdxBits;
-#pragma unroll 4
-  for (int kk = 0; kk < kBlk; kk++) {
-    const uint4 a4 = *reinterpret_cast<const uint4 *>(&sm.Kp[kk][ty * 4]);
-    const uint4 b4 = *reinterpret_cast<const uint4 *>(&sm.Kx[kk][tx * 4]);
-    const unsigned a[4] = {a4.x, a4.y, a4.z, a4.w};
-    const unsigned b[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int c = 0; c < 4; c++) acc[i][c] = __viaddmin_u32(a[i], b[c], acc[i][c]);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int li = ty * 4 + i;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-      const int lj = tx * 4 + c;
-      const unsigned key = min(min(cv[i][c], kPackH) << kIdxBits, acc[i][c]);
-      const unsigned idx = key & kIdxMask;
-      if (idx == 0) continue;
-      if (TO_SMEM) {
-        sm.D[li][lj] = key >> kIdxBits;
-        if (PRED) sm.P[li][lj] = sm.Xp[idx - 1][lj];
-      } else {
-        const int ci = cr * kBlk + li, cj = cc * kBlk + lj;
-        if (!inside(ci, cj)) continue;
-        Dg[(int64_t)ci * job.ld + cj] = key >> kIdxBits;
-        if (PRED) job.P[(int64_t)ci * job.ld + cj] = sm.Xp[idx - 1][lj];
-      }
-    }
-  }
-  __syncthreads();  // scratch free again
-}
-
-template <bool PRED>
-__global__ void __cluster_dims__(kPivotCtas, 1, 1) __launch_bounds__(kThreads, 2)
-    fw_pivot_kernel(const FwDiagJob *__restrict__ jobs) {
-  namespace cg = cooperative_groups;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  PivotSmem &sm = *reinterpret_cast<PivotSmem *>(smem_raw);
-  cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank();
-  const int role = rank / (kPivotCtas / 2);  // 0: row panel, 1: column panel
-  const int sub = rank % (kPivotCtas / 2);   // which of the panel's blocks
-  constexpr int kStride = kPivotCtas / 2;
-  const FwDiagJob job = jobs[blockIdx.x / kPivotCtas];
-  const int r = job.block;
-  const int nb = (job.size + kBlk - 1) / kBlk;
-  const int npanel = nb - 1;
-  const unsigned INF = Dist<uint32_t>::inf();
-  auto panel_block = [&](int i) { return i < r ? i : i + 1; };  // i-th block other than r
-  auto load_values = [&](int pi) {  // panel block pi's values -> Xv
-    const int b = panel_block(pi);
-    if (role == 0) pivot_load_block<false>(&sm.Xv[0][0], job, r, b);
-    else pivot_load_block<false>(&sm.Xv[0][0], job, b, r);
-  };
-  auto load_preds = [&](int pi) {  // row panel: block pi's predecessors -> Xp
-    if (PRED && role == 0)
-      pivot_load_block<true>(reinterpret_cast<unsigned *>(&sm.Xp[0][0]), job, r, panel_block(pi));
-  };
-  // Lookahead: the update of round job.prev to this block row and column
-  // (left out by that round's remaining-tile launch) comes first -- CTA 0
-  // applies it to the pivot block before the closure, the others to the
-  // panel blocks meanwhile.  Without it the first panel block's copy lands
-  // during the closure; with it, after the cluster barrier that publishes
-  // those updates.
-  const int prev = job.prev;
-  auto first_copy = [&]() {
-    if (sub < npanel) load_values(sub);
-    cp_async_commit();
-    if (sub < npanel) load_preds(sub);
-    cp_async_commit();
-  };
-  if (prev < 0) first_copy();
-
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  if (rank != 0 && prev >= 0) {
-    const int lo = min(r, prev), hi = max(r, prev);
-    auto other = [&](int t) {  // t-th block other than r and prev
-      int b = t;
-      if (b >= lo) b++;
-      if (b >= hi) b++;
-      return b;
-    };
-    const int nother = nb - 2;
-    for (int t = rank - 1; t < 2 * nother; t += kPivotCtas - 1) {
-      if (t < nother) pivot_prev_block<PRED, false>(sm, job, r, other(t), prev);
-      else pivot_prev_block<PRED, false>(sm, job, other(t - nother), r, prev);
-    }
-  }
-  if (rank == 0) {
-    unsigned *Dg = static_cast<unsigned *>(job.D);
-    const int base = r * kBlk;
-    for (int idx = threadIdx.x; idx < kBlk * kBlk; idx += kThreads) {
-      const int i = idx >> 6, j = idx & 63;
-      const int gi = base + i, gj = base + j;
-      const bool ok = gi < job.size && gj < job.size;
-      sm.D[i][j] = ok ? Dg[(int64_t)gi * job.ld + gj] : (i == j ? 0u : INF);
-      if (PRED) sm.P[i][j] = ok ? job.P[(int64_t)gi * job.ld + gj] : -1;
-    }
-    __syncthreads();
-    if (prev >= 0) pivot_prev_block<PRED, true>(sm, job, r, r, prev);
-    close_block<uint32_t, PRED>(sm.D, sm.P);
-    for (int idx = threadIdx.x; idx < kBlk * kBlk; idx += kThreads) {
-      const int i = idx >> 6, j = idx & 63;
-      const int gi = base + i, gj = base + j;
-      if (gi < job.size && gj < job.size) {
-        Dg[(int64_t)gi * job.ld + gj] = sm.D[i][j];
-        if (PRED) job.P[(int64_t)gi * job.ld + gj] = sm.P[i][j];
-      }
-    }
-  }
-  cluster.sync();  // the closed pivot block is in CTA 0's shared memory (and the lookahead updates are in memory)
-  if (prev >= 0) first_copy();
-  if (rank != 0) {
-    const unsigned *rD = cluster.map_shared_rank(&sm.D[0][0], 0);
-    const int32_t *rP = cluster.map_shared_rank(&sm.P[0][0], 0);
-    for (int idx = threadIdx.x; idx < kBlk * (kBlk + 1); idx += kThreads) {
-      (&sm.D[0][0])[idx] = rD[idx];
-      if (PRED) (&sm.P[0][0])[idx] = rP[idx];
-    }
-  }
-  cluster.sync();  // CTA 0's shared memory is no longer read; every copy is complete
-  for (int idx = threadIdx.x; idx < kBlk * kBlk; idx += kThreads) {
-    const int i = idx >> 6, j = idx & 63;
-    if (role == 0) sm.Kp[j][i] = min(sm.D[i][j], kPackH) << kIdxBits;  // A^T, idx 0
-    else sm.Kp[i][j] = (min(sm.D[i][j], kPackH) << kIdxBits) | (unsigned)(i + 1);  // B, idx k + 1
-  }
-
-  for (int pi = sub; pi < npanel; pi += kStride) {
-    const int b = panel_block(pi);
-    cp_async_wait_1();  // this block's values (its predecessors may still be in flight)
-    __syncthreads();    // ... for every thread's part (and Kp, on the first trip)
-    // Keys of this block from each thread's own 4x4 outputs, whose values
-    // stay in registers for the epilogue.
-    unsigned cv[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const uint4 v = *reinterpret_cast<const uint4 *>(&sm.Xv[ty * 4 + i][tx * 4]);
-      cv[i][0] = min(v.x, kPackH);
-      cv[i][1] = min(v.y, kPackH);
-      cv[i][2] = min(v.z, kPackH);
-      cv[i][3] = min(v.w, kPackH);
-    }
-    if (role == 0) {  // B = the block, row k carries idx k + 1
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const unsigned id = (unsigned)(ty * 4 + i + 1);
-        *reinterpret_cast<uint4 *>(&sm.Kx[ty * 4 + i][tx * 4]) =
-            make_uint4((cv[i][0] << kIdxBits) | id, (cv[i][1] << kIdxBits) | id,
-                       (cv[i][2] << kIdxBits) | id, (cv[i][3] << kIdxBits) | id);
-      }
-    } else {  // A^T of the block
-#pragma unroll
-      for (int c = 0; c < 4; c++)
-        *reinterpret_cast<uint4 *>(&sm.Kx[tx * 4 + c][ty * 4]) =
-            make_uint4(cv[0][c] << kIdxBits, cv[1][c] << kIdxBits, cv[2][c] << kIdxBits,
-                       cv[3][c] << kIdxBits);
-    }
-    __syncthreads();  // Kx complete; Xv free for the next block's copy
-    if (pi + kStride < npanel) load_values(pi + kStride);
-    cp_async_commit();
-    const unsigned *Aop = role == 0 ? &sm.Kp[0][0] : &sm.Kx[0][0];
-    const unsigned *Bop = role == 0 ? &sm.Kx[0][0] : &sm.Kp[0][0];
-    unsigned acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int c = 0; c < 4; c++) acc[i][c] = kPackH << kIdxBits;
-#pragma unroll 4
-    for (int kk = 0; kk < kBlk; kk++) {
-      const uint4 av = *reinterpret_cast<const uint4 *>(Aop + kk * kBlk + ty * 4);
-      const uint4 bv = *reinterpret_cast<const uint4 *>(Bop + kk * kBlk + tx * 4);
-      const unsigned a[4] = {av.x, av.y, av.z, av.w};
-      const unsigned bb[4] = {bv.x, bv.y, bv.z, bv.w};
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) acc[i][c] = __viaddmin_u32(a[i], bb[c], acc[i][c]);
-    }
-    cp_async_wait_1();  // this block's predecessors (the next block's values may be in flight)
-    __syncthreads();
-    unsigned *Dg = static_cast<unsigned *>(job.D);
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int li = ty * 4 + i;
-      const int gi = (role == 0 ? r : b) * kBlk + li;
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        const int lj = tx * 4 + c;
-        const int gj = (role == 0 ? b : r) * kBlk + lj;
-        const unsigned key = min(cv[i][c] << kIdxBits, acc[i][c]);
-        const unsigned idx = key & kIdxMask;
-        if (idx == 0 || gi >= job.size || gj >= job.size) continue;
-        Dg[(int64_t)gi * job.ld + gj] = key >> kIdxBits;
-        if (PRED) job.P[(int64_t)gi * job.ld + gj] = role == 0 ? sm.Xp[idx - 1][lj] : sm.P[idx - 1][lj];
-      }
-    }
-    __syncthreads();  // Kx and Xp are free again
-    if (pi + kStride < npanel) load_preds(pi + kStride);
-    cp_async_commit();
-  }
-  cp_async_wait_0();
-}
-
 template <typename T, bool PRED>
 cudaError_t launch_mp_t(const MpSegment *d_segs, int nseg, int tiles, int tile0, cudaStream_t st) {
   if (tiles <= 0 || nseg <= 0) return cudaSuccess;
@@ -2453,24 +2087,11 @@ cudaError_t strip_counters(unsigned long long out[3], bool reset) {
 }
 int max_packed_k() { return kMaxPackedK; }
 
-cudaError_t launch_fw_pivot(bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st) {
+cudaError_t launch_fw_diag(bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st) {
   if (njobs <= 0) return cudaSuccess;
-  const unsigned grid = (unsigned)(kPivotCtas * njobs);
-  if (pred) { ++launch_count(); fw_pivot_kernel<true><<<grid, kThreads, sizeof(PivotSmem), st>>>(d_jobs); }
-  else { ++launch_count(); fw_pivot_kernel<false><<<grid, kThreads, sizeof(PivotSmem), st>>>(d_jobs); }
-  return cudaGetLastError();
-}
-
-cudaError_t launch_fw_diag(bool f32, bool pred, const FwDiagJob *d_jobs, int njobs,
-                           cudaStream_t st) {
-  if (njobs <= 0) return cudaSuccess;
-  if (f32) {
-    if (pred) { ++launch_count(); fw_diag_kernel<float, true><<<njobs, 256, 0, st>>>(d_jobs); }
-    else { ++launch_count(); fw_diag_kernel<float, false><<<njobs, 256, 0, st>>>(d_jobs); }
-  } else {
-    if (pred) { ++launch_count(); fw_diag_kernel<uint32_t, true><<<njobs, 256, 0, st>>>(d_jobs); }
-    else { ++launch_count(); fw_diag_kernel<uint32_t, false><<<njobs, 256, 0, st>>>(d_jobs); }
-  }
+  ++launch_count();
+  if (pred) fw_diag_kernel<uint32_t, true><<<njobs, 256, 0, st>>>(d_jobs);
+  else fw_diag_kernel<uint32_t, false><<<njobs, 256, 0, st>>>(d_jobs);
   return cudaGetLastError();
 }
 
@@ -2504,12 +2125,6 @@ cudaError_t init_minplus_kernels() {
 #undef FAP_STRIP_ATTR
 #undef FAP_STRIP_ATTR1
 
-  if ((e = cudaFuncSetAttribute(fw_pivot_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(PivotSmem))) != cudaSuccess)
-    return e;
-  if ((e = cudaFuncSetAttribute(fw_pivot_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(PivotSmem))) != cudaSuccess)
-    return e;
 #define FAP_FWSTRIP_ATTR(P, F)                                                           \
   if ((e = cudaFuncSetAttribute(mp_fwstrip_kernel<P, kFwStripTN, F>,                     \
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,             \
