@@ -32,6 +32,7 @@
 #include "launch.h"
 
 using fapk::FwDiagJob;
+using fapk::FwRestJob;
 using fapk::MpSegment;
 using fapk::PartDesc;
 using fapk::SsspBatch;
@@ -140,11 +141,10 @@ struct Plan {
     std::vector<const MpSegment *> rest;
     std::vector<int> rest_nseg, rest_tiles;
     // lookahead (packed and FP32 forms): the remaining tiles of round r
-    // without block row and column r + 1 (which the pivot step or chain of
-    // round r + 1 updates itself), strip form
-    std::vector<const MpSegment *> rest2;
-    std::vector<int> rest2_nseg, rest2_strips;
-    const void *tmaps = nullptr;  // tensor-map pairs of the FW matrices (null: none)
+    // without block row and column r + 1 (which the pivot chain of round r + 1
+    // updates itself)
+    std::vector<const FwRestJob *> rest2;
+    std::vector<int> rest2_njob, rest2_strips, rest2_per;
     // boundary rows in their own buffer (host results): per part {element
     // offset in the results, element offset in the buffer, elements}, copied
     // out as soon as the SSSP has written them
@@ -191,11 +191,6 @@ struct Plan {
 
 // Host-side table builder: appends POD records into one byte buffer and
 // remembers offsets, which become device pointers after the upload.
-// Storage of one CUtensorMap (encoded by fapk::encode_fw_tmaps).
-struct alignas(64) TmapBlob {
-  unsigned char bytes[128];
-};
-
 struct TableBuilder {
   std::vector<unsigned char> bytes;
   template <typename T>
@@ -503,18 +498,14 @@ bool is_device_ptr(const void *p) {
   return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
 }
 
-// FW segments of one matrix for pivot block r (row panel + column panel, and
-// the remaining tiles).  Matrices are size x size with leading dimension ld.
+// Wide int32 form: FW segments of one matrix for pivot block r (row panel +
+// column panel, and the remaining tiles).  Matrices are size x size with leading dimension ld.
 void fw_segments(void *D, int32_t *P, int64_t ld, int size, int r, MpSegment &rowp,
-                 MpSegment &colp, MpSegment &rest, int &t_rowp, int &t_colp, int &t_rest,
-                 bool f32, int32_t tmap1 = 0) {
+                 MpSegment &colp, MpSegment &rest, int &t_rowp, int &t_colp, int &t_rest) {
   const int B = fapk::fw_block();
   const int nb = (size + B - 1) / B;
   const size_t es = 4;
-  (void)f32;
   MpSegment s{};
-  s.tmap1 = tmap1;  // the strips' bulk tensor copies, when the matrix has a map pair
-  s.b_row0 = r * B;
   s.A = static_cast<const unsigned char *>(D) + (size_t)r * B * es;
   s.lda = ld;
   s.B = static_cast<const unsigned char *>(D) + (size_t)r * B * ld * es;
@@ -552,29 +543,6 @@ void fw_segments(void *D, int32_t *P, int64_t ld, int size, int r, MpSegment &ro
   rest.col_fix = -1;
   rest.tiles_x = pairs;
   t_rest = pairs * pairs;
-}
-
-// Numbers the CTAs of one launch's FW segments in the strip form, with the
-// strip length that suits the launch; returns their count.
-int fw_number_strips(std::vector<MpSegment> &segs, int sm_count) {
-  const int T = fapk::fw_strip_tiles(segs.data(), (int)segs.size(), sm_count);
-  int strips = 0;
-  for (MpSegment &s : segs) {
-    s.strip_tiles = T;
-    s.strip_begin = strips;
-    strips += fapk::fw_strips_of(s, T);
-  }
-  return strips;
-}
-
-// Lookahead form of fw_segments' `rest` for pivot block r of nb: the rows and
-// columns other than r and r + 1 (block row and column r + 1 get round r's
-// update inside pivot step r + 1).
-void fw_rest_lookahead(MpSegment &rest, int nb, int r) {
-  const int pairs = (nb - 2 + 1) / 2;
-  rest.row_skip2 = r + 1;
-  rest.col_skip2 = r + 1;
-  rest.tiles_x = pairs;
 }
 
 // Min-plus segment C = A (x) B (fresh C), tiled in 128x128.
@@ -684,8 +652,6 @@ int build_plan(fap_engine *e, Plan &pl) {
   struct GroupOffs {
     size_t batches, batches_alt, pdesc, row_begin, dec_begin, mp, bjobs, bsrc;
     std::vector<size_t> diag, panel, rest, rest2;
-    size_t tmaps = 0;
-    bool has_tmaps = false;
   };
   std::vector<GroupOffs> goffs(groups.size());
   pl.groups.assign(groups.size(), Plan::Group{});
@@ -820,37 +786,18 @@ int build_plan(fap_engine *e, Plan &pl) {
     G.panel_tiles.assign(maxnb, 0);
     G.rest_nseg.assign(maxnb, 0);
     G.rest_tiles.assign(maxnb, 0);
-    G.rest2_nseg.assign(maxnb, 0);
+    G.rest2_njob.assign(maxnb, 0);
+    G.rest2_per.assign(maxnb, 1);
     G.rest2_strips.assign(maxnb, 0);
     G.diag_blocks.assign(maxnb, 0);
     O.diag.assign(maxnb, 0);
     O.panel.assign(maxnb, 0);
     O.rest.assign(maxnb, 0);
     O.rest2.assign(maxnb, 0);
-    // Tensor-map pairs (distances, predecessors) of the parts' FW matrices
-    // for the strips' bulk tensor copies; a part without one (no encoder)
-    // keeps the per-thread copies.
-    std::vector<int32_t> tmap1(pdesc.size(), 0);
-    {
-      std::vector<TmapBlob> maps;
-      for (size_t i = 0; i < pdesc.size(); i++) {
-        const PartDesc &d = pdesc[i];
-        TmapBlob two[2];
-        if (fapk::encode_fw_tmaps(two, fwd + (size_t)d.mat_off * 4, pred ? fwp + d.mat_off : nullptr, d.ld,
-                                  d.ld, d.ld)) {
-          tmap1[i] = (int32_t)(maps.size() / 2) + 1;
-          maps.push_back(two[0]);
-          maps.push_back(two[1]);
-        }
-      }
-      if (!maps.empty()) {
-        O.tmaps = tb.add(maps.data(), maps.size());
-        O.has_tmaps = true;
-      }
-    }
     for (int r = 0; r < maxnb; r++) {
       std::vector<FwDiagJob> dj;
-      std::vector<MpSegment> ps, rs, r2s;
+      std::vector<MpSegment> ps, rs;
+      std::vector<FwRestJob> r2s;
       int pt = 0, rt = 0, blocks = 0;
       for (size_t pi = 0; pi < pdesc.size(); pi++) {
         const PartDesc &d = pdesc[pi];
@@ -875,10 +822,11 @@ int build_plan(fap_engine *e, Plan &pl) {
           pl.fw_tile_work += blk * (unsigned long long)nb * nb;
         }
         if (nb > 1) {
-          MpSegment rp, cp, rest;
-          int a1, a2, a3;
-          fw_segments(D, P, d.ld, d.ld, r, rp, cp, rest, a1, a2, a3, e->f32(), tmap1[pi]);
+          r2s.push_back({D, P, d.ld, d.ld, r, r + 1 < nb ? 1 : 0, 0});
           if (!e->f32()) {  // the wide int32 form's tiles
+            MpSegment rp, cp, rest;
+            int a1, a2, a3;
+            fw_segments(D, P, d.ld, d.ld, r, rp, cp, rest, a1, a2, a3);
             rp.tile_begin = pt;
             pt += a1;
             ps.push_back(rp);
@@ -889,11 +837,9 @@ int build_plan(fap_engine *e, Plan &pl) {
             rt += a3;
             rs.push_back(rest);
           }
-          if (r + 1 < nb) fw_rest_lookahead(rest, nb, r);
-          if (rest.tiles_x > 0) r2s.push_back(rest);
         }
       }
-      const int r2strips = fw_number_strips(r2s, e->sm_count);
+      const int r2strips = fapk::number_fw_rest(r2s.data(), (int)r2s.size(), e->sm_count, &G.rest2_per[r]);
       G.diag_cnt[r] = (int)dj.size();
       G.diag_blocks[r] = blocks;
       O.diag[r] = tb.add(dj.data(), dj.size());
@@ -903,7 +849,7 @@ int build_plan(fap_engine *e, Plan &pl) {
       G.rest_nseg[r] = (int)rs.size();
       G.rest_tiles[r] = rt;
       O.rest[r] = tb.add(rs.data(), rs.size());
-      G.rest2_nseg[r] = (int)r2s.size();
+      G.rest2_njob[r] = (int)r2s.size();
       G.rest2_strips[r] = r2strips;
       O.rest2[r] = tb.add(r2s.data(), r2s.size());
     }
@@ -925,7 +871,6 @@ int build_plan(fap_engine *e, Plan &pl) {
     G.row_begin = reinterpret_cast<const int64_t *>(base + O.row_begin);
     G.dec_begin = reinterpret_cast<const int64_t *>(base + O.dec_begin);
     G.mp = reinterpret_cast<const MpSegment *>(base + O.mp);
-    G.tmaps = O.has_tmaps ? static_cast<const void *>(base + O.tmaps) : nullptr;
     size_t R = O.diag.size();
     G.diag.resize(R);
     G.panel.resize(R);
@@ -935,7 +880,7 @@ int build_plan(fap_engine *e, Plan &pl) {
       G.diag[r] = reinterpret_cast<const FwDiagJob *>(base + O.diag[r]);
       G.panel[r] = reinterpret_cast<const MpSegment *>(base + O.panel[r]);
       G.rest[r] = reinterpret_cast<const MpSegment *>(base + O.rest[r]);
-      G.rest2[r] = reinterpret_cast<const MpSegment *>(base + O.rest2[r]);
+      G.rest2[r] = reinterpret_cast<const FwRestJob *>(base + O.rest2[r]);
     }
   }
   return FAP_OK;
@@ -1085,9 +1030,8 @@ struct Issuer {
         FAP_CUDA(fapk::launch_fw_chain(f32, pred, G.diag[r], G.diag_cnt[r], G.diag_blocks[r], st));
         FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
         FAP_CUDA(cudaStreamWaitEvent(e->side, e->ev_fw[0], 0));
-        if (G.rest2_nseg[r] > 0)
-          FAP_CUDA(fapk::launch_fw_strips(pred, G.rest2[r], G.rest2_nseg[r], G.rest2_strips[r], e->side, f32,
-                                          G.tmaps));
+        FAP_CUDA(fapk::launch_fw_rest(f32, pred, G.rest2[r], G.rest2_njob[r], G.rest2_strips[r], G.rest2_per[r],
+                                      e->side));
         FAP_CUDA(cudaEventRecord(e->ev_fw[1 + r % 2], e->side));
       } else {
         FAP_CUDA(fapk::launch_fw_diag(pred, G.diag[r], G.diag_cnt[r], st));
@@ -1409,9 +1353,6 @@ int check_status(fap_engine *e) {
     if (h & fapk::kErrSsspCap) return set_error(FAP_ERR_NOT_CONVERGED, "SSSP reached its iteration cap");
     return set_error(FAP_ERR_INVALID, "a kernel saw an out-of-range index");
   }
-  unsigned t = 0;
-  FAP_CUDA(fapk::tma_status(&t, true));
-  if (t) return set_error(FAP_ERR_CUDA, "a bulk tensor copy of the Floyd-Warshall tiles did not complete");
   return FAP_OK;
 }
 
@@ -1641,6 +1582,7 @@ int init_device(fap_engine *e, int device) {
   FAP_CUDA(cudaMemset(e->d_stats, 0, 8 * sizeof(unsigned long long)));
   FAP_CUDA(fapk::init_minplus_kernels());
   FAP_CUDA(fapk::init_fw_pivot_kernels());
+  FAP_CUDA(fapk::init_fw_rest_kernels());
   FAP_CUDA(fapk::init_sssp_kernels());
   FAP_CUDA(fapk::init_sssp_row_kernels());
   FAP_CUDA(fapk::init_bg_kernels());
@@ -2204,7 +2146,7 @@ int fap_fw_counters(fap_engine *e, uint64_t *out2, int32_t reset) {
   std::lock_guard<std::mutex> lk(e->mu);
   DeviceGuard g(e->device);
   unsigned long long strip = 0;
-  FAP_CUDA(fapk::fw_strip_counter(&strip, reset != 0));
+  FAP_CUDA(fapk::fw_rest_counter(&strip, reset != 0));
   out2[0] = strip;
   out2[1] = e->fw_host_work;
   if (reset) e->fw_host_work = 0;
@@ -2293,32 +2235,13 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
   cudaStream_t st = pick_stream(e, stream);
   TableBuilder tb;
   std::vector<size_t> od(maxnb), op(maxnb), orr(maxnb), or2(maxnb);
-  std::vector<int> nd(maxnb), bd(maxnb), np(maxnb), tp(maxnb), nr(maxnb), tr(maxnb), nr2(maxnb), sr2(maxnb);
+  std::vector<int> nd(maxnb), bd(maxnb), np(maxnb), tp(maxnb), nr(maxnb), tr(maxnb), nr2(maxnb), sr2(maxnb), pr2(maxnb);
   int rc;
   if ((rc = e->fw_look.ensure((size_t)count * fapk::fw_look_bytes())) != FAP_OK) return rc;
-  // tensor-map pairs of the matrices that meet the copy unit's alignment
-  // rules (16-byte base and row stride); the others keep per-thread copies
-  std::vector<int32_t> tmap1(count, 0);
-  size_t o_tmaps = 0;
-  bool has_tmaps = false;
-  {
-    std::vector<TmapBlob> maps;
-    for (int32_t b = 0; b < count; b++) {
-      TmapBlob two[2];
-      if (sizes[b] > Bk && fapk::encode_fw_tmaps(two, D[b], pred ? P[b] : nullptr, ld[b], sizes[b], sizes[b])) {
-        tmap1[b] = (int32_t)(maps.size() / 2) + 1;
-        maps.push_back(two[0]);
-        maps.push_back(two[1]);
-      }
-    }
-    if (!maps.empty()) {
-      o_tmaps = tb.add(maps.data(), maps.size());
-      has_tmaps = true;
-    }
-  }
   for (int r = 0; r < maxnb; r++) {
     std::vector<FwDiagJob> dj;
-    std::vector<MpSegment> ps, rs, r2s;
+    std::vector<MpSegment> ps, rs;
+    std::vector<FwRestJob> r2s;
     int pt = 0, rt = 0, blocks = 0;
     for (int32_t b = 0; b < count; b++) {
       int nb = (sizes[b] + Bk - 1) / Bk;
@@ -2335,11 +2258,11 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
       blocks += 2 * (nb - 1);
       dj.push_back(j);
       if (nb > 1) {
-        MpSegment a, c, rest;
-        int t1, t2, t3;
-        fw_segments(D[b], pred ? P[b] : nullptr, ld[b], sizes[b], r, a, c, rest, t1, t2, t3,
-                    dtype == FAP_DTYPE_F32, tmap1[b]);
+        r2s.push_back({D[b], pred ? P[b] : nullptr, ld[b], sizes[b], r, r + 1 < nb ? 1 : 0, 0});
         if (dtype != FAP_DTYPE_F32) {  // the wide int32 form's tiles
+          MpSegment a, c, rest;
+          int t1, t2, t3;
+          fw_segments(D[b], pred ? P[b] : nullptr, ld[b], sizes[b], r, a, c, rest, t1, t2, t3);
           a.tile_begin = pt;
           pt += t1;
           ps.push_back(a);
@@ -2350,11 +2273,9 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
           rt += t3;
           rs.push_back(rest);
         }
-        if (r + 1 < nb) fw_rest_lookahead(rest, nb, r);
-        if (rest.tiles_x > 0) r2s.push_back(rest);
       }
     }
-    const int r2strips = fw_number_strips(r2s, e->sm_count);
+    const int r2strips = fapk::number_fw_rest(r2s.data(), (int)r2s.size(), e->sm_count, &pr2[r]);
     nr2[r] = (int)r2s.size();
     sr2[r] = r2strips;
     or2[r] = tb.add(r2s.data(), r2s.size());
@@ -2380,7 +2301,6 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
   if ((rc = e->small.ensure(std::max<size_t>(tb.bytes.size(), 64))) != FAP_OK) return rc;
   FAP_CUDA(cudaMemcpyAsync(e->small.p, tb.bytes.data(), tb.bytes.size(), cudaMemcpyHostToDevice, st));
   unsigned char *base = static_cast<unsigned char *>(e->small.p);
-  const void *tmaps = has_tmaps ? static_cast<const void *>(base + o_tmaps) : nullptr;
   bool packed = false;
   if (!f32) {
     // a finite shortest distance is at most (size - 1) * the largest entry
@@ -2399,9 +2319,8 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
       FAP_CUDA(fapk::launch_fw_chain(f32, pred, djobs, nd[r], bd[r], st));
       FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
       FAP_CUDA(cudaStreamWaitEvent(e->side, e->ev_fw[0], 0));
-      if (nr2[r] > 0)
-        FAP_CUDA(fapk::launch_fw_strips(pred, reinterpret_cast<const MpSegment *>(base + or2[r]), nr2[r], sr2[r],
-                                        e->side, f32, tmaps));
+      FAP_CUDA(fapk::launch_fw_rest(f32, pred, reinterpret_cast<const FwRestJob *>(base + or2[r]), nr2[r], sr2[r],
+                                    pr2[r], e->side));
       FAP_CUDA(cudaEventRecord(e->ev_fw[1 + r % 2], e->side));
     } else {
       FAP_CUDA(fapk::launch_fw_diag(pred, djobs, nd[r], st));

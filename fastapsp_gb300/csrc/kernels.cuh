@@ -63,7 +63,6 @@ struct MpSegment {
   int32_t tiles_x;     // CTA tiles along columns
   int32_t tile_begin;  // first global CTA index of this segment
   int32_t strip_begin; // first global CTA index in the strip form (min-plus)
-  int32_t strip_tiles; // Floyd-Warshall strips: 64-column tiles per CTA
   // Optional Floyd-Warshall override of the part's own columns (min-plus of
   // a part's inner rows): where col_part[col] == part, the output takes
   // F[row][col_local[col] - local0] (and Fp) instead of the product.
@@ -73,11 +72,6 @@ struct MpSegment {
   const int32_t *Fp;
   int64_t ldf;
   int32_t part, local0;
-  // Floyd-Warshall strips: 1 + the index of the matrix's tensor-map pair in
-  // the launch's table (0: none, per-thread copies) and the first row of B
-  // (the pivot block row) in the matrix.
-  int32_t tmap1;
-  int32_t b_row0;
 };
 
 // FW pivot job: close the 64x64 pivot block of one matrix and update its
@@ -93,6 +87,16 @@ struct FwDiagJob {
                  // remaining-tile launch of round prev left them out); -1: none
   int32_t panel_begin;  // first CTA of its panel blocks in the launch's numbering
   void *look;           // the matrix's scratch of fw_look_bytes() (used when prev >= 0)
+};
+
+// FW remaining tiles of one matrix in one round (fw_rest.cu): block rows and
+// columns other than `block` and, with look, `block` + 1.
+struct FwRestJob {
+  void *D;
+  int32_t *P;
+  int64_t ld;
+  int32_t size, block, look;
+  int32_t strip_begin;  // first CTA in the launch's numbering
 };
 
 // A strided row-major matrix of 4-byte values.

@@ -35,24 +35,6 @@ cudaError_t launch_minplus_strips(bool pred, const MpSegment *d_segs, int nseg, 
                                   bool aligned = true);
 int minplus_strip_class_cols(int c);
 int minplus_strip_tiles();
-// Strip form of the FW remaining-tile phase (packed int32, or FP32 with
-// f32; init_from_c = 1, K <= 64): CTAs numbered by MpSegment::strip_begin,
-// fw_strips_of(segment, strip_tiles) per segment.  tmaps:
-// device array of CUtensorMap pairs (distances, predecessors) indexed by
-// MpSegment::tmap1 - 1 (64-byte aligned; null: no segment uses one).
-cudaError_t launch_fw_strips(bool pred, const MpSegment *d_segs, int nseg, int strips,
-                             cudaStream_t st, bool f32 = false, const void *tmaps = nullptr);
-// Nonzero when a bulk tensor copy of the FW strips did not complete (the
-// strip was abandoned: the results are not valid); optionally reset.
-cudaError_t tma_status(unsigned *out, bool reset);
-// Encodes the tensor-map pair of one 4-byte matrix (rows x cols, row
-// stride ld elements) for the FW strips' 64 x 64 boxes into out[0] (d) and
-// out[1] (p, or d again when p is null); false when the matrix does not meet
-// the copy unit's alignment rules (16-byte base and row stride) or the
-// driver has no encoder.
-bool encode_fw_tmaps(void *out, const void *d, const void *p, int64_t ld, int rows, int cols);
-int fw_strips_of(const MpSegment &s, int tiles);  // CTAs of a segment with that many column tiles each
-int fw_strip_tiles(const MpSegment *segs, int nseg, int sm_count);  // column tiles per CTA for a launch of these
 int minplus_strip_max_k();   // largest K of the strip form
 // Segments go to the strip form in classes of K (one launch per class, each
 // with its own CTAs per SM): class c takes K <= minplus_strip_class_k(c)
@@ -66,9 +48,6 @@ unsigned pack_limit();
 // with no active step, active steps over all tiles]; optionally reset.
 cudaError_t strip_counters(unsigned long long out[3], bool reset);
 int max_packed_k();
-// Add-mins executed by the FW remaining-tile strips on the current device
-// since the last reset; optionally reset.
-cudaError_t fw_strip_counter(unsigned long long *out, bool reset);
 // Wide int32 form: closes each job's pivot block.
 cudaError_t launch_fw_diag(bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st);
 // fw_pivot.cu (packed int32 and FP32 forms): round job.prev's update of each
@@ -76,6 +55,15 @@ cudaError_t launch_fw_diag(bool pred, const FwDiagJob *d_jobs, int njobs, cudaSt
 // panels: two launches.  blocks = the jobs' panel blocks, 2 (blocks a side - 1)
 // each, numbered by FwDiagJob::panel_begin.
 cudaError_t launch_fw_chain(bool f32, bool pred, const FwDiagJob *d_jobs, int njobs, int blocks, cudaStream_t st);
+// fw_rest.cu: number_fw_rest numbers a launch's CTAs (returns their count)
+// and chooses the column tiles each takes.
+int number_fw_rest(FwRestJob *jobs, int njobs, int sm_count, int *per);
+cudaError_t launch_fw_rest(bool f32, bool pred, const FwRestJob *d_jobs, int njobs, int strips, int per,
+                           cudaStream_t st);
+// Add-mins executed by the remaining tiles on the current device since the
+// last reset; optionally reset.
+cudaError_t fw_rest_counter(unsigned long long *out, bool reset);
+cudaError_t init_fw_rest_kernels();
 size_t fw_look_bytes();  // device scratch per matrix
 cudaError_t init_fw_pivot_kernels();
 int minplus_tile_rows();  // CTA output tile edge (128)

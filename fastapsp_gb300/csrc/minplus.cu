@@ -29,8 +29,6 @@
 // min(D_ij, D_ir (x) D_rj).  Ties keep the current value, so predecessors
 // follow P[i][j] = P[k][j] on strict improvement as in the reference.
 
-#include <cuda.h>  // CUtensorMap (the type only; maps are encoded on the host)
-#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -68,60 +66,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 __device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;\n" ::); }
 __device__ __forceinline__ void cp_async_wait_2() { asm volatile("cp.async.wait_group 2;\n" ::); }
 __device__ __forceinline__ void cp_async_wait_0() { asm volatile("cp.async.wait_group 0;\n" ::); }
-
-// Bulk tensor copies (TMA): a 2-D box of a tensor map into shared memory,
-// completed on an mbarrier whose phase also waits for the expected bytes.
-__device__ __forceinline__ unsigned smem_u32(const void *p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ void mbar_init(unsigned long long *bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_init_fence() {
-  asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-}
-// One arrival that also expects `bytes` of copies on the barrier's phase.
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long *bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
-               : "memory");
-}
-// Waits for the phase with this parity to complete: false after `polls`
-// unsuccessful polls (each poll may suspend the thread for a short while).
-__device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned parity, int polls) {
-  const unsigned a = smem_u32(bar);
-  for (int i = 0; i < polls; i++) {
-    unsigned done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(done)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-// Orders this thread's earlier shared-memory accesses before later bulk
-// copies (the async proxy) into the same buffers.
-__device__ __forceinline__ void fence_proxy_async_smem() {
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-}
-// The tensor map, copied to global memory by the host before the launch,
-// made visible to the copy unit.
-__device__ __forceinline__ void tmap_acquire(const CUtensorMap *map) {
-  asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;\n" ::"l"(map) : "memory");
-}
-// Box of `map` at column x, row y (x a multiple of 4 elements of 4 bytes:
-// 16-byte aligned) into dst (16-byte aligned shared memory).  Elements
-// outside the tensor arrive as zeros.
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y,
-                                            unsigned long long *bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], "
-      "[%4];\n" ::"r"(smem_u32(dst)),
-      "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-      : "memory");
-}
 
 // Block index of list entry g of 0..nblocks-1 without block `skip` (and
 // `skip2`, when it is above `skip`), or of the one-block list `fix`; -1 past
@@ -790,71 +734,6 @@ __device__ __forceinline__ void strip_addmin(unsigned &acc, int &arg, unsigned a
   }
 }
 
-// FP32 add-mins of a thread's 8 x 4 outputs over steps [0, kseg) (kseg a
-// multiple of 4) in groups of four, then, with PRED, each output's group
-// resolved to the step idx (k + 1) of its last strict improvement -- the
-// same values and steps as single add-mins in ascending order.  As: A^T
-// [k][sa] and Bs: B [k][sb] in the swizzled layout (swz); the thread's rows
-// are a0 .. a0 + 3 and a0 + kBlk .. a0 + kBlk + 3, its columns b0 .. b0 + 3.
-// With LEAN, the B operands load two columns at a time (24 operands live
-// instead of 32).  Without `hi` (uniform over the CTA: the tile's second
-// 64-row block is empty) the rows a0 + kBlk .. are left as they are.
-template <bool PRED, bool LEAN = false>
-__device__ __forceinline__ void addmin_groups_f32(unsigned (&acc)[8][4], int (&arg)[8][4],
-                                                  const unsigned *As, int sa, int a0,
-                                                  const unsigned *Bs, int sb, int b0, int kseg,
-                                                  bool hi = true) {
-  for (int kk = 0; kk < kseg; kk += 4) {
-    const unsigned *acol = As + kk * sa + (a0 ^ swz<true>(kk));
-    const unsigned *bcol = Bs + kk * sb + (b0 ^ swz<true>(kk));
-    unsigned b[4][4];  // [column][step]
-    if (!LEAN) {
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const uint4 v = *reinterpret_cast<const uint4 *>(bcol + j * sb);
-        b[0][j] = v.x, b[1][j] = v.y, b[2][j] = v.z, b[3][j] = v.w;
-      }
-    }
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      if (h == 1 && !hi) break;
-      unsigned a[4][4];  // [row of the half][step]
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const uint4 v = *reinterpret_cast<const uint4 *>(acol + j * sa + h * kBlk);
-        a[0][j] = v.x, a[1][j] = v.y, a[2][j] = v.z, a[3][j] = v.w;
-      }
-#pragma unroll
-      for (int ch = 0; ch < 2; ch++) {
-        if (LEAN) {
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const uint2 v = *reinterpret_cast<const uint2 *>(bcol + j * sb + ch * 2);
-            b[ch * 2][j] = v.x, b[ch * 2 + 1][j] = v.y;
-          }
-        }
-#pragma unroll
-        for (int r = 0; r < 4; r++)
-#pragma unroll
-          for (int c = ch * 2; c < ch * 2 + 2; c++)
-            strip_addmin4_f32(acc[h * 4 + r][c], arg[h * 4 + r][c], a[r], b[c], kk + 1);
-      }
-    }
-  }
-  if (PRED) {
-#pragma unroll
-    for (int r = 0; r < 8; r++)
-#pragma unroll
-      for (int c = 0; c < 4; c++) {
-        if (r >= 4 && !hi) continue;
-        const int k0 = arg[r][c] > 0 ? arg[r][c] - 1 : 0;
-        const int sw = swz<true>(k0);
-        arg[r][c] = strip_resolve_f32(acc[r][c], arg[r][c], As + k0 * sa + (a0 ^ sw) + (r >> 2) * kBlk + (r & 3),
-                                      sa, Bs + k0 * sb + (b0 ^ sw) + c, sb);
-      }
-  }
-}
-
 // The same for the strip min-plus, from row-major copies of the operands:
 // Ar[128][ars] (row m's steps contiguous, ars = strip_ar_stride(kseg)) and
 // Bq, the tile's B by step group (16-byte unit g * 64 + col: steps 4g ..
@@ -1356,409 +1235,6 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
   }
 }
 
-// Strip form of the accumulating packed product of the Floyd-Warshall
-// remaining-tile phase: D_ij = min(D_ij, D_ir (x) D_rj) with K <= 64 (one
-// pivot block), ties keeping D_ij.  A CTA owns a strip: one 128-row tile of
-// the segment's row list (A = D_ir resident) and strip_tiles consecutive
-// column tiles of its column list (chosen per launch, fw_strip_tiles).  Everything a tile needs is
-// in flight before it is needed: B (= D_rj) double-buffered, the current
-// tile's C and B's predecessors staged behind its DPX loop.  The product starts from "unreached" and C joins in the
-// epilogue with index 0, which gives the same minimum and tie rule as
-// starting from C.
-// Column tile of the form used: one 64-column block (128 x 64 tiles, 8 x 4
-// outputs a thread, 112 KB of shared memory, two CTAs per SM, so that one
-// CTA's epilogue overlaps the other's add-mins).  TN = 128 (block pairs,
-// 197 KB, one CTA per SM) is the other form.
-constexpr int kFwStripTN = 64;
-
-template <int TN>
-struct FwStripSmem {
-  unsigned A[kBlk][kTile];     // A keys, transposed: pivot block x strip rows
-  unsigned B[2][kBlk][TN];     // B keys of the current / next tile
-  int32_t Bp[kBlk][TN];        // B's predecessors of the current tile
-  unsigned C[kTile][TN];       // C of the current tile
-};
-
-// Copies rows [0, 64) of B-like data (row k at src + k * ld, columns of the
-// tile's 64-column blocks starting at cbase.x / cbase.y, -1 for none) into
-// dst[64][TN] (SWZ: chunks permuted by swz); 16-byte copies of 4 columns
-// where aligned, `fill` outside the matrix.
-template <int TN, bool SWZ = false>
-__device__ __forceinline__ void fw_load_b(unsigned *dst, const unsigned *src, int64_t ld, int K,
-                                          int N, int2 cbase, bool vec, unsigned fill) {
-  constexpr int TPR = TN / 4;  // threads per row
-  const int t = threadIdx.x;
-  const int j = (t % TPR) * 4;
-  const int cb = (j >> 6) ? cbase.y : cbase.x;
-  const int col = cb + (j & 63);
-  for (int kk = t / TPR; kk < kBlk; kk += kThreads / TPR) {
-    unsigned *d = dst + kk * TN + (j ^ swz<SWZ>(kk));
-    const unsigned *g = src + (int64_t)kk * ld + col;
-    if (cb >= 0 && kk < K && vec && col + 3 < N) {
-      cp_async16(d, g);
-    } else {
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        if (cb >= 0 && kk < K && col + q < N) cp_async4(d + q, g + q);
-        else d[q] = fill;
-      }
-    }
-  }
-}
-
-// Work counter of the FW remaining-tile strips (diagnostics): add-mins
-// executed (steps run x the tile's 128 x TN outputs), summed per CTA.
-__device__ unsigned long long g_fw_counters[1];
-// Set when a bulk tensor copy of the FW strips did not complete within its
-// poll limit (the kernel then gives up on the strip; the host reports it).
-__device__ unsigned g_tma_status;
-constexpr int kTmaPolls = 1 << 22;
-constexpr unsigned kTmaBox = 64 * 64 * 4;  // bytes of one 64 x 64 box
-
-// F32: FP32 distances (value bits, "unreached" = the bits of 1e8): the
-// product keeps each output's value bits and the step (k + 1) of its last
-// strict improvement in two registers (the active steps, in order); the
-// epilogue stores the product where it is strictly below the current value,
-// with the predecessor of that step -- the same result as updating the
-// current value step by step.  TN = 64.  (Two steps per pass, as in the
-// strip min-plus, measured the same here and spills more.)
-// TMA: when the segment's matrix has a tensor-map pair (tmaps[2 (tmap1 - 1)]
-// for the distances, + 1 for the predecessors: 64 x 64 boxes of 4-byte
-// elements, x = column, y = row), thread 0 stages the tile's C (two boxes),
-// B's predecessors and, for packed keys, B itself with bulk tensor copies on
-// three mbarriers (the two B buffers, C with the predecessors); the FP32 B
-// tile keeps its swizzled layout through per-thread copies.  Without a map
-// the per-thread asynchronous copies stage everything.
-template <bool PRED, int TN, bool F32 = false>
-__global__ void __launch_bounds__(kThreads, TN == 128 ? 1 : 2)
-    mp_fwstrip_kernel(const MpSegment *__restrict__ segs, int nseg, const CUtensorMap *__restrict__ tmaps) {
-  static_assert(!F32 || TN == 64, "the FP32 form uses 64-column tiles");
-  constexpr int CH = TN / 64;   // 64-column blocks of a tile
-  constexpr int TPR = TN / 4;   // threads per row in the row-wise copies
-  // (a name of its own: the other kernels' dynamic shared memory, under
-  // one name, is declared 16-byte aligned; the bulk tensor copies want
-  // 128-byte aligned destinations, and B, Bp and C start at multiples of
-  // 16 KB of this array)
-  extern __shared__ __align__(128) unsigned char fw_smem[];
-  FwStripSmem<TN> &sm = *reinterpret_cast<FwStripSmem<TN> *>(fw_smem);
-  __shared__ MpSegment seg;
-  __shared__ unsigned s_kmask[2][2];  // rows k of B with a finite entry (per tile parity)
-  __shared__ unsigned s_amask[2];     // columns k of A with a finite entry (per strip)
-  __shared__ __align__(8) unsigned long long s_mbar[3];  // TMA: B buffers 0 and 1; C + B's predecessors
-  if (threadIdx.x == 0) {
-    seg = find_strip_segment(segs, nseg, blockIdx.x);
-    mbar_init(&s_mbar[0], 1);
-    mbar_init(&s_mbar[1], 1);
-    mbar_init(&s_mbar[2], 1);
-    mbar_init_fence();
-  }
-  if (threadIdx.x < 4) (&s_kmask[0][0])[threadIdx.x] = 0u;
-  if (threadIdx.x < 2) s_amask[threadIdx.x] = 0u;
-  __syncthreads();
-  const MpSegment &s = seg;
-  const CUtensorMap *tmap_d = (TN == 64 && tmaps != nullptr && s.tmap1 > 0) ? tmaps + 2 * (s.tmap1 - 1) : nullptr;
-  // (uniform over the CTA; the alignment tests only guard the copies' rules:
-  // 128-byte shared destinations, 64-byte tensor maps)
-  const bool tma = tmap_d != nullptr && (smem_u32(fw_smem) & 127u) == 0 &&
-                   (reinterpret_cast<uintptr_t>(tmap_d) & 63) == 0;
-  const bool tma_b = tma && !F32;
-  if (tma && threadIdx.x == 0) {
-    tmap_acquire(tmap_d);
-    if (PRED) tmap_acquire(tmap_d + 1);
-  }
-  const int local = blockIdx.x - s.strip_begin;
-  const int nbr = (s.M + kBlk - 1) / kBlk, nbc = (s.N + kBlk - 1) / kBlk;
-  // column list length, in tiles of CH blocks, and this strip's column tiles
-  const int nct = (list_len(s.col_skip, s.col_skip2, s.col_fix, nbc) + CH - 1) / CH;
-  const int per = s.strip_tiles, sx = (nct + per - 1) / per;
-  const int tyt = local / sx;
-  const int jt0 = (local - tyt * sx) * per;
-  const int jt1 = min(jt0 + per, nct);
-  const int rl0 = list_block(2 * tyt, s.row_skip, s.row_skip2, s.row_fix, nbr);
-  const int rl1 = list_block(2 * tyt + 1, s.row_skip, s.row_skip2, s.row_fix, nbr);
-  const int rbase0 = rl0 >= 0 ? rl0 * kBlk : -1, rbase1 = rl1 >= 0 ? rl1 * kBlk : -1;
-  auto col_bases = [&](int jt) {  // first columns of the tile's blocks (-1: none)
-    const int b0 = list_block(CH * jt, s.col_skip, s.col_skip2, s.col_fix, nbc);
-    const int b1 = CH == 2 ? list_block(CH * jt + 1, s.col_skip, s.col_skip2, s.col_fix, nbc) : -1;
-    return make_int2(b0 >= 0 ? b0 * kBlk : -1, b1 >= 0 ? b1 * kBlk : -1);
-  };
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  const unsigned INF = F32 ? __float_as_uint(Dist<float>::inf()) : Dist<uint32_t>::inf();
-  const unsigned FIN = F32 ? INF : kPackH;  // entries below are finite
-  const int kseg = (s.K + 3) & ~3;
-  const bool vec_b = (s.ldb & 3) == 0 && (reinterpret_cast<uintptr_t>(s.B) & 15) == 0;
-  const bool vec_bp = PRED && (s.ldbp & 3) == 0 && (reinterpret_cast<uintptr_t>(s.Bp) & 15) == 0;
-  const bool vec_c = (s.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(s.C) & 15) == 0;
-
-  // Prologue: A (transposed) and the first B | the first B's predecessors.
-  for (int idx = threadIdx.x; idx < kBlk * kTile; idx += kThreads) {
-    const int kk = idx >> 7, m = idx & (kTile - 1);
-    const int rb = (m >> 6) ? rbase1 : rbase0;
-    const int row = rb + (m & 63);
-    unsigned *d = &sm.A[kk][m ^ swz<F32>(kk)];
-    if (rb >= 0 && row < s.M && kk < s.K)
-      cp_async4(d, static_cast<const unsigned *>(s.A) + (int64_t)row * s.lda + kk);
-    else
-      *d = INF;
-  }
-  // B of a tile by TMA (thread 0): one box of pivot rows b_row0.. over the
-  // tile's column block, or an arrival without bytes when it has none.
-  auto tma_issue_b = [&](int b, int2 c) {
-    mbar_expect_tx(&s_mbar[b], c.x >= 0 ? kTmaBox : 0u);
-    if (c.x >= 0) tma_load_2d(&sm.B[b][0][0], tmap_d, c.x, s.b_row0, &s_mbar[b]);
-  };
-  int2 cb = col_bases(jt0);
-  if (!tma_b)
-    fw_load_b<TN, F32>(&sm.B[0][0][0], static_cast<const unsigned *>(s.B), s.ldb, s.K, s.N, cb, vec_b, INF);
-  else if (threadIdx.x == 0)
-    tma_issue_b(0, cb);
-  cp_async_commit();
-  // The epilogue's view of C in registers (the descriptor is in shared memory).
-  unsigned *const c_mat = static_cast<unsigned *>(s.C);
-  int32_t *const p_mat = s.Cp;
-  const int64_t ldc = s.ldc, ldcp = s.ldcp;
-  const int m_rows = s.M, n_cols = s.N;
-  unsigned long long n_work = 0;  // add-mins executed (thread 0)
-
-  for (int jt = jt0; jt < jt1; jt++) {
-    const int buf = (jt - jt0) & 1;
-    const unsigned use = (unsigned)(jt - jt0);  // tiles so far: B[buf] is on use >> 1, C on use
-    cb = col_bases(jt);
-    if (jt + 1 < jt1) {
-      if (!tma_b)
-        fw_load_b<TN, F32>(&sm.B[buf ^ 1][0][0], static_cast<const unsigned *>(s.B), s.ldb, s.K, s.N,
-                  col_bases(jt + 1), vec_b, INF);
-      else if (threadIdx.x == 0)
-        tma_issue_b(buf ^ 1, col_bases(jt + 1));
-    }
-    cp_async_commit();
-    cp_async_wait_1();  // A and this tile's B have landed
-    const bool b_ok = !tma_b || mbar_wait(&s_mbar[buf], (use >> 1) & 1u, kTmaPolls);
-    if (jt == jt0)  // A keys; a warp converts 32 entries of one step k and marks finite ones
-      for (int idx = threadIdx.x; idx < kBlk * kTile; idx += kThreads) {
-        const unsigned v = (&sm.A[0][0])[idx];
-        if (!F32) (&sm.A[0][0])[idx] = min(v, kPackH) << kIdxBits;
-        const int kk = idx >> 7;
-        if (__any_sync(0xffffffffu, v < FIN) && (threadIdx.x & 31) == 0)
-          atomicOr(&s_amask[kk >> 5], 1u << (kk & 31));
-      }
-    {  // B keys; TPR lanes convert a whole row and its first lane marks it when finite
-      const int j = (threadIdx.x % TPR) * 4;
-      const int lane = threadIdx.x & 31;
-      for (int kk = threadIdx.x / TPR; kk < kBlk; kk += kThreads / TPR) {
-        uint4 *p = reinterpret_cast<uint4 *>(&sm.B[buf][kk][j]);
-        const unsigned idx = (unsigned)kk + 1u;
-        uint4 v = *p;
-        if (tma_b) {  // steps past K and columns past N: the box brought other rows or zeros
-          const int col = cb.x + j;
-          const bool row_ok = cb.x >= 0 && kk < s.K;
-          if (!row_ok || col >= s.N) v.x = INF;
-          if (!row_ok || col + 1 >= s.N) v.y = INF;
-          if (!row_ok || col + 2 >= s.N) v.z = INF;
-          if (!row_ok || col + 3 >= s.N) v.w = INF;
-        }
-        const bool fin = min(min(v.x, v.y), min(v.z, v.w)) < FIN;
-        if (!F32) {
-          v.x = (min(v.x, kPackH) << kIdxBits) | idx;
-          v.y = (min(v.y, kPackH) << kIdxBits) | idx;
-          v.z = (min(v.z, kPackH) << kIdxBits) | idx;
-          v.w = (min(v.w, kPackH) << kIdxBits) | idx;
-          *p = v;
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, fin);  // every lane runs the same trips
-        const unsigned grp = TPR == 32 ? 0xffffffffu : ((1u << (TPR & 31)) - 1u);
-        if (lane % TPR == 0 && ((bal >> lane) & grp) != 0u)
-          atomicOr(&s_kmask[buf][kk >> 5], 1u << (kk & 31));
-      }
-      if (threadIdx.x < 2) s_kmask[buf ^ 1][threadIdx.x] = 0u;  // for the next tile
-    }
-    if (__syncthreads_or(!b_ok)) {  // a B copy never completed: give up on the strip
-      if (threadIdx.x == 0) atomicOr(&g_tma_status, 1u);
-      mbar_wait(&s_mbar[buf], (use >> 1) & 1u, kTmaPolls);
-      if (jt + 1 < jt1) mbar_wait(&s_mbar[buf ^ 1], ((use + 1) >> 1) & 1u, kTmaPolls);
-      cp_async_wait_0();
-      return;
-    }
-    // Stage this tile's C behind the DPX loop.
-    if (tma) {
-      // C's two 64-row boxes and B's predecessors (rows b_row0..), whatever
-      // lies outside the matrix arriving as zeros: the epilogue stores no
-      // such output and reads only predecessors of steps below K.
-      if (threadIdx.x == 0) {
-        const bool c0 = cb.x >= 0 && rbase0 >= 0, c1 = cb.x >= 0 && rbase1 >= 0, bp = PRED && cb.x >= 0;
-        mbar_expect_tx(&s_mbar[2], (c0 ? kTmaBox : 0u) + (c1 ? kTmaBox : 0u) + (bp ? kTmaBox : 0u));
-        if (c0) tma_load_2d(&sm.C[0][0], tmap_d, cb.x, rbase0, &s_mbar[2]);
-        if (c1) tma_load_2d(&sm.C[kBlk][0], tmap_d, cb.x, rbase1, &s_mbar[2]);
-        if (bp) tma_load_2d(&sm.Bp[0][0], tmap_d + 1, cb.x, s.b_row0, &s_mbar[2]);
-      }
-    } else {
-      const int j = (threadIdx.x % TPR) * 4;
-      const int cbj = (j >> 6) ? cb.y : cb.x;
-      const int col = cbj + (j & 63);
-      for (int m = threadIdx.x / TPR; m < kTile; m += kThreads / TPR) {
-        const int rb = (m >> 6) ? rbase1 : rbase0;
-        const int row = rb + (m & 63);
-        unsigned *d = &sm.C[m][j];
-        const unsigned *g = static_cast<const unsigned *>(s.C) + (int64_t)row * s.ldc + col;
-        if (rb >= 0 && row < s.M && cbj >= 0 && vec_c && col + 3 < s.N) {
-          cp_async16(d, g);
-        } else {
-#pragma unroll
-          for (int q = 0; q < 4; q++) {
-            if (rb >= 0 && row < s.M && cbj >= 0 && col + q < s.N) cp_async4(d + q, g + q);
-            else d[q] = INF;
-          }
-        }
-      }
-      // ... and B's predecessors of this tile, read in the epilogue only
-      if (PRED)
-        fw_load_b<TN>(reinterpret_cast<unsigned *>(&sm.Bp[0][0]), reinterpret_cast<const unsigned *>(s.Bp),
-                      s.ldbp, s.K, s.N, cb, vec_bp, 0xffffffffu);
-    }
-    cp_async_commit();
-
-    unsigned acc[8][4 * CH];
-    int arg[8][4 * CH];  // F32: step (k + 1) of the last strict improvement, 0: none
-#pragma unroll
-    for (int r = 0; r < 8; r++)
-#pragma unroll
-      for (int c = 0; c < 4 * CH; c++) {
-        acc[r][c] = F32 ? INF : kPackH << kIdxBits;
-        arg[r][c] = 0;
-      }
-    // Only steps k whose B row (pivot row k over this tile's columns) and A
-    // column (over this strip's rows) have a finite entry can improve an
-    // output: all k (unrolled) when every row
-    // has one, else the set bits of the row mask.  The next step's operands
-    // load while the current step's add-mins issue.
-    {
-      const unsigned *acol = &sm.A[0][ty * 4];
-      const unsigned *bcol = &sm.B[buf][0][tx * 4];
-      unsigned long long msk = (unsigned long long)(s_kmask[buf][0] & s_amask[0]) |
-                               ((unsigned long long)(s_kmask[buf][1] & s_amask[1]) << 32);
-      if (kseg < 64) msk &= (1ull << kseg) - 1ull;
-      const int nact = __popcll(msk);
-      // FP32 with at least half of the steps active: all steps in groups of
-      // four (steps that are not active hold "unreached" on one side)
-      const bool grouped = F32 && CH == 1 && nact > 0 && 2 * nact >= kseg;
-      // (the FP32 groups skip the rows of an empty second row block)
-      n_work += (unsigned long long)(nact == s.K || grouped ? kseg : nact) * (grouped && rbase1 < 0 ? kBlk : kTile) * TN;
-      if (grouped) {
-        if constexpr (F32 && CH == 1)
-          addmin_groups_f32<PRED>(acc, arg, &sm.A[0][0], kTile, ty * 4, &sm.B[buf][0][0], TN, tx * 4, kseg,
-                                  rbase1 >= 0);
-      } else if (F32 && msk) {
-        while (msk) {  // (the swizzled layout)
-          const int kk = __ffsll(msk) - 1;
-          msk &= msk - 1ull;
-          const unsigned *ak = &sm.A[kk][(ty * 4) ^ swz<true>(kk)];
-          const uint4 na0 = *reinterpret_cast<const uint4 *>(ak);
-          const uint4 na1 = *reinterpret_cast<const uint4 *>(ak + kBlk);
-          const uint4 nb0 = *reinterpret_cast<const uint4 *>(&sm.B[buf][kk][(tx * 4) ^ swz<true>(kk)]);
-          const unsigned a[8] = {na0.x, na0.y, na0.z, na0.w, na1.x, na1.y, na1.z, na1.w};
-          const unsigned b[4] = {nb0.x, nb0.y, nb0.z, nb0.w};
-#pragma unroll
-          for (int r = 0; r < 8; r++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) strip_addmin<true>(acc[r][c], arg[r][c], a[r], b[c], kk + 1);
-        }
-      } else if (__popcll(msk) == s.K && s.K > 0) {
-        uint4 na0 = *reinterpret_cast<const uint4 *>(acol);
-        uint4 na1 = *reinterpret_cast<const uint4 *>(acol + kBlk);
-        uint4 nb0 = *reinterpret_cast<const uint4 *>(bcol);
-        uint4 nb1 = CH == 2 ? *reinterpret_cast<const uint4 *>(bcol + kBlk) : nb0;
-#pragma unroll 2
-        for (int kk = 0; kk < kseg; kk++) {
-          const unsigned a[8] = {na0.x, na0.y, na0.z, na0.w, na1.x, na1.y, na1.z, na1.w};
-          const unsigned b[8] = {nb0.x, nb0.y, nb0.z, nb0.w, nb1.x, nb1.y, nb1.z, nb1.w};
-          const int kn = kk + 1 < kseg ? kk + 1 : kk;
-          na0 = *reinterpret_cast<const uint4 *>(acol + kn * kTile);
-          na1 = *reinterpret_cast<const uint4 *>(acol + kn * kTile + kBlk);
-          nb0 = *reinterpret_cast<const uint4 *>(bcol + kn * TN);
-          if (CH == 2) nb1 = *reinterpret_cast<const uint4 *>(bcol + kn * TN + kBlk);
-#pragma unroll
-          for (int r = 0; r < 8; r++)
-#pragma unroll
-            for (int c = 0; c < 4 * CH; c++) acc[r][c] = __viaddmin_u32(a[r], b[c], acc[r][c]);
-        }
-      } else if (msk) {
-        int kk = __ffsll(msk) - 1;
-        msk &= msk - 1ull;
-        uint4 na0 = *reinterpret_cast<const uint4 *>(acol + kk * kTile);
-        uint4 na1 = *reinterpret_cast<const uint4 *>(acol + kk * kTile + kBlk);
-        uint4 nb0 = *reinterpret_cast<const uint4 *>(bcol + kk * TN);
-        uint4 nb1 = CH == 2 ? *reinterpret_cast<const uint4 *>(bcol + kk * TN + kBlk) : nb0;
-        while (kk >= 0) {
-          const unsigned a[8] = {na0.x, na0.y, na0.z, na0.w, na1.x, na1.y, na1.z, na1.w};
-          const unsigned b[8] = {nb0.x, nb0.y, nb0.z, nb0.w, nb1.x, nb1.y, nb1.z, nb1.w};
-          kk = msk ? __ffsll(msk) - 1 : -1;
-          if (msk) msk &= msk - 1ull;
-          const int kn = kk >= 0 ? kk : 0;
-          na0 = *reinterpret_cast<const uint4 *>(acol + kn * kTile);
-          na1 = *reinterpret_cast<const uint4 *>(acol + kn * kTile + kBlk);
-          nb0 = *reinterpret_cast<const uint4 *>(bcol + kn * TN);
-          if (CH == 2) nb1 = *reinterpret_cast<const uint4 *>(bcol + kn * TN + kBlk);
-#pragma unroll
-          for (int r = 0; r < 8; r++)
-#pragma unroll
-            for (int c = 0; c < 4 * CH; c++) acc[r][c] = __viaddmin_u32(a[r], b[c], acc[r][c]);
-        }
-      }
-    }
-    cp_async_wait_0();
-    const bool c_ok = !tma || mbar_wait(&s_mbar[2], use & 1u, kTmaPolls);
-    if (__syncthreads_or(!c_ok)) {  // C and the predecessors staged (by every thread, or the copy unit)
-      if (threadIdx.x == 0) atomicOr(&g_tma_status, 1u);
-      mbar_wait(&s_mbar[2], use & 1u, kTmaPolls);
-      if (jt + 1 < jt1 && tma_b) mbar_wait(&s_mbar[buf ^ 1], ((use + 1) >> 1) & 1u, kTmaPolls);
-      cp_async_wait_0();
-      return;
-    }
-
-    // Epilogue: C joins with index 0; only strict improvements are stored.
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const int m = (r >> 2) * kBlk + ty * 4 + (r & 3);
-      const int rb = (r >> 2) ? rbase1 : rbase0;
-      const int row = rb + ty * 4 + (r & 3);
-      if (rb < 0 || row >= m_rows) continue;
-#pragma unroll
-      for (int h = 0; h < CH; h++) {
-        const int cbh = h ? cb.y : cb.x;
-        if (cbh < 0) continue;
-        const int sc0 = h * kBlk + tx * 4;
-        const uint4 cv = *reinterpret_cast<const uint4 *>(&sm.C[m][sc0]);
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const int col = cbh + tx * 4 + q;
-          const unsigned cq = q == 0 ? cv.x : q == 1 ? cv.y : q == 2 ? cv.z : cv.w;
-          if constexpr (F32) {  // strict improvements only: ties keep the current value
-            // (the addresses from the descriptor in shared memory, read
-            // again after every barrier: with the register copies the
-            // compiler kept the rows' 64-bit offsets live across the tile
-            // loop, beside the 64 value and step registers, and spilled)
-            if (!(acc[r][h * 4 + q] < cq) || col >= n_cols) continue;
-            static_cast<unsigned *>(s.C)[(int64_t)row * s.ldc + col] = acc[r][h * 4 + q];
-            if (PRED) s.Cp[(int64_t)row * s.ldcp + col] = sm.Bp[arg[r][h * 4 + q] - 1][sc0 + q];
-          } else {
-            const unsigned key = min(min(cq, kPackH) << kIdxBits, acc[r][h * 4 + q]);
-            const unsigned idx = key & kIdxMask;
-            if (idx == 0 || col >= n_cols) continue;
-            c_mat[(int64_t)row * ldc + col] = key >> kIdxBits;
-            if (PRED) p_mat[(int64_t)row * ldcp + col] = sm.Bp[idx - 1][sc0 + q];
-          }
-        }
-      }
-    }
-    // C, B[buf] and the predecessors are free again (the fence orders this
-    // thread's reads and writes of them before the bulk copies that refill them)
-    if (tma) fence_proxy_async_smem();
-    __syncthreads();
-  }
-  cp_async_wait_0();
-  if (threadIdx.x == 0 && n_work > 0) atomicAdd(&g_fw_counters[0], n_work);
-}
-
 template <typename T, bool PRED>
 __global__ void __launch_bounds__(kThreads, 1)
     mp_tile_kernel(const MpSegment *__restrict__ segs, int nseg, int tile0) {
@@ -1932,16 +1408,6 @@ cudaError_t launch_strip_t(const MpSegment *d_segs, int nseg, int strips, int ks
   return cudaGetLastError();
 }
 
-template <bool PRED, bool F32>
-cudaError_t launch_fwstrip_t(const MpSegment *d_segs, int nseg, int strips, cudaStream_t st,
-                             const void *tmaps) {
-  if (strips <= 0 || nseg <= 0) return cudaSuccess;
-  ++launch_count();
-  mp_fwstrip_kernel<PRED, kFwStripTN, F32><<<strips, kThreads, sizeof(FwStripSmem<kFwStripTN>), st>>>(
-      d_segs, nseg, static_cast<const CUtensorMap *>(tmaps));
-  return cudaGetLastError();
-}
-
 template <typename T, bool PRED>
 cudaError_t set_mp_attr() {
   return cudaFuncSetAttribute(mp_tile_kernel<T, PRED>,
@@ -1985,79 +1451,6 @@ cudaError_t launch_minplus_strips(bool pred, const MpSegment *d_segs, int nseg, 
 
 int minplus_strip_tiles() { return kStripTiles; }
 
-cudaError_t launch_fw_strips(bool pred, const MpSegment *d_segs, int nseg, int strips,
-                             cudaStream_t st, bool f32, const void *tmaps) {
-  if (f32)
-    return pred ? launch_fwstrip_t<true, true>(d_segs, nseg, strips, st, tmaps)
-                : launch_fwstrip_t<false, true>(d_segs, nseg, strips, st, tmaps);
-  return pred ? launch_fwstrip_t<true, false>(d_segs, nseg, strips, st, tmaps)
-              : launch_fwstrip_t<false, false>(d_segs, nseg, strips, st, tmaps);
-}
-
-// The driver's tensor-map encoder, looked up once through the runtime (the
-// library does not link the driver library itself); null when unavailable.
-static PFN_cuTensorMapEncodeTiled_v12000 tmap_encoder() {
-  static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-    void *f = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) !=
-            cudaSuccess ||
-        q != cudaDriverEntryPointSuccess) {
-      (void)cudaGetLastError();
-      f = nullptr;
-    }
-    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
-  }();
-  return fn;
-}
-
-bool encode_fw_tmaps(void *out, const void *d, const void *p, int64_t ld, int rows, int cols) {
-  static_assert(sizeof(CUtensorMap) == 128, "a tensor map is 128 bytes");
-  const PFN_cuTensorMapEncodeTiled_v12000 enc = tmap_encoder();
-  if (!enc || !d || rows <= 0 || cols <= 0 || ((ld * 4) & 15) != 0 ||
-      (reinterpret_cast<uintptr_t>(d) & 15) != 0 || (p && (reinterpret_cast<uintptr_t>(p) & 15) != 0))
-    return false;
-  CUtensorMap *m = static_cast<CUtensorMap *>(out);
-  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
-  const cuuint32_t box[2] = {64, 64};
-  const cuuint32_t elem[2] = {1, 1};
-  for (int i = 0; i < 2; i++) {
-    void *base = const_cast<void *>(i == 1 && p ? p : d);
-    if (enc(&m[i], CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, base, dims, strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return false;
-  }
-  return true;
-}
-
-cudaError_t tma_status(unsigned *out, bool reset) {
-  cudaError_t e = cudaMemcpyFromSymbol(out, g_tma_status, sizeof(unsigned));
-  if (e == cudaSuccess && reset && *out) {
-    const unsigned zero = 0;
-    e = cudaMemcpyToSymbol(g_tma_status, &zero, sizeof(unsigned));
-  }
-  return e;
-}
-int fw_strips_of(const MpSegment &s, int tiles) {
-  const int rows = list_len(s.row_skip, s.row_skip2, s.row_fix, (s.M + kBlk - 1) / kBlk);
-  const int cols = list_len(s.col_skip, s.col_skip2, s.col_fix, (s.N + kBlk - 1) / kBlk);
-  return (rows + 1) / 2 * ((cols + tiles - 1) / tiles);
-}
-// The column tiles a CTA takes: the most (up to 8, which amortise the staging
-// of A, about two tiles' time) that still give the launch one CTA for every
-// slot of the GPU (two per SM).  A single 910-vertex matrix then runs its
-// remaining tiles in 98 CTAs of one tile instead of 14 of eight: its 14
-// rounds took 2.33 ms in strips of 8 and take 1.15 ms.
-int fw_strip_tiles(const MpSegment *segs, int nseg, int sm_count) {
-  for (int tiles = 8; tiles > 1; tiles /= 2) {
-    long long strips = 0;
-    for (int i = 0; i < nseg; i++) strips += fw_strips_of(segs[i], tiles);
-    if (strips >= 2LL * sm_count) return tiles;
-  }
-  return 1;
-}
 int minplus_strip_max_k() { return kStripMaxK; }
 int minplus_strip_classes() { return kStripClasses; }
 int minplus_strip_class_k(int c) { return c >= 0 && c < kStripClasses ? kStripClassK[c] : -1; }
@@ -2071,13 +1464,6 @@ cudaError_t launch_max_finite(const MatRef *d_mats, int nmats, unsigned *out, cu
 }
 
 unsigned pack_limit() { return kPackH; }
-
-cudaError_t fw_strip_counter(unsigned long long *out, bool reset) {
-  cudaError_t e = cudaMemcpyFromSymbol(out, g_fw_counters, sizeof(unsigned long long));
-  if (e != cudaSuccess || !reset) return e;
-  const unsigned long long zero = 0;
-  return cudaMemcpyToSymbol(g_fw_counters, &zero, sizeof(zero));
-}
 
 cudaError_t strip_counters(unsigned long long out[3], bool reset) {
   cudaError_t e = cudaMemcpyFromSymbol(out, g_strip_counters, sizeof(unsigned long long) * 3);
@@ -2125,16 +1511,6 @@ cudaError_t init_minplus_kernels() {
 #undef FAP_STRIP_ATTR
 #undef FAP_STRIP_ATTR1
 
-#define FAP_FWSTRIP_ATTR(P, F)                                                           \
-  if ((e = cudaFuncSetAttribute(mp_fwstrip_kernel<P, kFwStripTN, F>,                     \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,             \
-                                (int)sizeof(FwStripSmem<kFwStripTN>))) != cudaSuccess)   \
-    return e;
-  FAP_FWSTRIP_ATTR(true, false)
-  FAP_FWSTRIP_ATTR(false, false)
-  FAP_FWSTRIP_ATTR(true, true)
-  FAP_FWSTRIP_ATTR(false, true)
-#undef FAP_FWSTRIP_ATTR
   return cudaSuccess;
 }
 

@@ -284,6 +284,15 @@ def test_floyd_strip_lengths_agree(ctx, oracle_lib, f32, size):
         first = first or (ds[0], ps[0])
         for d, q in zip(ds, ps):
             assert torch.equal(d, first[0]) and torch.equal(q, first[1])
+    for ld in (size + 1, (size + 7) // 4 * 4):  # rows past the matrix, aligned or not
+        d, q = torch.zeros((size, ld), dtype=first[0].dtype, device="cuda"), torch.zeros((size, ld), dtype=torch.int32,
+                                                                                          device="cuda")
+        d[:, :size], q[:, :size] = torch.from_numpy(a).cuda(), torch.from_numpy(p).cuda()
+        torch.cuda.synchronize()
+        ctx.floyd_batched(0 if f32 else 1, [d[:, :size]], [q[:, :size]])
+        torch.cuda.synchronize()
+        assert torch.equal(d[:, :size], first[0]) and torch.equal(q[:, :size], first[1])
+        assert not d[:, size:].any() and not q[:, size:].any()
     w = torch.from_numpy(np.where(a < inf, a, np.inf).astype(np.float64)).cuda()
     for k in range(size):
         w = torch.minimum(w, w[:, k:k + 1] + w[k:k + 1, :])
