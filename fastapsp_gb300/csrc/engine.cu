@@ -160,6 +160,7 @@ struct Plan {
     int mp_ncls = 0, mp_strip_tiles = 0;
     int mp_cls_first[kMaxCls] = {}, mp_cls_nseg[kMaxCls] = {};
     int mp_cls_strips[kMaxCls] = {}, mp_cls_max_k[kMaxCls] = {};
+    int mp_cls_per[kMaxCls] = {};   // 128-column tiles per strip
     int mp_cls_cols[kMaxCls] = {};  // tile columns the tuner chose (0: the class default)
     bool mp_aligned = true;  // every strip segment's result rows start on 16-byte boundaries
     int max_sub = 0;  // largest part of the group (bound of the packed form)
@@ -584,12 +585,6 @@ int mp_tiles_of(const MpSegment &s) {
   return ((s.M + T - 1) / T) * s.tiles_x;
 }
 
-// CTAs of a segment in the strip form of the min-plus.
-int mp_strips_of(const MpSegment &s) {
-  const int T = fapk::minplus_tile_rows(), S = fapk::minplus_strip_tiles();
-  return ((s.M + T - 1) / T) * ((s.tiles_x + S - 1) / S);
-}
-
 // Groups of a batched plan whose results are copied to host rows:
 // consecutive parts (indices into `parts`) in groups of about 8 GB of rows
 // (at most 8 groups), so that the copy of one group's rows runs while the
@@ -761,9 +756,9 @@ int build_plan(fap_engine *e, Plan &pl) {
     for (int c = 0; c < ncls; c++) {
       G.mp_cls_first[c] = (int)mps.size();
       G.mp_cls_nseg[c] = (int)mps_cls[c].size();
-      for (MpSegment &s : mps_cls[c]) {
-        s.strip_begin = G.mp_cls_strips[c];
-        G.mp_cls_strips[c] += mp_strips_of(s);
+      G.mp_cls_strips[c] = fapk::number_minplus_strips(mps_cls[c].data(), (int)mps_cls[c].size(), e->sm_count,
+                                                       &G.mp_cls_per[c]);
+      for (const MpSegment &s : mps_cls[c]) {
         G.mp_cls_max_k[c] = std::max(G.mp_cls_max_k[c], s.K);
         G.mp_aligned = G.mp_aligned && rows_aligned16(s);
       }
@@ -1067,7 +1062,7 @@ struct Issuer {
       }
       for (int c = 0; c < G.mp_ncls; c++)
         FAP_CUDA(fapk::launch_minplus_strips(pred, G.mp + G.mp_cls_first[c], G.mp_cls_nseg[c],
-                                             G.mp_cls_strips[c], G.mp_cls_max_k[c],
+                                             G.mp_cls_strips[c], G.mp_cls_max_k[c], G.mp_cls_per[c],
                                              fork && c > 0 ? e->side : st, f32,
                                              e->tile_cols ? e->tile_cols : G.mp_cls_cols[c], G.mp_aligned));
       FAP_CUDA(fapk::launch_minplus_tiles(f32, pred, G.mp, G.mp_nseg, G.mp_tiles - G.mp_strip_tiles,
@@ -1288,7 +1283,7 @@ int autotune_tiles(fap_engine *e, Plan &pl, cudaStream_t st) {
           cudaError_t ce = cudaEventRecord(a, st);
           if (ce == cudaSuccess)
             ce = fapk::launch_minplus_strips(pred, G.mp + G.mp_cls_first[c], G.mp_cls_nseg[c],
-                                             G.mp_cls_strips[c], G.mp_cls_max_k[c], st, false, cols,
+                                             G.mp_cls_strips[c], G.mp_cls_max_k[c], G.mp_cls_per[c], st, false, cols,
                                              G.mp_aligned);
           if (ce == cudaSuccess) ce = cudaEventRecord(b, st);
           if (ce == cudaSuccess) ce = cudaEventSynchronize(b);
@@ -2176,8 +2171,8 @@ int fap_minplus(fap_engine *e, int32_t dtype, int32_t M, int32_t N, int32_t K, c
   int tiles = 0;
   MpSegment s = mp_segment(A, lda, B, ldb, Bpath, ldbp, C, ldc, Cpath, ldcp, M, N, K, tiles);
   s.tile_begin = 0;
-  s.strip_begin = 0;
-  int rc;
+  int rc, per = 1;
+  const int strips = fapk::number_minplus_strips(&s, 1, e->sm_count, &per);
   const bool i32 = dtype == FAP_DTYPE_I32;
   TableBuilder tb;
   size_t o_seg = tb.add(&s, 1);
@@ -2203,7 +2198,7 @@ int fap_minplus(fap_engine *e, int32_t dtype, int32_t M, int32_t N, int32_t K, c
   // the strip form addresses C rows with 32-bit offsets within a 128-row strip
   if ((packed || (!i32 && K > 0)) && K <= fapk::minplus_strip_max_k() && ldc < (1 << 24) &&
       (!Cpath || ldcp < (1 << 24)))
-    FAP_CUDA(fapk::launch_minplus_strips(Cpath != nullptr, dseg, 1, mp_strips_of(s), K, st, !i32,
+    FAP_CUDA(fapk::launch_minplus_strips(Cpath != nullptr, dseg, 1, strips, K, per, st, !i32,
                                          e->tile_cols, rows_aligned16(s)));
   else
     FAP_CUDA(fapk::launch_minplus_tiles(!i32, Cpath != nullptr, dseg, 1, tiles, packed, st));

@@ -23,18 +23,20 @@ cudaError_t launch_minplus_tiles(bool f32, bool pred, const MpSegment *d_segs, i
 // Strip form of the packed min-plus: segments that do not accumulate into C
 // (init_from_c = 0), C's leading dimensions below 2^24, every
 // K <= max_k <= minplus_strip_max_k(), CTAs numbered by
-// MpSegment::strip_begin (ceil(M / 128) x ceil(tiles_x / minplus_strip_tiles())
-// strips per segment).  Same preconditions as the packed tile form.
+// MpSegment::strip_begin (ceil(M / 128) x ceil(tiles_x / per) strips per
+// segment).  Same preconditions as the packed tile form.
 // f32: FP32 distances (any range) instead of the packed int32 form.
 // tile_cols (packed form): 64 or 128-column tiles, 0 = the default of the
 // K class (minplus_strip_class_cols); the FP32 form always takes 64.
 // aligned: every segment's C (and Cp) rows start on 16-byte boundaries (the
 // other form realigns its 16-byte stores row by row).
 cudaError_t launch_minplus_strips(bool pred, const MpSegment *d_segs, int nseg, int strips,
-                                  int max_k, cudaStream_t st, bool f32 = false, int tile_cols = 0,
+                                  int max_k, int per, cudaStream_t st, bool f32 = false, int tile_cols = 0,
                                   bool aligned = true);
 int minplus_strip_class_cols(int c);
-int minplus_strip_tiles();
+// Numbers the CTAs of one strip launch (returns their count) and chooses the
+// 128-column tiles each takes (launch_minplus_strips' per).
+int number_minplus_strips(MpSegment *segs, int nseg, int sm_count, int *per);
 int minplus_strip_max_k();   // largest K of the strip form
 // Segments go to the strip form in classes of K (one launch per class, each
 // with its own CTAs per SM): class c takes K <= minplus_strip_class_k(c)

@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
 // Strip form of the packed min-plus for products that do not accumulate into
 // C (the inner rows of every part) with K <= kStripMaxK.  One CTA owns a
-// strip: one 128-row tile of a segment and the TN-column tiles of
+// strip: one 128-row tile of a segment and the TN-column tiles of up to
 // kStripTiles x 128 consecutive columns.  A's 128 x K block is staged once
 // per strip (transposed, so that a thread's 8 row operands of one k are two
 // 16-byte loads); B's K x TN tiles are double-buffered, so the next tile's
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 // outputs, summed over tiles)], summed per CTA.
 __device__ unsigned long long g_strip_counters[3];
 
-constexpr int kStripTiles = 16;  // a strip spans kStripTiles x 128 columns
+constexpr int kStripTiles = 16;  // a strip spans at most kStripTiles x 128 columns (minplus_strip_cols)
 constexpr int kStripMaxK = 100;  // largest K of the strip form
 constexpr int kOwnCap = 12;
 // Segments are launched in classes of K.  K <= 48: 128 x 64 tiles with 8 x
@@ -809,7 +809,7 @@ __device__ __forceinline__ void addmin_groups_rows_f32(unsigned (&acc)[8][4], in
 // only, two CTAs per SM.
 template <bool PRED, int TN, bool F32 = false, bool UA = false>
 __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
-    mp_strip_kernel(const MpSegment *__restrict__ segs, int nseg, int ks) {
+    mp_strip_kernel(const MpSegment *__restrict__ segs, int nseg, int ks, int per) {
   constexpr int CH = TN / 64;  // 64-column halves of a thread's outputs
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned *Bs = reinterpret_cast<unsigned *>(smem_raw);  // [2][ks][TN]
@@ -836,12 +836,12 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
   if (threadIdx.x < TN) Bps[threadIdx.x] = -1;  // predecessor of idx 0
   __syncthreads();
   const MpSegment &s = seg;
-  const int strips_x = (s.tiles_x + kStripTiles - 1) / kStripTiles;
+  const int strips_x = (s.tiles_x + per - 1) / per;
   const int local = blockIdx.x - s.strip_begin;
   const int rt = local / strips_x;
-  // column tiles of TN: this strip's 128-column tiles, split
-  const int jt0 = (local - rt * strips_x) * kStripTiles * (128 / TN);
-  const int jt1 = min(jt0 + kStripTiles * (128 / TN), (s.N + TN - 1) / TN);
+  // column tiles of TN: this strip's 128-column tiles (`per` of them), split
+  const int jt0 = (local - rt * strips_x) * per * (128 / TN);
+  const int jt1 = min(jt0 + per * (128 / TN), (s.N + TN - 1) / TN);
   const int row0 = rt * kTile;
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   const unsigned INF = F32 ? __float_as_uint(Dist<float>::inf()) : Dist<uint32_t>::inf();
@@ -1396,15 +1396,15 @@ cudaError_t launch_packed_t(const MpSegment *d_segs, int nseg, int tiles, int ti
 }
 
 template <bool PRED, int TN, bool F32 = false>
-cudaError_t launch_strip_t(const MpSegment *d_segs, int nseg, int strips, int ks, cudaStream_t st,
+cudaError_t launch_strip_t(const MpSegment *d_segs, int nseg, int strips, int ks, int per, cudaStream_t st,
                            bool aligned) {
   if (strips <= 0 || nseg <= 0) return cudaSuccess;
   ++launch_count();
   if (aligned || F32)  // the FP32 epilogue stores 4-byte words at any alignment
-    mp_strip_kernel<PRED, TN, F32><<<strips, kThreads, strip_smem_bytes<TN, F32>(ks), st>>>(d_segs, nseg, ks);
+    mp_strip_kernel<PRED, TN, F32><<<strips, kThreads, strip_smem_bytes<TN, F32>(ks), st>>>(d_segs, nseg, ks, per);
   else if constexpr (!F32)
     mp_strip_kernel<PRED, TN, false, true>
-        <<<strips, kThreads, strip_smem_bytes<TN, false>(ks), st>>>(d_segs, nseg, ks);
+        <<<strips, kThreads, strip_smem_bytes<TN, false>(ks), st>>>(d_segs, nseg, ks, per);
   return cudaGetLastError();
 }
 
@@ -1433,23 +1433,49 @@ cudaError_t launch_minplus_tiles(bool f32, bool pred, const MpSegment *d_segs, i
 }
 
 cudaError_t launch_minplus_strips(bool pred, const MpSegment *d_segs, int nseg, int strips,
-                                  int max_k, cudaStream_t st, bool f32, int tile_cols, bool aligned) {
-  if (max_k < 0 || max_k > kStripMaxK) return cudaErrorInvalidValue;
+                                  int max_k, int per, cudaStream_t st, bool f32, int tile_cols, bool aligned) {
+  if (max_k < 0 || max_k > kStripMaxK || per < 1) return cudaErrorInvalidValue;
   const int ks = (max_k + 3) & ~3;
   if (f32)  // 128 x 64 tiles at every K (the argmin registers leave no room for 128 x 128)
-    return pred ? launch_strip_t<true, 64, true>(d_segs, nseg, strips, ks, st, aligned)
-                : launch_strip_t<false, 64, true>(d_segs, nseg, strips, ks, st, aligned);
+    return pred ? launch_strip_t<true, 64, true>(d_segs, nseg, strips, ks, per, st, aligned)
+                : launch_strip_t<false, 64, true>(d_segs, nseg, strips, ks, per, st, aligned);
   const int tn = tile_cols ? tile_cols : kStripClassTN[max_k <= kStripClassK[0] ? 0 : 1];
   if (tn == 64)
-    return pred ? launch_strip_t<true, 64>(d_segs, nseg, strips, ks, st, aligned)
-                : launch_strip_t<false, 64>(d_segs, nseg, strips, ks, st, aligned);
+    return pred ? launch_strip_t<true, 64>(d_segs, nseg, strips, ks, per, st, aligned)
+                : launch_strip_t<false, 64>(d_segs, nseg, strips, ks, per, st, aligned);
   if (tn == 128)
-    return pred ? launch_strip_t<true, 128>(d_segs, nseg, strips, ks, st, aligned)
-                : launch_strip_t<false, 128>(d_segs, nseg, strips, ks, st, aligned);
+    return pred ? launch_strip_t<true, 128>(d_segs, nseg, strips, ks, per, st, aligned)
+                : launch_strip_t<false, 128>(d_segs, nseg, strips, ks, per, st, aligned);
   return cudaErrorInvalidValue;
 }
 
-int minplus_strip_tiles() { return kStripTiles; }
+namespace {
+int strips_of(const MpSegment &s, int per) { return (s.M + kTile - 1) / kTile * ((s.tiles_x + per - 1) / per); }
+}  // namespace
+
+// The strip length: the longest (it amortises the staging of A) that still
+// gives the launch a CTA for every slot of the GPU (three per SM at most).  A
+// 910-vertex part of a 24,575-vertex road graph has 84 strips of 2,048 columns
+// (207 us) and 588 of 256 (119 us); four parts of 576 vertices 4 and 20 (80 and
+// 27 us).
+int number_minplus_strips(MpSegment *segs, int nseg, int sm_count, int *per) {
+  *per = 1;
+  for (int tiles = kStripTiles; tiles > 1; tiles /= 2) {
+    long long strips = 0;
+    for (int i = 0; i < nseg; i++) strips += strips_of(segs[i], tiles);
+    if (strips >= 3LL * sm_count) {
+      *per = tiles;
+      break;
+    }
+  }
+  int strips = 0;
+  for (int i = 0; i < nseg; i++) {
+    segs[i].strip_begin = strips;
+    strips += strips_of(segs[i], *per);
+  }
+  return strips;
+}
+
 
 int minplus_strip_max_k() { return kStripMaxK; }
 int minplus_strip_classes() { return kStripClasses; }

@@ -331,3 +331,29 @@ def test_sssp_one_cta_per_source_matches_batches(gpu, f32, n, sources):
             for d, p in out[1:3]:
                 assert torch.equal(d, out[0][0]) and torch.equal(p, out[0][1])
             assert torch.equal(out[3][0], out[0][0]) and bool((out[3][1] == 7).all())
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("n", [130, 4100, 70001])
+def test_minplus_strip_lengths_agree(ctx, f32, n):
+    """Strips of 128 to 2,048 columns (by how many the product has) give the
+    rows of the same product in slices of 100 columns."""
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    m, k = 260, 19
+
+    def side(r, c):
+        x = torch.rand(r, c, device="cuda", generator=gen) * 100
+        x = x if f32 else x.int()
+        return x.masked_fill_(torch.rand(r, c, device="cuda", generator=gen) < 0.3, 1e8 if f32 else 1 << 30)
+
+    a, b = side(m, k), side(k, n)
+    bp = torch.randint(0, n, (k, n), device="cuda", generator=gen, dtype=torch.int32)
+    c, cp = torch.empty((m, n), dtype=a.dtype, device="cuda"), torch.empty((m, n), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ctx.minplus(0 if f32 else 1, a, b, c, Bp=bp, Cp=cp)
+    for j in range(0, n, max(100, n // 20)):
+        w = min(100, n - j)
+        d, dp = torch.empty((m, w), dtype=a.dtype, device="cuda"), torch.empty((m, w), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        ctx.minplus(0 if f32 else 1, a, b[:, j:j + w], d, Bp=bp[:, j:j + w], Cp=dp)
+        assert torch.equal(d, c[:, j:j + w]) and torch.equal(dp, cp[:, j:j + w])
