@@ -170,7 +170,6 @@ struct Plan {
   std::vector<Group> groups;
   size_t fw_elems = 0;  // FW arena elements needed
   int max_sub = 0;      // largest part of the plan
-  int max_mp_k = 0;     // largest min-plus K (boundary count) of the plan
   int pack = -1;        // packed int32 form: -1 undecided, 0 no, 1 yes
   int sssp_lanes = 32;  // sources per SSSP batch
   int sssp_lanes_alt = 0;  // the other width the autotuner tries (0: none)
@@ -546,10 +545,10 @@ void fw_segments(void *D, int32_t *P, int64_t ld, int size, int r, MpSegment &ro
   t_rest = pairs * pairs;
 }
 
-// Min-plus segment C = A (x) B (fresh C), tiled in 128x128.
+// Min-plus segment C = A (x) B (fresh C).
 MpSegment mp_segment(const void *A, int64_t lda, const void *B, int64_t ldb, const int32_t *Bp,
                      int64_t ldbp, void *C, int64_t ldc, int32_t *Cp, int64_t ldcp, int M, int N,
-                     int K, int &tiles) {
+                     int K) {
   MpSegment s{};
   s.A = A;
   s.lda = lda;
@@ -568,7 +567,6 @@ MpSegment mp_segment(const void *A, int64_t lda, const void *B, int64_t ldb, con
   s.init_from_c = 0;
   const int T = fapk::minplus_tile_rows();
   s.tiles_x = (N + T - 1) / T;
-  tiles = ((M + T - 1) / T) * s.tiles_x;
   return s;
 }
 
@@ -577,12 +575,6 @@ MpSegment mp_segment(const void *A, int64_t lda, const void *B, int64_t ldb, con
 bool rows_aligned16(const MpSegment &s) {
   const bool c = (s.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(s.C) & 15) == 0;
   return c && (s.Cp == nullptr || ((s.ldcp & 3) == 0 && (reinterpret_cast<uintptr_t>(s.Cp) & 15) == 0));
-}
-
-// CTAs of a segment in the tile form of the min-plus (no skipped blocks).
-int mp_tiles_of(const MpSegment &s) {
-  const int T = fapk::minplus_tile_rows();
-  return ((s.M + T - 1) / T) * s.tiles_x;
 }
 
 // Groups of a batched plan whose results are copied to host rows:
@@ -712,7 +704,7 @@ int build_plan(fap_engine *e, Plan &pl) {
                                  bdist + (size_t)boff * es, n, pred ? bpred + boff : nullptr, n,
                                  dist + (size_t)(roff + (int64_t)bdy * n) * es, n,
                                  pred ? pl.pred + roff + (int64_t)bdy * n : nullptr, n, inner,
-                                 (int)n, bdy, tiles);
+                                 (int)n, bdy);
         // the part's own columns come from the FW matrix (rows bdy..sub-1)
         s.col_part = e->d_gid;
         s.part = p;
@@ -721,7 +713,6 @@ int build_plan(fap_engine *e, Plan &pl) {
         s.F = fwd + (size_t)(mat_off[idx] + (int64_t)bdy * d.ld) * es;
         s.Fp = pred ? fwp + mat_off[idx] + (int64_t)bdy * d.ld : nullptr;
         s.ldf = d.ld;
-        pl.max_mp_k = std::max(pl.max_mp_k, bdy);
         int c = 0;
         while (c < ncls && bdy > fapk::minplus_strip_class_k(c)) c++;
         if (n >= (1 << 24)) c = ncls;  // the strip form needs leading dimensions below 2^24
@@ -766,14 +757,9 @@ int build_plan(fap_engine *e, Plan &pl) {
     }
     const int nstrip = (int)mps.size();
     mps.insert(mps.end(), mps_wide.begin(), mps_wide.end());
-    int mp_tiles = 0;
-    for (MpSegment &s : mps) {
-      s.tile_begin = mp_tiles;
-      mp_tiles += mp_tiles_of(s);
-      if (&s - mps.data() + 1 == nstrip) G.mp_strip_tiles = mp_tiles;
-    }
+    G.mp_strip_tiles = fapk::number_minplus_deep(mps.data(), nstrip, 0);
     G.mp_nseg = (int)mps.size();
-    G.mp_tiles = mp_tiles;
+    G.mp_tiles = fapk::number_minplus_deep(mps.data() + nstrip, G.mp_nseg - nstrip, G.mp_strip_tiles);
     O.mp = tb.add(mps.data(), mps.size());
     // FW rounds
     G.diag_cnt.assign(maxnb, 0);
@@ -1030,10 +1016,8 @@ struct Issuer {
         FAP_CUDA(cudaEventRecord(e->ev_fw[1 + r % 2], e->side));
       } else {
         FAP_CUDA(fapk::launch_fw_diag(pred, G.diag[r], G.diag_cnt[r], st));
-        {
-          FAP_CUDA(fapk::launch_minplus_tiles(f32, pred, G.panel[r], G.panel_nseg[r], G.panel_tiles[r], packed, st));
-          FAP_CUDA(fapk::launch_minplus_tiles(f32, pred, G.rest[r], G.rest_nseg[r], G.rest_tiles[r], packed, st));
-        }
+        FAP_CUDA(fapk::launch_minplus_tiles(pred, G.panel[r], G.panel_nseg[r], G.panel_tiles[r], st));
+        FAP_CUDA(fapk::launch_minplus_tiles(pred, G.rest[r], G.rest_nseg[r], G.rest_tiles[r], st));
       }
     }
     if ((packed || f32) && rounds > 0) FAP_CUDA(cudaStreamWaitEvent(st, e->ev_fw[1 + (rounds - 1) % 2], 0));  // join
@@ -1065,14 +1049,14 @@ struct Issuer {
                                              G.mp_cls_strips[c], G.mp_cls_max_k[c], G.mp_cls_per[c],
                                              fork && c > 0 ? e->side : st, f32,
                                              e->tile_cols ? e->tile_cols : G.mp_cls_cols[c], G.mp_aligned));
-      FAP_CUDA(fapk::launch_minplus_tiles(f32, pred, G.mp, G.mp_nseg, G.mp_tiles - G.mp_strip_tiles,
-                                          packed, st, G.mp_strip_tiles));
+      FAP_CUDA(fapk::launch_minplus_deep(f32, packed, pred, G.mp, G.mp_nseg, G.mp_tiles - G.mp_strip_tiles,
+                                         G.mp_strip_tiles, st));
       if (fork) {  // join
         FAP_CUDA(cudaEventRecord(e->ev_fw[1], e->side));
         FAP_CUDA(cudaStreamWaitEvent(st, e->ev_fw[1], 0));
       }
     } else {
-      FAP_CUDA(fapk::launch_minplus_tiles(f32, pred, G.mp, G.mp_nseg, G.mp_tiles, packed, st));
+      FAP_CUDA(fapk::launch_minplus_deep(f32, packed, pred, G.mp, G.mp_nseg, G.mp_tiles, 0, st));
     }
     if (last) FAP_CUDA(rec(4));
     if (decode_aside) FAP_CUDA(cudaStreamWaitEvent(st, e->ev_copy[1], 0));  // join
@@ -1331,8 +1315,7 @@ int first_run(fap_engine *e, Plan &pl, cudaStream_t st) {
   FAP_CUDA(cudaStreamSynchronize(st));
   const unsigned long long bound =
       (unsigned long long)maxd + (unsigned long long)std::max(pl.max_sub - 1, 0) * e->wmax;
-  const bool k_ok = pl.pred == nullptr || pl.max_mp_k <= fapk::max_packed_k();
-  pl.pack = (e->int32_form == 0 && bound < fapk::pack_limit() && k_ok) ? 1 : 0;
+  pl.pack = (e->int32_form == 0 && bound < fapk::pack_limit()) ? 1 : 0;
   for (size_t g = 0; g < pl.groups.size(); g++) {
     if ((rc = is.rest(g, g + 1 == pl.groups.size())) != FAP_OK) return rc;
     if ((rc = is.copy_out(g)) != FAP_OK) return rc;
@@ -1576,6 +1559,7 @@ int init_device(fap_engine *e, int device) {
   FAP_CUDA(cudaMalloc(&e->d_stats, 8 * sizeof(unsigned long long)));
   FAP_CUDA(cudaMemset(e->d_stats, 0, 8 * sizeof(unsigned long long)));
   FAP_CUDA(fapk::init_minplus_kernels());
+  FAP_CUDA(fapk::init_mp_deep_kernels());
   FAP_CUDA(fapk::init_fw_pivot_kernels());
   FAP_CUDA(fapk::init_fw_rest_kernels());
   FAP_CUDA(fapk::init_sssp_kernels());
@@ -2168,9 +2152,8 @@ int fap_minplus(fap_engine *e, int32_t dtype, int32_t M, int32_t N, int32_t K, c
   std::lock_guard<std::mutex> lk(e->mu);
   DeviceGuard g(e->device);
   cudaStream_t st = pick_stream(e, stream);
-  int tiles = 0;
-  MpSegment s = mp_segment(A, lda, B, ldb, Bpath, ldbp, C, ldc, Cpath, ldcp, M, N, K, tiles);
-  s.tile_begin = 0;
+  MpSegment s = mp_segment(A, lda, B, ldb, Bpath, ldbp, C, ldc, Cpath, ldcp, M, N, K);
+  const int tiles = fapk::number_minplus_deep(&s, 1, 0);
   int rc, per = 1;
   const int strips = fapk::number_minplus_strips(&s, 1, e->sm_count, &per);
   const bool i32 = dtype == FAP_DTYPE_I32;
@@ -2186,13 +2169,11 @@ int fap_minplus(fap_engine *e, int32_t dtype, int32_t M, int32_t N, int32_t K, c
     // packed form only if max finite A + max finite B stays below the limit
     const fapk::MatRef *dr = reinterpret_cast<const fapk::MatRef *>(base + o_ref);
     FAP_CUDA(cudaMemsetAsync(e->d_status + 1, 0, 2 * sizeof(unsigned), st));
-    FAP_CUDA(fapk::launch_max_finite(dr, 1, e->d_status + 1, st));
-    FAP_CUDA(fapk::launch_max_finite(dr + 1, 1, e->d_status + 2, st));
+    FAP_CUDA(fapk::launch_max_finite(dr, 2, e->d_status + 1, 1, st));
     unsigned mx[2] = {0, 0};
     FAP_CUDA(cudaMemcpyAsync(mx, e->d_status + 1, sizeof(mx), cudaMemcpyDeviceToHost, st));
     FAP_CUDA(cudaStreamSynchronize(st));
-    packed = (unsigned long long)mx[0] + mx[1] < fapk::pack_limit() &&
-             (Cpath == nullptr || K <= fapk::max_packed_k());
+    packed = (unsigned long long)mx[0] + mx[1] < fapk::pack_limit();
   }
   const MpSegment *dseg = reinterpret_cast<const MpSegment *>(base + o_seg);
   // the strip form addresses C rows with 32-bit offsets within a 128-row strip
@@ -2201,7 +2182,7 @@ int fap_minplus(fap_engine *e, int32_t dtype, int32_t M, int32_t N, int32_t K, c
     FAP_CUDA(fapk::launch_minplus_strips(Cpath != nullptr, dseg, 1, strips, K, per, st, !i32,
                                          e->tile_cols, rows_aligned16(s)));
   else
-    FAP_CUDA(fapk::launch_minplus_tiles(!i32, Cpath != nullptr, dseg, 1, tiles, packed, st));
+    FAP_CUDA(fapk::launch_minplus_deep(!i32, packed, Cpath != nullptr, dseg, 1, tiles, 0, st));
   FAP_CUDA(cudaStreamSynchronize(st));
   return check_status(e);
 }
@@ -2301,7 +2282,7 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
     // a finite shortest distance is at most (size - 1) * the largest entry
     FAP_CUDA(cudaMemsetAsync(e->d_status + 1, 0, sizeof(unsigned), st));
     FAP_CUDA(fapk::launch_max_finite(reinterpret_cast<const fapk::MatRef *>(base + o_ref),
-                                     (int)refs.size(), e->d_status + 1, st));
+                                     (int)refs.size(), e->d_status + 1, 0, st));
     unsigned mx = 0;
     FAP_CUDA(cudaMemcpyAsync(&mx, e->d_status + 1, sizeof(mx), cudaMemcpyDeviceToHost, st));
     FAP_CUDA(cudaStreamSynchronize(st));
@@ -2319,12 +2300,8 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
       FAP_CUDA(cudaEventRecord(e->ev_fw[1 + r % 2], e->side));
     } else {
       FAP_CUDA(fapk::launch_fw_diag(pred, djobs, nd[r], st));
-      {
-        FAP_CUDA(fapk::launch_minplus_tiles(f32, pred, reinterpret_cast<const MpSegment *>(base + op[r]), np[r],
-                                            tp[r], packed, st));
-        FAP_CUDA(fapk::launch_minplus_tiles(f32, pred, reinterpret_cast<const MpSegment *>(base + orr[r]),
-                                            nr[r], tr[r], packed, st));
-      }
+      FAP_CUDA(fapk::launch_minplus_tiles(pred, reinterpret_cast<const MpSegment *>(base + op[r]), np[r], tp[r], st));
+      FAP_CUDA(fapk::launch_minplus_tiles(pred, reinterpret_cast<const MpSegment *>(base + orr[r]), nr[r], tr[r], st));
     }
   }
   if ((packed || f32) && maxnb > 0) FAP_CUDA(cudaStreamWaitEvent(st, e->ev_fw[1 + (maxnb - 1) % 2], 0));  // join

@@ -13,18 +13,15 @@ namespace fapk {
 int &launch_count();
 
 // minplus.cu
-// packed = true selects the packed int32 form (uint32 distances only); the
-// caller must have checked that every finite result stays below
-// pack_limit() and, with predecessors, that every segment has K <=
-// max_packed_k().
-// CTAs take tiles tile0 .. tile0 + tiles - 1 of the segments' numbering.
-cudaError_t launch_minplus_tiles(bool f32, bool pred, const MpSegment *d_segs, int nseg,
-                                 int tiles, bool packed, cudaStream_t st, int tile0 = 0);
+// Tiles of the Floyd-Warshall panels and remaining blocks of wide int32
+// matrices (numbered by MpSegment::tile_begin).
+cudaError_t launch_minplus_tiles(bool pred, const MpSegment *d_segs, int nseg, int tiles, cudaStream_t st);
 // Strip form of the packed min-plus: segments that do not accumulate into C
 // (init_from_c = 0), C's leading dimensions below 2^24, every
 // K <= max_k <= minplus_strip_max_k(), CTAs numbered by
 // MpSegment::strip_begin (ceil(M / 128) x ceil(tiles_x / per) strips per
-// segment).  Same preconditions as the packed tile form.
+// segment).  The caller must have checked that every finite int32 result stays
+// below pack_limit().
 // f32: FP32 distances (any range) instead of the packed int32 form.
 // tile_cols (packed form): 64 or 128-column tiles, 0 = the default of the
 // K class (minplus_strip_class_cols); the FP32 form always takes 64.
@@ -43,13 +40,20 @@ int minplus_strip_max_k();   // largest K of the strip form
 // above the previous bound; -1 past the last class.
 int minplus_strip_classes();
 int minplus_strip_class_k(int c);
-// Largest finite int32 entry of the matrices, atomicMax-ed into *out.
-cudaError_t launch_max_finite(const MatRef *d_mats, int nmats, unsigned *out, cudaStream_t st);
+// mp_deep.cu: products of any K and leading dimensions (init_from_c = 0), int32
+// packed (finite results below pack_limit()) or wide.  number_minplus_deep
+// sets the segments' tile_begin (64 x 64 tiles) from `first` and returns the
+// number after the last; the launch takes tiles tile0 .. tile0 + tiles - 1.
+int number_minplus_deep(MpSegment *segs, int nseg, int first);
+cudaError_t launch_minplus_deep(bool f32, bool packed, bool pred, const MpSegment *d_segs, int nseg, int tiles,
+                                int tile0, cudaStream_t st);
+cudaError_t init_mp_deep_kernels();
+// Largest finite int32 entry of each matrix, atomicMax-ed into out[its index * step].
+cudaError_t launch_max_finite(const MatRef *d_mats, int nmats, unsigned *out, int step, cudaStream_t st);
 unsigned pack_limit();
 // Work counters of the strip min-plus on the current device: [tiles, tiles
 // with no active step, active steps over all tiles]; optionally reset.
 cudaError_t strip_counters(unsigned long long out[3], bool reset);
-int max_packed_k();
 // Wide int32 form: closes each job's pivot block.
 cudaError_t launch_fw_diag(bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st);
 // fw_pivot.cu (packed int32 and FP32 forms): round job.prev's update of each

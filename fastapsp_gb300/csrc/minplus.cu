@@ -7,21 +7,21 @@
 // fw_kernel1 / FW_kernel1A2 / fw_kernel3, fap/kernel/cuda/floyd.cu:26-267).
 //
 // Kernels of this file:
-//  - mp_tile_kernel (FP32 and wide int32): the generic tile form.  One CTA
-//    computes C = min(C0, A (x) B) for a 128x128 output tile with 256
+//  - mp_strip_kernel (FP32, and int32 whose finite results stay below 2^24 - 1;
+//    at most 100 steps): packed keys (d << 7) | idx, one DPX __viaddmin_u32 per
+//    add-min, which gives the minimum and, on ties, the smallest idx -- the
+//    current value (idx 0) first, then the first k.  A stays resident for a
+//    strip of column tiles, and the steps k whose A column or B row has no
+//    finite entry in the tile are skipped (such a candidate never wins).
+//    Other products: mp_deep.cu.
+//  - mp_tile_kernel (Floyd-Warshall panels and remaining tiles of wide int32).
+//    One CTA computes C = min(C, A (x) B) for a 128x128 output tile with 256
 //    threads, 8x8 outputs per thread in registers, k staged in chunks of 32
 //    by cp.async with a two-stage pipeline; the argmin is the chunk-local k
 //    of the last strict improvement, resolved against the staged
-//    B-predecessor tile after each chunk.  A batch of segments (one per
-//    matrix or FW panel) is one launch; each CTA finds its segment by binary
-//    search over the segments' first tile.
-//  - mp_tile_packed_kernel, mp_strip_kernel, mp_fwstrip_kernel
-//    (int32 whose finite results stay below 2^24 - 1): packed keys
-//    (d << 7) | idx, one DPX __viaddmin_u32 per add-min, which gives the
-//    minimum and, on ties, the smallest idx -- the current value (idx 0)
-//    first, then the first k.  The strip kernels keep A resident for a strip
-//    of column tiles and skip the steps k whose A column or B row has no
-//    finite entry in the tile (such a candidate never wins).
+//    B-predecessor tile after each chunk.  A batch of segments (one per FW
+//    panel) is one launch; each CTA finds its segment by binary search over
+//    the segments' first tile.
 //
 // Floyd-Warshall over 64-wide pivot blocks: once the pivot block is closed
 // (shortest paths through its own vertices, zero diagonal), the row panel is
@@ -37,6 +37,7 @@
 #include "fw_tile.cuh"
 #include "kernels.cuh"
 #include "launch.h"
+#include "mp_common.cuh"
 
 namespace fapk {
 
@@ -47,25 +48,11 @@ constexpr int kBK = 32;      // k chunk staged in shared memory
 constexpr int kThreads = 256;
 constexpr int kApad = kBK + 1;  // A rows padded against bank conflicts
 
-template <typename T>
 struct MpSmem {
-  T A[2][kTile][kApad];
-  T B[2][kBK][kTile];
+  unsigned A[2][kTile][kApad];
+  unsigned B[2][kBK][kTile];
   int32_t Bp[2][kBK][kTile];
 };
-
-__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem));
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
-__device__ __forceinline__ void cp_async_wait_1() { asm volatile("cp.async.wait_group 1;\n" ::); }
-__device__ __forceinline__ void cp_async_wait_2() { asm volatile("cp.async.wait_group 2;\n" ::); }
-__device__ __forceinline__ void cp_async_wait_0() { asm volatile("cp.async.wait_group 0;\n" ::); }
 
 // Block index of list entry g of 0..nblocks-1 without block `skip` (and
 // `skip2`, when it is above `skip`), or of the one-block list `fix`; -1 past
@@ -95,11 +82,11 @@ __host__ __device__ __forceinline__ int list_len(int skip, int skip2, int fix, i
 // rows) and B (128 columns), and of B's predecessors when WITH_BP (16-byte
 // cp.async of 4 columns where aligned); entries outside the matrices are
 // written directly as "unreached" / -1.
-template <typename T, bool WITH_BP, typename SM>
-__device__ __forceinline__ void load_chunk(SM &sm, int buf, const MpSegment &s, const int rbase[2],
+template <bool WITH_BP>
+__device__ __forceinline__ void load_chunk(MpSmem &sm, int buf, const MpSegment &s, const int rbase[2],
                                            const int cbase[2], int k0) {
   const int t = threadIdx.x;
-  const T INF = Dist<T>::inf();
+  const unsigned INF = Dist<uint32_t>::inf();
   // A: 128 rows x 32 k; consecutive threads take consecutive k of one row.
   {
     const int kk = t & 31;
@@ -109,16 +96,16 @@ __device__ __forceinline__ void load_chunk(SM &sm, int buf, const MpSegment &s, 
       const int m = (t >> 5) + 8 * it;
       const int rb = rbase[m >> 6];
       const int row = rb + (m & 63);
-      T *dst = &sm.A[buf][m][kk];
+      unsigned *dst = &sm.A[buf][m][kk];
       if (rb >= 0 && row < s.M && kg < s.K) {
-        cp_async4(dst, static_cast<const T *>(s.A) + (int64_t)row * s.lda + kg);
+        cp_async4(dst, static_cast<const unsigned *>(s.A) + (int64_t)row * s.lda + kg);
       } else {
         *dst = INF;
       }
     }
   }
   // B (and its predecessors): 32 k x 128 columns; a warp takes one row k,
-  // 4 consecutive columns a lane (keys_from_values relies on this mapping).
+  // 4 consecutive columns a lane.
   {
     const int j4 = (t & 31) * 4;
     const int cb = cbase[j4 >> 6];
@@ -130,8 +117,8 @@ __device__ __forceinline__ void load_chunk(SM &sm, int buf, const MpSegment &s, 
     for (int it = 0; it < kBK / 8; it++) {
       const int kk = (t >> 5) + 8 * it;
       const int kg = k0 + kk;
-      T *dst = &sm.B[buf][kk][j4];
-      const T *src = static_cast<const T *>(s.B) + (int64_t)kg * s.ldb + col;
+      unsigned *dst = &sm.B[buf][kk][j4];
+      const unsigned *src = static_cast<const unsigned *>(s.B) + (int64_t)kg * s.ldb + col;
       if (kg < s.K && vec) {
         cp_async16(dst, src);
       } else {
@@ -164,16 +151,6 @@ struct TileGeom {
   int ty, tx;
 };
 
-__device__ __forceinline__ const MpSegment &find_segment(const MpSegment *__restrict__ segs,
-                                                         int nseg, int tile) {
-  int lo = 0, hi = nseg - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (segs[mid].tile_begin <= tile) lo = mid; else hi = mid - 1;
-  }
-  return segs[lo];
-}
-
 __device__ __forceinline__ TileGeom tile_geom(const MpSegment &s, int tile) {
   TileGeom g;
   const int local = tile - s.tile_begin;
@@ -200,105 +177,15 @@ __device__ __forceinline__ int out_col(const TileGeom &g, int c) {
 __device__ __forceinline__ int smem_row(const TileGeom &g, int r) { return (r >> 2) * kBlk + g.ty * 4 + (r & 3); }
 __device__ __forceinline__ int smem_col(const TileGeom &g, int c) { return (c >> 2) * kBlk + g.tx * 4 + (c & 3); }
 
-// In-part columns of the inner rows take the part's Floyd-Warshall values
-// (the decode of MysubMatDecode_path, util_Myalgorithm.h:236-247, for these
-// rows), so the min-plus epilogue writes every column once.
-__device__ __forceinline__ bool fw_column(const MpSegment &s, int col, int64_t &off) {
-  if (s.col_part == nullptr || s.col_part[col] != s.part) return false;
-  off = (int64_t)(s.col_local[col] - s.local0);
-  return true;
-}
-
-// Whether the output rows allow 16-byte stores of 4 consecutive columns.
-// Stores the values of a 64-column row segment held by 16 lanes (4
-// consecutive columns a lane; p = this lane's first column) where the row is
-// not 16-byte aligned: each lane stores the aligned 16-byte chunk that starts
-// inside its quad, completed with the next lane's first values; the ragged
-// ends of the segment (lane 0's values before the first boundary, lane 15's
-// after the last) go as single stores.  All 32 lanes call it (the values
-// move by shuffles within each half-warp); `ok` drops the stores of a row
-// outside the matrix.  (A case split on the misalignment, which is the same
-// for the whole warp, measured slower than these selects.)
-template <typename V>
-__device__ __forceinline__ void store_quad_unaligned(V *p, const V v[4], int tx, bool ok) {
-  V nx[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) nx[q] = __shfl_down_sync(0xffffffffu, v[q], 1, 16);
-  if (!ok) return;
-  const int o = (int)((reinterpret_cast<uintptr_t>(p) >> 2) & 3);  // the same for the whole segment
-  if (o == 0) {
-    __stcs(reinterpret_cast<uint4 *>(p), make_uint4((unsigned)v[0], (unsigned)v[1], (unsigned)v[2], (unsigned)v[3]));
-    return;
-  }
-  if (tx < 15) {  // chunk [p + 4 - o, p + 8 - o): v[4 - o .. 3], then nx[0 .. 3 - o]
-    const V w0 = o == 1 ? v[3] : o == 2 ? v[2] : v[1];
-    const V w1 = o == 1 ? nx[0] : o == 2 ? v[3] : v[2];
-    const V w2 = o == 1 ? nx[1] : o == 2 ? nx[0] : v[3];
-    const V w3 = o == 1 ? nx[2] : o == 2 ? nx[1] : nx[0];
-    __stcs(reinterpret_cast<uint4 *>(p + 4 - o), make_uint4((unsigned)w0, (unsigned)w1, (unsigned)w2, (unsigned)w3));
-  } else {
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (q >= 4 - o) p[q] = v[q];
-  }
-  if (tx == 0) {
-#pragma unroll
-    for (int q = 0; q < 4; q++)
-      if (q < 4 - o) p[q] = v[q];
-  }
-}
-
-template <bool PRED>
-__device__ __forceinline__ bool vec_stores_ok(const MpSegment &s) {
-  bool ok = (s.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(s.C) & 15) == 0;
-  if (PRED) ok = ok && (s.ldcp & 3) == 0 && (reinterpret_cast<uintptr_t>(s.Cp) & 15) == 0;
-  return ok;
-}
-
-// Stores the 4 outputs of columns col0..col0+3 of `row` (those < N), after
-// the part-column override; one 16-byte store per array when all 4 are in
-// range and the rows are aligned.
-template <typename T, bool PRED>
-__device__ __forceinline__ void store_quad(const MpSegment &s, int row, int col0, T d[4],
-                                           int32_t p[4], bool vec) {
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    int64_t j;
-    if (col0 + q < s.N && fw_column(s, col0 + q, j)) {
-      d[q] = static_cast<const T *>(s.F)[(int64_t)row * s.ldf + j];
-      if (PRED) p[q] = s.Fp[(int64_t)row * s.ldf + j];
-    }
-  }
-  T *crow = static_cast<T *>(s.C) + (int64_t)row * s.ldc;
-  int32_t *prow = PRED ? s.Cp + (int64_t)row * s.ldcp : nullptr;
-  if (vec && col0 + 3 < s.N) {
-    uint4 dv;
-    dv.x = Dist<T>::bits(d[0]);
-    dv.y = Dist<T>::bits(d[1]);
-    dv.z = Dist<T>::bits(d[2]);
-    dv.w = Dist<T>::bits(d[3]);
-    *reinterpret_cast<uint4 *>(crow + col0) = dv;
-    if (PRED) *reinterpret_cast<int4 *>(prow + col0) = make_int4(p[0], p[1], p[2], p[3]);
-    return;
-  }
-#pragma unroll
-  for (int q = 0; q < 4; q++)
-    if (col0 + q < s.N) {
-      crow[col0 + q] = d[q];
-      if (PRED) prow[col0 + q] = p[q];
-    }
-}
-
-// Wide form (FP32, and int32 outside the packed range).  Distances are kept
-// as their bit patterns, which order like the values (non-negative floats and
-// the int32 encoding), so one __vibmin_u32 gives both the new minimum and
-// whether the current value was kept (ties keep it: strict improvement).  An
-// add-min is then add + vibmin + select; the argmin is the chunk-local k of
+// Floyd-Warshall tiles of int32 matrices outside the packed range.  One
+// __vibmin_u32 gives both the new minimum and whether the current value was
+// kept (ties keep it: strict improvement).  An add-min is then add + vibmin +
+// select; the argmin is the chunk-local k of
 // the last strict improvement, resolved against the staged predecessor tile
 // after each chunk.
-template <typename T, bool PRED>
-__device__ __forceinline__ void tile_wide(MpSmem<T> &sm, const MpSegment &s, const TileGeom &g) {
-  const unsigned INF = Dist<T>::bits(Dist<T>::inf());
+template <bool PRED>
+__device__ __forceinline__ void tile_wide(MpSmem &sm, const MpSegment &s, const TileGeom &g) {
+  const unsigned INF = Dist<uint32_t>::inf();
   unsigned acc[8][8];
   int32_t pred[8][8];
   int arg[8][8];
@@ -318,18 +205,18 @@ __device__ __forceinline__ void tile_wide(MpSmem<T> &sm, const MpSegment &s, con
     }
   }
   const int nchunks = (s.K + kBK - 1) / kBK;
-  if (nchunks > 0) load_chunk<T, PRED>(sm, 0, s, g.rbase, g.cbase, 0);
+  if (nchunks > 0) load_chunk<PRED>(sm, 0, s, g.rbase, g.cbase, 0);
   cp_async_commit();
   for (int ch = 0; ch < nchunks; ch++) {
     const int buf = ch & 1;
-    if (ch + 1 < nchunks) load_chunk<T, PRED>(sm, buf ^ 1, s, g.rbase, g.cbase, (ch + 1) * kBK);
+    if (ch + 1 < nchunks) load_chunk<PRED>(sm, buf ^ 1, s, g.rbase, g.cbase, (ch + 1) * kBK);
     cp_async_commit();
     cp_async_wait_1();
     __syncthreads();
     const int kn = min(kBK, s.K - ch * kBK);  // steps of this chunk (the rest is fill)
 #pragma unroll 2
     for (int kk = 0; kk < kn; kk++) {
-      T a[8], b[8];
+      unsigned a[8], b[8];
 #pragma unroll
       for (int r = 0; r < 8; r++) a[r] = sm.A[buf][smem_row(g, r)][kk];
 #pragma unroll
@@ -338,7 +225,7 @@ __device__ __forceinline__ void tile_wide(MpSmem<T> &sm, const MpSegment &s, con
       for (int r = 0; r < 8; r++)
 #pragma unroll
         for (int c = 0; c < 8; c++) {
-          const unsigned v = Dist<T>::bits(Dist<T>::add(a[r], b[c]));
+          const unsigned v = a[r] + b[c];
           if (PRED) {
             bool keep;
             acc[r][c] = __vibmin_u32(acc[r][c], v, &keep);
@@ -371,208 +258,14 @@ __device__ __forceinline__ void tile_wide(MpSmem<T> &sm, const MpSegment &s, con
       if (g.cbase[h] < 0) continue;
       const int col0 = g.cbase[h] + g.tx * 4;
       if (col0 >= s.N) continue;
-      T d[4];
-      int32_t p[4];
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        d[q] = Dist<T>::from_bits(acc[r][h * 4 + q]);
-        p[q] = pred[r][h * 4 + q];
-      }
-      store_quad<T, PRED>(s, row, col0, d, p, vec);
-    }
-  }
-}
-
-constexpr int kStagedBpRows = 64;  // B-predecessor rows kept in shared memory
-
-struct KeySmem {
-  unsigned A[2][kTile][kApad];
-  unsigned B[2][kBK][kTile];
-  int32_t Bp[kStagedBpRows][kTile];  // rows k of B's predecessors when K <= 64
-  int32_t fwcol[kTile];  // FW-matrix column of each tile column of the own part, else -1
-};
-
-// Stages B-predecessor rows [k0, k0+32) into Bp[k0..] (not double-buffered:
-// every row of the whole K range keeps its own slot); read only after a
-// barrier, so any thread mapping does.
-__device__ __forceinline__ void load_bp_rows(KeySmem &sm, const MpSegment &s, const int cbase[2],
-                                             int k0) {
-  const int t = threadIdx.x;
-  const int j = t & 127;
-  const int cb = cbase[j >> 6];
-  const int col = cb + (j & 63);
-  const bool colok = cb >= 0 && col < s.N;
-#pragma unroll 4
-  for (int it = 0; it < kBK / 2; it++) {
-    const int kk = (t >> 7) + 2 * it;
-    const int kg = k0 + kk;
-    int32_t *dst = &sm.Bp[kg][j];
-    if (colok && kg < s.K) cp_async4(dst, s.Bp + (int64_t)kg * s.ldbp + col);
-    else *dst = -1;
-  }
-}
-
-// After this thread's copies of a chunk have landed, turns the elements it
-// loaded (same index mapping as load_chunk) into keys.
-__device__ __forceinline__ void keys_from_values(KeySmem &sm, int buf, int k0) {
-  const int t = threadIdx.x;
-  {
-    const int kk = t & 31;
-#pragma unroll 4
-    for (int it = 0; it < kTile / 8; it++) {
-      const int m = (t >> 5) + 8 * it;
-      sm.A[buf][m][kk] = min(sm.A[buf][m][kk], kPackH) << kIdxBits;
-    }
-  }
-  {
-    const int j4 = (t & 31) * 4;
-#pragma unroll 4
-    for (int it = 0; it < kBK / 8; it++) {
-      const int kk = (t >> 5) + 8 * it;
-      const unsigned idx = ((unsigned)((k0 + kk) & kMaxPackedK) + 1u) & kIdxMask;
-      uint4 *p = reinterpret_cast<uint4 *>(&sm.B[buf][kk][j4]);
-      uint4 v = *p;
-      v.x = (min(v.x, kPackH) << kIdxBits) | idx;
-      v.y = (min(v.y, kPackH) << kIdxBits) | idx;
-      v.z = (min(v.z, kPackH) << kIdxBits) | idx;
-      v.w = (min(v.w, kPackH) << kIdxBits) | idx;
-      *p = v;
-    }
-  }
-}
-
-template <bool PRED>
-__global__ void __launch_bounds__(kThreads, 2)
-    mp_tile_packed_kernel(const MpSegment *__restrict__ segs, int nseg, int tile0) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  KeySmem &sm = *reinterpret_cast<KeySmem *>(smem_raw);
-  __shared__ MpSegment seg;
-  const int tile = tile0 + blockIdx.x;
-  if (threadIdx.x == 0) seg = find_segment(segs, nseg, tile);
-  __syncthreads();
-  const MpSegment &s = seg;
-  const TileGeom g = tile_geom(s, tile);
-  unsigned acc[8][8];
-#pragma unroll
-  for (int r = 0; r < 8; r++) {
-    const int row = out_row(g, r);
-#pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const int col = out_col(g, c);
-      acc[r][c] = kPackH << kIdxBits;
-      if (s.init_from_c && row >= 0 && row < s.M && col >= 0 && col < s.N)
-        acc[r][c] = min(static_cast<const unsigned *>(s.C)[(int64_t)row * s.ldc + col], kPackH) << kIdxBits;
-    }
-  }
-  // Own-part columns of the tile (min-plus of inner rows): FW column or -1.
-  if (threadIdx.x < kTile) {
-    const int j = threadIdx.x;
-    const int cb = g.cbase[j >> 6];
-    const int col = cb + (j & 63);
-    int32_t f = -1;
-    if (s.col_part != nullptr && cb >= 0 && col < s.N && s.col_part[col] == s.part)
-      f = s.col_local[col] - s.local0;
-    sm.fwcol[j] = f;
-  }
-  const int nchunks = (s.K + kBK - 1) / kBK;
-  // B's predecessor rows (K <= 64) go to shared memory in their own cp.async
-  // group, waited for only before the epilogue, so their latency hides under
-  // the DPX loop.  Groups: chunk 0 | predecessor rows | chunk 1 | ...
-  const bool stage_bp = PRED && s.K <= kStagedBpRows;
-  if (nchunks > 0) load_chunk<uint32_t, false>(sm, 0, s, g.rbase, g.cbase, 0);
-  cp_async_commit();
-  if (stage_bp) {
-    for (int k0 = 0; k0 < s.K; k0 += kBK) load_bp_rows(sm, s, g.cbase, k0);
-    cp_async_commit();
-  }
-  for (int ch = 0; ch < nchunks; ch++) {
-    const int buf = ch & 1;
-    if (ch + 1 < nchunks) load_chunk<uint32_t, false>(sm, buf ^ 1, s, g.rbase, g.cbase, (ch + 1) * kBK);
-    cp_async_commit();
-    if (ch == 0 && stage_bp) cp_async_wait_2(); else cp_async_wait_1();
-    keys_from_values(sm, buf, ch * kBK);
-    __syncthreads();
-    const int kn = min(kBK, s.K - ch * kBK);  // steps of this chunk (the rest is fill)
-#pragma unroll 2
-    for (int kk = 0; kk < kn; kk++) {
-      unsigned a[8], b[8];
-#pragma unroll
-      for (int r = 0; r < 8; r++) a[r] = sm.A[buf][smem_row(g, r)][kk];
-#pragma unroll
-      for (int c = 0; c < 8; c++) b[c] = sm.B[buf][kk][smem_col(g, c)];
-#pragma unroll
-      for (int r = 0; r < 8; r++)
-#pragma unroll
-        for (int c = 0; c < 8; c++) acc[r][c] = __viaddmin_u32(a[r], b[c], acc[r][c]);
-    }
-    __syncthreads();
-  }
-  cp_async_wait_0();
-  __syncthreads();  // staged predecessor rows and column flags visible to every thread
-  if (s.init_from_c) {
-    // Accumulating product (FW phases): idx 0 means the output kept its value,
-    // so neither its distance nor its predecessor is stored again.
-#pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const int row = out_row(g, r);
-      if (row < 0 || row >= s.M) continue;
-#pragma unroll
-      for (int c = 0; c < 8; c++) {
-        const int col = out_col(g, c);
-        if (col < 0 || col >= s.N) continue;
-        const unsigned key = acc[r][c];
-        const unsigned idx = key & kIdxMask;
-        if (idx == 0) continue;
-        static_cast<unsigned *>(s.C)[(int64_t)row * s.ldc + col] = key >> kIdxBits;
-        if (PRED)
-          s.Cp[(int64_t)row * s.ldcp + col] =
-              stage_bp ? sm.Bp[idx - 1][smem_col(g, c)] : s.Bp[(int64_t)(idx - 1) * s.ldbp + col];
-      }
-    }
-    return;
-  }
-  const bool vec = vec_stores_ok<PRED>(s);
-#pragma unroll
-  for (int r = 0; r < 8; r++) {
-    const int row = out_row(g, r);
-    if (row < 0 || row >= s.M) continue;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      if (g.cbase[h] < 0) continue;
-      const int col0 = g.cbase[h] + g.tx * 4;
-      if (col0 >= s.N) continue;
       unsigned d[4];
       int32_t p[4];
 #pragma unroll
       for (int q = 0; q < 4; q++) {
-        const int col = col0 + q;
-        const int sc = smem_col(g, h * 4 + q);
-        const unsigned key = acc[r][h * 4 + q];
-        const unsigned dist = key >> kIdxBits;
-        const unsigned idx = key & kIdxMask;
-        d[q] = dist >= kPackH ? Dist<uint32_t>::inf() : dist;
-        p[q] = -1;
-        if (PRED && col < s.N && dist < kPackH && idx != 0)
-          p[q] = stage_bp ? sm.Bp[idx - 1][sc] : s.Bp[(int64_t)(idx - 1) * s.ldbp + col];
-        const int fj = sm.fwcol[sc];
-        if (fj >= 0) {  // own-part column: the FW value (the decode of this row)
-          d[q] = static_cast<const unsigned *>(s.F)[(int64_t)row * s.ldf + fj];
-          if (PRED) p[q] = s.Fp[(int64_t)row * s.ldf + fj];
-        }
+        d[q] = acc[r][h * 4 + q];
+        p[q] = pred[r][h * 4 + q];
       }
-      unsigned *crow = static_cast<unsigned *>(s.C) + (int64_t)row * s.ldc;
-      int32_t *prow = PRED ? s.Cp + (int64_t)row * s.ldcp : nullptr;
-      if (vec && col0 + 3 < s.N) {  // streaming stores: the rows are not read again here
-        __stcs(reinterpret_cast<uint4 *>(crow + col0), make_uint4(d[0], d[1], d[2], d[3]));
-        if (PRED) __stcs(reinterpret_cast<int4 *>(prow + col0), make_int4(p[0], p[1], p[2], p[3]));
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-          if (col0 + q < s.N) {
-            crow[col0 + q] = d[q];
-            if (PRED) prow[col0 + q] = p[q];
-          }
-      }
+      store_quad<uint32_t, PRED>(s, row, col0, d, p, vec);
     }
   }
 }
@@ -1235,37 +928,53 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
   }
 }
 
-template <typename T, bool PRED>
+template <bool PRED>
 __global__ void __launch_bounds__(kThreads, 1)
-    mp_tile_kernel(const MpSegment *__restrict__ segs, int nseg, int tile0) {
+    mp_tile_kernel(const MpSegment *__restrict__ segs, int nseg) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  MpSmem<T> &sm = *reinterpret_cast<MpSmem<T> *>(smem_raw);
+  MpSmem &sm = *reinterpret_cast<MpSmem *>(smem_raw);
   // The segment descriptor stays in shared memory (read where needed) so that
   // the accumulators, argmins and predecessors keep the registers.
   __shared__ MpSegment seg;
-  const int tile = tile0 + blockIdx.x;
+  const int tile = blockIdx.x;
   if (threadIdx.x == 0) seg = find_segment(segs, nseg, tile);
   __syncthreads();
   const MpSegment &s = seg;
   const TileGeom g = tile_geom(s, tile);
-  tile_wide<T, PRED>(sm, s, g);
+  tile_wide<PRED>(sm, s, g);
 }
 
-// Largest finite int32 value (< 2^30) of a strided matrix, atomicMax-ed into
-// *out; CTAs (blockIdx.x) row-stride over matrix blockIdx.y.
-__global__ void max_finite_kernel(const MatRef *__restrict__ mats, unsigned *out) {
+// Largest finite int32 value (< 2^30) of the strided matrix blockIdx.y,
+// atomicMax-ed into out[blockIdx.y * step] once a CTA.  The CTAs (blockIdx.x)
+// stride over pieces of kMaxCols columns of a row, so that few long rows keep
+// as many loads in flight as many short ones.
+constexpr int kMaxCols = 1024;
+__global__ void __launch_bounds__(256)
+    max_finite_kernel(const MatRef *__restrict__ mats, unsigned *out, int step) {
+  __shared__ unsigned s_max;
   const MatRef mr = mats[blockIdx.y];
   const unsigned *D = static_cast<const unsigned *>(mr.p);
+  if (threadIdx.x == 0) s_max = 0u;
+  __syncthreads();
+  const int per_row = (mr.cols + kMaxCols - 1) / kMaxCols;
+  const int64_t pieces = (int64_t)mr.rows * per_row;
   unsigned m = 0;
-  for (int r = blockIdx.x; r < mr.rows; r += gridDim.x)
-    for (int c = threadIdx.x; c < mr.cols; c += blockDim.x) {
-      const unsigned v = D[(int64_t)r * mr.ld + c];
+  for (int64_t p = blockIdx.x; p < pieces; p += gridDim.x) {
+    const int64_t r = p / per_row;
+    const int c0 = (int)(p - r * per_row) * kMaxCols + threadIdx.x;
+    const unsigned *row = D + r * mr.ld;
+#pragma unroll
+    for (int i = 0; i < kMaxCols / 256; i++) {
+      const int c = c0 + 256 * i;
+      const unsigned v = c < mr.cols ? row[c] : 0u;
       if (v < Dist<uint32_t>::inf()) m = max(m, v);
     }
+  }
   m = __reduce_max_sync(0xffffffffu, m);
-  if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(&s_max, m);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_max) atomicMax(out + blockIdx.y * step, s_max);
 }
-
 
 // Closes a 64x64 block held in shared memory (D values, P predecessors, row
 // pitch 65): sequential k as the reference's floyd_CPU_path
@@ -1379,19 +1088,11 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-template <typename T, bool PRED>
-cudaError_t launch_mp_t(const MpSegment *d_segs, int nseg, int tiles, int tile0, cudaStream_t st) {
-  if (tiles <= 0 || nseg <= 0) return cudaSuccess;
-  ++launch_count();
-  mp_tile_kernel<T, PRED><<<tiles, kThreads, sizeof(MpSmem<T>), st>>>(d_segs, nseg, tile0);
-  return cudaGetLastError();
-}
-
 template <bool PRED>
-cudaError_t launch_packed_t(const MpSegment *d_segs, int nseg, int tiles, int tile0, cudaStream_t st) {
+cudaError_t launch_mp_t(const MpSegment *d_segs, int nseg, int tiles, cudaStream_t st) {
   if (tiles <= 0 || nseg <= 0) return cudaSuccess;
   ++launch_count();
-  mp_tile_packed_kernel<PRED><<<tiles, kThreads, sizeof(KeySmem), st>>>(d_segs, nseg, tile0);
+  mp_tile_kernel<PRED><<<tiles, kThreads, sizeof(MpSmem), st>>>(d_segs, nseg);
   return cudaGetLastError();
 }
 
@@ -1408,28 +1109,15 @@ cudaError_t launch_strip_t(const MpSegment *d_segs, int nseg, int strips, int ks
   return cudaGetLastError();
 }
 
-template <typename T, bool PRED>
-cudaError_t set_mp_attr() {
-  return cudaFuncSetAttribute(mp_tile_kernel<T, PRED>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MpSmem<T>));
-}
-
 template <bool PRED>
-cudaError_t set_packed_attr() {
-  return cudaFuncSetAttribute(mp_tile_packed_kernel<PRED>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KeySmem));
+cudaError_t set_mp_attr() {
+  return cudaFuncSetAttribute(mp_tile_kernel<PRED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MpSmem));
 }
 
 }  // namespace
 
-cudaError_t launch_minplus_tiles(bool f32, bool pred, const MpSegment *d_segs, int nseg,
-                                 int tiles, bool packed, cudaStream_t st, int tile0) {
-  if (f32) return pred ? launch_mp_t<float, true>(d_segs, nseg, tiles, tile0, st)
-                       : launch_mp_t<float, false>(d_segs, nseg, tiles, tile0, st);
-  if (packed) return pred ? launch_packed_t<true>(d_segs, nseg, tiles, tile0, st)
-                          : launch_packed_t<false>(d_segs, nseg, tiles, tile0, st);
-  return pred ? launch_mp_t<uint32_t, true>(d_segs, nseg, tiles, tile0, st)
-              : launch_mp_t<uint32_t, false>(d_segs, nseg, tiles, tile0, st);
+cudaError_t launch_minplus_tiles(bool pred, const MpSegment *d_segs, int nseg, int tiles, cudaStream_t st) {
+  return pred ? launch_mp_t<true>(d_segs, nseg, tiles, st) : launch_mp_t<false>(d_segs, nseg, tiles, st);
 }
 
 cudaError_t launch_minplus_strips(bool pred, const MpSegment *d_segs, int nseg, int strips,
@@ -1482,10 +1170,11 @@ int minplus_strip_classes() { return kStripClasses; }
 int minplus_strip_class_k(int c) { return c >= 0 && c < kStripClasses ? kStripClassK[c] : -1; }
 int minplus_strip_class_cols(int c) { return c >= 0 && c < kStripClasses ? kStripClassTN[c] : -1; }
 
-cudaError_t launch_max_finite(const MatRef *d_mats, int nmats, unsigned *out, cudaStream_t st) {
+cudaError_t launch_max_finite(const MatRef *d_mats, int nmats, unsigned *out, int step, cudaStream_t st) {
   if (nmats <= 0) return cudaSuccess;
   ++launch_count();
-  max_finite_kernel<<<dim3(32, nmats), 256, 0, st>>>(d_mats, out);
+  // (CTAs for every SM whatever the number of matrices)
+  max_finite_kernel<<<dim3(max(32, 1216 / nmats), nmats), 256, 0, st>>>(d_mats, out, step);
   return cudaGetLastError();
 }
 
@@ -1497,7 +1186,6 @@ cudaError_t strip_counters(unsigned long long out[3], bool reset) {
   const unsigned long long zero[3] = {0, 0, 0};
   return cudaMemcpyToSymbol(g_strip_counters, zero, sizeof(zero));
 }
-int max_packed_k() { return kMaxPackedK; }
 
 cudaError_t launch_fw_diag(bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st) {
   if (njobs <= 0) return cudaSuccess;
@@ -1509,12 +1197,8 @@ cudaError_t launch_fw_diag(bool pred, const FwDiagJob *d_jobs, int njobs, cudaSt
 
 cudaError_t init_minplus_kernels() {
   cudaError_t e;
-  if ((e = set_mp_attr<float, true>()) != cudaSuccess) return e;
-  if ((e = set_mp_attr<float, false>()) != cudaSuccess) return e;
-  if ((e = set_mp_attr<uint32_t, true>()) != cudaSuccess) return e;
-  if ((e = set_mp_attr<uint32_t, false>()) != cudaSuccess) return e;
-  if ((e = set_packed_attr<true>()) != cudaSuccess) return e;
-  if ((e = set_packed_attr<false>()) != cudaSuccess) return e;
+  if ((e = set_mp_attr<true>()) != cudaSuccess) return e;
+  if ((e = set_mp_attr<false>()) != cudaSuccess) return e;
   // either tile width serves any K of the strip form (tile_cols)
   static_assert(kStripClassTN[0] == 64 && kStripClassTN[1] == 128, "strip tile widths");
   const int smax0 = (int)strip_smem_bytes<64>((kStripMaxK + 3) & ~3);

@@ -357,3 +357,61 @@ def test_minplus_strip_lengths_agree(ctx, f32, n):
         torch.cuda.synchronize()
         ctx.minplus(0 if f32 else 1, a, b[:, j:j + w], d, Bp=bp[:, j:j + w], Cp=dp)
         assert torch.equal(d, c[:, j:j + w]) and torch.equal(dp, cp[:, j:j + w])
+
+
+@pytest.mark.parametrize("pred", [True, False])
+@pytest.mark.parametrize("kind", ["f32", "packed", "wide"])
+@pytest.mark.parametrize("m, n, k, pad", [(64, 64, 101, 0), (65, 63, 128, 1), (1, 130, 192, 0), (130, 257, 500, 3),
+                                          (200, 64, 129, 3), (61, 192, 260, 4)])
+def test_minplus_of_many_steps(ctx, kind, pred, m, n, k, pad):
+    """More steps than the strip form takes: the rows of a step-by-step product
+    (strict improvements, ascending steps), at edges of tiles, chunks and
+    alignments; `wide` has int32 values past the packed range."""
+    gen = torch.Generator(device="cuda").manual_seed(m * 1000 + n + k)
+    dt, inf = (torch.float32, 1e8) if kind == "f32" else (torch.int32, 1 << 30)
+
+    def side(r, c):  # few distinct values: ties within and across groups and chunks
+        x = torch.randint(0, 40, (r, c + pad), device="cuda", generator=gen) * ((1 << 22) if kind == "wide" else 1)
+        x = (x * 0.1 if kind == "f32" else x).to(dt)
+        return x.masked_fill_(torch.rand(r, c + pad, device="cuda", generator=gen) < 0.4, inf)[:, :c]
+
+    a, b = side(m, k), side(k, n)
+    b[:, n // 2] = inf  # a column that nothing reaches
+    bp = torch.randint(0, n, (k, n), device="cuda", generator=gen, dtype=torch.int32)
+    ref = torch.full((m, n), inf, dtype=dt, device="cuda")
+    refp = torch.full((m, n), -1, dtype=torch.int32, device="cuda")
+    for i in range(k):
+        v = a[:, i, None] + b[i]
+        better = (v < ref) & (a[:, i, None] < inf) & (b[i] < inf)
+        ref, refp = torch.where(better, v, ref), torch.where(better, bp[i].expand(m, n), refp)
+    c = torch.full((m, n + pad), 7, dtype=dt, device="cuda")
+    cp = torch.full((m, n + pad), 7, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    if pred:
+        ctx.minplus(0 if kind == "f32" else 1, a, b, c[:, :n], Bp=bp, Cp=cp[:, :n])
+        assert torch.equal(cp[:, :n], refp) and bool((cp[:, n:] == 7).all())
+    else:
+        ctx.minplus(0 if kind == "f32" else 1, a, b, c[:, :n])
+    assert torch.equal(c[:, :n], ref) and bool((c[:, n:] == 7).all())
+
+
+@pytest.mark.parametrize("f32", [False, True])
+def test_solve_with_many_boundary_vertices(gpu, f32):
+    """Parts whose boundaries exceed the strip form's steps and the packed index:
+    int32 rows equal the wide form's, FP32 rows (integer weights) the same values."""
+    g = graphs.small_random_graph(901, 5000, True, True, seed=9)
+    gid, _ = gpu.partition(g.row_offset, g.col_val, 3)
+    outs = []
+    for dtype, form in ((gpu.DTYPE_I32, 1), (gpu.DTYPE_F32 if f32 else gpu.DTYPE_I32, 0)):
+        with gpu.Engine(g.n, g.row_offset, g.col_val, g.weight, 3, graph_id=gid, dtype=dtype) as eng:
+            assert max(eng.part_info(p)[1] for p in range(1, 4)) > 127
+            if dtype == gpu.DTYPE_I32:
+                eng.set_option(gpu._lib.OPT_INT32_FORM, form)
+            d = torch.empty((g.n, g.n), dtype=torch.int32 if dtype == gpu.DTYPE_I32 else torch.float32, device="cuda")
+            p = torch.empty((g.n, g.n), dtype=torch.int32, device="cuda")
+            eng.solve(d, p, gpu.MODE_BATCHED)
+            eng.solve(d, p, gpu.MODE_BATCHED)  # the captured graph
+            torch.cuda.synchronize()
+            outs.append((as_oracle(d.cpu().numpy()), p.cpu().numpy()))
+    assert np.array_equal(outs[0][0], outs[1][0])
+    assert np.array_equal(outs[0][1], outs[1][1])
