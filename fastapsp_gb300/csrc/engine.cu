@@ -162,7 +162,7 @@ struct Plan {
     int mp_cls_strips[kMaxCls] = {}, mp_cls_max_k[kMaxCls] = {};
     int mp_cls_per[kMaxCls] = {};   // 128-column tiles per strip
     int mp_cls_cols[kMaxCls] = {};  // tile columns the tuner chose (0: the class default)
-    bool mp_aligned = true;  // every strip segment's result rows start on 16-byte boundaries
+    bool mp_rows = false;    // packed int32 rows off 16-byte boundaries: mp_rows.cu instead of the strips
     int max_sub = 0;  // largest part of the group (bound of the packed form)
     int64_t out_lo = 0, out_elems = 0;  // the group's result rows: elements [out_lo, out_lo + out_elems)
     int64_t dev_lo = 0;                 // where they are computed in dist/pred (out_lo, or its slot)
@@ -571,7 +571,10 @@ MpSegment mp_segment(const void *A, int64_t lda, const void *B, int64_t ldb, con
 }
 
 // Whether a min-plus segment's result rows (and predecessor rows) all start
-// on 16-byte boundaries.
+// on 16-byte boundaries.  Packed int32 products of other rows take mp_rows.cu
+// (geometric graph, 55 parts, min-plus phase: 57,301 vertices 12.5 ms in the
+// strip form, 8.4 ms there; 57,300 vertices 8.2 and 9.0 ms); FP32 ones are bound
+// by their add-mins (road-like graph: 57,301 vertices 13.4 ms, 57,304 12.9 ms).
 bool rows_aligned16(const MpSegment &s) {
   const bool c = (s.ldc & 3) == 0 && (reinterpret_cast<uintptr_t>(s.C) & 15) == 0;
   return c && (s.Cp == nullptr || ((s.ldcp & 3) == 0 && (reinterpret_cast<uintptr_t>(s.Cp) & 15) == 0));
@@ -744,15 +747,14 @@ int build_plan(fap_engine *e, Plan &pl) {
     O.dec_begin = tb.add(dec_begin.data(), dec_begin.size());
     std::vector<MpSegment> mps;
     G.mp_ncls = ncls;
+    for (int c = 0; c < ncls; c++)
+      for (const MpSegment &s : mps_cls[c]) G.mp_rows = G.mp_rows || (!e->f32() && !rows_aligned16(s));
     for (int c = 0; c < ncls; c++) {
       G.mp_cls_first[c] = (int)mps.size();
       G.mp_cls_nseg[c] = (int)mps_cls[c].size();
-      G.mp_cls_strips[c] = fapk::number_minplus_strips(mps_cls[c].data(), (int)mps_cls[c].size(), e->sm_count,
-                                                       &G.mp_cls_per[c]);
-      for (const MpSegment &s : mps_cls[c]) {
-        G.mp_cls_max_k[c] = std::max(G.mp_cls_max_k[c], s.K);
-        G.mp_aligned = G.mp_aligned && rows_aligned16(s);
-      }
+      auto *number = G.mp_rows ? fapk::number_minplus_rows : fapk::number_minplus_strips;
+      G.mp_cls_strips[c] = number(mps_cls[c].data(), (int)mps_cls[c].size(), e->sm_count, &G.mp_cls_per[c]);
+      for (const MpSegment &s : mps_cls[c]) G.mp_cls_max_k[c] = std::max(G.mp_cls_max_k[c], s.K);
       mps.insert(mps.end(), mps_cls[c].begin(), mps_cls[c].end());
     }
     const int nstrip = (int)mps.size();
@@ -1044,11 +1046,16 @@ struct Issuer {
         FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
         FAP_CUDA(cudaStreamWaitEvent(e->side, e->ev_fw[0], 0));
       }
-      for (int c = 0; c < G.mp_ncls; c++)
-        FAP_CUDA(fapk::launch_minplus_strips(pred, G.mp + G.mp_cls_first[c], G.mp_cls_nseg[c],
-                                             G.mp_cls_strips[c], G.mp_cls_max_k[c], G.mp_cls_per[c],
-                                             fork && c > 0 ? e->side : st, f32,
-                                             e->tile_cols ? e->tile_cols : G.mp_cls_cols[c], G.mp_aligned));
+      for (int c = 0; c < G.mp_ncls; c++) {
+        cudaStream_t sc = fork && c > 0 ? e->side : st;
+        if (G.mp_rows)
+          FAP_CUDA(fapk::launch_minplus_rows(pred, G.mp + G.mp_cls_first[c], G.mp_cls_nseg[c], G.mp_cls_strips[c],
+                                             G.mp_cls_max_k[c], G.mp_cls_per[c], sc));
+        else
+          FAP_CUDA(fapk::launch_minplus_strips(pred, G.mp + G.mp_cls_first[c], G.mp_cls_nseg[c], G.mp_cls_strips[c],
+                                               G.mp_cls_max_k[c], G.mp_cls_per[c], sc, f32,
+                                               e->tile_cols ? e->tile_cols : G.mp_cls_cols[c]));
+      }
       FAP_CUDA(fapk::launch_minplus_deep(f32, packed, pred, G.mp, G.mp_nseg, G.mp_tiles - G.mp_strip_tiles,
                                          G.mp_strip_tiles, st));
       if (fork) {  // join
@@ -1258,7 +1265,7 @@ int autotune_tiles(fap_engine *e, Plan &pl, cudaStream_t st) {
   int rc = FAP_OK;
   for (auto &G : pl.groups) {
     for (int c = 0; c < G.mp_ncls && rc == FAP_OK; c++) {
-      if (G.mp_cls_strips[c] <= 0) continue;
+      if (G.mp_cls_strips[c] <= 0 || G.mp_rows) continue;
       float best_ms = 1e30f;
       int best = 0;
       for (int cols : {64, 128}) {
@@ -1267,8 +1274,7 @@ int autotune_tiles(fap_engine *e, Plan &pl, cudaStream_t st) {
           cudaError_t ce = cudaEventRecord(a, st);
           if (ce == cudaSuccess)
             ce = fapk::launch_minplus_strips(pred, G.mp + G.mp_cls_first[c], G.mp_cls_nseg[c],
-                                             G.mp_cls_strips[c], G.mp_cls_max_k[c], G.mp_cls_per[c], st, false, cols,
-                                             G.mp_aligned);
+                                             G.mp_cls_strips[c], G.mp_cls_max_k[c], G.mp_cls_per[c], st, false, cols);
           if (ce == cudaSuccess) ce = cudaEventRecord(b, st);
           if (ce == cudaSuccess) ce = cudaEventSynchronize(b);
           float ms = 0;
@@ -1560,6 +1566,7 @@ int init_device(fap_engine *e, int device) {
   FAP_CUDA(cudaMemset(e->d_stats, 0, 8 * sizeof(unsigned long long)));
   FAP_CUDA(fapk::init_minplus_kernels());
   FAP_CUDA(fapk::init_mp_deep_kernels());
+  FAP_CUDA(fapk::init_mp_rows_kernels());
   FAP_CUDA(fapk::init_fw_pivot_kernels());
   FAP_CUDA(fapk::init_fw_rest_kernels());
   FAP_CUDA(fapk::init_sssp_kernels());
@@ -2155,8 +2162,8 @@ int fap_minplus(fap_engine *e, int32_t dtype, int32_t M, int32_t N, int32_t K, c
   MpSegment s = mp_segment(A, lda, B, ldb, Bpath, ldbp, C, ldc, Cpath, ldcp, M, N, K);
   const int tiles = fapk::number_minplus_deep(&s, 1, 0);
   int rc, per = 1;
-  const int strips = fapk::number_minplus_strips(&s, 1, e->sm_count, &per);
-  const bool i32 = dtype == FAP_DTYPE_I32;
+  const bool i32 = dtype == FAP_DTYPE_I32, by_rows = i32 && !rows_aligned16(s);
+  const int strips = (by_rows ? fapk::number_minplus_rows : fapk::number_minplus_strips)(&s, 1, e->sm_count, &per);
   TableBuilder tb;
   size_t o_seg = tb.add(&s, 1);
   fapk::MatRef refs[2] = {{A, lda, M, K}, {B, ldb, K, N}};
@@ -2178,11 +2185,14 @@ int fap_minplus(fap_engine *e, int32_t dtype, int32_t M, int32_t N, int32_t K, c
   const MpSegment *dseg = reinterpret_cast<const MpSegment *>(base + o_seg);
   // the strip form addresses C rows with 32-bit offsets within a 128-row strip
   if ((packed || (!i32 && K > 0)) && K <= fapk::minplus_strip_max_k() && ldc < (1 << 24) &&
-      (!Cpath || ldcp < (1 << 24)))
-    FAP_CUDA(fapk::launch_minplus_strips(Cpath != nullptr, dseg, 1, strips, K, per, st, !i32,
-                                         e->tile_cols, rows_aligned16(s)));
-  else
+      (!Cpath || (ldcp < (1 << 24) && ldbp < (1 << 24)))) {
+    if (by_rows)
+      FAP_CUDA(fapk::launch_minplus_rows(Cpath != nullptr, dseg, 1, strips, K, per, st));
+    else
+      FAP_CUDA(fapk::launch_minplus_strips(Cpath != nullptr, dseg, 1, strips, K, per, st, !i32, e->tile_cols));
+  } else {
     FAP_CUDA(fapk::launch_minplus_deep(!i32, packed, Cpath != nullptr, dseg, 1, tiles, 0, st));
+  }
   FAP_CUDA(cudaStreamSynchronize(st));
   return check_status(e);
 }

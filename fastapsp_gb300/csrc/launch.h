@@ -25,11 +25,8 @@ cudaError_t launch_minplus_tiles(bool pred, const MpSegment *d_segs, int nseg, i
 // f32: FP32 distances (any range) instead of the packed int32 form.
 // tile_cols (packed form): 64 or 128-column tiles, 0 = the default of the
 // K class (minplus_strip_class_cols); the FP32 form always takes 64.
-// aligned: every segment's C (and Cp) rows start on 16-byte boundaries (the
-// other form realigns its 16-byte stores row by row).
 cudaError_t launch_minplus_strips(bool pred, const MpSegment *d_segs, int nseg, int strips,
-                                  int max_k, int per, cudaStream_t st, bool f32 = false, int tile_cols = 0,
-                                  bool aligned = true);
+                                  int max_k, int per, cudaStream_t st, bool f32 = false, int tile_cols = 0);
 int minplus_strip_class_cols(int c);
 // Numbers the CTAs of one strip launch (returns their count) and chooses the
 // 128-column tiles each takes (launch_minplus_strips' per).
@@ -40,6 +37,14 @@ int minplus_strip_max_k();   // largest K of the strip form
 // above the previous bound; -1 past the last class.
 int minplus_strip_classes();
 int minplus_strip_class_k(int c);
+// mp_rows.cu: the packed strip form for result rows that do not start on 16-byte
+// boundaries; same preconditions (B's predecessors' leading dimension below 2^24
+// too), numbering and counters.
+int number_minplus_rows(MpSegment *segs, int nseg, int sm_count, int *per);
+cudaError_t launch_minplus_rows(bool pred, const MpSegment *d_segs, int nseg, int strips, int max_k, int per,
+                                cudaStream_t st);
+cudaError_t rows_counters(unsigned long long out[3], bool reset);
+cudaError_t init_mp_rows_kernels();
 // mp_deep.cu: products of any K and leading dimensions (init_from_c = 0), int32
 // packed (finite results below pack_limit()) or wide.  number_minplus_deep
 // sets the segments' tile_begin (64 x 64 tiles) from `first` and returns the

@@ -500,7 +500,7 @@ __device__ __forceinline__ void addmin_groups_rows_f32(unsigned (&acc)[8][4], in
 // current value was kept (non-negative floats order like their bits) -- the
 // reference's strict-<, ascending-k rule, as in the packed form.  TN = 64
 // only, two CTAs per SM.
-template <bool PRED, int TN, bool F32 = false, bool UA = false>
+template <bool PRED, int TN, bool F32 = false>
 __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
     mp_strip_kernel(const MpSegment *__restrict__ segs, int nseg, int ks, int per) {
   constexpr int CH = TN / 64;  // 64-column halves of a thread's outputs
@@ -856,15 +856,12 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
       for (int c = 0; c < 4 * CH; c++)
         if (ownidx[buf * TN + (c >> 2) * kBlk + tx * 4 + (c & 3)] != -1) ownmask |= 1u << c;
     }
-    // The unaligned store form (UA) masks rows and columns outside the
-    // matrix per lane instead of skipping them: it moves values between lanes.
-    const bool cols_full = colbase + TN <= n_cols;  // uniform over the CTA
 #pragma unroll
     for (int r = 0; r < 8; r++) {
       const int rr = (r >> 2) * kBlk + (r & 3);  // row offset from this thread's first row
       const int row = row0 + ty * 4 + rr;
       const bool row_ok = row < m_rows;
-      if (!UA && !row_ok) continue;
+      if (!row_ok) continue;
       unsigned *crow = c_thr + rr * ldc;
       int32_t *prow = PRED ? p_thr + rr * ldcp : nullptr;
 #pragma unroll
@@ -872,7 +869,7 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
         const int sc0 = h * kBlk + tx * 4;
         const int col0 = colbase + sc0;
         const bool ok = row_ok && col0 < n_cols;
-        if (!UA && !ok) continue;
+        if (!ok) continue;
         unsigned d[4] = {INF, INF, INF, INF};
         int32_t p[4] = {-1, -1, -1, -1};
         // a quad of unreached outputs (the common case on sparse graphs)
@@ -906,9 +903,6 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
         if (vec_c && ok && col0 + 3 < n_cols) {  // streaming stores: the rows are not read again here
           __stcs(reinterpret_cast<uint4 *>(crow + col0), make_uint4(d[0], d[1], d[2], d[3]));
           if (PRED) __stcs(reinterpret_cast<int4 *>(prow + col0), make_int4(p[0], p[1], p[2], p[3]));
-        } else if (UA && !vec_c && cols_full) {  // rows not 16-byte aligned: realigned 16-byte stores
-          store_quad_unaligned(crow + col0, d, tx, row_ok);
-          if (PRED) store_quad_unaligned(prow + col0, p, tx, row_ok);
         } else if (ok) {
 #pragma unroll
           for (int q = 0; q < 4; q++)
@@ -1097,15 +1091,10 @@ cudaError_t launch_mp_t(const MpSegment *d_segs, int nseg, int tiles, cudaStream
 }
 
 template <bool PRED, int TN, bool F32 = false>
-cudaError_t launch_strip_t(const MpSegment *d_segs, int nseg, int strips, int ks, int per, cudaStream_t st,
-                           bool aligned) {
+cudaError_t launch_strip_t(const MpSegment *d_segs, int nseg, int strips, int ks, int per, cudaStream_t st) {
   if (strips <= 0 || nseg <= 0) return cudaSuccess;
   ++launch_count();
-  if (aligned || F32)  // the FP32 epilogue stores 4-byte words at any alignment
-    mp_strip_kernel<PRED, TN, F32><<<strips, kThreads, strip_smem_bytes<TN, F32>(ks), st>>>(d_segs, nseg, ks, per);
-  else if constexpr (!F32)
-    mp_strip_kernel<PRED, TN, false, true>
-        <<<strips, kThreads, strip_smem_bytes<TN, false>(ks), st>>>(d_segs, nseg, ks, per);
+  mp_strip_kernel<PRED, TN, F32><<<strips, kThreads, strip_smem_bytes<TN, F32>(ks), st>>>(d_segs, nseg, ks, per);
   return cudaGetLastError();
 }
 
@@ -1121,19 +1110,19 @@ cudaError_t launch_minplus_tiles(bool pred, const MpSegment *d_segs, int nseg, i
 }
 
 cudaError_t launch_minplus_strips(bool pred, const MpSegment *d_segs, int nseg, int strips,
-                                  int max_k, int per, cudaStream_t st, bool f32, int tile_cols, bool aligned) {
+                                  int max_k, int per, cudaStream_t st, bool f32, int tile_cols) {
   if (max_k < 0 || max_k > kStripMaxK || per < 1) return cudaErrorInvalidValue;
   const int ks = (max_k + 3) & ~3;
   if (f32)  // 128 x 64 tiles at every K (the argmin registers leave no room for 128 x 128)
-    return pred ? launch_strip_t<true, 64, true>(d_segs, nseg, strips, ks, per, st, aligned)
-                : launch_strip_t<false, 64, true>(d_segs, nseg, strips, ks, per, st, aligned);
+    return pred ? launch_strip_t<true, 64, true>(d_segs, nseg, strips, ks, per, st)
+                : launch_strip_t<false, 64, true>(d_segs, nseg, strips, ks, per, st);
   const int tn = tile_cols ? tile_cols : kStripClassTN[max_k <= kStripClassK[0] ? 0 : 1];
   if (tn == 64)
-    return pred ? launch_strip_t<true, 64>(d_segs, nseg, strips, ks, per, st, aligned)
-                : launch_strip_t<false, 64>(d_segs, nseg, strips, ks, per, st, aligned);
+    return pred ? launch_strip_t<true, 64>(d_segs, nseg, strips, ks, per, st)
+                : launch_strip_t<false, 64>(d_segs, nseg, strips, ks, per, st);
   if (tn == 128)
-    return pred ? launch_strip_t<true, 128>(d_segs, nseg, strips, ks, per, st, aligned)
-                : launch_strip_t<false, 128>(d_segs, nseg, strips, ks, per, st, aligned);
+    return pred ? launch_strip_t<true, 128>(d_segs, nseg, strips, ks, per, st)
+                : launch_strip_t<false, 128>(d_segs, nseg, strips, ks, per, st);
   return cudaErrorInvalidValue;
 }
 
@@ -1181,8 +1170,12 @@ cudaError_t launch_max_finite(const MatRef *d_mats, int nmats, unsigned *out, in
 unsigned pack_limit() { return kPackH; }
 
 cudaError_t strip_counters(unsigned long long out[3], bool reset) {
-  cudaError_t e = cudaMemcpyFromSymbol(out, g_strip_counters, sizeof(unsigned long long) * 3);
-  if (e != cudaSuccess || !reset) return e;
+  cudaError_t e = rows_counters(out, reset);
+  unsigned long long strip[3];
+  if (e == cudaSuccess) e = cudaMemcpyFromSymbol(strip, g_strip_counters, sizeof(strip));
+  if (e != cudaSuccess) return e;
+  for (int i = 0; i < 3; i++) out[i] += strip[i];
+  if (!reset) return e;
   const unsigned long long zero[3] = {0, 0, 0};
   return cudaMemcpyToSymbol(g_strip_counters, zero, sizeof(zero));
 }
@@ -1203,24 +1196,18 @@ cudaError_t init_minplus_kernels() {
   static_assert(kStripClassTN[0] == 64 && kStripClassTN[1] == 128, "strip tile widths");
   const int smax0 = (int)strip_smem_bytes<64>((kStripMaxK + 3) & ~3);
   const int smax1 = (int)strip_smem_bytes<128>((kStripMaxK + 3) & ~3);
-#define FAP_STRIP_ATTR1(P, TN, F, UA, SMAX)                                                    \
-  if ((e = cudaFuncSetAttribute(mp_strip_kernel<P, TN, F, UA>,                                    \
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, SMAX)) != cudaSuccess) \
+#define FAP_STRIP_ATTR(P, TN, F, SMAX)                                                               \
+  if ((e = cudaFuncSetAttribute(mp_strip_kernel<P, TN, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                SMAX)) != cudaSuccess)                                                \
     return e;
-#define FAP_STRIP_ATTR(P, TN, SMAX)  \
-  FAP_STRIP_ATTR1(P, TN, false, false, SMAX) \
-  FAP_STRIP_ATTR1(P, TN, false, true, SMAX)
-  FAP_STRIP_ATTR(true, 64, smax0)
-  FAP_STRIP_ATTR(false, 64, smax0)
-  FAP_STRIP_ATTR(true, 128, smax1)
-  FAP_STRIP_ATTR(false, 128, smax1)
-  // FP32: one form for every row alignment
+  FAP_STRIP_ATTR(true, 64, false, smax0)
+  FAP_STRIP_ATTR(false, 64, false, smax0)
+  FAP_STRIP_ATTR(true, 128, false, smax1)
+  FAP_STRIP_ATTR(false, 128, false, smax1)
   const int smaxf = (int)strip_smem_bytes<64, true>((kStripMaxK + 3) & ~3);
-  FAP_STRIP_ATTR1(true, 64, true, false, smaxf)
-  FAP_STRIP_ATTR1(false, 64, true, false, smaxf)
+  FAP_STRIP_ATTR(true, 64, true, smaxf)
+  FAP_STRIP_ATTR(false, 64, true, smaxf)
 #undef FAP_STRIP_ATTR
-#undef FAP_STRIP_ATTR1
-
   return cudaSuccess;
 }
 

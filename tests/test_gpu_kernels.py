@@ -415,3 +415,46 @@ def test_solve_with_many_boundary_vertices(gpu, f32):
             outs.append((as_oracle(d.cpu().numpy()), p.cpu().numpy()))
     assert np.array_equal(outs[0][0], outs[1][0])
     assert np.array_equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("pred", [True, False])
+@pytest.mark.parametrize("m, n, k, off", [(128, 57, 1, 1), (129, 64, 4, 3), (3, 1001, 19, 0), (300, 2049, 33, 5),
+                                          (130, 130, 100, 7), (64, 4095, 48, 2)])
+def test_minplus_of_rows_off_boundaries(ctx, m, n, k, off, pred):
+    """Packed products into rows that start off 16-byte boundaries (odd lengths and
+    offsets) equal those into aligned rows."""
+    gen = torch.Generator(device="cuda").manual_seed(m + n * k)
+
+    def side(r, c):
+        x = torch.randint(0, 50, (r, c), device="cuda", generator=gen, dtype=torch.int32)
+        return x.masked_fill_(torch.rand(r, c, device="cuda", generator=gen) < 0.5, 1 << 30)
+
+    a, b = side(m, k), side(k, n)
+    b[:, : min(n, 200)] = 1 << 30  # tiles without a step
+    bp = torch.randint(0, n, (k, n), device="cuda", generator=gen, dtype=torch.int32)
+    outs = []
+    for ld, o in ((n + 32 - n % 32, 0), (n | 1, off)):
+        c, p = (torch.full((m * ld + 64,), 7, dtype=torch.int32, device="cuda") for _ in range(2))
+        cv, pv = (x[o:o + m * ld].view(m, ld)[:, :n] for x in (c, p))
+        torch.cuda.synchronize()
+        ctx.minplus(1, a, b, cv, Bp=bp if pred else None, Cp=pv if pred else None)
+        outs.append((cv.clone(), pv.clone()))
+        cv[:], pv[:] = 7, 7
+        assert bool((c == 7).all()) and bool((p == 7).all())  # nothing outside the rows
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+@pytest.mark.parametrize("n, parts", [(3001, 3), (1537, 12)])
+def test_solve_of_odd_rows_matches_wide_form(gpu, n, parts):
+    g = graphs.geometric_knn(n, seed=n)
+    gid, _ = gpu.partition(g.row_offset, g.col_val, parts)
+    outs = []
+    for form in (0, 1):
+        with gpu.Engine(g.n, g.row_offset, g.col_val, g.weight, parts, graph_id=gid, dtype=gpu.DTYPE_I32) as eng:
+            eng.set_option(gpu._lib.OPT_INT32_FORM, form)
+            d, p = (torch.empty((g.n, g.n), dtype=torch.int32, device="cuda") for _ in range(2))
+            eng.solve(d, p, gpu.MODE_BATCHED)
+            eng.solve(d, p, gpu.MODE_BATCHED)  # the captured graph
+            torch.cuda.synchronize()
+            outs.append((d, p))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
