@@ -152,16 +152,12 @@ struct Plan {
     // min-plus
     const MpSegment *mp = nullptr;
     int mp_nseg = 0, mp_tiles = 0;
-    // strip form: class c (K up to fapk::minplus_strip_class_k(c)) holds
-    // mp_cls_nseg[c] segments from mp_cls_first[c], one launch each with CTAs
-    // numbered from 0; mp_strip_tiles = tiles of all of them in the tile
-    // numbering, which the tile form's launch skips
-    static constexpr int kMaxCls = 4;
-    int mp_ncls = 0, mp_strip_tiles = 0;
-    int mp_cls_first[kMaxCls] = {}, mp_cls_nseg[kMaxCls] = {};
-    int mp_cls_strips[kMaxCls] = {}, mp_cls_max_k[kMaxCls] = {};
-    int mp_cls_per[kMaxCls] = {};   // 128-column tiles per strip
-    int mp_cls_cols[kMaxCls] = {};  // tile columns the tuner chose (0: the class default)
+    // strip form (K <= fapk::minplus_strip_max_k(f32)): the first mp_strip_nseg
+    // segments, one launch; mp_strip_tiles = their tiles in the numbering of
+    // the other form (mp_deep.cu), whose launch skips them
+    int mp_strip_nseg = 0, mp_strip_tiles = 0;
+    int mp_strips = 0, mp_strip_k = 0;  // CTAs, largest K
+    int mp_strip_per = 0;               // 128-column tiles per strip
     bool mp_rows = false;    // packed int32 rows off 16-byte boundaries: mp_rows.cu instead of the strips
     int max_sub = 0;  // largest part of the group (bound of the packed form)
     int64_t out_lo = 0, out_elems = 0;  // the group's result rows: elements [out_lo, out_lo + out_elems)
@@ -223,7 +219,7 @@ struct fap_engine {
   int autotune = 1;        // tune the SSSP step on the first solve
   int sssp_lanes = 0;      // sources per SSSP batch: 16, 32, 0 = chosen per solve
   int sssp_lanes_tuned = 0;  // the width the autotuner chose (0: none yet)
-  int tile_cols = 0;       // min-plus strip tile columns: 64, 128, 0 = per class
+  int tile_cols = 0;       // FAP_OPT_TILE_COLS: accepted, chooses nothing
   int host_results = 0;    // FAP_OPT_HOST_RESULTS: 0 staged when the device has room, 1 direct
   double host_group_mb = 8192.0;  // FAP_OPT_HOST_GROUP_MB: result rows per group of a host-results solve
   int int32_form = 0;      // FAP_OPT_INT32_FORM: 0 packed keys when provably exact, 1 always wide
@@ -653,10 +649,9 @@ int build_plan(fap_engine *e, Plan &pl) {
     std::vector<PartDesc> pdesc;
     std::vector<int> mat_index;  // pdesc entry -> index in pl.parts
     std::vector<int64_t> row_begin(1, 0), dec_begin(1, 0);
-    // min-plus segments: the strip form's classes of K in order, then those
-    // above its limit; tiles are numbered over all of them
-    std::vector<MpSegment> mps_cls[Plan::Group::kMaxCls], mps_wide;
-    const int ncls = std::min(fapk::minplus_strip_classes(), (int)Plan::Group::kMaxCls);
+    // min-plus segments: the strip form's, then those above its limit; tiles are
+    // numbered over all of them
+    std::vector<MpSegment> mps, mps_deep;
     int maxnb = 0;
     {
       const int first = groups[g].front(), last = groups[g].back();
@@ -716,11 +711,8 @@ int build_plan(fap_engine *e, Plan &pl) {
         s.F = fwd + (size_t)(mat_off[idx] + (int64_t)bdy * d.ld) * es;
         s.Fp = pred ? fwp + mat_off[idx] + (int64_t)bdy * d.ld : nullptr;
         s.ldf = d.ld;
-        int c = 0;
-        while (c < ncls && bdy > fapk::minplus_strip_class_k(c)) c++;
-        if (n >= (1 << 24)) c = ncls;  // the strip form needs leading dimensions below 2^24
-        if (c < ncls) mps_cls[c].push_back(s);
-        else mps_wide.push_back(s);
+        // (the strip form needs leading dimensions below 2^24)
+        (bdy <= fapk::minplus_strip_max_k(e->f32()) && n < (1 << 24) ? mps : mps_deep).push_back(s);
       }
     }
     G.nbatches = (int)batches.size();
@@ -745,20 +737,14 @@ int build_plan(fap_engine *e, Plan &pl) {
     O.pdesc = tb.add(pdesc.data(), pdesc.size());
     O.row_begin = tb.add(row_begin.data(), row_begin.size());
     O.dec_begin = tb.add(dec_begin.data(), dec_begin.size());
-    std::vector<MpSegment> mps;
-    G.mp_ncls = ncls;
-    for (int c = 0; c < ncls; c++)
-      for (const MpSegment &s : mps_cls[c]) G.mp_rows = G.mp_rows || (!e->f32() && !rows_aligned16(s));
-    for (int c = 0; c < ncls; c++) {
-      G.mp_cls_first[c] = (int)mps.size();
-      G.mp_cls_nseg[c] = (int)mps_cls[c].size();
-      auto *number = G.mp_rows ? fapk::number_minplus_rows : fapk::number_minplus_strips;
-      G.mp_cls_strips[c] = number(mps_cls[c].data(), (int)mps_cls[c].size(), e->sm_count, &G.mp_cls_per[c]);
-      for (const MpSegment &s : mps_cls[c]) G.mp_cls_max_k[c] = std::max(G.mp_cls_max_k[c], s.K);
-      mps.insert(mps.end(), mps_cls[c].begin(), mps_cls[c].end());
+    for (const MpSegment &s : mps) {
+      G.mp_rows = G.mp_rows || (!e->f32() && !rows_aligned16(s));
+      G.mp_strip_k = std::max(G.mp_strip_k, s.K);
     }
-    const int nstrip = (int)mps.size();
-    mps.insert(mps.end(), mps_wide.begin(), mps_wide.end());
+    const int nstrip = G.mp_strip_nseg = (int)mps.size();
+    auto *number = G.mp_rows ? fapk::number_minplus_rows : fapk::number_minplus_strips;
+    G.mp_strips = number(mps.data(), nstrip, e->sm_count, &G.mp_strip_per);
+    mps.insert(mps.end(), mps_deep.begin(), mps_deep.end());
     G.mp_strip_tiles = fapk::number_minplus_deep(mps.data(), nstrip, 0);
     G.mp_nseg = (int)mps.size();
     G.mp_tiles = fapk::number_minplus_deep(mps.data() + nstrip, G.mp_nseg - nstrip, G.mp_strip_tiles);
@@ -1035,29 +1021,23 @@ struct Issuer {
       FAP_CUDA(fapk::launch_decode(f32, pred, ba, pl.dist, pl.pred, e->copy));
       FAP_CUDA(cudaEventRecord(e->ev_copy[1], e->copy));
     }
-    if (packed || f32) {  // strip form for the segments with K <= 100, tiles for the rest
-      // The first class on the issuing stream, the later ones (a few parts
-      // with larger K) on the low-priority side stream, whose CTAs take the
-      // SMs the first launch leaves as it drains.  They write other parts'
-      // rows and read only the FW matrices and the boundary rows.
-      bool fork = false;
-      for (int c = 1; c < G.mp_ncls; c++) fork = fork || (G.mp_cls_strips[c] > 0 && G.mp_cls_strips[0] > 0);
+    if (packed || f32) {
+      // The strip form's parts on the issuing stream, those with a larger K on
+      // the low-priority side stream, whose CTAs take the SMs the first launch
+      // leaves as it drains.  They write other parts' rows and read only the FW
+      // matrices and the boundary rows.
+      const bool fork = G.mp_strips > 0 && G.mp_tiles > G.mp_strip_tiles;
       if (fork) {
         FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
         FAP_CUDA(cudaStreamWaitEvent(e->side, e->ev_fw[0], 0));
       }
-      for (int c = 0; c < G.mp_ncls; c++) {
-        cudaStream_t sc = fork && c > 0 ? e->side : st;
-        if (G.mp_rows)
-          FAP_CUDA(fapk::launch_minplus_rows(pred, G.mp + G.mp_cls_first[c], G.mp_cls_nseg[c], G.mp_cls_strips[c],
-                                             G.mp_cls_max_k[c], G.mp_cls_per[c], sc));
-        else
-          FAP_CUDA(fapk::launch_minplus_strips(pred, G.mp + G.mp_cls_first[c], G.mp_cls_nseg[c], G.mp_cls_strips[c],
-                                               G.mp_cls_max_k[c], G.mp_cls_per[c], sc, f32,
-                                               e->tile_cols ? e->tile_cols : G.mp_cls_cols[c]));
-      }
+      if (G.mp_rows)
+        FAP_CUDA(fapk::launch_minplus_rows(pred, G.mp, G.mp_strip_nseg, G.mp_strips, G.mp_strip_k, G.mp_strip_per, st));
+      else
+        FAP_CUDA(fapk::launch_minplus_strips(f32, pred, G.mp, G.mp_strip_nseg, G.mp_strips, G.mp_strip_k,
+                                             G.mp_strip_per, st));
       FAP_CUDA(fapk::launch_minplus_deep(f32, packed, pred, G.mp, G.mp_nseg, G.mp_tiles - G.mp_strip_tiles,
-                                         G.mp_strip_tiles, st));
+                                         G.mp_strip_tiles, fork ? e->side : st));
       if (fork) {  // join
         FAP_CUDA(cudaEventRecord(e->ev_fw[1], e->side));
         FAP_CUDA(cudaStreamWaitEvent(st, e->ev_fw[1], 0));
@@ -1244,61 +1224,6 @@ int trial_sssp_method(fap_engine *e, Plan &pl, cudaStream_t st) {
   return FAP_OK;
 }
 
-// Tile autotuner of the packed min-plus (strip form): on a plan's first run,
-// once the product's inputs are in place (closed FW matrices, boundary
-// rows), times every strip class launch of every group with 128 x 64 and
-// 128 x 128 tiles (best of two launches each) and keeps the faster for the
-// plan's later runs and its CUDA graph.  The product is a pure function of
-// those inputs -- the part's own columns come from its FW matrix, every
-// other output from the product, whatever the output held -- so the trial
-// launches rewrite the same rows.  Not run for results in mapped host
-// memory, where the host link bounds every tile width.
-int autotune_tiles(fap_engine *e, Plan &pl, cudaStream_t st) {
-  if (pl.pack != 1 || pl.bdist != nullptr) return FAP_OK;
-  const bool pred = pl.pred != nullptr;
-  cudaEvent_t a, b;
-  FAP_CUDA(cudaEventCreate(&a));
-  if (cudaEventCreate(&b) != cudaSuccess) {
-    cudaEventDestroy(a);
-    return set_error(FAP_ERR_CUDA, "autotune: event failed");
-  }
-  int rc = FAP_OK;
-  for (auto &G : pl.groups) {
-    for (int c = 0; c < G.mp_ncls && rc == FAP_OK; c++) {
-      if (G.mp_cls_strips[c] <= 0 || G.mp_rows) continue;
-      float best_ms = 1e30f;
-      int best = 0;
-      for (int cols : {64, 128}) {
-        float t = 1e30f;
-        for (int rep = 0; rep < 2 && rc == FAP_OK; rep++) {
-          cudaError_t ce = cudaEventRecord(a, st);
-          if (ce == cudaSuccess)
-            ce = fapk::launch_minplus_strips(pred, G.mp + G.mp_cls_first[c], G.mp_cls_nseg[c],
-                                             G.mp_cls_strips[c], G.mp_cls_max_k[c], G.mp_cls_per[c], st, false, cols);
-          if (ce == cudaSuccess) ce = cudaEventRecord(b, st);
-          if (ce == cudaSuccess) ce = cudaEventSynchronize(b);
-          float ms = 0;
-          if (ce == cudaSuccess) ce = cudaEventElapsedTime(&ms, a, b);
-          if (ce != cudaSuccess) {
-            rc = set_error(FAP_ERR_CUDA, std::string("tile autotune: ") + cudaGetErrorString(ce));
-            break;
-          }
-          t = std::min(t, ms);
-        }
-        if (rc == FAP_OK && t < best_ms) {
-          best_ms = t;
-          best = cols;
-        }
-      }
-      G.mp_cls_cols[c] = best;
-    }
-  }
-  cudaEventDestroy(a);
-  cudaEventDestroy(b);
-  if (rc != FAP_OK) return rc;
-  return check_status(e);
-}
-
 // Decides the packed int32 form for a plan on its first run: runs every
 // group's SSSP, reads back the largest finite SSSP distance, and checks the
 // bound of every finite result: a path inside a part to its first boundary
@@ -1348,7 +1273,6 @@ std::vector<const void *> buffer_signature(const fap_engine *e) {
           reinterpret_cast<const void *>((intptr_t)e->sssp_slots_alloc),
           reinterpret_cast<const void *>((intptr_t)e->sssp_fp64),
           reinterpret_cast<const void *>((intptr_t)e->sssp_lanes),
-          reinterpret_cast<const void *>((intptr_t)e->tile_cols),
           reinterpret_cast<const void *>((intptr_t)e->sssp_method),
           reinterpret_cast<const void *>((intptr_t)e->int32_form),
           e->bg_tab.p,
@@ -1467,7 +1391,6 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
     }
     if ((rc = first_run(e, *pl, st)) != FAP_OK) return rc;
     e->fw_host_work += pl->pack == 1 || e->f32() ? pl->fw_pivot_work : pl->fw_tile_work;
-    if (e->autotune && e->tile_cols == 0 && (rc = autotune_tiles(e, *pl, st)) != FAP_OK) return rc;
     e->last_launches = fapk::launch_count() - c0;  // every kernel of this call, trials included
     return FAP_OK;
   }
@@ -2183,13 +2106,17 @@ int fap_minplus(fap_engine *e, int32_t dtype, int32_t M, int32_t N, int32_t K, c
     packed = (unsigned long long)mx[0] + mx[1] < fapk::pack_limit();
   }
   const MpSegment *dseg = reinterpret_cast<const MpSegment *>(base + o_seg);
-  // the strip form addresses C rows with 32-bit offsets within a 128-row strip
-  if ((packed || (!i32 && K > 0)) && K <= fapk::minplus_strip_max_k() && ldc < (1 << 24) &&
+  // The strip form addresses C rows with 32-bit offsets within a 128-row strip,
+  // and pays from about 6 million outputs and up to 40 steps: FP32 K = 19, 1,000 x
+  // 5,000 62 us there and 56 us in mp_deep.cu, 2,000 x 4,000 68 and 70, 4,000 x
+  // 4,000 102 and 109, 2,000 x 20,000 205 and 225; packed K = 48, 4,000 x 4,000 150
+  // and 141 us, FP32 192 and 141.
+  if ((packed || (!i32 && K > 0)) && K <= 40 && (int64_t)M * N >= 6000000 && ldc < (1 << 24) &&
       (!Cpath || (ldcp < (1 << 24) && ldbp < (1 << 24)))) {
     if (by_rows)
       FAP_CUDA(fapk::launch_minplus_rows(Cpath != nullptr, dseg, 1, strips, K, per, st));
     else
-      FAP_CUDA(fapk::launch_minplus_strips(Cpath != nullptr, dseg, 1, strips, K, per, st, !i32, e->tile_cols));
+      FAP_CUDA(fapk::launch_minplus_strips(!i32, Cpath != nullptr, dseg, 1, strips, K, per, st));
   } else {
     FAP_CUDA(fapk::launch_minplus_deep(!i32, packed, Cpath != nullptr, dseg, 1, tiles, 0, st));
   }

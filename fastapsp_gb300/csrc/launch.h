@@ -16,27 +16,18 @@ int &launch_count();
 // Tiles of the Floyd-Warshall panels and remaining blocks of wide int32
 // matrices (numbered by MpSegment::tile_begin).
 cudaError_t launch_minplus_tiles(bool pred, const MpSegment *d_segs, int nseg, int tiles, cudaStream_t st);
-// Strip form of the packed min-plus: segments that do not accumulate into C
+// Strip form of the min-plus (f32: FP32, else packed int32): segments that do not accumulate into C
 // (init_from_c = 0), C's leading dimensions below 2^24, every
-// K <= max_k <= minplus_strip_max_k(), CTAs numbered by
+// K <= max_k <= minplus_strip_max_k(f32), CTAs numbered by
 // MpSegment::strip_begin (ceil(M / 128) x ceil(tiles_x / per) strips per
 // segment).  The caller must have checked that every finite int32 result stays
 // below pack_limit().
-// f32: FP32 distances (any range) instead of the packed int32 form.
-// tile_cols (packed form): 64 or 128-column tiles, 0 = the default of the
-// K class (minplus_strip_class_cols); the FP32 form always takes 64.
-cudaError_t launch_minplus_strips(bool pred, const MpSegment *d_segs, int nseg, int strips,
-                                  int max_k, int per, cudaStream_t st, bool f32 = false, int tile_cols = 0);
-int minplus_strip_class_cols(int c);
+cudaError_t launch_minplus_strips(bool f32, bool pred, const MpSegment *d_segs, int nseg, int strips, int max_k,
+                                  int per, cudaStream_t st);
 // Numbers the CTAs of one strip launch (returns their count) and chooses the
 // 128-column tiles each takes (launch_minplus_strips' per).
 int number_minplus_strips(MpSegment *segs, int nseg, int sm_count, int *per);
-int minplus_strip_max_k();   // largest K of the strip form
-// Segments go to the strip form in classes of K (one launch per class, each
-// with its own CTAs per SM): class c takes K <= minplus_strip_class_k(c)
-// above the previous bound; -1 past the last class.
-int minplus_strip_classes();
-int minplus_strip_class_k(int c);
+int minplus_strip_max_k(bool f32);   // largest K of the strip form
 // mp_rows.cu: the packed strip form for result rows that do not start on 16-byte
 // boundaries; same preconditions (B's predecessors' leading dimension below 2^24
 // too), numbering and counters.

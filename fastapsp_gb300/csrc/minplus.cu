@@ -8,7 +8,7 @@
 //
 // Kernels of this file:
 //  - mp_strip_kernel (FP32, and int32 whose finite results stay below 2^24 - 1;
-//    at most 100 steps): packed keys (d << 7) | idx, one DPX __viaddmin_u32 per
+//    at most 48 steps): packed keys (d << 7) | idx, one DPX __viaddmin_u32 per
 //    add-min, which gives the minimum and, on ties, the smallest idx -- the
 //    current value (idx 0) first, then the first k.  A stays resident for a
 //    strip of column tiles, and the steps k whose A column or B row has no
@@ -272,7 +272,7 @@ __device__ __forceinline__ void tile_wide(MpSmem &sm, const MpSegment &s, const 
 
 // Strip form of the packed min-plus for products that do not accumulate into
 // C (the inner rows of every part) with K <= kStripMaxK.  One CTA owns a
-// strip: one 128-row tile of a segment and the TN-column tiles of up to
+// strip: one 128-row tile of a segment and the 64-column tiles of up to
 // kStripTiles x 128 consecutive columns.  A's 128 x K block is staged once
 // per strip (transposed, so that a thread's 8 row operands of one k are two
 // 16-byte loads); B's K x TN tiles are double-buffered, so the next tile's
@@ -297,31 +297,34 @@ __device__ __forceinline__ void tile_wide(MpSmem &sm, const MpSegment &s, const 
 // outputs, summed over tiles)], summed per CTA.
 __device__ unsigned long long g_strip_counters[3];
 
-constexpr int kStripTiles = 16;  // a strip spans at most kStripTiles x 128 columns (minplus_strip_cols)
-constexpr int kStripMaxK = 100;  // largest K of the strip form
+constexpr int kStripTiles = 16;  // a strip spans at most kStripTiles x 128 columns 
+constexpr int kStripCols = 64;   // columns of a tile
+// Largest K of the strip form.  128 x 64 tiles with 8 x 4 outputs a thread,
+// three CTAs per SM: on sparse products most of a tile's time is its fixed work
+// (B keys, masks, epilogue), whose latencies only more resident warps hide
+// (against 128 x 128 tiles at two CTAs per SM 16 % faster on a 65,536-vertex
+// geometric graph; four CTAs per SM for K <= 32, at 64 registers a thread, no
+// faster).  Above, mp_deep.cu's tiles, which share the staging of A among fewer
+// columns but keep three CTAs per SM at any K, are faster: products of 2,000 x
+// 20,000 at K = 36 / 48 / 72 / 100, packed 223 / 272 / 381 / 482 us here and 237 /
+// 260 / 334 / 412 us there, FP32 285 / 400 / 521 / 667 and 277 / 305 / 439 / 560 us;
+// the min-plus of a 128 x 128 grid in 16 parts (K from 41 to 92) 2.07 ms with
+// every part here (128 x 128 tiles above 48), 1.79 ms with those above 48 there.
+// (FP32, whose tiles take more shared memory: 40.)
+constexpr int kStripMaxK = 48, kStripMaxKF32 = 40;
 constexpr int kOwnCap = 12;
-// Segments are launched in classes of K.  K <= 48: 128 x 64 tiles with 8 x
-// 4 outputs a thread, three CTAs per SM.  On sparse products most of a
-// tile's time is its fixed work (B keys, masks, epilogue), whose latencies
-// only more resident warps hide; against 128 x 128 tiles at two CTAs per SM
-// it measured 16 % faster on a 65,536-vertex geometric graph.  (Four CTAs per
-// SM for K <= 32, at 64 registers a thread, measured no faster.)  K <= 100:
-// 128 x 128 tiles with 8 x 8 outputs a thread (twice the add-mins per shared
-// load), one CTA per SM either way at that K.
-constexpr int kStripClassK[] = {48, kStripMaxK};
-constexpr int kStripClassTN[] = {64, 128};
-constexpr int kStripClasses = 2;
 
 // Row stride of the FP32 strip kernel's row-major copy of A for kseg
 // steps: kseg, or kseg + 4 when kseg / 4 is even, so that the stride in
 // 16-byte units is odd.
 __host__ __device__ constexpr int strip_ar_stride(int kseg) { return ((kseg >> 2) & 1) ? kseg : kseg + 4; }
 
-// Shared memory of the strip kernel with TN-column tiles, in bytes; F32 adds
+// Shared memory of the strip kernel, in bytes; F32 adds
 // the row-major copy of A ([128][ks + 4] at most) and the step-group copy
 // of B ([ks / 4][64] 16-byte units, within [64][ks + 4] words).
-template <int TN, bool F32 = false>
+template <bool F32>
 __host__ __device__ constexpr size_t strip_smem_bytes(int ks) {
+  constexpr int TN = kStripCols;
   return ((size_t)2 * ks * TN + (size_t)(ks + 1) * TN + 6 * TN + (size_t)2 * kOwnCap * kTile +
           (size_t)ks * kTile + (F32 ? (size_t)(kTile + TN) * (ks + 4) : 0)) * 4;
 }
@@ -498,12 +501,12 @@ __device__ __forceinline__ void addmin_groups_rows_f32(unsigned (&acc)[8][4], in
 // bits and the step idx (k + 1, 0 = none) of its last strict improvement in
 // two registers: fl(a + b), then __vibmin_u32 for the minimum and whether the
 // current value was kept (non-negative floats order like their bits) -- the
-// reference's strict-<, ascending-k rule, as in the packed form.  TN = 64
-// only, two CTAs per SM.
-template <bool PRED, int TN, bool F32 = false>
-__global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
+// reference's strict-<, ascending-k rule, as in the packed form.  Two
+// CTAs per SM.
+template <bool PRED, bool F32>
+__global__ void __launch_bounds__(kThreads, F32 ? 2 : 3)
     mp_strip_kernel(const MpSegment *__restrict__ segs, int nseg, int ks, int per) {
-  constexpr int CH = TN / 64;  // 64-column halves of a thread's outputs
+  constexpr int TN = kStripCols;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned *Bs = reinterpret_cast<unsigned *>(smem_raw);  // [2][ks][TN]
   int32_t *Bps = reinterpret_cast<int32_t *>(Bs + 2 * ks * TN);  // [1 + ks][TN]
@@ -686,7 +689,7 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
     n_tiles++;
     n_empty += nact == 0;
     // (FP32 with at least half of the steps active runs all of them)
-    n_steps += (unsigned long long)(F32 && CH == 1 && nact > 0 && 2 * nact >= kseg ? kseg : nact) * kTile * TN;
+    n_steps += (unsigned long long)(F32 && nact > 0 && 2 * nact >= kseg ? kseg : nact) * kTile * TN;
     if (PRED && nact == s.K && s.K > 0)  // every step active: all rows, 16-byte copies spread over the CTA
       strip_load_rows<TN>(reinterpret_cast<unsigned *>(Bps + TN), reinterpret_cast<const unsigned *>(s.Bp),
                           s.ldbp, s.K, s.N, kseg, jt * TN, vec_bp, 0xffffffffu);
@@ -698,12 +701,12 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
                           s.N, kseg, (jt + 1) * TN, vec_b, INF);
     cp_async_commit();
 
-    unsigned acc[8][4 * CH];
-    int arg[8][4 * CH];  // F32: step idx of the last strict improvement (0: none)
+    unsigned acc[8][4];
+    int arg[8][4];  // F32: step idx of the last strict improvement (0: none)
 #pragma unroll
     for (int r = 0; r < 8; r++)
 #pragma unroll
-      for (int c = 0; c < 4 * CH; c++) {
+      for (int c = 0; c < 4; c++) {
         acc[r][c] = F32 ? INF : kPackH << kIdxBits;
         arg[r][c] = 0;
       }
@@ -728,27 +731,25 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
       // FP32 with at least half of the steps active: all steps in groups
       // of four (steps that are not active, or at or past K, hold
       // "unreached" on one side and never win).
-      const bool grouped = F32 && CH == 1 && nact > 0 && 2 * nact >= kseg;
+      const bool grouped = F32 && nact > 0 && 2 * nact >= kseg;
       if (grouped) {
-        if constexpr (F32 && CH == 1) addmin_groups_rows_f32<PRED>(acc, arg, Ar, ars, kseg, ty * 4, Bq, tx);
+        if constexpr (F32) addmin_groups_rows_f32<PRED>(acc, arg, Ar, ars, kseg, ty * 4, Bq, tx);
       } else if (nact == s.K && s.K > 0) {
         uint4 na0 = *reinterpret_cast<const uint4 *>(a_at(0));
         uint4 na1 = *reinterpret_cast<const uint4 *>(a_at(0) + kBlk);
-        uint4 nb0 = load_b(0);
-        uint4 nb1 = CH == 2 ? *reinterpret_cast<const uint4 *>(b_at(0) + kBlk) : nb0;
+        uint4 nb = load_b(0);
 #pragma unroll 2
         for (int kk = 0; kk < kseg; kk++) {
           const unsigned a[8] = {na0.x, na0.y, na0.z, na0.w, na1.x, na1.y, na1.z, na1.w};
-          const unsigned b[8] = {nb0.x, nb0.y, nb0.z, nb0.w, nb1.x, nb1.y, nb1.z, nb1.w};
+          const unsigned b[4] = {nb.x, nb.y, nb.z, nb.w};
           const int kn = kk + 1 < kseg ? kk + 1 : kk;
           na0 = *reinterpret_cast<const uint4 *>(a_at(kn));
           na1 = *reinterpret_cast<const uint4 *>(a_at(kn) + kBlk);
-          nb0 = load_b(kn);
-          if (CH == 2) nb1 = *reinterpret_cast<const uint4 *>(b_at(kn) + kBlk);
+          nb = load_b(kn);
 #pragma unroll
           for (int r = 0; r < 8; r++)
 #pragma unroll
-            for (int c = 0; c < 4 * CH; c++) strip_addmin<F32>(acc[r][c], arg[r][c], a[r], b[c], kk + 1);
+            for (int c = 0; c < 4; c++) strip_addmin<F32>(acc[r][c], arg[r][c], a[r], b[c], kk + 1);
         }
       } else if (nact > 0) {
         auto next_k = [&]() {  // lowest remaining step, or -1
@@ -767,22 +768,20 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
         int kk = next_k();
         uint4 na0 = *reinterpret_cast<const uint4 *>(a_at(kk));
         uint4 na1 = *reinterpret_cast<const uint4 *>(a_at(kk) + kBlk);
-        uint4 nb0 = load_b(kk);
-        uint4 nb1 = CH == 2 ? *reinterpret_cast<const uint4 *>(b_at(kk) + kBlk) : nb0;
+        uint4 nb = load_b(kk);
         while (kk >= 0) {
           const unsigned a[8] = {na0.x, na0.y, na0.z, na0.w, na1.x, na1.y, na1.z, na1.w};
-          const unsigned b[8] = {nb0.x, nb0.y, nb0.z, nb0.w, nb1.x, nb1.y, nb1.z, nb1.w};
+          const unsigned b[4] = {nb.x, nb.y, nb.z, nb.w};
           const int cur = kk;
           kk = next_k();
           const int kn = kk >= 0 ? kk : 0;
           na0 = *reinterpret_cast<const uint4 *>(a_at(kn));
           na1 = *reinterpret_cast<const uint4 *>(a_at(kn) + kBlk);
-          nb0 = load_b(kn);
-          if (CH == 2) nb1 = *reinterpret_cast<const uint4 *>(b_at(kn) + kBlk);
+          nb = load_b(kn);
 #pragma unroll
           for (int r = 0; r < 8; r++)
 #pragma unroll
-            for (int c = 0; c < 4 * CH; c++) strip_addmin<F32>(acc[r][c], arg[r][c], a[r], b[c], cur + 1);
+            for (int c = 0; c < 4; c++) strip_addmin<F32>(acc[r][c], arg[r][c], a[r], b[c], cur + 1);
         }
       }
     }
@@ -850,67 +849,59 @@ __global__ void __launch_bounds__(kThreads, TN == 128 || F32 ? 2 : 3)
       }
       continue;
     }
-    unsigned ownmask = 0;  // bit h * 4 + q: this thread's column sc0 + q of half h is the part's own
+    const int sc0 = tx * 4, col0 = colbase + sc0;
+    unsigned ownmask = 0;  // bit q: this thread's column sc0 + q is the part's own
     if (nown > 0) {
 #pragma unroll
-      for (int c = 0; c < 4 * CH; c++)
-        if (ownidx[buf * TN + (c >> 2) * kBlk + tx * 4 + (c & 3)] != -1) ownmask |= 1u << c;
+      for (int q = 0; q < 4; q++)
+        if (ownidx[buf * TN + sc0 + q] != -1) ownmask |= 1u << q;
     }
 #pragma unroll
     for (int r = 0; r < 8; r++) {
       const int rr = (r >> 2) * kBlk + (r & 3);  // row offset from this thread's first row
       const int row = row0 + ty * 4 + rr;
-      const bool row_ok = row < m_rows;
-      if (!row_ok) continue;
+      if (row >= m_rows || col0 >= n_cols) continue;
       unsigned *crow = c_thr + rr * ldc;
       int32_t *prow = PRED ? p_thr + rr * ldcp : nullptr;
+      unsigned d[4] = {INF, INF, INF, INF};
+      int32_t p[4] = {-1, -1, -1, -1};
+      // a quad of unreached outputs (the common case on sparse graphs)
+      // needs no decode and no predecessor gathers
+      const unsigned qmin = min(min(acc[r][0], acc[r][1]), min(acc[r][2], acc[r][3]));
+      if (qmin < (kPackH << kIdxBits)) {
 #pragma unroll
-      for (int h = 0; h < CH; h++) {
-        const int sc0 = h * kBlk + tx * 4;
-        const int col0 = colbase + sc0;
-        const bool ok = row_ok && col0 < n_cols;
-        if (!ok) continue;
-        unsigned d[4] = {INF, INF, INF, INF};
-        int32_t p[4] = {-1, -1, -1, -1};
-        // a quad of unreached outputs (the common case on sparse graphs)
-        // needs no decode and no predecessor gathers
-        const unsigned qmin = min(min(acc[r][h * 4], acc[r][h * 4 + 1]),
-                                  min(acc[r][h * 4 + 2], acc[r][h * 4 + 3]));
-        if (qmin < (kPackH << kIdxBits)) {
+        for (int q = 0; q < 4; q++) {
+          const unsigned key = acc[r][q];
+          const unsigned dist = key >> kIdxBits;
+          d[q] = dist >= kPackH ? INF : dist;
+          if (PRED) p[q] = Bps[(key & kIdxMask) * TN + sc0 + q];
+        }
+      }
+      if (ownmask) {
 #pragma unroll
-          for (int q = 0; q < 4; q++) {
-            const unsigned key = acc[r][h * 4 + q];
-            const unsigned dist = key >> kIdxBits;
-            d[q] = dist >= kPackH ? INF : dist;
-            if (PRED) p[q] = Bps[(key & kIdxMask) * TN + sc0 + q];
+        for (int q = 0; q < 4; q++) {
+          if (!((ownmask >> q) & 1u)) continue;
+          const int oi = ownidx[buf * TN + sc0 + q];
+          if (oi >= 0) {  // own-part column: the FW value, staged
+            d[q] = Fst[oi * kTile + row - row0];
+            if (PRED) p[q] = Fpst[oi * kTile + row - row0];
+          } else if (oi == -2) {  // own-part column beyond the staging slots
+            const int64_t fj = coll[buf * TN + sc0 + q] - s.local0;
+            d[q] = static_cast<const unsigned *>(s.F)[(int64_t)row * s.ldf + fj];
+            if (PRED) p[q] = s.Fp[(int64_t)row * s.ldf + fj];
           }
         }
-        if ((ownmask >> (h * 4)) & 0xfu) {
+      }
+      if (vec_c && col0 + 3 < n_cols) {  // streaming stores: the rows are not read again here
+        __stcs(reinterpret_cast<uint4 *>(crow + col0), make_uint4(d[0], d[1], d[2], d[3]));
+        if (PRED) __stcs(reinterpret_cast<int4 *>(prow + col0), make_int4(p[0], p[1], p[2], p[3]));
+      } else {
 #pragma unroll
-          for (int q = 0; q < 4; q++) {
-            if (!((ownmask >> (h * 4 + q)) & 1u)) continue;
-            const int oi = ownidx[buf * TN + sc0 + q];
-            if (oi >= 0) {  // own-part column: the FW value, staged
-              d[q] = Fst[oi * kTile + row - row0];
-              if (PRED) p[q] = Fpst[oi * kTile + row - row0];
-            } else if (oi == -2 && ok) {  // own-part column beyond the staging slots
-              const int64_t fj = coll[buf * TN + sc0 + q] - s.local0;
-              d[q] = static_cast<const unsigned *>(s.F)[(int64_t)row * s.ldf + fj];
-              if (PRED) p[q] = s.Fp[(int64_t)row * s.ldf + fj];
-            }
+        for (int q = 0; q < 4; q++)
+          if (col0 + q < n_cols) {
+            crow[col0 + q] = d[q];
+            if (PRED) prow[col0 + q] = p[q];
           }
-        }
-        if (vec_c && ok && col0 + 3 < n_cols) {  // streaming stores: the rows are not read again here
-          __stcs(reinterpret_cast<uint4 *>(crow + col0), make_uint4(d[0], d[1], d[2], d[3]));
-          if (PRED) __stcs(reinterpret_cast<int4 *>(prow + col0), make_int4(p[0], p[1], p[2], p[3]));
-        } else if (ok) {
-#pragma unroll
-          for (int q = 0; q < 4; q++)
-            if (col0 + q < n_cols) {
-              crow[col0 + q] = d[q];
-              if (PRED) prow[col0 + q] = p[q];
-            }
-        }
       }
     }
   }
@@ -1090,12 +1081,18 @@ cudaError_t launch_mp_t(const MpSegment *d_segs, int nseg, int tiles, cudaStream
   return cudaGetLastError();
 }
 
-template <bool PRED, int TN, bool F32 = false>
+template <bool PRED, bool F32>
 cudaError_t launch_strip_t(const MpSegment *d_segs, int nseg, int strips, int ks, int per, cudaStream_t st) {
   if (strips <= 0 || nseg <= 0) return cudaSuccess;
   ++launch_count();
-  mp_strip_kernel<PRED, TN, F32><<<strips, kThreads, strip_smem_bytes<TN, F32>(ks), st>>>(d_segs, nseg, ks, per);
+  mp_strip_kernel<PRED, F32><<<strips, kThreads, strip_smem_bytes<F32>(ks), st>>>(d_segs, nseg, ks, per);
   return cudaGetLastError();
+}
+
+template <bool PRED, bool F32>
+cudaError_t set_strip_attr() {
+  return cudaFuncSetAttribute(mp_strip_kernel<PRED, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)strip_smem_bytes<F32>((minplus_strip_max_k(F32) + 3) & ~3));
 }
 
 template <bool PRED>
@@ -1109,21 +1106,15 @@ cudaError_t launch_minplus_tiles(bool pred, const MpSegment *d_segs, int nseg, i
   return pred ? launch_mp_t<true>(d_segs, nseg, tiles, st) : launch_mp_t<false>(d_segs, nseg, tiles, st);
 }
 
-cudaError_t launch_minplus_strips(bool pred, const MpSegment *d_segs, int nseg, int strips,
-                                  int max_k, int per, cudaStream_t st, bool f32, int tile_cols) {
-  if (max_k < 0 || max_k > kStripMaxK || per < 1) return cudaErrorInvalidValue;
+cudaError_t launch_minplus_strips(bool f32, bool pred, const MpSegment *d_segs, int nseg, int strips, int max_k,
+                                  int per, cudaStream_t st) {
+  if (max_k < 0 || max_k > minplus_strip_max_k(f32) || per < 1) return cudaErrorInvalidValue;
   const int ks = (max_k + 3) & ~3;
-  if (f32)  // 128 x 64 tiles at every K (the argmin registers leave no room for 128 x 128)
-    return pred ? launch_strip_t<true, 64, true>(d_segs, nseg, strips, ks, per, st)
-                : launch_strip_t<false, 64, true>(d_segs, nseg, strips, ks, per, st);
-  const int tn = tile_cols ? tile_cols : kStripClassTN[max_k <= kStripClassK[0] ? 0 : 1];
-  if (tn == 64)
-    return pred ? launch_strip_t<true, 64>(d_segs, nseg, strips, ks, per, st)
-                : launch_strip_t<false, 64>(d_segs, nseg, strips, ks, per, st);
-  if (tn == 128)
-    return pred ? launch_strip_t<true, 128>(d_segs, nseg, strips, ks, per, st)
-                : launch_strip_t<false, 128>(d_segs, nseg, strips, ks, per, st);
-  return cudaErrorInvalidValue;
+  if (f32)
+    return pred ? launch_strip_t<true, true>(d_segs, nseg, strips, ks, per, st)
+                : launch_strip_t<false, true>(d_segs, nseg, strips, ks, per, st);
+  return pred ? launch_strip_t<true, false>(d_segs, nseg, strips, ks, per, st)
+              : launch_strip_t<false, false>(d_segs, nseg, strips, ks, per, st);
 }
 
 namespace {
@@ -1153,11 +1144,7 @@ int number_minplus_strips(MpSegment *segs, int nseg, int sm_count, int *per) {
   return strips;
 }
 
-
-int minplus_strip_max_k() { return kStripMaxK; }
-int minplus_strip_classes() { return kStripClasses; }
-int minplus_strip_class_k(int c) { return c >= 0 && c < kStripClasses ? kStripClassK[c] : -1; }
-int minplus_strip_class_cols(int c) { return c >= 0 && c < kStripClasses ? kStripClassTN[c] : -1; }
+int minplus_strip_max_k(bool f32) { return f32 ? kStripMaxKF32 : kStripMaxK; }
 
 cudaError_t launch_max_finite(const MatRef *d_mats, int nmats, unsigned *out, int step, cudaStream_t st) {
   if (nmats <= 0) return cudaSuccess;
@@ -1192,22 +1179,10 @@ cudaError_t init_minplus_kernels() {
   cudaError_t e;
   if ((e = set_mp_attr<true>()) != cudaSuccess) return e;
   if ((e = set_mp_attr<false>()) != cudaSuccess) return e;
-  // either tile width serves any K of the strip form (tile_cols)
-  static_assert(kStripClassTN[0] == 64 && kStripClassTN[1] == 128, "strip tile widths");
-  const int smax0 = (int)strip_smem_bytes<64>((kStripMaxK + 3) & ~3);
-  const int smax1 = (int)strip_smem_bytes<128>((kStripMaxK + 3) & ~3);
-#define FAP_STRIP_ATTR(P, TN, F, SMAX)                                                               \
-  if ((e = cudaFuncSetAttribute(mp_strip_kernel<P, TN, F>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                SMAX)) != cudaSuccess)                                                \
-    return e;
-  FAP_STRIP_ATTR(true, 64, false, smax0)
-  FAP_STRIP_ATTR(false, 64, false, smax0)
-  FAP_STRIP_ATTR(true, 128, false, smax1)
-  FAP_STRIP_ATTR(false, 128, false, smax1)
-  const int smaxf = (int)strip_smem_bytes<64, true>((kStripMaxK + 3) & ~3);
-  FAP_STRIP_ATTR(true, 64, true, smaxf)
-  FAP_STRIP_ATTR(false, 64, true, smaxf)
-#undef FAP_STRIP_ATTR
+  if ((e = set_strip_attr<true, false>()) != cudaSuccess) return e;
+  if ((e = set_strip_attr<false, false>()) != cudaSuccess) return e;
+  if ((e = set_strip_attr<true, true>()) != cudaSuccess) return e;
+  if ((e = set_strip_attr<false, true>()) != cudaSuccess) return e;
   return cudaSuccess;
 }
 

@@ -128,8 +128,9 @@ __global__ void __launch_bounds__(kDeepThreads, 3)
     load_rows<kDeepTile, kDeepPitch, false>(&sm[buf].A[0][0], Ag + k0, lda, vec_a && kn >= kDeepK, M - row0, kn, INF);
     load_rows<kDeepK, kDeepTile, true>(&sm[buf].B[0][0], Bg + k0 * ldb, ldb, vec_b, kn, N - col0, INF);
   };
-  // Packed: the entries this thread copied become keys.
+  // Packed: the entries this thread copied become keys; whether it saw a finite one in B.
   auto to_keys = [&](int buf, int kn) {
+    unsigned least = INF;
     auto key = [](unsigned v, unsigned idx) { return min(v, kPackH) * (1u << kIdxBits) + idx; };
     if (vec_a && kn >= kDeepK) {
 #pragma unroll
@@ -149,15 +150,18 @@ __global__ void __launch_bounds__(kDeepThreads, 3)
         const unsigned idx = PRED ? k + 1 : 0;
         uint4 *p = reinterpret_cast<uint4 *>(&sm[buf].B[k][(tx * 4) ^ swz<true>(k)]);
         const uint4 v = *p;
+        least = min(least, min(min(v.x, v.y), min(v.z, v.w)));
         *p = make_uint4(key(v.x, idx), key(v.y, idx), key(v.z, idx), key(v.w, idx));
       }
     } else {
 #pragma unroll 4
       for (int k = t >> 6; k < kDeepK; k += 4) {
         unsigned *p = &sm[buf].B[k][(t & 63) ^ swz<true>(k)];
+        least = min(least, *p);
         *p = key(*p, PRED ? k + 1 : 0);
       }
     }
+    return least < kPackH;
   };
 
   unsigned acc[4][4];
@@ -175,10 +179,13 @@ __global__ void __launch_bounds__(kDeepThreads, 3)
   for (int ch = 0; ch < nchunks; ch++) {
     const int buf = ch & 1, k0 = ch * kDeepK;
     cp_async_wait_0();
-    if (FORM == kDeepPacked) to_keys(buf, K - k0);
-    __syncthreads();  // the chunk is there; every thread is done with the last one
+    // the chunk is there; every thread is done with the last one
+    bool work = true;
+    if (FORM == kDeepPacked) work = __syncthreads_or(to_keys(buf, K - k0));
+    else __syncthreads();
     if (ch + 1 < nchunks) load(ch + 1, buf ^ 1);
     cp_async_commit();
+    if (!work) continue;  // columns that nothing reaches (unconnected parts)
     const int ng = (min(kDeepK, K - k0) + 3) >> 2;
 #pragma unroll 1
     for (int g = 0; g < ng; g++) {

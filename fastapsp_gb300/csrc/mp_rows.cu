@@ -374,7 +374,7 @@ int number_minplus_rows(MpSegment *segs, int nseg, int sm_count, int *per) {
 cudaError_t launch_minplus_rows(bool pred, const MpSegment *d_segs, int nseg, int strips, int max_k, int per,
                                 cudaStream_t st) {
   if (strips <= 0 || nseg <= 0) return cudaSuccess;
-  if (max_k < 0 || max_k > minplus_strip_max_k() || per < 1) return cudaErrorInvalidValue;
+  if (max_k < 0 || max_k > minplus_strip_max_k(false) || per < 1) return cudaErrorInvalidValue;
   const int ks = std::max((max_k + 3) & ~3, 4);
   ++launch_count();
   if (pred) mp_rows_kernel<true><<<strips, kMpThreads, mp_rows_smem(ks), st>>>(d_segs, nseg, ks, per);
@@ -390,7 +390,7 @@ cudaError_t rows_counters(unsigned long long out[3], bool reset) {
 }
 
 cudaError_t init_mp_rows_kernels() {
-  const int smem = (int)mp_rows_smem((minplus_strip_max_k() + 3) & ~3);
+  const int smem = (int)mp_rows_smem((minplus_strip_max_k(false) + 3) & ~3);
   cudaError_t e = cudaFuncSetAttribute(mp_rows_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(mp_rows_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);

@@ -208,12 +208,8 @@ int fap_precondition(fap_engine *e);
  *                      keeps the faster, which fap_get_option then reports
  *                      (not with FAP_OPT_SSSP_FP64, which takes 16 unless 32
  *                      is set).  Changes speed only, never results.
- *   FAP_OPT_TILE_COLS  column width of the packed int32 min-plus tiles (128
- *                      rows): 64 or 128, or 0 (default) = chosen per K class
- *                      of each plan: while FAP_OPT_AUTOTUNE is on, the first
- *                      run times both widths and keeps the faster (not for
- *                      results in mapped host memory); otherwise 64 for
- *                      K <= 48 and 128 above.  Changes speed only.
+ *   FAP_OPT_TILE_COLS  0, 64 or 128; accepted for programs that set it, chooses
+ *                      nothing (the min-plus has one tile width).
  *   FAP_OPT_SSSP_METHOD how the boundary SSSP rows of a solve are made.
  *                      The boundary-graph method (local rows of every part
  *                      from its boundary vertices, shortest paths between

@@ -339,7 +339,7 @@ def test_minplus_strip_lengths_agree(ctx, f32, n):
     """Strips of 128 to 2,048 columns (by how many the product has) give the
     rows of the same product in slices of 100 columns."""
     gen = torch.Generator(device="cuda").manual_seed(n)
-    m, k = 260, 19
+    m, k = max(260, 6100000 // n), 19
 
     def side(r, c):
         x = torch.rand(r, c, device="cuda", generator=gen) * 100
@@ -418,8 +418,8 @@ def test_solve_with_many_boundary_vertices(gpu, f32):
 
 
 @pytest.mark.parametrize("pred", [True, False])
-@pytest.mark.parametrize("m, n, k, off", [(128, 57, 1, 1), (129, 64, 4, 3), (3, 1001, 19, 0), (300, 2049, 33, 5),
-                                          (130, 130, 100, 7), (64, 4095, 48, 2)])
+@pytest.mark.parametrize("m, n, k, off", [(128, 65537, 1, 1), (129, 65600, 4, 3), (3, 2800001, 19, 0),
+                                          (4100, 2049, 33, 5), (6100, 1001, 40, 7)])
 def test_minplus_of_rows_off_boundaries(ctx, m, n, k, off, pred):
     """Packed products into rows that start off 16-byte boundaries (odd lengths and
     offsets) equal those into aligned rows."""
