@@ -1490,6 +1490,8 @@ int init_device(fap_engine *e, int device) {
   FAP_CUDA(fapk::init_minplus_kernels());
   FAP_CUDA(fapk::init_mp_deep_kernels());
   FAP_CUDA(fapk::init_mp_rows_kernels());
+  FAP_CUDA(fapk::init_query_kernels());
+  FAP_CUDA(fapk::init_backward_kernels());
   FAP_CUDA(fapk::init_fw_pivot_kernels());
   FAP_CUDA(fapk::init_fw_rest_kernels());
   FAP_CUDA(fapk::init_sssp_kernels());
@@ -2015,6 +2017,16 @@ int fap_minplus_counters(fap_engine *e, uint64_t *out3, int32_t reset) {
   return FAP_OK;
 }
 
+// Scratch of the walks along predecessor rows: a counter and an entry a walk;
+// null: no memory for it.
+static int32_t *walk_scratch(fap_engine *e, int32_t walks) {
+  if (e->small.ensure(((size_t)walks + 1) * sizeof(int32_t)) != FAP_OK) {
+    fapi::clear_error();
+    return nullptr;
+  }
+  return static_cast<int32_t *>(e->small.p);
+}
+
 int fap_query(fap_engine *e, const void *dist, const int32_t *pred, int32_t nq, const int32_t *src,
               const int32_t *dst, void *out_dist, int32_t *out_len, int32_t *out_path, int32_t max_len,
               void *stream) {
@@ -2045,7 +2057,9 @@ int fap_query(fap_engine *e, const void *dist, const int32_t *pred, int32_t nq, 
   a.out_path = out_path;
   a.max_len = max_len;
   a.status = e->d_status;
-  FAP_CUDA(fapk::launch_query(e->f32(), a, st));
+  a.nrest = fapk::queries_by_row(e->n, nq) ? walk_scratch(e, nq) : nullptr;
+  a.rest = a.nrest ? a.nrest + 1 : nullptr;
+  FAP_CUDA(fapk::launch_query(e->f32(), a, e->sm_count, st));
   FAP_CUDA(cudaStreamSynchronize(st));
   return check_status(e);
 }
@@ -2320,8 +2334,22 @@ int fap_backward(fap_engine *e, const int32_t *pred, int32_t num_pairs, const in
   std::lock_guard<std::mutex> lk(e->mu);
   DeviceGuard dg(e->device);
   cudaStream_t st = pick_stream(e, stream);
-  FAP_CUDA(fapk::launch_backward_graph(e->n, e->d_ro, e->d_col, static_cast<const float *>(e->d_w),
-                                       e->d_ed2st, pred, num_pairs, s, t, g, dw, e->d_status, st));
+  fapk::BackwardArgs a{};
+  a.n = e->n;
+  a.ro = e->d_ro;
+  a.col = e->d_col;
+  a.w = static_cast<const float *>(e->d_w);
+  a.ed2st = e->d_ed2st;
+  a.pred = pred;
+  a.npairs = num_pairs;
+  a.s = s;
+  a.t = t;
+  a.g = g;
+  a.dw = dw;
+  a.status = e->d_status;
+  a.nrest = fapk::pairs_by_row(e->n, num_pairs) ? walk_scratch(e, num_pairs) : nullptr;
+  a.rest = a.nrest ? a.nrest + 1 : nullptr;
+  FAP_CUDA(fapk::launch_backward_graph(a, e->sm_count, st));
   FAP_CUDA(cudaStreamSynchronize(st));
   return check_status(e);
 }

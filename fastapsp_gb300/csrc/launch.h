@@ -195,8 +195,11 @@ struct QueryArgs {
   int32_t *out_path;       // nq x max_len, may be null
   int32_t max_len;
   unsigned *status;
+  int32_t *nrest, *rest;   // scratch: a counter and nq entries (null: queries_by_row() is false)
 };
-cudaError_t launch_query(bool f32, const QueryArgs &a, cudaStream_t st);
+bool queries_by_row(int32_t n, int32_t walks);
+cudaError_t init_query_kernels();
+cudaError_t launch_query(bool f32, const QueryArgs &a, int sm_count, cudaStream_t st);
 
 // transform.cu
 struct PartDesc {
@@ -228,10 +231,22 @@ cudaError_t launch_decode(bool f32, bool pred, const BuildArgs &a, void *rows, i
                           cudaStream_t st);
 
 // adjoint.cu
-cudaError_t launch_backward_graph(int32_t n, const int32_t *ro, const int32_t *col, const float *w,
-                                  const int32_t *ed2st, const int32_t *pred, int32_t npairs,
-                                  const int32_t *s, const int32_t *t, const float *g, float *dw,
-                                  unsigned *status, cudaStream_t st);
+struct BackwardArgs {
+  int32_t n;
+  const int32_t *ro, *col;  // out-edge CSR
+  const float *w;
+  const int32_t *ed2st;     // vertex -> row
+  const int32_t *pred;      // n x n solve() rows
+  int32_t npairs;
+  const int32_t *s, *t;
+  const float *g;
+  float *dw;
+  unsigned *status;
+  int32_t *nrest, *rest;    // scratch as QueryArgs'
+};
+bool pairs_by_row(int32_t n, int32_t walks);
+cudaError_t init_backward_kernels();
+cudaError_t launch_backward_graph(const BackwardArgs &a, int sm_count, cudaStream_t st);
 cudaError_t launch_backward_dense(const void *inst, int32_t ninst, int32_t npairs,
                                   const int32_t *b, const int32_t *s, const int32_t *t,
                                   const float *g, unsigned *status, cudaStream_t st);

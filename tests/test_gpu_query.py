@@ -196,3 +196,64 @@ def test_part_shares_equal_the_full_solve(gpu, world):
                 r0 += sub
         with pytest.raises(gpu._lib.FapError):
             eng.solve_parts([1, 1], d, p)
+
+
+@pytest.mark.parametrize("n, nq", [(17, 400), (18, 400), (257, 400), (2600, 400), (2600, 160000)])
+def test_walks_along_a_chain(gpu, n, nq):
+    """Paths of every length of a two-way chain (and an isolated vertex): the
+    vertices, slots left alone where the path does not fit, the gradient of each
+    edge, and broken chains reported."""
+    k = n - 1  # vertex k is isolated
+    edges = sorted([(i, i + 1) for i in range(k - 1)] + [(i + 1, i) for i in range(k - 1)])
+    ro = np.zeros(n + 1, np.int32)
+    for u, _ in edges:
+        ro[u + 1] += 1
+    ro = np.cumsum(ro).astype(np.int32)
+    col, w = np.array([v for _, v in edges], np.int32), np.ones(len(edges), np.float32)
+    rng = np.random.default_rng(n)
+    s, t = (rng.integers(0, n, size=nq).astype(np.int32) for _ in range(2))
+    s[:3], t[:3] = (0, k, 0), (k - 1, k, k)
+    hops = np.where((s == t) | ((s < k) & (t < k)), np.abs(s - t), -1)
+    with gpu.Engine(n, ro, col, w, 2, dtype=gpu.DTYPE_F32) as eng:
+        d = torch.empty((n, n), device="cuda")
+        p = torch.empty((n, n), dtype=torch.int32, device="cuda")
+        eng.solve(d, p)
+        sd, td = torch.from_numpy(s).cuda(), torch.from_numpy(t).cuda()
+        od, ol = torch.empty(nq, device="cuda"), torch.empty(nq, dtype=torch.int32, device="cuda")
+        fit = max(3, n // 2) if nq == 400 else 20
+        op = torch.full((nq, fit), -7, dtype=torch.int32, device="cuda")
+        dw = torch.zeros(len(edges), device="cuda")
+        torch.cuda.synchronize()
+        eng.query(d, p, sd, td, od, ol, op, fit)
+        eng.backward(p, sd, td, torch.ones(nq, device="cuda"), dw)
+        want = np.zeros(len(edges))
+        index = {e: i for i, e in enumerate(edges)}
+        diff = {1: np.zeros(n), -1: np.zeros(n)}
+        paths = op.cpu().numpy()
+        assert np.array_equal(ol.cpu().numpy(), hops + 1)
+        for q in range(nq):
+            if hops[q] > 0:  # the edges that the walk crosses
+                step = 1 if t[q] > s[q] else -1
+                diff[step][min(s[q], t[q])] += 1
+                diff[step][max(s[q], t[q])] -= 1
+        sums = {step: np.cumsum(diff[step]) for step in diff}
+        for (u, v), i in index.items():
+            want[i] = sums[v - u][min(u, v)]
+        for q in range(400):
+            step = 1 if t[q] > s[q] else -1
+            path = [int(s[q]) + step * i for i in range(hops[q] + 1)]
+            wrote = len(path) if len(path) <= fit else 0
+            assert list(paths[q, :wrote]) == path[:wrote] and (paths[q, wrote:] == -7).all()
+        assert np.array_equal(dw.cpu().numpy(), want)
+        row = int(np.flatnonzero(eng.mapping() == 0)[0])
+        for u, bad in ((k // 2, k // 2), (k // 2, n), (k // 2, -1)):  # a cycle, a bad vertex, an end
+            q = p.clone()
+            q[row, u] = bad
+            torch.cuda.synchronize()
+            with pytest.raises(gpu.FapError):
+                eng.query(d, q, sd[:1], td[:1], od[:1], ol[:1], None, 0)
+            if bad != -1:
+                with pytest.raises(gpu.FapError):
+                    eng.backward(q, sd[:1], td[:1], torch.ones(1, device="cuda"), dw)
+        eng.query(d, p, sd, td, od, ol, None, 0)  # still usable
+        assert np.array_equal(ol.cpu().numpy(), hops + 1)
