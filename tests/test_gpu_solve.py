@@ -284,3 +284,27 @@ def test_set_partition_matches_a_fresh_engine(gpu):
         d2, p2 = d2.cpu(), p2.cpu()
     for d, p in outs:
         assert torch.equal(d, d2) and torch.equal(p, p2)
+
+
+@pytest.mark.parametrize("n", [700, 1501, 3001])
+def test_solve_into_fresh_host_arrays(gpu, n):
+    """Host results whose pages are brought in beside the solve (none, one and
+    both arrays' worth of them) equal the device results, written over what the
+    arrays held."""
+    from fastapsp_gb300 import graphs
+
+    g = graphs.road_like(n, seed=n)
+    with gpu.Engine(n, g.row_offset, g.col_val, g.weight, max(2, n // 700), dtype=gpu.DTYPE_F32) as eng:
+        d, p = torch.empty((n, n), device="cuda"), torch.empty((n, n), dtype=torch.int32, device="cuda")
+        eng.solve(d, p, 0)
+        torch.cuda.synchronize()
+        for fresh in (True, False):
+            hd = np.empty(n * n + 3, np.float32) if fresh else np.full(n * n + 3, 7, np.float32)
+            hp = np.empty(n * n + 3, np.int32) if fresh else np.full(n * n + 3, 7, np.int32)
+            hd[[0, 1, -1]], hp[[0, 1, -1]] = 5, 5  # outside the rows
+            eng.solve(hd[2:-1].reshape(n, n), hp[2:-1].reshape(n, n), 0)
+            assert np.array_equal(hd[2:-1].reshape(n, n), d.cpu().numpy())
+            assert np.array_equal(hp[2:-1].reshape(n, n), p.cpu().numpy())
+            assert (hd[[0, 1, -1]] == 5).all() and (hp[[0, 1, -1]] == 5).all()
+            eng.solve(hd[2:-1].reshape(n, n), None, 0)
+            assert np.array_equal(hd[2:-1].reshape(n, n), d.cpu().numpy())
