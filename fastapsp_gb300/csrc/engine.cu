@@ -747,8 +747,8 @@ int build_plan(fap_engine *e, Plan &pl) {
       G.mp_strip_k = std::max(G.mp_strip_k, s.K);
     }
     const int nstrip = G.mp_strip_nseg = (int)mps.size();
-    auto *number = G.mp_rows ? fapk::number_minplus_rows : fapk::number_minplus_strips;
-    G.mp_strips = number(mps.data(), nstrip, e->sm_count, &G.mp_strip_per);
+    G.mp_strips = G.mp_rows ? fapk::number_minplus_rows(mps.data(), nstrip, e->sm_count, &G.mp_strip_per)
+                            : fapk::number_minplus_strips(e->f32(), mps.data(), nstrip, e->sm_count, &G.mp_strip_per);
     mps.insert(mps.end(), mps_deep.begin(), mps_deep.end());
     G.mp_strip_tiles = fapk::number_minplus_deep(mps.data(), nstrip, 0);
     G.mp_nseg = (int)mps.size();
@@ -2162,7 +2162,8 @@ int fap_minplus(fap_engine *e, int32_t dtype, int32_t M, int32_t N, int32_t K, c
   const int tiles = fapk::number_minplus_deep(&s, 1, 0);
   int rc, per = 1;
   const bool i32 = dtype == FAP_DTYPE_I32, by_rows = i32 && !rows_aligned16(s);
-  const int strips = (by_rows ? fapk::number_minplus_rows : fapk::number_minplus_strips)(&s, 1, e->sm_count, &per);
+  const int strips = by_rows ? fapk::number_minplus_rows(&s, 1, e->sm_count, &per)
+                             : fapk::number_minplus_strips(!i32, &s, 1, e->sm_count, &per);
   TableBuilder tb;
   size_t o_seg = tb.add(&s, 1);
   fapk::MatRef refs[2] = {{A, lda, M, K}, {B, ldb, K, N}};

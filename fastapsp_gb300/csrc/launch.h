@@ -26,7 +26,7 @@ cudaError_t launch_minplus_strips(bool f32, bool pred, const MpSegment *d_segs, 
                                   int per, cudaStream_t st);
 // Numbers the CTAs of one strip launch (returns their count) and chooses the
 // 128-column tiles each takes (launch_minplus_strips' per).
-int number_minplus_strips(MpSegment *segs, int nseg, int sm_count, int *per);
+int number_minplus_strips(bool f32, MpSegment *segs, int nseg, int sm_count, int *per);
 int minplus_strip_max_k(bool f32);   // largest K of the strip form
 // mp_rows.cu: the packed strip form for result rows that do not start on 16-byte
 // boundaries; same preconditions (B's predecessors' leading dimension below 2^24

@@ -273,7 +273,7 @@ __device__ __forceinline__ void tile_wide(MpSmem &sm, const MpSegment &s, const 
 // Strip form of the packed min-plus for products that do not accumulate into
 // C (the inner rows of every part) with K <= kStripMaxK.  One CTA owns a
 // strip: one 128-row tile of a segment and the 64-column tiles of up to
-// kStripTiles x 128 consecutive columns.  A's 128 x K block is staged once
+// 16 x 128 consecutive columns.  A's 128 x K block is staged once
 // per strip (transposed, so that a thread's 8 row operands of one k are two
 // 16-byte loads); B's K x TN tiles are double-buffered, so the next tile's
 // copy is in flight while the current one is multiplied; B's predecessor
@@ -297,7 +297,6 @@ __device__ __forceinline__ void tile_wide(MpSmem &sm, const MpSegment &s, const 
 // outputs, summed over tiles)], summed per CTA.
 __device__ unsigned long long g_strip_counters[3];
 
-constexpr int kStripTiles = 16;  // a strip spans at most kStripTiles x 128 columns 
 constexpr int kStripCols = 64;   // columns of a tile
 // Largest K of the strip form.  128 x 64 tiles with 8 x 4 outputs a thread,
 // three CTAs per SM: on sparse products most of a tile's time is its fixed work
@@ -1121,27 +1120,8 @@ namespace {
 int strips_of(const MpSegment &s, int per) { return (s.M + kTile - 1) / kTile * ((s.tiles_x + per - 1) / per); }
 }  // namespace
 
-// The strip length: the longest (it amortises the staging of A) that still
-// gives the launch a CTA for every slot of the GPU (three per SM at most).  A
-// 910-vertex part of a 24,575-vertex road graph has 84 strips of 2,048 columns
-// (207 us) and 588 of 256 (119 us); four parts of 576 vertices 4 and 20 (80 and
-// 27 us).
-int number_minplus_strips(MpSegment *segs, int nseg, int sm_count, int *per) {
-  *per = 1;
-  for (int tiles = kStripTiles; tiles > 1; tiles /= 2) {
-    long long strips = 0;
-    for (int i = 0; i < nseg; i++) strips += strips_of(segs[i], tiles);
-    if (strips >= 3LL * sm_count) {
-      *per = tiles;
-      break;
-    }
-  }
-  int strips = 0;
-  for (int i = 0; i < nseg; i++) {
-    segs[i].strip_begin = strips;
-    strips += strips_of(segs[i], *per);
-  }
-  return strips;
+int number_minplus_strips(bool f32, MpSegment *segs, int nseg, int sm_count, int *per) {
+  return number_strips(segs, nseg, sm_count, f32 ? 2 : 3, per, strips_of);
 }
 
 int minplus_strip_max_k(bool f32) { return f32 ? kStripMaxKF32 : kStripMaxK; }

@@ -352,23 +352,8 @@ int strips_of(const MpSegment &s, int per) {
 
 }  // namespace
 
-// The strip length, as in number_minplus_strips (minplus.cu).
 int number_minplus_rows(MpSegment *segs, int nseg, int sm_count, int *per) {
-  *per = 1;
-  for (int units = 16; units > 1; units /= 2) {
-    long long strips = 0;
-    for (int i = 0; i < nseg; i++) strips += strips_of(segs[i], units);
-    if (strips >= 3LL * sm_count) {
-      *per = units;
-      break;
-    }
-  }
-  int strips = 0;
-  for (int i = 0; i < nseg; i++) {
-    segs[i].strip_begin = strips;
-    strips += strips_of(segs[i], *per);
-  }
-  return strips;
+  return number_strips(segs, nseg, sm_count, 3, per, strips_of);
 }
 
 cudaError_t launch_minplus_rows(bool pred, const MpSegment *d_segs, int nseg, int strips, int max_k, int per,
