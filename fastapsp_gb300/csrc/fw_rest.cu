@@ -52,9 +52,19 @@ namespace {
 constexpr int kRestThreads = 256;
 constexpr int kRows = 128;  // tile rows: two blocks of the row list
 
+// FP32: A and B in 16-byte units of the four steps of a group of a row or a
+// column, unit (g, m) of A at g * kAUnits + m, (g, j) of B at g * kBlk + j: the
+// adds go in pairs (six instructions a group instead of eight), and the look-up
+// of an improved entry's step is two loads instead of six.  256 matrices of 256 to
+// 1,024: 15.45 -> 15.21 ms; a road-like graph's 64 matrices of 895: 5.83 -> 5.67.
+// (A's extra row is FP32's alone: with it the packed form's three CTAs ask for
+// the next larger shared memory, and the smaller L1 costs 8 %.)
+constexpr int kAUnits = kRows + 1;  // (odd: the stores of a row's groups hit different banks)
+
+template <bool F32>
 struct RestSmem {
-  unsigned A[kBlk][kRows];    // step k: keys (FP32: values) of the strip's rows, row m at m ^ swz(k)
-  unsigned B[kBlk][kBlk];     // step k: of the tile's columns, column j at 4 (j % 16) + j / 16 (FP32: that ^ swz(k))
+  unsigned A[F32 ? kBlk + 1 : kBlk][kRows];  // step k: keys of the strip's rows, row m at m ^ swz(k)
+  unsigned B[kBlk][kBlk];     // step k: of the tile's columns, column j at 4 (j % 16) + j / 16
   unsigned next[kBlk][kBlk];  // the next tile's values as they are in memory
 };
 
@@ -91,7 +101,7 @@ template <bool F32, bool PRED>
 __global__ void __launch_bounds__(kRestThreads, F32 ? 2 : 3)
     fw_rest_kernel(const FwRestJob *__restrict__ jobs, int njobs, int per) {
   extern __shared__ __align__(16) unsigned char rest_smem[];
-  RestSmem &sm = *reinterpret_cast<RestSmem *>(rest_smem);
+  RestSmem<F32> &sm = *reinterpret_cast<RestSmem<F32> *>(rest_smem);
   __shared__ FwRestJob s;
   __shared__ unsigned s_amask[2];     // steps with a finite entry in the strip's rows
   __shared__ unsigned s_bmask[2][2];  // ... and in the tile's columns (per tile parity)
@@ -164,8 +174,10 @@ __global__ void __launch_bounds__(kRestThreads, F32 ? 2 : 3)
 #pragma unroll
         for (int q = 0; q < 4; q++) {
           nib |= v[i][q] < FIN ? 1u << q : 0u;
-          sm.A[k + q][m ^ swz<true>(k)] = F32 ? v[i][q] : min(v[i][q], kPackH) << kIdxBits;
+          if (!F32) sm.A[k + q][m ^ swz<true>(k)] = min(v[i][q], kPackH) << kIdxBits;
         }
+        if (F32)
+          reinterpret_cast<uint4 *>(&sm.A[0][0])[tx * kAUnits + m] = make_uint4(v[i][0], v[i][1], v[i][2], v[i][3]);
       }
     }
     const unsigned lo = __reduce_or_sync(0xffffffffu, tx < 8 ? nib << (4 * tx) : 0u);
@@ -182,7 +194,16 @@ __global__ void __launch_bounds__(kRestThreads, F32 ? 2 : 3)
     asm volatile("cp.async.wait_group 0;\n" ::);
     __syncthreads();  // the tile's values are here; every thread is done with the last tile's keys and mask
     if (t < 2) s_bmask[par ^ 1][t] = 0u;
-    {  // values to keys; the rows with a finite entry
+    if constexpr (F32) {  // values to units; the groups with a finite entry
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int g = (t >> 6) + 4 * i, j = t & 63;
+        const uint4 v = make_uint4(sm.next[4 * g][j], sm.next[4 * g + 1][j], sm.next[4 * g + 2][j], sm.next[4 * g + 3][j]);
+        reinterpret_cast<uint4 *>(&sm.B[0][0])[g * kBlk + j] = v;
+        if (__any_sync(0xffffffffu, min(min(v.x, v.y), min(v.z, v.w)) < FIN) && (t & 31) == 0)
+          atomicOr(&s_bmask[par][g >> 3], 15u << (4 * (g & 7)));
+      }
+    } else {  // values to keys; the rows with a finite entry
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         unsigned bits = 0;
@@ -191,14 +212,12 @@ __global__ void __launch_bounds__(kRestThreads, F32 ? 2 : 3)
           const int kk = ty + 16 * (2 * h + i);
           uint4 v = make_uint4(sm.next[kk][tx], sm.next[kk][tx + 16], sm.next[kk][tx + 32], sm.next[kk][tx + 48]);
           const bool fin = min(min(v.x, v.y), min(v.z, v.w)) < FIN;
-          if (!F32) {
-            const unsigned id = (unsigned)kk + 1u;
-            v.x = (min(v.x, kPackH) << kIdxBits) | id;
-            v.y = (min(v.y, kPackH) << kIdxBits) | id;
-            v.z = (min(v.z, kPackH) << kIdxBits) | id;
-            v.w = (min(v.w, kPackH) << kIdxBits) | id;
-          }
-          *reinterpret_cast<uint4 *>(&sm.B[kk][(tx * 4) ^ swz<F32>(kk)]) = v;
+          const unsigned id = (unsigned)kk + 1u;
+          v.x = (min(v.x, kPackH) << kIdxBits) | id;
+          v.y = (min(v.y, kPackH) << kIdxBits) | id;
+          v.z = (min(v.z, kPackH) << kIdxBits) | id;
+          v.w = (min(v.w, kPackH) << kIdxBits) | id;
+          *reinterpret_cast<uint4 *>(&sm.B[kk][tx * 4]) = v;
           const unsigned bal = __ballot_sync(0xffffffffu, fin);  // rows kk of the warp's two ty
           bits |= (((bal & 0xffffu) ? 1u : 0u) | ((bal >> 16) ? 2u : 0u)) << (16 * i);
         }
@@ -231,27 +250,20 @@ __global__ void __launch_bounds__(kRestThreads, F32 ? 2 : 3)
       for (int k = 0; k < kBlk; k += 4) {
         if (!((unsigned)(msk >> k) & 15u)) continue;
         n_work += (two ? kRows : kBlk) * kBlk * 4;
-        const unsigned *ap = &sm.A[k][(ty * 4) ^ swz<true>(k)];
-        const unsigned *bp = &sm.B[k][(tx * 4) ^ swz<true>(k)];
-        unsigned b[4][4];  // [column][step]
+        const ulonglong2 *ap = reinterpret_cast<const ulonglong2 *>(&sm.A[0][0]) + (k >> 2) * kAUnits + ty * 4;
+        const ulonglong2 *bp = reinterpret_cast<const ulonglong2 *>(&sm.B[0][0]) + (k >> 2) * kBlk + tx;
+        ulonglong2 b[4];
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const uint4 v = *reinterpret_cast<const uint4 *>(bp + j * kBlk);
-          b[0][j] = v.x, b[1][j] = v.y, b[2][j] = v.z, b[3][j] = v.w;
-        }
+        for (int c = 0; c < 4; c++) b[c] = bp[16 * c];
 #pragma unroll
         for (int h = 0; h < 2; h++) {
           if (h == 1 && !two) break;
-          unsigned a[4][4];  // [row of the half][step]
 #pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const uint4 v = *reinterpret_cast<const uint4 *>(ap + j * kRows + h * kBlk);
-            a[0][j] = v.x, a[1][j] = v.y, a[2][j] = v.z, a[3][j] = v.w;
+          for (int i = 0; i < 4; i++) {
+            const ulonglong2 a = ap[h * kBlk + i];
+#pragma unroll
+            for (int c = 0; c < 4; c++) unit_addmin_f32(acc[h * 4 + i][c], arg[h * 4 + i][c], a, b[c], k + 1);
           }
-#pragma unroll
-          for (int i = 0; i < 4; i++)
-#pragma unroll
-            for (int c = 0; c < 4; c++) strip_addmin4_f32(acc[h * 4 + i][c], arg[h * 4 + i][c], a[i], b[c], k + 1);
         }
       }
     } else {
@@ -326,10 +338,12 @@ __global__ void __launch_bounds__(kRestThreads, F32 ? 2 : 3)
           k[q] = 0;
           if constexpr (F32) {
             if (v < c[i][q]) {
-              const int k0 = max(arg[h * 4 + i][q] - 1, 0), sw = swz<true>(k0);
+              const int g = max(arg[h * 4 + i][q] - 1, 0) >> 2;
               // (no step: a value above "unreached" that none reaches)
-              k[q] = PRED ? (unsigned)strip_resolve_f32(v, arg[h * 4 + i][q], &sm.A[k0][(ty * 4) ^ sw] + h * kBlk + i,
-                                                        kRows, &sm.B[k0][(tx * 4) ^ sw] + q, kBlk)
+              k[q] = PRED ? (unsigned)unit_resolve_f32(
+                                v, arg[h * 4 + i][q],
+                                reinterpret_cast<const ulonglong2 *>(&sm.A[0][0])[g * kAUnits + ty * 4 + h * kBlk + i],
+                                reinterpret_cast<const ulonglong2 *>(&sm.B[0][0])[g * kBlk + tx + 16 * q])
                           : (unsigned)arg[h * 4 + i][q];
             }
           } else {
@@ -365,7 +379,7 @@ __global__ void __launch_bounds__(kRestThreads, F32 ? 2 : 3)
 template <bool F32, bool PRED>
 cudaError_t launch_rest(const FwRestJob *d_jobs, int njobs, int strips, int per, cudaStream_t st) {
   ++launch_count();
-  fw_rest_kernel<F32, PRED><<<strips, kRestThreads, sizeof(RestSmem), st>>>(d_jobs, njobs, per);
+  fw_rest_kernel<F32, PRED><<<strips, kRestThreads, sizeof(RestSmem<F32>), st>>>(d_jobs, njobs, per);
   return cudaGetLastError();
 }
 
@@ -420,7 +434,7 @@ cudaError_t init_fw_rest_kernels() {
   cudaError_t e;
 #define FAP_REST_ATTR(F, P)                                                                           \
   if ((e = cudaFuncSetAttribute(fw_rest_kernel<F, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                (int)sizeof(RestSmem))) != cudaSuccess)                               \
+                                (int)sizeof(RestSmem<F>))) != cudaSuccess)                            \
     return e;
   FAP_REST_ATTR(true, true)
   FAP_REST_ATTR(true, false)

@@ -56,6 +56,29 @@ __device__ __forceinline__ void strip_addmin4_f32(unsigned &acc, int &tag, const
   acc = nacc;
 }
 
+// Two FP32 sums (steps k and k + 1) of operands held as pairs; their bits.
+__device__ __forceinline__ uint2 add2_f32(unsigned long long a, unsigned long long b) {
+  unsigned long long z;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(z) : "l"(a), "l"(b));
+  return make_uint2((unsigned)z, (unsigned)(z >> 32));
+}
+
+// strip_addmin4_f32 on units of four steps: two paired adds instead of four.
+__device__ __forceinline__ void unit_addmin_f32(unsigned &acc, int &tag, const ulonglong2 &a, const ulonglong2 &b,
+                                                int grp) {
+  const uint2 v = add2_f32(a.x, b.x), w = add2_f32(a.y, b.y);
+  const unsigned nacc = __vimin3_u32(acc, __vimin3_u32(v.x, v.y, w.x), w.y);
+  tag = nacc != acc ? grp : tag;
+  acc = nacc;
+}
+
+// strip_resolve_f32 on the units of the tagged group.
+__device__ __forceinline__ int unit_resolve_f32(unsigned acc, int tag, const ulonglong2 &a, const ulonglong2 &b) {
+  const uint2 v = add2_f32(a.x, b.x), w = add2_f32(a.y, b.y);
+  const int j = v.x == acc ? 0 : v.y == acc ? 1 : w.x == acc ? 2 : 3;
+  return tag > 0 ? tag + j : 0;
+}
+
 // The step idx (k + 1) of an output whose last strict improvement fell in the
 // group tagged `tag` (0: none): the group's first step whose sum has the
 // final value's bits.  ap / bp point at the output's A and B entries of the
