@@ -317,8 +317,8 @@ def run_solve(args, name, rank, world, local_rank):
     sssp_bytes = srcs * (4 * (n + 1) + 8 * g.m + 8 * n)
     mp_bytes = int(((subs - bdys) * n * 8).sum() + (bdys * n * 8).sum())  # C written + B read once
     mp_gbs = rate(mp_bytes, ph["min_plus"]) / 1e9
-    # add-min steps the strip kernels actually ran (they skip the k-steps whose
-    # B row or A column is unreached over a tile): one more solve with counters
+    # add-min steps the min-plus and FW kernels actually ran (they skip the k-steps
+    # whose B row or A column is unreached over a tile): one more solve with counters
     eng.minplus_counters(reset=True)
     eng.fw_counters(reset=True)
     step()
@@ -433,7 +433,8 @@ def run_solve(args, name, rank, world, local_rank):
             # add-min work is data-dependent: steps that cannot change a tile
             # are skipped), so its roofline is HBM; alu_view gives the same
             # launch against the add-min issue rate of its arithmetic.
-            "kernel": "mp_strip_kernel (min-plus of the inner rows and decode of their own-part columns)",
+            "kernel": "mp_strip_kernel, mp_rows_kernel, mp_deep_kernel (min-plus of the inner rows and decode of "
+                      "their own-part columns)",
             "bound": "hbm",
             "achieved": mp_gbs, "peak": hbm, "unit": "GB/s", "frac": mp_gbs / hbm,
             "peak_source": peak_src,

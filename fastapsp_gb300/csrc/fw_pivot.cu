@@ -5,8 +5,8 @@
 // fap/kernel/cuda/floyd.cu:26-267).
 //
 // Round r of the blocked form closes the pivot block (r, r) and updates block
-// row and column r with it (the panels); the remaining tiles follow on the
-// strip kernel (minplus.cu), except block row and column r + 1, which get
+// row and column r with it (the panels); the remaining tiles follow in
+// fw_rest.cu, except block row and column r + 1, which get
 // round r's update here, at the start of round r + 1, so that they need not
 // wait for the other tiles (lookahead).  Two launches a round over all the
 // matrices of a batch:
@@ -50,7 +50,8 @@ constexpr int kPivC = 2;
 
 // Operands of a 64^3 product in shared memory.  A by step: entry (k, row) at
 // k * 64 + (row ^ swz(k)); B the same with columns (the packed form's B
-// unswizzled): a thread's four rows or two columns of a step are one chunk, and A's transposing stores and the FP32 resolve hit different banks.
+// unswizzled): a thread's four rows or two columns of a step are one chunk, and
+// A's transposing stores and the FP32 resolve hit different banks.
 
 // A block as a thread holds it: rows 4 ty + i, columns 2 tx + c.
 template <typename V>

@@ -43,12 +43,14 @@ cudaError_t init_mp_rows_kernels();
 int number_minplus_deep(MpSegment *segs, int nseg, int first);
 cudaError_t launch_minplus_deep(bool f32, bool packed, bool pred, const MpSegment *d_segs, int nseg, int tiles,
                                 int tile0, cudaStream_t st);
+cudaError_t deep_counters(unsigned long long out[3], bool reset);
 cudaError_t init_mp_deep_kernels();
 // Largest finite int32 entry of each matrix, atomicMax-ed into out[its index * step].
 cudaError_t launch_max_finite(const MatRef *d_mats, int nmats, unsigned *out, int step, cudaStream_t st);
 unsigned pack_limit();
-// Work counters of the strip min-plus on the current device: [tiles, tiles
-// with no active step, active steps over all tiles]; optionally reset.
+// Work counters of the min-plus kernels on the current device: [tiles, tiles
+// with no active step, add-mins executed (active steps x the tile's outputs)];
+// optionally reset.
 cudaError_t strip_counters(unsigned long long out[3], bool reset);
 // Wide int32 form: closes each job's pivot block.
 cudaError_t launch_fw_diag(bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st);

@@ -1138,10 +1138,11 @@ unsigned pack_limit() { return kPackH; }
 
 cudaError_t strip_counters(unsigned long long out[3], bool reset) {
   cudaError_t e = rows_counters(out, reset);
-  unsigned long long strip[3];
+  unsigned long long strip[3], deep[3];
+  if (e == cudaSuccess) e = deep_counters(deep, reset);
   if (e == cudaSuccess) e = cudaMemcpyFromSymbol(strip, g_strip_counters, sizeof(strip));
   if (e != cudaSuccess) return e;
-  for (int i = 0; i < 3; i++) out[i] += strip[i];
+  for (int i = 0; i < 3; i++) out[i] += strip[i] + deep[i];
   if (!reset) return e;
   const unsigned long long zero[3] = {0, 0, 0};
   return cudaMemcpyToSymbol(g_strip_counters, zero, sizeof(zero));

@@ -62,6 +62,9 @@ struct DeepChunk {
   unsigned B[kDeepK][kDeepTile];  // columns permuted by swz: lookups of different steps hit different banks
 };
 
+// Work counters as mp_strip_kernel's (minplus.cu).
+__device__ unsigned long long g_deep_counters[3];
+
 template <DeepForm FORM>
 __device__ __forceinline__ unsigned deep_add(unsigned a, unsigned b) {
   return FORM == kDeepF32 ? __float_as_uint(__fadd_rn(__uint_as_float(a), __uint_as_float(b))) : a + b;
@@ -174,6 +177,7 @@ __global__ void __launch_bounds__(kDeepThreads, 3)
       arg[i][c] = 0;
     }
   const int nchunks = (K + kDeepK - 1) / kDeepK;
+  int n_groups = 0;  // groups of four steps run
   if (nchunks > 0) load(0, 0);
   cp_async_commit();
   for (int ch = 0; ch < nchunks; ch++) {
@@ -187,6 +191,7 @@ __global__ void __launch_bounds__(kDeepThreads, 3)
     cp_async_commit();
     if (!work) continue;  // columns that nothing reaches (unconnected parts)
     const int ng = (min(kDeepK, K - k0) + 3) >> 2;
+    n_groups += ng;
 #pragma unroll 1
     for (int g = 0; g < ng; g++) {
       uint4 a[4], b[4];
@@ -242,6 +247,12 @@ __global__ void __launch_bounds__(kDeepThreads, 3)
 #pragma unroll
       for (int c = 0; c < 4; c++)
         arg[i][c] = arg[i][c] && col0 + tx * 4 + c < N ? bp[(arg[i][c] - 1) * ldbp + c] : -1;
+  }
+
+  if (t == 0) {
+    atomicAdd(&g_deep_counters[0], 1ull);
+    if (n_groups == 0) atomicAdd(&g_deep_counters[1], 1ull);
+    atomicAdd(&g_deep_counters[2], (unsigned long long)n_groups * 4 * kDeepTile * kDeepTile);
   }
 
   const bool own = s.col_part != nullptr, full = col0 + kDeepTile <= N;  // (uniform over the CTA)
@@ -325,6 +336,13 @@ cudaError_t launch_minplus_deep(bool f32, bool packed, bool pred, const MpSegmen
                           : launch_deep_t<kDeepPacked, false>(d_segs, nseg, tiles, tile0, st);
   return pred ? launch_deep_t<kDeepWide, true>(d_segs, nseg, tiles, tile0, st)
               : launch_deep_t<kDeepWide, false>(d_segs, nseg, tiles, tile0, st);
+}
+
+cudaError_t deep_counters(unsigned long long out[3], bool reset) {
+  cudaError_t e = cudaMemcpyFromSymbol(out, g_deep_counters, sizeof(unsigned long long) * 3);
+  if (e != cudaSuccess || !reset) return e;
+  const unsigned long long zero[3] = {0, 0, 0};
+  return cudaMemcpyToSymbol(g_deep_counters, zero, sizeof(zero));
 }
 
 cudaError_t init_mp_deep_kernels() {

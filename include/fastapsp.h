@@ -25,9 +25,10 @@
  *    of the engine's GPU; the engine detects which.  Streams are passed as
  *    `void *` (a cudaStream_t) so that this header needs no CUDA headers;
  *    NULL means the engine's own stream.  Work issued on a caller's stream
- *    is ordered on that stream: the Floyd-Warshall phase of the packed int32
- *    form forks part of its launches to an internal stream of the engine
- *    and joins it back on the caller's stream before the next phase.
+ *    is ordered on that stream: the Floyd-Warshall phase (packed int32 and
+ *    FP32) and the min-plus fork part of their launches to internal streams
+ *    of the engine and join them back on the caller's stream before the next
+ *    phase.
  */
 #ifndef FASTAPSP_H_
 #define FASTAPSP_H_
@@ -271,11 +272,11 @@ int fap_last_times(const fap_engine *e, double *times5);
 /* Number of kernels the last solve launched (no reference counterpart; the
  * bench reports it as the GPU launch count of a step). */
 int fap_last_launches(const fap_engine *e, int64_t *count);
-/* Work counters of the min-plus strip kernel on the engine's GPU since the
- * last reset (no reference counterpart; diagnostics of the sparsity skip):
- * [tiles, tiles with no active k-step, add-mins executed: active k-steps x
- * the tile's outputs (128 x 64 or 128 x 128), summed over tiles].  reset != 0
- * clears them after reading. */
+/* Work counters of the min-plus kernels on the engine's GPU since the last
+ * reset (no reference counterpart; diagnostics of the sparsity skip):
+ * [tiles, tiles with no active k-step, add-mins executed: k-steps run x the
+ * tile's outputs (128 x 64, and 64 x 64 for parts of many boundary vertices),
+ * summed over tiles].  reset != 0 clears them after reading. */
 int fap_minplus_counters(fap_engine *e, uint64_t *out3, int32_t reset);
 /* Floyd-Warshall work of the solves since the last reset (no reference
  * counterpart; the executed-work view of the FW roofline): [add-mins the
