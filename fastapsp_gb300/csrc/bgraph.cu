@@ -9,12 +9,12 @@
 //   1. local rows: for every part q and every boundary vertex b of q, the
 //      distances from b to the vertices of q along edges inside q
 //      (L_q[b][v]; bdy_q x sub_q per part), by a frontier Bellman-Ford in
-//      shared memory, one CTA per (part, 8 sources);
+//      shared memory, one CTA per (part, 8 or 4 sources);
 //   2. boundary graph: its nodes are all boundary vertices, its edges the
 //      cut edges (both ends are boundary vertices by the definition of
 //      findBoundry, fap/utils/util_preprocess.h:32-58) and, inside every
 //      part, b -> b' with weight L_q[b][b'].  A frontier Bellman-Ford in
-//      shared memory per 8 sources gives D_S[s][t] for all boundary s, t;
+//      shared memory per 8 or 4 sources gives D_S[s][t] for all boundary s, t;
 //   3. rows: for v in part q, D[s][v] = min over boundary b of q of
 //      D_S[s][b] + L_q[b][v] -- a min-plus per (source batch, part).
 //
@@ -51,8 +51,7 @@ namespace {
 
 constexpr int kBgThreads = 512;
 constexpr int kBgWarps = kBgThreads / 32;
-constexpr int kBgLanes = 8;          // sources per CTA in steps 1 and 2
-constexpr int kBgGroups = 32 / kBgLanes;  // frontier nodes a warp relaxes at once
+constexpr int kBgLanes = 8;               // sources of a CTA in steps 1 and 2, or half as many (bg_lanes)
 constexpr int kBgEdges = 8;               // edges of a node whose loads are in flight together
 constexpr int kRowThreads = 256;     // step 3
 constexpr int kRowTA = 32;           // boundary vertices per step-3 chunk
@@ -67,15 +66,15 @@ __device__ __forceinline__ bool bg_set_bit(unsigned *bits, int v) {
   return (atomicOr(&bits[v >> 5], m) & m) == 0u;
 }
 
-// Shared-memory layout of steps 1 and 2 for N nodes: d[N][kBgLanes] (V) |
+// Shared-memory layout of steps 1 and 2 for N nodes: d[N][lanes] (V) |
 // list[2][N] | bits[2][words].
 template <typename V>
-__host__ __device__ inline size_t bg_smem(int N) {
+__host__ __device__ inline size_t bg_smem(int N, int lanes) {
   const size_t words = (size_t)(N + 31) / 32;
-  return (size_t)N * kBgLanes * sizeof(V) + (size_t)2 * N * 4 + 2 * words * 4;
+  return (size_t)N * lanes * sizeof(V) + (size_t)2 * N * 4 + 2 * words * 4;
 }
 
-// Frontier Bellman-Ford over N nodes with kBgLanes sources at once, in
+// Frontier Bellman-Ford over N nodes with LANES sources at once, in
 // shared memory.  `relax(u, lane, du, push)` relaxes node u's out-edges for
 // one lane (du = that lane's distance of u) and calls push(v, improved) once
 // per edge in lockstep across the group's lanes.  The sources' own entries
@@ -90,14 +89,15 @@ __host__ __device__ inline size_t bg_smem(int N) {
 // road-like graph each node was relaxed about ten times).  The order of the
 // relaxations never changes the fixpoint the distances converge to.
 // Returns false at the round cap.
-template <typename V, typename Relax>
+template <int LANES, typename V, typename Relax>
 __device__ bool bg_bellman_ford(V *d, int *list0, unsigned *bits0, int N, int *s_cnt, V delta, Relax relax,
                                 unsigned long long &rounds, unsigned long long &visited) {
   __shared__ int s_done[2];                  // nodes relaxed in the round (by round parity)
   __shared__ unsigned long long s_defer[2];  // smallest deferred distance (by round parity)
+  constexpr int kGroups = 32 / LANES;  // frontier nodes a warp relaxes at once
   const int words = (N + 31) / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int grp = lane / kBgLanes, gl = lane % kBgLanes;
+  const int grp = lane / LANES, gl = lane % LANES;
   if (threadIdx.x < 2) {
     s_done[threadIdx.x] = 0;
     s_defer[threadIdx.x] = ~0ull;
@@ -117,13 +117,13 @@ __device__ bool bg_bellman_ford(V *d, int *list0, unsigned *bits0, int N, int *s
     const int *lcur = list0 + cur * N;
     int *lnxt = list0 + nxt * N;
     unsigned *bcur = bits0 + cur * words, *bnxt = bits0 + nxt * words;
-    for (int base = warp * kBgGroups; base < f; base += kBgWarps * kBgGroups) {
+    for (int base = warp * kGroups; base < f; base += kBgWarps * kGroups) {
       const int idx = base + grp;
       int u = idx < f ? lcur[idx] : -1;
-      V du = u >= 0 ? d[(size_t)u * kBgLanes + gl] : bg_inf<V>();
+      V du = u >= 0 ? d[(size_t)u * LANES + gl] : bg_inf<V>();
       V key = du;
 #pragma unroll
-      for (int o = 1; o < kBgLanes; o <<= 1) {
+      for (int o = 1; o < LANES; o <<= 1) {
         const V other = __shfl_xor_sync(0xffffffffu, key, o);
         key = other < key ? other : key;
       }
@@ -142,7 +142,7 @@ __device__ bool bg_bellman_ford(V *d, int *list0, unsigned *bits0, int N, int *s
       relax(u, gl, u >= 0 ? du : bg_inf<V>(), [&](int v, bool improved) {
         // one lane of the group files v when any lane improved it
         const unsigned bal = __ballot_sync(0xffffffffu, improved);
-        const unsigned gmask = ((1u << kBgLanes) - 1u) << (grp * kBgLanes);
+        const unsigned gmask = ((1u << LANES) - 1u) << (grp * LANES);
         if (gl == 0 && (bal & gmask) && bg_set_bit(bnxt, v)) lnxt[atomicAdd(&s_cnt[nxt], 1)] = v;
       });
     }
@@ -165,7 +165,7 @@ __device__ __forceinline__ bool bg_try(V *slot, V c) {
 }
 
 // Step 1: local rows.  Job = (part, first local boundary index, count).
-template <typename V>
+template <typename V, int LANES>
 __global__ void __launch_bounds__(kBgThreads) bg_local_kernel(BgArgs a) {
   extern __shared__ __align__(16) unsigned char bg_smem_raw[];
   __shared__ int s_cnt[2];
@@ -173,16 +173,16 @@ __global__ void __launch_bounds__(kBgThreads) bg_local_kernel(BgArgs a) {
   const BgPart q = a.parts[job.unit];
   const int N = q.sub;
   V *d = reinterpret_cast<V *>(bg_smem_raw);
-  int *list0 = reinterpret_cast<int *>(d + (size_t)N * kBgLanes);
+  int *list0 = reinterpret_cast<int *>(d + (size_t)N * LANES);
   unsigned *bits0 = reinterpret_cast<unsigned *>(list0 + 2 * N);
   const int words = (N + 31) / 32;
-  for (int i = threadIdx.x; i < N * kBgLanes; i += blockDim.x) d[i] = bg_inf<V>();
+  for (int i = threadIdx.x; i < N * LANES; i += blockDim.x) d[i] = bg_inf<V>();
   for (int i = threadIdx.x; i < 2 * words; i += blockDim.x) bits0[i] = 0u;
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
   __syncthreads();
   if (threadIdx.x < job.count) {
     const int s = job.first + threadIdx.x;  // local index of the source (boundary vertices come first)
-    d[(size_t)s * kBgLanes + threadIdx.x] = 0;
+    d[(size_t)s * LANES + threadIdx.x] = 0;
     bg_set_bit(bits0, s);
     list0[atomicAdd(&s_cnt[0], 1)] = s;
   }
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(kBgThreads) bg_local_kernel(BgArgs a) {
   const V *lw = static_cast<const V *>(a.lw);
   const int lane = threadIdx.x & 31;
   unsigned long long rounds = 0, visited = 0;
-  const bool ok = bg_bellman_ford<V>(
+  const bool ok = bg_bellman_ford<LANES, V>(
       d, list0, bits0, N, s_cnt, (V)a.delta_local,
       [&](int u, int gl, V du, auto push) {
         int e0 = 0, deg = 0;
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(kBgThreads) bg_local_kernel(BgArgs a) {
         }
         int dmax = deg;
 #pragma unroll
-        for (int o = kBgLanes; o < 32; o <<= 1) dmax = max(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+        for (int o = LANES; o < 32; o <<= 1) dmax = max(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
         // kBgEdges edges at a time: their loads issue together
         for (int t0 = 0; t0 < dmax; t0 += kBgEdges) {
           int v[kBgEdges];
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(kBgThreads) bg_local_kernel(BgArgs a) {
           for (int q = 0; q < kBgEdges; q++) {
             if (t0 + q >= dmax) break;  // uniform over the warp
             bool imp = false;
-            if (t0 + q < deg && du < bg_inf<V>()) imp = bg_try(&d[(size_t)v[q] * kBgLanes + gl], (V)(du + w[q]));
+            if (t0 + q < deg && du < bg_inf<V>()) imp = bg_try(&d[(size_t)v[q] * LANES + gl], (V)(du + w[q]));
             push(v[q], imp);
           }
         }
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kBgThreads) bg_local_kernel(BgArgs a) {
   V *L = static_cast<V *>(a.L) + q.loff;
   for (int i = threadIdx.x; i < job.count * N; i += blockDim.x) {
     const int l = i / N, v = i - l * N;
-    L[(size_t)(job.first + l) * N + v] = d[(size_t)v * kBgLanes + l];
+    L[(size_t)(job.first + l) * N + v] = d[(size_t)v * LANES + l];
   }
   if (threadIdx.x == 0 && a.stats) {
     atomicAdd(&a.stats[0], rounds);
@@ -238,17 +238,17 @@ __global__ void __launch_bounds__(kBgThreads) bg_local_kernel(BgArgs a) {
 
 // Step 2: boundary graph.  Job = (batch of the solve's SSSP sources, first
 // lane, count): sources are the boundary indices a.bsrc[batch][first + l].
-template <typename V>
+template <typename V, int LANES>
 __global__ void __launch_bounds__(kBgThreads) bg_boundary_kernel(BgArgs a) {
   extern __shared__ __align__(16) unsigned char bg_smem_raw[];
   __shared__ int s_cnt[2];
   const BgJob job = a.bjobs[blockIdx.x];
   const int N = a.B;
   V *d = reinterpret_cast<V *>(bg_smem_raw);
-  int *list0 = reinterpret_cast<int *>(d + (size_t)N * kBgLanes);
+  int *list0 = reinterpret_cast<int *>(d + (size_t)N * LANES);
   unsigned *bits0 = reinterpret_cast<unsigned *>(list0 + 2 * N);
   const int words = (N + 31) / 32;
-  for (int i = threadIdx.x; i < N * kBgLanes; i += blockDim.x) d[i] = bg_inf<V>();
+  for (int i = threadIdx.x; i < N * LANES; i += blockDim.x) d[i] = bg_inf<V>();
   for (int i = threadIdx.x; i < 2 * words; i += blockDim.x) bits0[i] = 0u;
   if (threadIdx.x < 2) s_cnt[threadIdx.x] = 0;
   __syncthreads();
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(kBgThreads) bg_boundary_kernel(BgArgs a) {
   if (threadIdx.x < job.count) {
     const int s = srcs[threadIdx.x];
     if (s >= 0 && s < N) {
-      d[(size_t)s * kBgLanes + threadIdx.x] = 0;
+      d[(size_t)s * LANES + threadIdx.x] = 0;
       if (bg_set_bit(bits0, s)) list0[atomicAdd(&s_cnt[0], 1)] = s;
     } else {
       atomicOr(a.status, kErrBadInput);
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(kBgThreads) bg_boundary_kernel(BgArgs a) {
   const V *L = static_cast<const V *>(a.L);
   const V *cw = static_cast<const V *>(a.cw);
   unsigned long long rounds = 0, visited = 0;
-  const bool ok = bg_bellman_ford<V>(
+  const bool ok = bg_bellman_ford<LANES, V>(
       d, list0, bits0, N, s_cnt, (V)a.delta_boundary,
       [&](int u, int gl, V du, auto push) {
         // the node's part-mates (row of its part's local rows), then its cut edges
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kBgThreads) bg_boundary_kernel(BgArgs a) {
         int tot = nb + ncut;
         int tmax = tot;
 #pragma unroll
-        for (int o = kBgLanes; o < 32; o <<= 1) tmax = max(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
+        for (int o = LANES; o < 32; o <<= 1) tmax = max(tmax, __shfl_xor_sync(0xffffffffu, tmax, o));
         const bool live = du < bg_inf<V>();
         // kBgEdges edges at a time: their loads issue together
         for (int t0 = 0; t0 < tmax; t0 += kBgEdges) {
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kBgThreads) bg_boundary_kernel(BgArgs a) {
             if (t0 + q >= tmax) break;  // uniform over the warp
             bool imp = false;
             if (live && t0 + q < tot && v[q] != u && w[q] < bg_inf<V>())
-              imp = bg_try(&d[(size_t)v[q] * kBgLanes + gl], (V)(du + w[q]));
+              imp = bg_try(&d[(size_t)v[q] * LANES + gl], (V)(du + w[q]));
             push(v[q], imp);
           }
         }
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kBgThreads) bg_boundary_kernel(BgArgs a) {
   for (int l = 0; l < job.count; l++) {
     const int s = srcs[l];
     if (s < 0 || s >= N) continue;
-    for (int v = threadIdx.x; v < N; v += blockDim.x) DS[(size_t)s * N + v] = d[(size_t)v * kBgLanes + l];
+    for (int v = threadIdx.x; v < N; v += blockDim.x) DS[(size_t)s * N + v] = d[(size_t)v * LANES + l];
   }
   if (threadIdx.x == 0 && a.stats) {
     atomicAdd(&a.stats[0], rounds);
@@ -419,12 +419,12 @@ __global__ void __launch_bounds__(kRowThreads) bg_rows_kernel(BgArgs a, BgRowArg
   }
 }
 
-template <typename V>
+template <typename V, int LANES>
 cudaError_t set_bg_attrs() {
-  cudaError_t e = cudaFuncSetAttribute(bg_local_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(bg_local_kernel<V, LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kBgSmemMax);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(bg_boundary_kernel<V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(bg_boundary_kernel<V, LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)kBgSmemMax);
 }
 
@@ -445,13 +445,25 @@ cudaError_t set_rows_attr() {
 }  // namespace
 
 size_t bg_smem_bytes(bool wide, int nodes) {
-  return wide ? bg_smem<unsigned long long>(nodes) : bg_smem<uint32_t>(nodes);
+  return wide ? bg_smem<unsigned long long>(nodes, kBgLanes) : bg_smem<uint32_t>(nodes, kBgLanes);
 }
-int bg_lanes() { return kBgLanes; }
+
+// The sources of a CTA: eight, whose relaxations of a node share its edges, or
+// four, which make twice the CTAs and half the table: where eight do not give
+// the GPU enough CTAs, and where their table leaves an SM one CTA.  SSSP phase
+// with eight and four, ms: road-like graphs of 8,000 vertices 0.60 / 0.48, 20,000
+// 0.92 / 0.77, 40,000 1.65 / 1.40 (960 boundary vertices), 80,000 5.54 / 5.14 (table),
+// 114,599 10.97 / 9.81 (table); geometric 20,000 0.44 / 0.40, 65,536 (1,848
+// boundary vertices) 1.35 / 1.37; near the line, road-like graphs of 57,301 with
+// 1,408 3.44 / 3.20, with fewer 2.57 / 2.70.
+int bg_lanes(bool wide, int nodes, int sm_count) {
+  return nodes <= 10 * sm_count || bg_smem_bytes(wide, nodes) > 113 * 1024 ? kBgLanes / 2 : kBgLanes;
+}
 
 cudaError_t init_bg_kernels() {
   cudaError_t e;
-  if ((e = set_bg_attrs<uint32_t>()) != cudaSuccess || (e = set_bg_attrs<unsigned long long>()) != cudaSuccess ||
+  if ((e = set_bg_attrs<uint32_t, 8>()) != cudaSuccess || (e = set_bg_attrs<unsigned long long, 8>()) != cudaSuccess ||
+      (e = set_bg_attrs<uint32_t, 4>()) != cudaSuccess || (e = set_bg_attrs<unsigned long long, 4>()) != cudaSuccess ||
       (e = set_rows_attr<unsigned long long, 16, true>()) != cudaSuccess ||
       (e = set_rows_attr<unsigned long long, 32, true>()) != cudaSuccess ||
       (e = set_rows_attr<uint32_t, 8, false>()) != cudaSuccess ||
@@ -461,27 +473,33 @@ cudaError_t init_bg_kernels() {
   return cudaSuccess;
 }
 
-cudaError_t launch_bg_local(bool wide, const BgArgs &a, int njobs, int max_sub, cudaStream_t st) {
+cudaError_t launch_bg_local(bool wide, int lanes, const BgArgs &a, int njobs, int max_sub, cudaStream_t st) {
   if (njobs <= 0) return cudaSuccess;
-  const size_t smem = bg_smem_bytes(wide, max_sub);
+  const size_t smem = wide ? bg_smem<unsigned long long>(max_sub, lanes) : bg_smem<uint32_t>(max_sub, lanes);
   if (smem > kBgSmemMax) return cudaErrorInvalidValue;
   ++launch_count();
-  if (wide)
-    bg_local_kernel<unsigned long long><<<njobs, kBgThreads, smem, st>>>(a);
-  else
-    bg_local_kernel<uint32_t><<<njobs, kBgThreads, smem, st>>>(a);
+  if (lanes == 4) {
+    if (wide) bg_local_kernel<unsigned long long, 4><<<njobs, kBgThreads, smem, st>>>(a);
+    else bg_local_kernel<uint32_t, 4><<<njobs, kBgThreads, smem, st>>>(a);
+  } else {
+    if (wide) bg_local_kernel<unsigned long long, 8><<<njobs, kBgThreads, smem, st>>>(a);
+    else bg_local_kernel<uint32_t, 8><<<njobs, kBgThreads, smem, st>>>(a);
+  }
   return cudaGetLastError();
 }
 
-cudaError_t launch_bg_boundary(bool wide, const BgArgs &a, int njobs, cudaStream_t st) {
+cudaError_t launch_bg_boundary(bool wide, int lanes, const BgArgs &a, int njobs, cudaStream_t st) {
   if (njobs <= 0) return cudaSuccess;
-  const size_t smem = bg_smem_bytes(wide, a.B);
+  const size_t smem = wide ? bg_smem<unsigned long long>(a.B, lanes) : bg_smem<uint32_t>(a.B, lanes);
   if (smem > kBgSmemMax) return cudaErrorInvalidValue;
   ++launch_count();
-  if (wide)
-    bg_boundary_kernel<unsigned long long><<<njobs, kBgThreads, smem, st>>>(a);
-  else
-    bg_boundary_kernel<uint32_t><<<njobs, kBgThreads, smem, st>>>(a);
+  if (lanes == 4) {
+    if (wide) bg_boundary_kernel<unsigned long long, 4><<<njobs, kBgThreads, smem, st>>>(a);
+    else bg_boundary_kernel<uint32_t, 4><<<njobs, kBgThreads, smem, st>>>(a);
+  } else {
+    if (wide) bg_boundary_kernel<unsigned long long, 8><<<njobs, kBgThreads, smem, st>>>(a);
+    else bg_boundary_kernel<uint32_t, 8><<<njobs, kBgThreads, smem, st>>>(a);
+  }
   return cudaGetLastError();
 }
 

@@ -236,6 +236,7 @@ struct fap_engine {
   bool bg_ready = false;
   bool bg_ok = false;      // usable: exact arithmetic and both shared-memory tables fit
   int bg_B = 0, bg_max_sub = 0, bg_nljobs = 0;
+  int bg_lanes = 8;        // sources per CTA of its kernels
   std::vector<int32_t> bg_bidx;  // vertex -> boundary index (-1: inner vertex)
   DevBuf bg_tab, bg_L, bg_DS;
   fapk::BgArgs bg_args{};
@@ -426,10 +427,11 @@ int prepare_bgraph(fap_engine *e) {
     for (int32_t u = 0; u < n; u++)
       for (int32_t j = e->ro[u]; j < e->ro[u + 1]; j++) iwfix[fill[e->col[j]]++] = weight(j);
   }
+  e->bg_lanes = fapk::bg_lanes(wide, B, e->sm_count);
   std::vector<fapk::BgJob> ljobs;
   for (int q = 0; q < K; q++)
-    for (int a0 = 0; a0 < parts[q].bdy; a0 += fapk::bg_lanes())
-      ljobs.push_back({q, a0, std::min(fapk::bg_lanes(), parts[q].bdy - a0)});
+    for (int a0 = 0; a0 < parts[q].bdy; a0 += e->bg_lanes)
+      ljobs.push_back({q, a0, std::min(e->bg_lanes, parts[q].bdy - a0)});
   e->bg_nljobs = (int)ljobs.size();
   TableBuilder tb;
   const size_t o_parts = tb.add(parts.data(), parts.size());
@@ -727,8 +729,8 @@ int build_plan(fap_engine *e, Plan &pl) {
       std::vector<fapk::BgJob> bjobs;
       for (size_t b = 0; b < batches.size(); b++) {
         for (int l = 0; l < batches[b].count; l++) bsrc[b * 32 + l] = e->bg_bidx[batches[b].src[l]];
-        for (int l0 = 0; l0 < batches[b].count; l0 += fapk::bg_lanes())
-          bjobs.push_back({(int32_t)b, l0, std::min(fapk::bg_lanes(), batches[b].count - l0)});
+        for (int l0 = 0; l0 < batches[b].count; l0 += e->bg_lanes)
+          bjobs.push_back({(int32_t)b, l0, std::min(e->bg_lanes, batches[b].count - l0)});
       }
       G.nbjobs = (int)bjobs.size();
       O.bjobs = tb.add(bjobs.data(), bjobs.size());
@@ -932,8 +934,8 @@ struct Issuer {
       ba.bsrc = G.bsrc;
       ba.status = e->d_status;
       ba.stats = e->d_stats;
-      if (g == 0) FAP_CUDA(fapk::launch_bg_local(wide, ba, e->bg_nljobs, e->bg_max_sub, st));
-      FAP_CUDA(fapk::launch_bg_boundary(wide, ba, G.nbjobs, st));
+      if (g == 0) FAP_CUDA(fapk::launch_bg_local(wide, e->bg_lanes, ba, e->bg_nljobs, e->bg_max_sub, st));
+      FAP_CUDA(fapk::launch_bg_boundary(wide, e->bg_lanes, ba, G.nbjobs, st));
       fapk::BgRowArgs ra{};
       ra.batches = G.batches;
       ra.nbatches = G.nbatches;

@@ -178,10 +178,10 @@ struct BgRowArgs {
 };
 constexpr size_t kBgSmemMax = 226 * 1024;  // dynamic; the 227 KB per-block limit also holds the static part
 size_t bg_smem_bytes(bool wide, int nodes);  // shared memory of steps 1 and 2 over `nodes` nodes
-int bg_lanes();                              // sources per CTA in steps 1 and 2
+int bg_lanes(bool wide, int nodes, int sm_count);  // sources per CTA in steps 1 and 2 (8 or 4)
 cudaError_t init_bg_kernels();
-cudaError_t launch_bg_local(bool wide, const BgArgs &a, int njobs, int max_sub, cudaStream_t st);
-cudaError_t launch_bg_boundary(bool wide, const BgArgs &a, int njobs, cudaStream_t st);
+cudaError_t launch_bg_local(bool wide, int lanes, const BgArgs &a, int njobs, int max_sub, cudaStream_t st);
+cudaError_t launch_bg_boundary(bool wide, int lanes, const BgArgs &a, int njobs, cudaStream_t st);
 cudaError_t launch_bg_rows(bool wide, int lanes, const BgArgs &a, const BgRowArgs &r, cudaStream_t st);
 
 // query.cu -- point-to-point queries on solve() rows in device memory
