@@ -450,20 +450,21 @@ size_t bg_smem_bytes(bool wide, int nodes) {
 
 // The sources of a CTA: eight, whose relaxations of a node share its edges, or
 // four, which make twice the CTAs and half the table: where eight do not give
-// the GPU enough CTAs, and where their table leaves an SM one CTA.  SSSP phase
+// the GPU enough CTAs, and where their table leaves an SM one CTA (that of 8-byte
+// distances does as soon as they give it enough).  SSSP phase
 // with eight and four, ms: road-like graphs of 8,000 vertices 0.60 / 0.48, 20,000
 // 0.92 / 0.77, 40,000 1.65 / 1.40 (960 boundary vertices), 80,000 5.54 / 5.14 (table),
 // 114,599 10.97 / 9.81 (table); geometric 20,000 0.44 / 0.40, 65,536 (1,848
 // boundary vertices) 1.35 / 1.37; near the line, road-like graphs of 57,301 with
 // 1,408 3.44 / 3.20, with fewer 2.57 / 2.70.
 int bg_lanes(bool wide, int nodes, int sm_count) {
-  return nodes <= 10 * sm_count || bg_smem_bytes(wide, nodes) > 113 * 1024 ? kBgLanes / 2 : kBgLanes;
+  return wide || nodes <= 10 * sm_count || bg_smem_bytes(wide, nodes) > 113 * 1024 ? kBgLanes / 2 : kBgLanes;
 }
 
 cudaError_t init_bg_kernels() {
   cudaError_t e;
-  if ((e = set_bg_attrs<uint32_t, 8>()) != cudaSuccess || (e = set_bg_attrs<unsigned long long, 8>()) != cudaSuccess ||
-      (e = set_bg_attrs<uint32_t, 4>()) != cudaSuccess || (e = set_bg_attrs<unsigned long long, 4>()) != cudaSuccess ||
+  if ((e = set_bg_attrs<uint32_t, 8>()) != cudaSuccess || (e = set_bg_attrs<uint32_t, 4>()) != cudaSuccess ||
+      (e = set_bg_attrs<unsigned long long, 4>()) != cudaSuccess ||
       (e = set_rows_attr<unsigned long long, 16, true>()) != cudaSuccess ||
       (e = set_rows_attr<unsigned long long, 32, true>()) != cudaSuccess ||
       (e = set_rows_attr<uint32_t, 8, false>()) != cudaSuccess ||
@@ -478,13 +479,10 @@ cudaError_t launch_bg_local(bool wide, int lanes, const BgArgs &a, int njobs, in
   const size_t smem = wide ? bg_smem<unsigned long long>(max_sub, lanes) : bg_smem<uint32_t>(max_sub, lanes);
   if (smem > kBgSmemMax) return cudaErrorInvalidValue;
   ++launch_count();
-  if (lanes == 4) {
-    if (wide) bg_local_kernel<unsigned long long, 4><<<njobs, kBgThreads, smem, st>>>(a);
-    else bg_local_kernel<uint32_t, 4><<<njobs, kBgThreads, smem, st>>>(a);
-  } else {
-    if (wide) bg_local_kernel<unsigned long long, 8><<<njobs, kBgThreads, smem, st>>>(a);
-    else bg_local_kernel<uint32_t, 8><<<njobs, kBgThreads, smem, st>>>(a);
-  }
+  if (wide && lanes == 4) bg_local_kernel<unsigned long long, 4><<<njobs, kBgThreads, smem, st>>>(a);
+  else if (!wide && lanes == 4) bg_local_kernel<uint32_t, 4><<<njobs, kBgThreads, smem, st>>>(a);
+  else if (!wide && lanes == 8) bg_local_kernel<uint32_t, 8><<<njobs, kBgThreads, smem, st>>>(a);
+  else return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
 
@@ -493,13 +491,10 @@ cudaError_t launch_bg_boundary(bool wide, int lanes, const BgArgs &a, int njobs,
   const size_t smem = wide ? bg_smem<unsigned long long>(a.B, lanes) : bg_smem<uint32_t>(a.B, lanes);
   if (smem > kBgSmemMax) return cudaErrorInvalidValue;
   ++launch_count();
-  if (lanes == 4) {
-    if (wide) bg_boundary_kernel<unsigned long long, 4><<<njobs, kBgThreads, smem, st>>>(a);
-    else bg_boundary_kernel<uint32_t, 4><<<njobs, kBgThreads, smem, st>>>(a);
-  } else {
-    if (wide) bg_boundary_kernel<unsigned long long, 8><<<njobs, kBgThreads, smem, st>>>(a);
-    else bg_boundary_kernel<uint32_t, 8><<<njobs, kBgThreads, smem, st>>>(a);
-  }
+  if (wide && lanes == 4) bg_boundary_kernel<unsigned long long, 4><<<njobs, kBgThreads, smem, st>>>(a);
+  else if (!wide && lanes == 4) bg_boundary_kernel<uint32_t, 4><<<njobs, kBgThreads, smem, st>>>(a);
+  else if (!wide && lanes == 8) bg_boundary_kernel<uint32_t, 8><<<njobs, kBgThreads, smem, st>>>(a);
+  else return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
 
