@@ -396,13 +396,32 @@ int number_fw_rest(FwRestJob *jobs, int njobs, int sm_count, int *per) {
   // GPU (two per SM).  A single 910-vertex matrix then runs its remaining
   // tiles in 98 CTAs of one tile instead of 14 of eight (its 14 rounds took
   // 2.33 ms in strips of 8, 1.15 ms in single tiles).
-  *per = 1;
-  for (int tiles = 8; tiles > 1; tiles /= 2) {
+  auto count = [&](int tiles) {
     long long strips = 0;
     for (int i = 0; i < njobs; i++) strips += strips_of(jobs[i], tiles);
+    return strips;
+  };
+  *per = 1;
+  long long longest = 0;
+  for (int tiles = 8; tiles > 1; tiles /= 2) {
+    const long long strips = count(tiles);
+    if (tiles == 8) longest = strips;
     if (strips >= 2LL * sm_count) {
       *per = tiles;
       break;
+    }
+  }
+  // Of 8 to 4 tiles, where a few strips an SM are all there is, the length that
+  // gives the busiest SM the least (a strip's start counted as a tile and a
+  // half): the twelve listed block columns of a 64-matrix road-like graph go in
+  // three strips of four instead of eight and four (whole solve 22.75 -> 22.45
+  // ms), a geometric graph's fifteen in fives (14.81 -> 14.61).  Shorter ones, or
+  // those of launches that take less than 8 anyway, measured the same or slower.
+  if (*per == 8 && longest < 8LL * sm_count) {
+    long long best = 0;
+    for (int tiles = 8; tiles >= 4; tiles--) {
+      const long long cost = (count(tiles) + sm_count - 1) / sm_count * (2 * tiles + 3);
+      if (tiles == 8 || cost < best) best = cost, *per = tiles;
     }
   }
   int strips = 0;
