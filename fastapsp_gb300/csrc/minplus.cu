@@ -67,17 +67,6 @@ __device__ __forceinline__ int list_block(int g, int skip, int skip2, int fix, i
   return b < nblocks ? b : -1;
 }
 
-// Length of such a list.
-__host__ __device__ __forceinline__ int list_len(int skip, int skip2, int fix, int nblocks) {
-  if (fix >= 0) return 1;
-  int len = nblocks;
-  if (skip >= 0 && skip < nblocks) {
-    len--;
-    if (skip2 > skip && skip2 < nblocks) len--;
-  }
-  return len;
-}
-
 // Stages k-chunk [k0, k0+32) of A (128 rows, 4-byte cp.async into the padded
 // rows) and B (128 columns), and of B's predecessors when WITH_BP (16-byte
 // cp.async of 4 columns where aligned); entries outside the matrices are
