@@ -35,6 +35,7 @@
 #include "fap_internal.h"
 #include "kernels.cuh"
 #include "launch.h"
+#include "sssp_scratch.h"
 
 using fapk::FwDiagJob;
 using fapk::FwRestJob;
@@ -262,10 +263,8 @@ struct fap_engine {
   // work buffers
   DevBuf fw_d, fw_p;           // FW matrices arena
   DevBuf fw_look;              // the pivot chain's copies, per matrix (fapk::fw_look_bytes)
-  DevBuf sssp_scratch, sssp_bits;
+  fapk::SsspScratch<DevBuf> sssp;  // (the search with one CTA per source takes its tables too)
   DevBuf row_edges;             // the graph's edge records for the search with one CTA per source
-  int sssp_slots_alloc = 0;
-  bool sssp_wide = false;       // the scratch holds FP64 32-lane slots
   DevBuf res_d, res_p;         // device results when the caller passes host memory
   DevBuf bnd_d, bnd_p;         // boundary rows when the inner rows go straight to mapped host memory
   DevBuf small;                // tables of standalone calls
@@ -311,22 +310,9 @@ int max_sssp_slots(fap_engine *e, bool wide = false) {
   return slots;
 }
 
-// wide: slots of the FP64 search with 32 lanes (twice the distance table);
-// sssp_slots_alloc counts slots of the layout last ensured.
+// wide: slots of the FP64 search with 32 lanes (twice the distance table).
 int ensure_sssp_scratch(fap_engine *e, int slots, bool wide = false) {
-  if (wide != e->sssp_wide) {
-    e->sssp_wide = wide;
-    size_t fit = e->sssp_scratch.bytes / fapk::sssp_slot_bytes(e->n, wide);
-    if (fapk::sssp_bits_bytes(e->n) > 0) fit = std::min(fit, e->sssp_bits.bytes / fapk::sssp_bits_bytes(e->n));
-    e->sssp_slots_alloc = (int)fit;
-  }
-  if (slots <= e->sssp_slots_alloc) return FAP_OK;
-  int st;
-  if ((st = e->sssp_scratch.ensure(fapk::sssp_slot_bytes(e->n, wide) * slots)) != FAP_OK) return st;
-  if ((st = e->sssp_bits.ensure(std::max<size_t>(fapk::sssp_bits_bytes(e->n) * slots, 4))) != FAP_OK)
-    return st;
-  e->sssp_slots_alloc = slots;
-  return FAP_OK;
+  return e->sssp.ensure(slots, wide, fapk::sssp_slot_bytes(e->n, wide), fapk::sssp_bits_bytes(e->n));
 }
 
 // CTAs of that search for `jobs` sources, within a 4 GiB scratch budget; the
@@ -336,12 +322,14 @@ int ensure_row_scratch(fap_engine *e, int64_t jobs, int *ctas, cudaStream_t st) 
   if (!e->row_edges.p) {
     int rc = e->row_edges.ensure(std::max<size_t>((size_t)e->m * 16, 16));
     if (rc != FAP_OK) return rc;
-    FAP_CUDA(fapk::launch_row_edges(e->m, e->d_ro, e->d_col, e->d_w, e->row_edges.p, st));
+    const cudaError_t ce = fapk::launch_row_edges(e->m, e->d_ro, e->d_col, e->d_w, e->row_edges.p, st);
+    if (ce != cudaSuccess) e->row_edges.release();  // (a buffer that is there holds the records)
+    FAP_CUDA(ce);
   }
   const size_t per = std::max<size_t>(fapk::sssp_row_scratch_bytes(e->n), 4);
   const int64_t fit = std::max<int64_t>(1, (int64_t)(((size_t)4 << 30) / per));
   *ctas = (int)std::min<int64_t>(fapk::sssp_row_ctas(e->n, jobs, e->sm_count), fit);
-  return e->sssp_scratch.ensure(per * (size_t)*ctas);
+  return e->sssp.tables.ensure(per * (size_t)*ctas);
 }
 
 // Host tables of the boundary graph for the current partition (bgraph.cu):
@@ -912,9 +900,9 @@ struct Issuer {
     sa.nbatches = G.nbatches;
     sa.dist = pl.bdist ? pl.bdist : pl.dist;  // SSSP rows are the boundary rows
     sa.pred = pl.bdist ? pl.bpred : pl.pred;
-    sa.scratch = e->sssp_scratch.p;
-    sa.slots = std::min(G.nbatches, e->sssp_slots_alloc);
-    sa.bits = e->sssp_bits.p;
+    sa.scratch = e->sssp.tables.p;
+    sa.slots = std::min(G.nbatches, e->sssp.slots);
+    sa.bits = e->sssp.bits.p;
     sa.status = e->d_status;
     sa.maxd = e->f32() ? nullptr : e->d_status + 1;
     sa.iter_cap = 8 * e->n + 64;
@@ -940,7 +928,7 @@ struct Issuer {
       ra.batches = G.batches;
       ra.nbatches = G.nbatches;
       ra.st2ed = e->d_st2ed;
-      ra.scratch = e->sssp_scratch.p;
+      ra.scratch = e->sssp.tables.p;
       ra.slot_bytes = fapk::sssp_slot_bytes(e->n, sa.acc64 && sa.lanes == 32);
       ra.fix_inf = e->bg_fix_inf;
       FAP_CUDA(fapk::launch_bg_rows(wide, sa.lanes, ba, ra, st));
@@ -1276,8 +1264,8 @@ std::vector<const void *> buffer_signature(const fap_engine *e) {
   double d = sssp_delta_of(e);
   intptr_t dbits;
   std::memcpy(&dbits, &d, sizeof(dbits));
-  return {e->fw_d.p, e->fw_p.p, e->fw_look.p, e->sssp_scratch.p, e->sssp_bits.p,
-          reinterpret_cast<const void *>((intptr_t)e->sssp_slots_alloc),
+  return {e->fw_d.p, e->fw_p.p, e->fw_look.p, e->sssp.tables.p, e->sssp.bits.p,
+          reinterpret_cast<const void *>((intptr_t)e->sssp.slots),
           reinterpret_cast<const void *>((intptr_t)e->sssp_fp64),
           reinterpret_cast<const void *>((intptr_t)e->sssp_lanes),
           reinterpret_cast<const void *>((intptr_t)e->sssp_method),
@@ -1744,8 +1732,8 @@ int fap_destroy(fap_engine *e) {
     e->fw_d.release();
     e->fw_p.release();
     e->fw_look.release();
-    e->sssp_scratch.release();
-    e->sssp_bits.release();
+    e->sssp.tables.release();
+    e->sssp.bits.release();
     e->row_edges.release();
     e->res_d.release();
     e->res_p.release();
@@ -2373,9 +2361,9 @@ int fap_sssp(fap_engine *e, const int32_t *sources, int32_t num_sources, void *d
   sa.nbatches = (int)batches.size();
   sa.dist = dist;
   sa.pred = pred;
-  sa.scratch = e->sssp_scratch.p;
-  sa.slots = row ? slots : std::min(sa.nbatches, e->sssp_slots_alloc);
-  sa.bits = e->sssp_bits.p;
+  sa.scratch = e->sssp.tables.p;
+  sa.slots = row ? slots : std::min(sa.nbatches, e->sssp.slots);
+  sa.bits = e->sssp.bits.p;
   sa.status = e->d_status;
   sa.maxd = nullptr;
   sa.iter_cap = 8 * e->n + 64;
