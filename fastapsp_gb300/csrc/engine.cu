@@ -998,7 +998,7 @@ struct Issuer {
                                       e->side));
         FAP_CUDA(cudaEventRecord(e->ev_fw[1 + r % 2], e->side));
       } else {
-        FAP_CUDA(fapk::launch_fw_diag(pred, G.diag[r], G.diag_cnt[r], st));
+        FAP_CUDA(fapk::launch_fw_diag(false, pred, G.diag[r], G.diag_cnt[r], st));
         FAP_CUDA(fapk::launch_minplus_tiles(pred, G.panel[r], G.panel_nseg[r], G.panel_tiles[r], st));
         FAP_CUDA(fapk::launch_minplus_tiles(pred, G.rest[r], G.rest_nseg[r], G.rest_tiles[r], st));
       }
@@ -2218,6 +2218,9 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
   std::vector<int> nd(maxnb), bd(maxnb), np(maxnb), tp(maxnb), nr(maxnb), tr(maxnb), nr2(maxnb), sr2(maxnb), pr2(maxnb);
   int rc;
   if ((rc = e->fw_look.ensure((size_t)count * fapk::fw_look_bytes())) != FAP_OK) return rc;
+  // FP32 matrices of one block are closed in FP32 comparisons, which order
+  // negative entries and -0.0 too; the other kernels compare bit patterns.
+  std::vector<FwDiagJob> single;
   for (int r = 0; r < maxnb; r++) {
     std::vector<FwDiagJob> dj;
     std::vector<MpSegment> ps, rs;
@@ -2236,7 +2239,7 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
       j.panel_begin = blocks;
       j.look = static_cast<char *>(e->fw_look.p) + (size_t)b * fapk::fw_look_bytes();
       blocks += 2 * (nb - 1);
-      dj.push_back(j);
+      (nb == 1 && dtype == FAP_DTYPE_F32 ? single : dj).push_back(j);
       if (nb > 1) {
         r2s.push_back({D[b], pred ? P[b] : nullptr, ld[b], sizes[b], r, r + 1 < nb ? 1 : 0, 0});
         if (dtype != FAP_DTYPE_F32) {  // the wide int32 form's tiles
@@ -2278,6 +2281,7 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
       max_size = std::max(max_size, sizes[b]);
     }
   size_t o_ref = tb.add(refs.data(), refs.size());
+  const size_t o_single = tb.add(single.data(), single.size());
   if ((rc = e->small.ensure(std::max<size_t>(tb.bytes.size(), 64))) != FAP_OK) return rc;
   FAP_CUDA(cudaMemcpyAsync(e->small.p, tb.bytes.data(), tb.bytes.size(), cudaMemcpyHostToDevice, st));
   unsigned char *base = static_cast<unsigned char *>(e->small.p);
@@ -2292,7 +2296,16 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
     FAP_CUDA(cudaStreamSynchronize(st));
     packed = (unsigned long long)mx * (unsigned long long)std::max(max_size - 1, 1) < fapk::pack_limit();
   }
+  if (!single.empty()) {  // beside the others' first round, if there are others
+    if (maxnb > 1) {
+      FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
+      FAP_CUDA(cudaStreamWaitEvent(e->side, e->ev_fw[0], 0));
+    }
+    FAP_CUDA(fapk::launch_fw_diag(true, pred, reinterpret_cast<const FwDiagJob *>(base + o_single),
+                                  (int)single.size(), maxnb > 1 ? e->side : st));
+  }
   for (int r = 0; r < maxnb; r++) {
+    if (nd[r] == 0) continue;
     const FwDiagJob *djobs = reinterpret_cast<const FwDiagJob *>(base + od[r]);
     if (packed || f32) {  // lookahead, as in the solve's issue order
       if (r >= 2) FAP_CUDA(cudaStreamWaitEvent(st, e->ev_fw[1 + r % 2], 0));
@@ -2303,7 +2316,7 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
                                     pr2[r], e->side));
       FAP_CUDA(cudaEventRecord(e->ev_fw[1 + r % 2], e->side));
     } else {
-      FAP_CUDA(fapk::launch_fw_diag(pred, djobs, nd[r], st));
+      FAP_CUDA(fapk::launch_fw_diag(false, pred, djobs, nd[r], st));
       FAP_CUDA(fapk::launch_minplus_tiles(pred, reinterpret_cast<const MpSegment *>(base + op[r]), np[r], tp[r], st));
       FAP_CUDA(fapk::launch_minplus_tiles(pred, reinterpret_cast<const MpSegment *>(base + orr[r]), nr[r], tr[r], st));
     }

@@ -52,8 +52,9 @@ unsigned pack_limit();
 // with no active step, add-mins executed (active steps x the tile's outputs)];
 // optionally reset.
 cudaError_t strip_counters(unsigned long long out[3], bool reset);
-// Wide int32 form: closes each job's pivot block.
-cudaError_t launch_fw_diag(bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st);
+// Closes each job's pivot block: the wide int32 form's, and FP32 matrices of one
+// block.
+cudaError_t launch_fw_diag(bool f32, bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st);
 // fw_pivot.cu (packed int32 and FP32 forms): round job.prev's update of each
 // job's block row and column job.block, the closure of the pivot block and the
 // panels: two launches.  blocks = the jobs' panel blocks, 2 (blocks a side - 1)

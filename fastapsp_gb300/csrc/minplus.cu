@@ -1137,10 +1137,12 @@ cudaError_t strip_counters(unsigned long long out[3], bool reset) {
   return cudaMemcpyToSymbol(g_strip_counters, zero, sizeof(zero));
 }
 
-cudaError_t launch_fw_diag(bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st) {
+cudaError_t launch_fw_diag(bool f32, bool pred, const FwDiagJob *d_jobs, int njobs, cudaStream_t st) {
   if (njobs <= 0) return cudaSuccess;
   ++launch_count();
-  if (pred) fw_diag_kernel<uint32_t, true><<<njobs, 256, 0, st>>>(d_jobs);
+  if (f32 && pred) fw_diag_kernel<float, true><<<njobs, 256, 0, st>>>(d_jobs);
+  else if (f32) fw_diag_kernel<float, false><<<njobs, 256, 0, st>>>(d_jobs);
+  else if (pred) fw_diag_kernel<uint32_t, true><<<njobs, 256, 0, st>>>(d_jobs);
   else fw_diag_kernel<uint32_t, false><<<njobs, 256, 0, st>>>(d_jobs);
   return cudaGetLastError();
 }

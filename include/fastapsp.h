@@ -307,7 +307,9 @@ int fap_minplus(fap_engine *e, int32_t dtype, int32_t M, int32_t N, int32_t K,
  * sequence.  D[b] is sizes[b] x sizes[b] with leading dimension ld[b]; P[b]
  * (same shape and leading dimension, may be NULL for all b) is updated as
  * P[i][j] = P[k][j] on every strict improvement.  The pointer arrays live in
- * host memory; the matrices in device memory. */
+ * host memory; the matrices in device memory.  Entries are non-negative with a
+ * zero diagonal; FP32 matrices of at most 64 vertices may hold negative ones
+ * (and -0.0), without negative cycles. */
 int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count,
                       const int32_t *sizes, void *const *D, const int64_t *ld,
                       int32_t *const *P, void *stream);

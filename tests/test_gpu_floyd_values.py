@@ -1,0 +1,77 @@
+"""Batched FP32 Floyd-Warshall on entries outside the plain range: negative
+entries and -0.0 of small matrices."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+UNREACHED = np.float32(1e8)
+
+
+@pytest.fixture(scope="module")
+def ctx(gpu):
+    c = gpu.Context(0)
+    yield c
+    c.close()
+
+
+def digraph(rng, n):
+    """Whole-number weights, about two edges out of a vertex, zero diagonal, predecessors."""
+    a = np.full((n, n), UNREACHED)
+    edge = rng.random((n, n)) < 2.0 / n
+    a[edge] = rng.integers(1, 9, edge.sum())
+    np.fill_diagonal(a, 0)
+    return a, edge & ~np.eye(n, dtype=bool)
+
+
+def preds_of(a):
+    n = a.shape[0]
+    return np.where(a < UNREACHED, np.arange(n, dtype=np.int32)[:, None], -1).astype(np.int32)
+
+
+def sequential(a, p):
+    """Floyd-Warshall in ascending steps, strict improvements only."""
+    d, p = a.copy(), p.copy()
+    for k in range(a.shape[0]):
+        via = d[:, k:k + 1] + d[k:k + 1]
+        better = via < d
+        d, p = np.where(better, via, d), np.where(better, np.broadcast_to(p[k], p.shape), p)
+    return d, p
+
+
+def run(ctx, mats, preds):
+    ds = [torch.from_numpy(a).cuda() for a in mats]
+    ps = [torch.from_numpy(p).cuda() for p in preds] if preds else None
+    torch.cuda.synchronize()
+    ctx.floyd_batched(0, ds, ps)
+    torch.cuda.synchronize()
+    return [d.cpu().numpy() for d in ds], [p.cpu().numpy() for p in ps] if preds else None
+
+
+@pytest.mark.parametrize("kind", ["negative", "minus_zero"])
+@pytest.mark.parametrize("sizes", [(1, 2, 40, 63, 64), (64, 200, 33, 65)])
+def test_negative_entries_of_small_matrices(ctx, kind, sizes):
+    """Matrices of at most 64 vertices close with negative entries (without
+    negative cycles) and -0.0, alone and in a batch with larger ones."""
+    rng = np.random.default_rng(sum(sizes))
+    mats = []
+    for n in sizes:
+        a, edge = digraph(rng, n)
+        if n <= 64 and kind == "negative":  # potentials: every cycle keeps its length
+            h = rng.integers(0, 6, n).astype(np.float32)
+            a[edge] += (h[:, None] - h[None, :])[edge]
+        elif n <= 64:
+            a[edge & (rng.random((n, n)) < 0.3)] = -0.0
+        mats.append(a)
+    preds = [preds_of(a) for a in mats]
+    got, gotp = run(ctx, mats, preds)
+    plain, _ = run(ctx, mats, None)
+    for a, p, d, q, e in zip(mats, preds, got, gotp, plain):
+        ref, refp = sequential(a, p)
+        reached = ref < UNREACHED / 2
+        assert np.array_equal(d[reached], ref[reached])
+        if a.shape[0] <= 64:  # (blocks take equal paths in another order)
+            assert np.array_equal(q[reached], refp[reached])
+        assert (d[~reached] > UNREACHED / 2).all() and (q[~reached] == -1).all()
+        assert np.array_equal(e, d)
