@@ -1691,6 +1691,10 @@ int fap_create(int32_t n, int64_t m, const int32_t *row_offset, const int32_t *c
     if (dtype == FAP_DTYPE_F32) {
       std::memcpy(&wbits[j], &weight[j], 4);
       std::memcpy(&iwbits[j], &iw[j], 4);
+      // no weight is negative, but -0.0 passes for 0, and its bits (which the
+      // kernels compare) are above every other's
+      wbits[j] &= 0x7fffffffu;
+      iwbits[j] &= 0x7fffffffu;
     } else {
       wbits[j] = (uint32_t)weight[j];
       iwbits[j] = (uint32_t)iw[j];

@@ -1,8 +1,10 @@
-"""Batched FP32 Floyd-Warshall on entries outside the plain range: negative
-entries and -0.0 of small matrices."""
+"""FP32 values outside the plain range: negative entries and -0.0 of small
+matrices of a batched Floyd-Warshall, graph weights of -0.0."""
 import numpy as np
 import pytest
 import torch
+
+from fastapsp_gb300 import graphs
 
 pytestmark = pytest.mark.gpu
 
@@ -75,3 +77,20 @@ def test_negative_entries_of_small_matrices(ctx, kind, sizes):
             assert np.array_equal(q[reached], refp[reached])
         assert (d[~reached] > UNREACHED / 2).all() and (q[~reached] == -1).all()
         assert np.array_equal(e, d)
+
+
+@pytest.mark.parametrize("n, parts", [(50, 2), (400, 3)])
+def test_graph_weights_of_minus_zero(gpu, n, parts):
+    """Weights of -0.0 count as 0: the same rows as with +0.0."""
+    g = graphs.small_random_graph(n, 4 * n, True, True, seed=n)
+    gid, _ = gpu.partition(g.row_offset, g.col_val, parts)
+    w = g.weight.copy()
+    w[::5] = -0.0
+    outs = []
+    for weight in (w, np.abs(w)):
+        with gpu.Engine(n, g.row_offset, g.col_val, weight, parts, graph_id=gid, dtype=gpu.DTYPE_F32) as eng:
+            d, p = np.empty((n, n), np.float32), np.empty((n, n), np.int32)
+            eng.solve(d, p)
+            outs.append((d, p))
+    assert np.array_equal(outs[0][0].view(np.uint32), outs[1][0].view(np.uint32))
+    assert np.array_equal(outs[0][1], outs[1][1])
