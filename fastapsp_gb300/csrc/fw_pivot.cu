@@ -81,6 +81,18 @@ __device__ __forceinline__ void block_load(V (&out)[4][kPivC], const V *base, in
     for (int c = 0; c < kPivC; c++) out[i][c] = r0 + i < size && c0 + c < size ? p[i * ld + c] : fill;
 }
 
+// FP32: entries above "unreached" (infinities) are unreached.  Every block is a
+// panel once or twice, or the pivot block, and these write unreached entries too,
+// so a closed matrix holds one value for them.
+template <bool F32>
+__device__ __forceinline__ void cap_unreached(unsigned (&v)[4][kPivC]) {
+  if (!F32) return;
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int c = 0; c < kPivC; c++) v[i][c] = min(v[i][c], __float_as_uint(Dist<float>::inf()));
+}
+
 // A thread's part of an operand into shared memory, and the step groups (of
 // four) that it has a finite entry in: as A (transposed; its columns are the
 // steps) or as B (its rows are).
@@ -236,6 +248,7 @@ __global__ void __launch_bounds__(kPivThreads, 2) fw_close_kernel(const FwDiagJo
   int32_t p[4][kPivC];
   int step[4][kPivC];
   block_load(d, const_cast<const unsigned *>(D), job.ld, q, q, job.size, INF, vec);
+  cap_unreached<F32>(d);
   if (PRED) block_load(p, const_cast<const int32_t *>(job.P), job.ld, q, q, job.size, -1, vecp);
   if (r >= 0) {
     unsigned a[4][kPivC], b[4][kPivC];
@@ -463,6 +476,7 @@ __global__ void __launch_bounds__(kPivThreads, 2)
   unsigned x[4][kPivC], t[4][kPivC];
   int step1[4][kPivC], step[4][kPivC];
   block_load(x, const_cast<const unsigned *>(D), ld, rb, cb, size, INF, vec);
+  cap_unreached<F32>(x);
   block_load(t, const_cast<const unsigned *>(D), ld, q, q, size, INF, vec);
   __syncthreads();
   if (rowp) mask_or(&s_groups[0], store_a<F32>(sm.Q, t));
@@ -521,9 +535,10 @@ __global__ void __launch_bounds__(kPivThreads, 2)
 #pragma unroll
     for (int c = 0; c < kPivC; c++) {
       const int j = tx * kPivC + c, col = cb * kBlk + j, s = step[i][c];
-      if ((!s && !step1[i][c]) || row >= size || col >= size) continue;
+      const bool kept = !s && !step1[i][c];
+      if ((kept && !(F32 && x[i][c] == INF)) || row >= size || col >= size) continue;
       D[(int64_t)row * ld + col] = x[i][c];
-      if (PRED)
+      if (PRED && !kept)
         P[(int64_t)row * ld + col] = !s ? p1[i][c]
                                      : rowp ? sm.X[s - 1][j]
                                             : P[(int64_t)(q * kBlk + s - 1) * ld + q * kBlk + j];

@@ -309,7 +309,8 @@ int fap_minplus(fap_engine *e, int32_t dtype, int32_t M, int32_t N, int32_t K,
  * P[i][j] = P[k][j] on every strict improvement.  The pointer arrays live in
  * host memory; the matrices in device memory.  Entries are non-negative with a
  * zero diagonal; FP32 matrices of at most 64 vertices may hold negative ones
- * (and -0.0), without negative cycles. */
+ * (and -0.0), without negative cycles.  FP32 entries above 1e8 (infinities) are
+ * unreached, and come out as 1e8 from matrices of more than 64 vertices. */
 int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count,
                       const int32_t *sizes, void *const *D, const int64_t *ld,
                       int32_t *const *P, void *stream);

@@ -1,5 +1,6 @@
 """FP32 values outside the plain range: negative entries and -0.0 of small
-matrices of a batched Floyd-Warshall, graph weights of -0.0."""
+matrices of a batched Floyd-Warshall, values above "unreached", graph weights of
+-0.0."""
 import numpy as np
 import pytest
 import torch
@@ -77,6 +78,24 @@ def test_negative_entries_of_small_matrices(ctx, kind, sizes):
             assert np.array_equal(q[reached], refp[reached])
         assert (d[~reached] > UNREACHED / 2).all() and (q[~reached] == -1).all()
         assert np.array_equal(e, d)
+
+
+@pytest.mark.parametrize("absent", [np.inf, 3e8, np.nan])
+@pytest.mark.parametrize("n", [65, 128, 130, 300])
+def test_values_above_unreached(ctx, n, absent):
+    """Matrices of more than one block with missing edges at infinity (or any value
+    above "unreached") close as with 1e8 there, with predecessors and without."""
+    rng = np.random.default_rng(n)
+    a, _ = digraph(rng, n)
+    preds = [preds_of(a)] * 3
+    above, some = a.copy(), a.copy()
+    above[a >= UNREACHED] = absent
+    some[(a >= UNREACHED) & (rng.random((n, n)) < 0.5)] = absent
+    for p in (preds, None):
+        got, gotp = run(ctx, [a, above, some], p)
+        assert np.array_equal(got[0], got[1]) and np.array_equal(got[0], got[2])
+        if p:
+            assert np.array_equal(gotp[0], gotp[1]) and np.array_equal(gotp[0], gotp[2])
 
 
 @pytest.mark.parametrize("n, parts", [(50, 2), (400, 3)])
