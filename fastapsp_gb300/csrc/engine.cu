@@ -777,7 +777,7 @@ int build_plan(fap_engine *e, Plan &pl) {
         j.block = r;
         j.prev = r - 1;
         j.panel_begin = blocks;
-        j.look = static_cast<char *>(e->fw_look.p) + (size_t)mat_index[pi] * fapk::fw_look_bytes();
+        j.look = mat_index[pi];
         blocks += 2 * (nb - 1);
         dj.push_back(j);
         {  // 64^3 block products: pivot step (lookahead update, closure, panels); tile form (all blocks)
@@ -991,7 +991,7 @@ struct Issuer {
         // and writes r + 1; `rest2` reads block row and column r outside
         // blocks r and r + 1 and writes neither.
         if (r >= 2) FAP_CUDA(cudaStreamWaitEvent(st, e->ev_fw[1 + r % 2], 0));
-        FAP_CUDA(fapk::launch_fw_chain(f32, pred, G.diag[r], G.diag_cnt[r], G.diag_blocks[r], st));
+        FAP_CUDA(fapk::launch_fw_chain(f32, pred, G.diag[r], G.diag_cnt[r], G.diag_blocks[r], e->fw_look.p, st));
         FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
         FAP_CUDA(cudaStreamWaitEvent(e->side, e->ev_fw[0], 0));
         FAP_CUDA(fapk::launch_fw_rest(f32, pred, G.rest2[r], G.rest2_njob[r], G.rest2_strips[r], G.rest2_per[r],
@@ -2221,7 +2221,10 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
   std::vector<size_t> od(maxnb), op(maxnb), orr(maxnb), or2(maxnb);
   std::vector<int> nd(maxnb), bd(maxnb), np(maxnb), tp(maxnb), nr(maxnb), tr(maxnb), nr2(maxnb), sr2(maxnb), pr2(maxnb);
   int rc;
-  if ((rc = e->fw_look.ensure((size_t)count * fapk::fw_look_bytes())) != FAP_OK) return rc;
+  std::vector<int32_t> look(count, 0);  // matrices of two or more blocks, numbered
+  int32_t nlook = 0;
+  for (int32_t b = 0; b < count; b++)
+    if (sizes[b] > Bk) look[b] = nlook++;
   // FP32 matrices of one block are closed in FP32 comparisons, which order
   // negative entries and -0.0 too; the other kernels compare bit patterns.
   std::vector<FwDiagJob> single;
@@ -2241,7 +2244,7 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
       j.block = r;
       j.prev = r - 1;
       j.panel_begin = blocks;
-      j.look = static_cast<char *>(e->fw_look.p) + (size_t)b * fapk::fw_look_bytes();
+      j.look = look[b];
       blocks += 2 * (nb - 1);
       (nb == 1 && dtype == FAP_DTYPE_F32 ? single : dj).push_back(j);
       if (nb > 1) {
@@ -2300,6 +2303,8 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
     FAP_CUDA(cudaStreamSynchronize(st));
     packed = (unsigned long long)mx * (unsigned long long)std::max(max_size - 1, 1) < fapk::pack_limit();
   }
+  // (the wide form and matrices of one block have no lookahead)
+  if ((packed || f32) && (rc = e->fw_look.ensure((size_t)nlook * fapk::fw_look_bytes())) != FAP_OK) return rc;
   if (!single.empty()) {  // beside the others' first round, if there are others
     if (maxnb > 1) {
       FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
@@ -2313,7 +2318,7 @@ int fap_floyd_batched(fap_engine *e, int32_t dtype, int32_t count, const int32_t
     const FwDiagJob *djobs = reinterpret_cast<const FwDiagJob *>(base + od[r]);
     if (packed || f32) {  // lookahead, as in the solve's issue order
       if (r >= 2) FAP_CUDA(cudaStreamWaitEvent(st, e->ev_fw[1 + r % 2], 0));
-      FAP_CUDA(fapk::launch_fw_chain(f32, pred, djobs, nd[r], bd[r], st));
+      FAP_CUDA(fapk::launch_fw_chain(f32, pred, djobs, nd[r], bd[r], e->fw_look.p, st));
       FAP_CUDA(cudaEventRecord(e->ev_fw[0], st));
       FAP_CUDA(cudaStreamWaitEvent(e->side, e->ev_fw[0], 0));
       FAP_CUDA(fapk::launch_fw_rest(f32, pred, reinterpret_cast<const FwRestJob *>(base + or2[r]), nr2[r], sr2[r],

@@ -48,6 +48,10 @@ namespace {
 constexpr int kPivThreads = 512;
 constexpr int kPivC = 2;
 
+// Words of a matrix's copies of blocks (r + 1, r) and (r, r + 1), and of the
+// latter's predecessors.
+constexpr int64_t kLookWords = 3 * kBlk * kBlk;
+
 // Operands of a 64^3 product in shared memory.  A by step: entry (k, row) at
 // k * 64 + (row ^ swz(k)); B the same with columns (the packed form's B
 // unswizzled): a thread's four rows or two columns of a step are one chunk, and
@@ -233,7 +237,8 @@ __device__ __forceinline__ unsigned close_resolve(const CloseSmem &sm, unsigned 
 // An entry's predecessor is that of (its last step, column) as it stood at
 // that step; the rows' steps are kept as they pass and followed afterwards.
 template <bool F32, bool PRED>
-__global__ void __launch_bounds__(kPivThreads, 2) fw_close_kernel(const FwDiagJob *__restrict__ jobs) {
+__global__ void __launch_bounds__(kPivThreads, 2)
+    fw_close_kernel(const FwDiagJob *__restrict__ jobs, unsigned *looks) {
   extern __shared__ __align__(16) unsigned char piv_smem[];
   CloseSmem &sm = *reinterpret_cast<CloseSmem *>(piv_smem);
   __shared__ unsigned s_groups[2];
@@ -262,7 +267,7 @@ __global__ void __launch_bounds__(kPivThreads, 2) fw_close_kernel(const FwDiagJo
     mask_or(&s_groups[1], store_b<F32>(sm.B, b));
 #pragma unroll
     for (int i = 0; i < 4; i++) {  // the copies that the panel kernel reads
-      uint2 *look = reinterpret_cast<uint2 *>(job.look) + (ty * 4 + i) * (kBlk / 2) + tx;
+      uint2 *look = reinterpret_cast<uint2 *>(looks + job.look * kLookWords) + (ty * 4 + i) * (kBlk / 2) + tx;
       look[0] = make_uint2(a[i][0], a[i][1]);
       look[kBlk * kBlk / 2] = make_uint2(b[i][0], b[i][1]);
       if (PRED) {
@@ -454,7 +459,7 @@ struct PanelSmem {
 // block (x) pivot).
 template <bool F32, bool PRED>
 __global__ void __launch_bounds__(kPivThreads, 2)
-    fw_panel_kernel(const FwDiagJob *__restrict__ jobs, int njobs) {
+    fw_panel_kernel(const FwDiagJob *__restrict__ jobs, int njobs, const unsigned *looks) {
   extern __shared__ __align__(16) unsigned char piv_smem[];
   PanelSmem &sm = *reinterpret_cast<PanelSmem *>(piv_smem);
   __shared__ unsigned s_groups[4];
@@ -494,7 +499,7 @@ __global__ void __launch_bounds__(kPivThreads, 2)
     for (int c = 0; c < kPivC; c++) step1[i][c] = 0;
   int32_t p1[4][kPivC];  // predecessors that round prev's update brought
   if (r >= 0 && b != r) {
-    const unsigned *look = static_cast<const unsigned *>(job.look);
+    const unsigned *look = looks + job.look * kLookWords;
     if (rowp) {  // A: block (q, r) as it was, B: block (r, b)
       block_load(t, look, kBlk, 0, 0, kBlk, INF, true);
       mask_or(&s_groups[1], store_a<F32>(sm.A, t));
@@ -547,16 +552,16 @@ __global__ void __launch_bounds__(kPivThreads, 2)
 }
 
 template <bool F32, bool PRED>
-cudaError_t launch_close(const FwDiagJob *d_jobs, int njobs, cudaStream_t st) {
+cudaError_t launch_close(const FwDiagJob *d_jobs, int njobs, unsigned *looks, cudaStream_t st) {
   ++launch_count();
-  fw_close_kernel<F32, PRED><<<njobs, kPivThreads, sizeof(CloseSmem), st>>>(d_jobs);
+  fw_close_kernel<F32, PRED><<<njobs, kPivThreads, sizeof(CloseSmem), st>>>(d_jobs, looks);
   return cudaGetLastError();
 }
 
 template <bool F32, bool PRED>
-cudaError_t launch_panel(const FwDiagJob *d_jobs, int njobs, int blocks, cudaStream_t st) {
+cudaError_t launch_panel(const FwDiagJob *d_jobs, int njobs, int blocks, const unsigned *looks, cudaStream_t st) {
   ++launch_count();
-  fw_panel_kernel<F32, PRED><<<blocks, kPivThreads, sizeof(PanelSmem), st>>>(d_jobs, njobs);
+  fw_panel_kernel<F32, PRED><<<blocks, kPivThreads, sizeof(PanelSmem), st>>>(d_jobs, njobs, looks);
   return cudaGetLastError();
 }
 
@@ -571,7 +576,7 @@ cudaError_t set_attrs() {
 
 }  // namespace
 
-size_t fw_look_bytes() { return (size_t)3 * kBlk * kBlk * 4; }
+size_t fw_look_bytes() { return (size_t)kLookWords * 4; }
 
 cudaError_t init_fw_pivot_kernels() {
   cudaError_t e;
@@ -581,17 +586,19 @@ cudaError_t init_fw_pivot_kernels() {
   return cudaSuccess;
 }
 
-cudaError_t launch_fw_chain(bool f32, bool pred, const FwDiagJob *d_jobs, int njobs, int blocks, cudaStream_t st) {
+cudaError_t launch_fw_chain(bool f32, bool pred, const FwDiagJob *d_jobs, int njobs, int blocks, void *look,
+                            cudaStream_t st) {
   if (njobs <= 0) return cudaSuccess;
+  unsigned *const at = static_cast<unsigned *>(look);
   cudaError_t e;
-  if (f32) e = pred ? launch_close<true, true>(d_jobs, njobs, st) : launch_close<true, false>(d_jobs, njobs, st);
-  else e = pred ? launch_close<false, true>(d_jobs, njobs, st) : launch_close<false, false>(d_jobs, njobs, st);
+  if (f32) e = pred ? launch_close<true, true>(d_jobs, njobs, at, st) : launch_close<true, false>(d_jobs, njobs, at, st);
+  else e = pred ? launch_close<false, true>(d_jobs, njobs, at, st) : launch_close<false, false>(d_jobs, njobs, at, st);
   if (e != cudaSuccess || blocks <= 0) return e;
   if (f32)
-    return pred ? launch_panel<true, true>(d_jobs, njobs, blocks, st)
-                : launch_panel<true, false>(d_jobs, njobs, blocks, st);
-  return pred ? launch_panel<false, true>(d_jobs, njobs, blocks, st)
-              : launch_panel<false, false>(d_jobs, njobs, blocks, st);
+    return pred ? launch_panel<true, true>(d_jobs, njobs, blocks, at, st)
+                : launch_panel<true, false>(d_jobs, njobs, blocks, at, st);
+  return pred ? launch_panel<false, true>(d_jobs, njobs, blocks, at, st)
+              : launch_panel<false, false>(d_jobs, njobs, blocks, at, st);
 }
 
 }  // namespace fapk

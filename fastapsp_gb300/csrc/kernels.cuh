@@ -86,7 +86,8 @@ struct FwDiagJob {
                  // block row and column is applied first (lookahead: the
                  // remaining-tile launch of round prev left them out); -1: none
   int32_t panel_begin;  // first CTA of its panel blocks in the launch's numbering
-  void *look;           // the matrix's scratch of fw_look_bytes() (used when prev >= 0)
+  int32_t look;         // the matrix's scratch (used when prev >= 0): the launch's look + this many
+                        // times fw_look_bytes()
 };
 
 // FW remaining tiles of one matrix in one round (fw_rest.cu): block rows and

@@ -59,7 +59,8 @@ cudaError_t launch_fw_diag(bool f32, bool pred, const FwDiagJob *d_jobs, int njo
 // job's block row and column job.block, the closure of the pivot block and the
 // panels: two launches.  blocks = the jobs' panel blocks, 2 (blocks a side - 1)
 // each, numbered by FwDiagJob::panel_begin.
-cudaError_t launch_fw_chain(bool f32, bool pred, const FwDiagJob *d_jobs, int njobs, int blocks, cudaStream_t st);
+cudaError_t launch_fw_chain(bool f32, bool pred, const FwDiagJob *d_jobs, int njobs, int blocks, void *look,
+                            cudaStream_t st);
 // fw_rest.cu: number_fw_rest numbers a launch's CTAs (returns their count)
 // and chooses the column tiles each takes.
 int number_fw_rest(FwRestJob *jobs, int njobs, int sm_count, int *per);
@@ -69,7 +70,7 @@ cudaError_t launch_fw_rest(bool f32, bool pred, const FwRestJob *d_jobs, int njo
 // last reset; optionally reset.
 cudaError_t fw_rest_counter(unsigned long long *out, bool reset);
 cudaError_t init_fw_rest_kernels();
-size_t fw_look_bytes();  // device scratch per matrix
+size_t fw_look_bytes();  // device scratch per matrix of two or more blocks
 cudaError_t init_fw_pivot_kernels();
 int minplus_tile_rows();  // CTA output tile edge (128)
 int fw_block();           // FW pivot block edge (64)
