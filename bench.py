@@ -382,7 +382,8 @@ def run_solve(args, name, rank, world, local_rank):
             t0 = time.perf_counter()
             e = fap.Engine(n, ro_h.numpy(), col_h.numpy(), w_h.numpy(), K, graph_id=gid_h.numpy(),
                            dtype=dtype, device=dev)
-            for o, v in {**options, **tuned}.items():
+            # (a width set explicitly would select the batched search)
+            for o, v in {**options, **{o: v for o, v in tuned.items() if o != fap._lib.OPT_SSSP_LANES}}.items():
                 e.set_option(o, v)
             tc = time.perf_counter()
             if share is None:

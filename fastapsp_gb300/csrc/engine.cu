@@ -221,10 +221,11 @@ struct fap_engine {
   int32_t max_deg = 0; // largest out- or in-degree
   // SSSP options (fap_set_option)
   int sssp_fp64 = 0;       // FP32 engines: search in FP64
-  double sssp_delta = 0;   // near-far threshold step; 0 = auto (tuned on first solve)
+  double sssp_delta = 0;   // near-far threshold step; 0 = auto
+  double sssp_delta_tuned = 0;  // the batched search's, which the autotuner chose (0: none yet)
   int autotune = 1;        // tune the SSSP step on the first solve
   int sssp_lanes = 0;      // sources per SSSP batch: 16, 32, 0 = chosen per solve
-  int sssp_lanes_tuned = 0;  // the width the autotuner chose (0: none yet)
+  int sssp_lanes_tuned = 0;  // the width the autotuner chose, or of the last one-CTA-per-source plan (0: none yet)
   int tile_cols = 0;       // FAP_OPT_TILE_COLS: accepted, chooses nothing
   int host_results = 0;    // FAP_OPT_HOST_RESULTS: 0 staged when the device has room, 1 direct
   double host_group_mb = 8192.0;  // FAP_OPT_HOST_GROUP_MB: result rows per group of a host-results solve
@@ -291,12 +292,19 @@ bool sssp_row_form(const fap_engine *e) {
 // batched search's, 5 to 30 % slower), so no trial runs choose it.
 constexpr double kRowDelta = 64.0;
 
-double sssp_delta_of(const fap_engine *e) {
+// Near-far step of a search: with one CTA per source (row), or batched.
+double sssp_delta_of(const fap_engine *e, bool row) {
   if (e->delta_try > 0) return e->delta_try;
   if (e->sssp_delta > 0) return e->sssp_delta;
+  if (!row && e->sssp_delta_tuned > 0) return e->sssp_delta_tuned;
   // a few mean edge weights per near-far step (at least one unit for int32)
-  double d = (sssp_row_form(e) ? kRowDelta : 8.0) * e->wmean;
+  double d = (row ? kRowDelta : 8.0) * e->wmean;
   return e->f32() ? std::max(d, 1e-30) : std::max(1.0, std::floor(d));
+}
+
+// The batched search's step is still to be tuned.
+bool sssp_untuned(const fap_engine *e) {
+  return e->autotune && e->sssp_delta <= 0 && e->sssp_delta_tuned <= 0;
 }
 
 int max_sssp_slots(fap_engine *e, bool wide = false) {
@@ -908,7 +916,7 @@ struct Issuer {
     sa.iter_cap = 8 * e->n + 64;
     sa.lanes = pl.sssp_lanes;
     sa.acc64 = e->f32() && e->sssp_fp64;
-    sa.delta = sssp_delta_of(e);
+    sa.delta = sssp_delta_of(e, pl.sssp_row);
     sa.row_edges = e->row_edges.p;
     sa.stats = e->d_stats;
     if (g == 0) FAP_CUDA(cudaMemsetAsync(e->d_stats, 0, 8 * sizeof(unsigned long long), st));
@@ -1165,7 +1173,7 @@ int autotune_sssp(fap_engine *e, Plan &pl, cudaStream_t st) {
   cudaEventDestroy(b);
   if (rc != FAP_OK) return rc;
   if ((rc = check_status(e)) != FAP_OK) return rc;
-  e->sssp_delta = best;
+  e->sssp_delta_tuned = best;
   e->tuned_ms = best_ms;
   pl.sig = buffer_signature(e);
   return FAP_OK;
@@ -1261,7 +1269,7 @@ int check_status(fap_engine *e) {
 }
 
 std::vector<const void *> buffer_signature(const fap_engine *e) {
-  double d = sssp_delta_of(e);
+  double d = sssp_delta_of(e, sssp_row_form(e));
   intptr_t dbits;
   std::memcpy(&dbits, &d, sizeof(dbits));
   return {e->fw_d.p, e->fw_p.p, e->fw_look.p, e->sssp.tables.p, e->sssp.bits.p,
@@ -1330,7 +1338,7 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
   // 32 -> 16; not for the FP64 search, whose 32-source slots have another
   // layout); scratch for the larger batch count of the two.
   const bool row = sssp_row_form(e);
-  const bool tune_lanes = e->autotune && e->sssp_delta <= 0 && e->sssp_lanes == 0 && !acc64 && !bs && !row;
+  const bool tune_lanes = sssp_untuned(e) && e->sssp_lanes == 0 && !acc64 && !bs && !row;
   const int alt_lanes = lanes == 16 ? 32 : 16;
   const bool wide = acc64 && lanes == 32;
   const int count_lanes = tune_lanes ? std::min(lanes, alt_lanes) : lanes;
@@ -1376,13 +1384,9 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
   if (pl->pack < 0) {  // first run: trials and tuners, then the plan without a graph
     const int c0 = fapk::launch_count();
     if (pl->method_trial && (rc = trial_sssp_method(e, *pl, st)) != FAP_OK) return rc;
-    if (e->autotune && e->sssp_delta <= 0 && !pl->bsssp) {
-      if (pl->sssp_row) {  // nothing to try: the step as it is, and the width of its tables
-        e->sssp_delta = sssp_delta_of(e);
-        e->sssp_lanes_tuned = pl->sssp_lanes;
-      } else if ((rc = autotune_sssp(e, *pl, st)) != FAP_OK) {
-        return rc;
-      }
+    if (sssp_untuned(e) && !pl->bsssp) {
+      if (pl->sssp_row) e->sssp_lanes_tuned = pl->sssp_lanes;  // nothing to try; the width of its tables
+      else if ((rc = autotune_sssp(e, *pl, st)) != FAP_OK) return rc;
     }
     if ((rc = first_run(e, *pl, st)) != FAP_OK) return rc;
     e->fw_host_work += pl->pack == 1 || e->f32() ? pl->fw_pivot_work : pl->fw_tile_work;
@@ -2391,7 +2395,7 @@ int fap_sssp(fap_engine *e, const int32_t *sources, int32_t num_sources, void *d
   sa.iter_cap = 8 * e->n + 64;
   sa.lanes = lanes;
   sa.acc64 = acc64;
-  sa.delta = sssp_delta_of(e);
+  sa.delta = sssp_delta_of(e, row);
   sa.row_edges = e->row_edges.p;
   if (row) FAP_CUDA(fapk::launch_sssp_rows(e->f32(), sa, e->sm_count, st));
   else FAP_CUDA(fapk::launch_sssp(e->f32(), sa, st));
@@ -2471,6 +2475,7 @@ int fap_set_option(fap_engine *e, int32_t option, double value) {
     case FAP_OPT_SSSP_DELTA:
       if (!(value >= 0.0) || std::isinf(value)) return set_error(FAP_ERR_INVALID, "SSSP delta must be >= 0");
       e->sssp_delta = (!e->f32() && value > 0.0) ? std::max(1.0, std::floor(value)) : value;
+      e->sssp_delta_tuned = 0;
       return FAP_OK;
     case FAP_OPT_AUTOTUNE:
       e->autotune = value != 0.0 ? 1 : 0;
@@ -2513,7 +2518,7 @@ int fap_get_option(const fap_engine *e, int32_t option, double *value) {
   if (!e || !value) return set_error(FAP_ERR_INVALID, "null argument");
   switch (option) {
     case FAP_OPT_SSSP_FP64: *value = e->sssp_fp64; return FAP_OK;
-    case FAP_OPT_SSSP_DELTA: *value = sssp_delta_of(e); return FAP_OK;
+    case FAP_OPT_SSSP_DELTA: *value = sssp_delta_of(e, sssp_row_form(e)); return FAP_OK;
     case FAP_OPT_AUTOTUNE: *value = e->autotune; return FAP_OK;
     case FAP_OPT_SSSP_LANES: *value = e->sssp_lanes ? e->sssp_lanes : e->sssp_lanes_tuned; return FAP_OK;
     case FAP_OPT_TILE_COLS: *value = e->tile_cols; return FAP_OK;

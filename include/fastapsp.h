@@ -193,12 +193,13 @@ int fap_precondition(fap_engine *e);
  *                      Automatic is 64 x the mean weight where the search
  *                      runs one CTA per source (4-byte distances, automatic
  *                      batch width, no vertex of more than 64 edges), else
- *                      8 x, or what FAP_OPT_AUTOTUNE finds.
+ *                      8 x, or what FAP_OPT_AUTOTUNE finds for it.
  *   FAP_OPT_AUTOTUNE   1 (default) = while the step is automatic, the first
  *                      run of a solve with the batched search times the SSSP
  *                      phase with a few steps (multiples of the mean edge
- *                      weight, and plain Bellman-Ford) and keeps the fastest;
- *                      fap_get_option then reports the chosen step.
+ *                      weight, and plain Bellman-Ford) and keeps the fastest
+ *                      for that search; fap_get_option reports the step of
+ *                      the search that the options at the time select.
  *   FAP_OPT_SSSP_LANES sources per SSSP batch (one CTA each; 8 = four lane
  *                      groups a warp, 16 = two, 32 = one): 8, 16 or 32, which
  *                      also selects the batched search, or 0 (default) =
@@ -207,6 +208,8 @@ int fap_precondition(fap_engine *e);
  *                      and while the step is tuned (above), the first run
  *                      also times a second width at the chosen step and
  *                      keeps the faster, which fap_get_option then reports
+ *                      (after a solve with one CTA per source, the width its
+ *                      sources are listed in; setting it selects batches)
  *                      (not with FAP_OPT_SSSP_FP64, which takes 16 unless 32
  *                      is set).  Changes speed only, never results.
  *   FAP_OPT_TILE_COLS  0, 64 or 128; accepted for programs that set it, chooses

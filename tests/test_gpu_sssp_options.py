@@ -1,0 +1,58 @@
+"""Options of the boundary searches on one engine, changed between solves."""
+import numpy as np
+import pytest
+import torch
+
+from fastapsp_gb300 import graphs
+
+pytestmark = pytest.mark.gpu
+
+
+def solve(eng, n):
+    d = torch.empty((n, n), device="cuda")
+    p = torch.empty((n, n), dtype=torch.int32, device="cuda")
+    eng.solve(d, p)
+    launches = eng.last_launches()
+    eng.solve(d, p)
+    torch.cuda.synchronize()
+    return d, p, launches - eng.last_launches()  # kernels of the first run's trials
+
+
+def test_each_search_has_its_own_step(gpu):
+    """The search with one CTA per source leaves the batched one's step to be
+    tuned on its own first run, and keeps 64 x the mean weight before and after;
+    the rows are the same, the FP64 search's within its rounding."""
+    g = graphs.road_like(3001, seed=5)
+    gid, _ = gpu.partition(g.row_offset, g.col_val, 4)
+    mean = float(np.mean(g.weight.astype(np.float64)))
+    L = gpu._lib
+    with gpu.Engine(g.n, g.row_offset, g.col_val, g.weight, 4, graph_id=gid, dtype=gpu.DTYPE_F32) as eng:
+        d0, p0, _ = solve(eng, g.n)
+        assert eng.get_option(L.OPT_SSSP_DELTA) == pytest.approx(64 * mean)
+        eng.set_option(L.OPT_SSSP_FP64, 1)
+        assert eng.get_option(L.OPT_SSSP_DELTA) == pytest.approx(8 * mean)
+        eng.set_option(L.OPT_SSSP_FP64, 0)
+        eng.set_option(L.OPT_SSSP_LANES, 16)
+        assert eng.get_option(L.OPT_SSSP_DELTA) == pytest.approx(8 * mean)
+        d1, p1, trials = solve(eng, g.n)
+        assert trials >= 9  # nine steps were tried
+        tuned = eng.get_option(L.OPT_SSSP_DELTA)
+        eng.set_option(L.OPT_SSSP_LANES, 0)
+        assert eng.get_option(L.OPT_SSSP_DELTA) == pytest.approx(64 * mean)
+        d2, p2, _ = solve(eng, g.n)
+        assert all(torch.equal(a, d0) for a in (d1, d2)) and all(torch.equal(a, p0) for a in (p1, p2))
+        eng.set_option(L.OPT_SSSP_LANES, 8)
+        assert eng.get_option(L.OPT_SSSP_DELTA) == tuned
+        assert solve(eng, g.n)[2] == 0
+        eng.set_option(L.OPT_SSSP_DELTA, 3.0)  # a step of the program's own is every search's
+        for lanes in (0, 16):
+            eng.set_option(L.OPT_SSSP_LANES, lanes)
+            assert eng.get_option(L.OPT_SSSP_DELTA) == 3.0
+            d, p, trials = solve(eng, g.n)
+            assert trials == 0 and torch.equal(d, d0) and torch.equal(p, p0)
+        eng.set_option(L.OPT_SSSP_LANES, 0)
+        eng.set_option(L.OPT_SSSP_DELTA, 0)
+        eng.set_option(L.OPT_SSSP_FP64, 1)
+        d, _, _ = solve(eng, g.n)
+        # FP32 sums of at most n weights against one rounding
+        assert bool(((d - d0).abs() <= g.n * 2.0 ** -24 * d).all())
