@@ -124,6 +124,7 @@ struct Plan {
     // SSSP
     const SsspBatch *batches = nullptr;
     int nbatches = 0;
+    int64_t nsources = 0;  // sources of all the batches
     // the same sources in batches of the other width (sssp_lanes_alt), for
     // the autotuner; swapped with the above when that width wins
     const SsspBatch *batches_alt = nullptr;
@@ -323,10 +324,10 @@ int ensure_sssp_scratch(fap_engine *e, int slots, bool wide = false) {
   return e->sssp.ensure(slots, wide, fapk::sssp_slot_bytes(e->n, wide), fapk::sssp_bits_bytes(e->n));
 }
 
-// CTAs of that search for `jobs` sources, within a 4 GiB scratch budget; the
+// CTAs of that search for `sources` sources, within a 4 GiB scratch budget; the
 // scratch is the batched search's buffer.  The edge records are made on
 // first use, on the calling stream (calls end with a synchronize).
-int ensure_row_scratch(fap_engine *e, int64_t jobs, int *ctas, cudaStream_t st) {
+int ensure_row_scratch(fap_engine *e, int64_t sources, int *ctas, cudaStream_t st) {
   if (!e->row_edges.p) {
     int rc = e->row_edges.ensure(std::max<size_t>((size_t)e->m * 16, 16));
     if (rc != FAP_OK) return rc;
@@ -336,7 +337,7 @@ int ensure_row_scratch(fap_engine *e, int64_t jobs, int *ctas, cudaStream_t st) 
   }
   const size_t per = std::max<size_t>(fapk::sssp_row_scratch_bytes(e->n), 4);
   const int64_t fit = std::max<int64_t>(1, (int64_t)(((size_t)4 << 30) / per));
-  *ctas = (int)std::min<int64_t>(fapk::sssp_row_ctas(e->n, jobs, e->sm_count), fit);
+  *ctas = (int)std::min<int64_t>(fapk::sssp_row_ctas(e->n, sources, e->sm_count), fit);
   return e->sssp.tables.ensure(per * (size_t)*ctas);
 }
 
@@ -718,6 +719,10 @@ int build_plan(fap_engine *e, Plan &pl) {
         (bdy <= fapk::minplus_strip_max_k(e->f32()) && n < (1 << 24) ? mps : mps_deep).push_back(s);
       }
     }
+    for (SsspBatch &sb : batches) {
+      sb.first = (int32_t)G.nsources;
+      G.nsources += sb.count;
+    }
     G.nbatches = (int)batches.size();
     O.batches = tb.add(batches.data(), batches.size());
     if (pl.bsssp) {  // boundary-graph SSSP: each batch's sources as boundary indices, step-2 jobs
@@ -906,6 +911,7 @@ struct Issuer {
     sa.iw = e->d_iw;
     sa.batches = G.batches;
     sa.nbatches = G.nbatches;
+    sa.sources = G.nsources;
     sa.dist = pl.bdist ? pl.bdist : pl.dist;  // SSSP rows are the boundary rows
     sa.pred = pl.bdist ? pl.bpred : pl.pred;
     sa.scratch = e->sssp.tables.p;
@@ -952,7 +958,7 @@ struct Issuer {
       return FAP_OK;
     }
     if (pl.sssp_row) {
-      sa.slots = std::min(fapk::sssp_row_ctas(e->n, (int64_t)G.nbatches * sa.lanes, e->sm_count), pl.row_ctas);
+      sa.slots = std::min(fapk::sssp_row_ctas(e->n, G.nsources, e->sm_count), pl.row_ctas);
       FAP_CUDA(fapk::launch_sssp_rows(e->f32(), sa, e->sm_count, st));
       return FAP_OK;
     }
@@ -1306,12 +1312,13 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
   int rc;
   // work buffers
   size_t fw_elems = 0;
-  int64_t batches8 = 0, batches32 = 0;
+  int64_t batches8 = 0, batches32 = 0, sources = 0;
   for (int p : parts) {
     size_t ld = align_up((size_t)e->ver_num[p], (size_t)fapk::fw_block());
     fw_elems += ld * ld;
     batches8 += (e->bdy_num[p] + 7) / 8;
     batches32 += (e->bdy_num[p] + 31) / 32;
+    sources += e->bdy_num[p];
   }
   const bool acc64 = e->f32() && e->sssp_fp64;
   int lanes = e->sssp_lanes                        ? e->sssp_lanes
@@ -1352,8 +1359,7 @@ int run_parts(fap_engine *e, int mode, void *dist, int32_t *pred, const std::vec
     int slots = std::min(std::max(max_batches, 1), max_sssp_slots(e, wide));
     if ((rc = ensure_sssp_scratch(e, slots, wide)) != FAP_OK) return rc;
   }
-  if (row && (!bs || trial) && (rc = ensure_row_scratch(e, (int64_t)max_batches * lanes, &row_ctas, st)) != FAP_OK)
-    return rc;
+  if (row && (!bs || trial) && (rc = ensure_row_scratch(e, sources, &row_ctas, st)) != FAP_OK) return rc;
 
   Plan *pl = find_plan(e, mode, dist, pred, parts, offs, bdist, bpred, hdist, hpred, ring_elems);
   if (!pl) {
@@ -2360,6 +2366,7 @@ int fap_sssp(fap_engine *e, const int32_t *sources, int32_t num_sources, void *d
   for (int b0 = 0; b0 < num_sources; b0 += lanes) {
     SsspBatch sb{};
     sb.count = std::min(lanes, num_sources - b0);
+    sb.first = b0;
     for (int l = 0; l < sb.count; l++) {
       sb.src[l] = sources[b0 + l];
       sb.row_off[l] = (int64_t)(b0 + l) * ld;
@@ -2369,7 +2376,7 @@ int fap_sssp(fap_engine *e, const int32_t *sources, int32_t num_sources, void *d
   int rc;
   int slots = std::min((int)batches.size(), max_sssp_slots(e, wide));
   const bool row = sssp_row_form(e) && is_device_ptr(dist);
-  if (row) rc = ensure_row_scratch(e, (int64_t)batches.size() * lanes, &slots, st);
+  if (row) rc = ensure_row_scratch(e, num_sources, &slots, st);
   else rc = ensure_sssp_scratch(e, slots, wide);
   if (rc != FAP_OK) return rc;
   if ((rc = e->small.ensure(batches.size() * sizeof(SsspBatch))) != FAP_OK) return rc;
@@ -2385,6 +2392,7 @@ int fap_sssp(fap_engine *e, const int32_t *sources, int32_t num_sources, void *d
   sa.iw = e->d_iw;
   sa.batches = static_cast<const SsspBatch *>(e->small.p);
   sa.nbatches = (int)batches.size();
+  sa.sources = num_sources;
   sa.dist = dist;
   sa.pred = pred;
   sa.scratch = e->sssp.tables.p;

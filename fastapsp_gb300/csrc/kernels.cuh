@@ -112,6 +112,7 @@ struct MatRef {
 // given as element offsets into the output arrays.
 struct SsspBatch {
   int32_t count;
+  int32_t first;  // sources in the batches before it (sssp_row.cu)
   int32_t src[32];
   int64_t row_off[32];
 };

@@ -85,6 +85,7 @@ struct SsspArgs {
   const void *iw;
   const SsspBatch *batches;
   int32_t nbatches;
+  int64_t sources;            // launch_sssp_rows: sources of all batches
   void *dist;                 // output base (rows addressed by SsspBatch::row_off)
   int32_t *pred;              // may be null
   void *scratch;              // per-slot scratch, sssp_slot_bytes(n, acc64 && lanes == 32) each
@@ -119,7 +120,7 @@ int sssp_threads();
 cudaError_t launch_sssp(bool f32, const SsspArgs &a, cudaStream_t st);
 
 // sssp_row.cu: the same search and rows with one CTA per source (4-byte
-// distances; the batch width plays no part).  slots = CTAs
+// distances; the batch width only lists the sources).  slots = CTAs
 // (sssp_row_ctas), scratch = slots * sssp_row_scratch_bytes(n), dist in device
 // memory.
 bool sssp_row_fits(int32_t n, int32_t max_deg);  // bitmaps fit in shared memory, no vertex has too many edges
@@ -127,7 +128,7 @@ bool sssp_row_fits(int32_t n, int32_t max_deg);  // bitmaps fit in shared memory
 cudaError_t launch_row_edges(int64_t m, const int32_t *ro, const int32_t *col, const void *w, void *edges,
                              cudaStream_t st);
 size_t sssp_row_scratch_bytes(int32_t n);
-int sssp_row_ctas(int32_t n, int64_t jobs, int sm_count);
+int sssp_row_ctas(int32_t n, int64_t sources, int sm_count);
 cudaError_t init_sssp_row_kernels();
 cudaError_t launch_sssp_rows(bool f32, const SsspArgs &a, int sm_count, cudaStream_t st);
 

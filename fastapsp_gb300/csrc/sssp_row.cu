@@ -82,8 +82,8 @@ template <bool SMEM>
 __host__ __device__ inline size_t row_smem_bytes(int32_t n) {
   return (size_t)2 * kRowCap * sizeof(uint2) + (size_t)3 * row_words(n) * 4 + (SMEM ? (size_t)n * 4 : 0);
 }
-inline RowForm row_form(int32_t n, int64_t jobs, int sm_count) {
-  if (jobs > sm_count) return kRowMany;
+inline RowForm row_form(int32_t n, int64_t sources, int sm_count) {
+  if (sources > sm_count) return kRowMany;
   return row_smem_bytes<true>(n) <= kRowSmem ? kRowFewSmem : kRowFew;
 }
 
@@ -97,6 +97,17 @@ __device__ __forceinline__ bool row_set_bit(unsigned *bits, int v) {
 template <bool SMEM>
 __device__ __forceinline__ unsigned row_dist(const unsigned *d, int v) {
   return SMEM ? d[v] : __ldcg(d + v);
+}
+
+// The batch of a search's source number `job`: batches hold at most a.lanes, so
+// it is no earlier than job / a.lanes (and there where they are full); a warp
+// probes 32 at a time.
+__device__ __forceinline__ int row_batch(const SsspArgs &a, int64_t job) {
+  const int lane = threadIdx.x & 31;
+  for (int b = (int)(job / a.lanes);; b += 31) {
+    const unsigned from = __ballot_sync(0xffffffffu, b + lane < a.nbatches && a.batches[b + lane].first <= job);
+    if (from != 0xffffffffu) return b + __popc(from) - 1;
+  }
 }
 
 // Predecessor of v at distance bits dk (below "unreached").
@@ -157,10 +168,9 @@ __global__ void __launch_bounds__(kRowThreadsOf<SMEM, WIDE>, WIDE ? 1 : 4)
     else over[(size_t)par * n + i] = x;
   };
   unsigned long long st_steps = 0, st_splits = 0, st_relaxed = 0, st_scanned = 0, st_batches = 0;
-  for (int64_t job = blockIdx.x; job < (int64_t)a.nbatches * a.lanes; job += gridDim.x) {
-    const SsspBatch &sb = a.batches[job / a.lanes];
-    const int slot = (int)(job % a.lanes);
-    if (slot >= sb.count) continue;
+  for (int64_t job = blockIdx.x; job < a.sources; job += gridDim.x) {
+    const SsspBatch &sb = a.batches[row_batch(a, job)];
+    const int slot = (int)(job - sb.first);
     const int src = sb.src[slot];
     unsigned *const row = static_cast<unsigned *>(a.dist) + sb.row_off[slot];
     unsigned *const d = SMEM ? s_dist : row;
@@ -367,11 +377,11 @@ cudaError_t launch_rows_t(const SsspArgs &a, RowForm form, cudaStream_t st) {
 
 size_t sssp_row_scratch_bytes(int32_t n) { return row_scratch(n); }
 
-int sssp_row_ctas(int32_t n, int64_t jobs, int sm_count) {
-  if (row_form(n, jobs, sm_count) != kRowMany) return (int)jobs;
+int sssp_row_ctas(int32_t n, int64_t sources, int sm_count) {
+  if (row_form(n, sources, sm_count) != kRowMany) return (int)sources;
   const size_t smem = row_smem_bytes<false>(n) + 1024;
   const int per_sm = (int)std::min<size_t>(8, std::max<size_t>(1, (size_t)228 * 1024 / smem));
-  return (int)std::min<int64_t>(jobs, (int64_t)per_sm * sm_count);
+  return (int)std::min<int64_t>(sources, (int64_t)per_sm * sm_count);
 }
 
 cudaError_t launch_row_edges(int64_t m, const int32_t *ro, const int32_t *col, const void *w, void *edges,
@@ -406,9 +416,9 @@ cudaError_t init_sssp_row_kernels() {
 }
 
 cudaError_t launch_sssp_rows(bool f32, const SsspArgs &a, int sm_count, cudaStream_t st) {
-  if (a.nbatches <= 0 || a.slots <= 0) return cudaSuccess;
+  if (a.sources <= 0 || a.slots <= 0) return cudaSuccess;
   if (!sssp_row_fits(a.n, 0) || !(a.delta > 0.0) || a.row_edges == nullptr) return cudaErrorInvalidValue;
-  const RowForm form = row_form(a.n, (int64_t)a.nbatches * a.lanes, sm_count);
+  const RowForm form = row_form(a.n, a.sources, sm_count);
   const bool pred = a.pred != nullptr;
   if (f32) return pred ? launch_rows_t<float, true>(a, form, st) : launch_rows_t<float, false>(a, form, st);
   return pred ? launch_rows_t<uint32_t, true>(a, form, st) : launch_rows_t<uint32_t, false>(a, form, st);

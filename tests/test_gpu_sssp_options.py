@@ -1,4 +1,5 @@
-"""Options of the boundary searches on one engine, changed between solves."""
+"""The boundary searches of one engine: options changed between solves, parts with
+few boundary vertices."""
 import numpy as np
 import pytest
 import torch
@@ -56,3 +57,31 @@ def test_each_search_has_its_own_step(gpu):
         d, _, _ = solve(eng, g.n)
         # FP32 sums of at most n weights against one rounding
         assert bool(((d - d0).abs() <= g.n * 2.0 ** -24 * d).all())
+
+
+def test_parts_with_few_boundary_vertices(gpu):
+    """60 parts of a chain have 118 boundary vertices, whose lists of eight have 480
+    places: the search takes a CTA, and its scratch (24 bytes a vertex), a source."""
+    n, parts = 20001, 60
+    src = np.arange(n - 1)
+    g = graphs.csr_from_lines(n, src, src + 1, np.random.default_rng(1).integers(1, 9, n - 1), False, True)
+    gid = (np.arange(n) * parts // n + 1).astype(np.int32)
+    L = gpu._lib
+    with gpu.Engine(n, g.row_offset, g.col_val, g.weight, parts, graph_id=gid, dtype=gpu.DTYPE_F32) as eng:
+        info = [eng.part_info(q) for q in range(1, parts + 1)]
+        sources = sum(b for _, b, _ in info)
+        assert sources == 118
+        d = torch.empty((n, n), device="cuda")
+        p = torch.empty((n, n), dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        eng.solve(d, p)
+        torch.cuda.synchronize()
+        taken = before - torch.cuda.mem_get_info()[0]
+        closures = sum(8 * (-(-s // 64) * 64) ** 2 + 49152 for s, _, _ in info)
+        assert taken < closures + sources * 24 * n + (48 << 20)
+        e, q = torch.empty_like(d), torch.empty_like(p)
+        eng.set_option(L.OPT_SSSP_LANES, 8)
+        eng.solve(e, q)
+        torch.cuda.synchronize()
+        assert torch.equal(d, e) and torch.equal(p, q)
