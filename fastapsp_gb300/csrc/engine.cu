@@ -324,7 +324,7 @@ int ensure_sssp_scratch(fap_engine *e, int slots, bool wide = false) {
   return e->sssp.ensure(slots, wide, fapk::sssp_slot_bytes(e->n, wide), fapk::sssp_bits_bytes(e->n));
 }
 
-// CTAs of that search for `sources` sources, within a 4 GiB scratch budget; the
+// CTAs of that search for up to `sources` sources, within a 4 GiB scratch budget; the
 // scratch is the batched search's buffer.  The edge records are made on
 // first use, on the calling stream (calls end with a synchronize).
 int ensure_row_scratch(fap_engine *e, int64_t sources, int *ctas, cudaStream_t st) {
@@ -337,7 +337,7 @@ int ensure_row_scratch(fap_engine *e, int64_t sources, int *ctas, cudaStream_t s
   }
   const size_t per = std::max<size_t>(fapk::sssp_row_scratch_bytes(e->n), 4);
   const int64_t fit = std::max<int64_t>(1, (int64_t)(((size_t)4 << 30) / per));
-  *ctas = (int)std::min<int64_t>(fapk::sssp_row_ctas(e->n, sources, e->sm_count), fit);
+  *ctas = (int)std::min<int64_t>(fapk::sssp_row_ctas_up_to(e->n, e->m, sources, e->sm_count), fit);
   return e->sssp.tables.ensure(per * (size_t)*ctas);
 }
 
@@ -912,6 +912,7 @@ struct Issuer {
     sa.batches = G.batches;
     sa.nbatches = G.nbatches;
     sa.sources = G.nsources;
+    sa.m = e->m;
     sa.dist = pl.bdist ? pl.bdist : pl.dist;  // SSSP rows are the boundary rows
     sa.pred = pl.bdist ? pl.bpred : pl.pred;
     sa.scratch = e->sssp.tables.p;
@@ -958,7 +959,7 @@ struct Issuer {
       return FAP_OK;
     }
     if (pl.sssp_row) {
-      sa.slots = std::min(fapk::sssp_row_ctas(e->n, G.nsources, e->sm_count), pl.row_ctas);
+      sa.slots = std::min(fapk::sssp_row_ctas(e->n, e->m, G.nsources, e->sm_count), pl.row_ctas);
       FAP_CUDA(fapk::launch_sssp_rows(e->f32(), sa, e->sm_count, st));
       return FAP_OK;
     }
@@ -2393,10 +2394,12 @@ int fap_sssp(fap_engine *e, const int32_t *sources, int32_t num_sources, void *d
   sa.batches = static_cast<const SsspBatch *>(e->small.p);
   sa.nbatches = (int)batches.size();
   sa.sources = num_sources;
+  sa.m = e->m;
   sa.dist = dist;
   sa.pred = pred;
   sa.scratch = e->sssp.tables.p;
-  sa.slots = row ? slots : std::min(sa.nbatches, e->sssp.slots);
+  sa.slots = row ? std::min(slots, fapk::sssp_row_ctas(e->n, e->m, num_sources, e->sm_count))
+                 : std::min(sa.nbatches, e->sssp.slots);
   sa.bits = e->sssp.bits.p;
   sa.status = e->d_status;
   sa.maxd = nullptr;

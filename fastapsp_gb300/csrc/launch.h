@@ -85,7 +85,7 @@ struct SsspArgs {
   const void *iw;
   const SsspBatch *batches;
   int32_t nbatches;
-  int64_t sources;            // launch_sssp_rows: sources of all batches
+  int64_t sources, m;         // launch_sssp_rows: sources of all batches, edges
   void *dist;                 // output base (rows addressed by SsspBatch::row_off)
   int32_t *pred;              // may be null
   void *scratch;              // per-slot scratch, sssp_slot_bytes(n, acc64 && lanes == 32) each
@@ -128,7 +128,8 @@ bool sssp_row_fits(int32_t n, int32_t max_deg);  // bitmaps fit in shared memory
 cudaError_t launch_row_edges(int64_t m, const int32_t *ro, const int32_t *col, const void *w, void *edges,
                              cudaStream_t st);
 size_t sssp_row_scratch_bytes(int32_t n);
-int sssp_row_ctas(int32_t n, int64_t sources, int sm_count);
+int sssp_row_ctas(int32_t n, int64_t m, int64_t sources, int sm_count);
+int sssp_row_ctas_up_to(int32_t n, int64_t m, int64_t sources, int sm_count);  // ... or of any fewer sources
 cudaError_t init_sssp_row_kernels();
 cudaError_t launch_sssp_rows(bool f32, const SsspArgs &a, int sm_count, cudaStream_t st);
 

@@ -41,6 +41,15 @@ namespace {
 // a CTA an SM); 2,448 of 114,599 104 -> 27.8 (38 with the edge records).
 // Four lanes a vertex instead of one: 0.72 -> 0.58 and 3.1 -> 2.5 for few
 // sources, 6.0 -> 9.4 for 1,200 of 57,301.
+// Small CTAs also need their rows in L2, where their frontiers hop: on random
+// graphs of 100,000 vertices 1,500 sources took 474 ms (24 edges a vertex, 243 MB
+// of rows at once), the batched search 220; wide CTAs, one an SM, one source after
+// the other, 139.  12 edges 229 / 134 / 75, 6 edges 112 / 84 / 41; nearest-neighbour
+// graphs of 65,536 with 8 edges 321 / 311 / 170.  So where the graph has more than
+// four edges a vertex, rows past shared memory and more of them at once than L2
+// holds, the wide ones go on.  Below, frontiers are narrow (roads; 114,599 vertices
+// 18.7 ms against 24.4 in the wide form) or little is reached, and with shorter rows
+// small CTAs are as fast: 40,000 vertices of 24 edges 43.5 / 42.8, of 8 17.0 / 18.7.
 enum RowForm { kRowMany, kRowFew, kRowFewSmem };
 template <bool SMEM, bool WIDE>
 constexpr int kRowThreadsOf = SMEM ? 512 : WIDE ? 1024 : 256;
@@ -82,9 +91,17 @@ template <bool SMEM>
 __host__ __device__ inline size_t row_smem_bytes(int32_t n) {
   return (size_t)2 * kRowCap * sizeof(uint2) + (size_t)3 * row_words(n) * 4 + (SMEM ? (size_t)n * 4 : 0);
 }
-inline RowForm row_form(int32_t n, int64_t sources, int sm_count) {
-  if (sources > sm_count) return kRowMany;
-  return row_smem_bytes<true>(n) <= kRowSmem ? kRowFewSmem : kRowFew;
+constexpr int64_t kRowL2 = (int64_t)128 << 20;
+// CTAs of the form for many sources.
+inline int64_t many_ctas(int32_t n, int64_t sources, int sm_count) {
+  const size_t smem = row_smem_bytes<false>(n) + 1024;
+  return std::min<int64_t>(sources, (int64_t)std::min<size_t>(8, std::max<size_t>(1, (size_t)228 * 1024 / smem)) * sm_count);
+}
+inline RowForm row_form(int32_t n, int64_t m, int64_t sources, int sm_count) {
+  const bool fits = row_smem_bytes<true>(n) <= kRowSmem;
+  if (sources > sm_count && (fits || m <= 4 * (int64_t)n || many_ctas(n, sources, sm_count) * n * 4 <= kRowL2))
+    return kRowMany;
+  return fits ? kRowFewSmem : kRowFew;
 }
 
 __device__ __forceinline__ bool row_set_bit(unsigned *bits, int v) {
@@ -377,11 +394,15 @@ cudaError_t launch_rows_t(const SsspArgs &a, RowForm form, cudaStream_t st) {
 
 size_t sssp_row_scratch_bytes(int32_t n) { return row_scratch(n); }
 
-int sssp_row_ctas(int32_t n, int64_t sources, int sm_count) {
-  if (row_form(n, sources, sm_count) != kRowMany) return (int)sources;
-  const size_t smem = row_smem_bytes<false>(n) + 1024;
-  const int per_sm = (int)std::min<size_t>(8, std::max<size_t>(1, (size_t)228 * 1024 / smem));
-  return (int)std::min<int64_t>(sources, (int64_t)per_sm * sm_count);
+int sssp_row_ctas(int32_t n, int64_t m, int64_t sources, int sm_count) {
+  if (row_form(n, m, sources, sm_count) == kRowMany) return (int)many_ctas(n, sources, sm_count);
+  return (int)std::min<int64_t>(sources, sm_count);
+}
+
+int sssp_row_ctas_up_to(int32_t n, int64_t m, int64_t sources, int sm_count) {
+  const int ctas = sssp_row_ctas(n, m, sources, sm_count);
+  if (sources <= sm_count || row_form(n, m, sources, sm_count) == kRowMany) return ctas;
+  return std::max(ctas, (int)(kRowL2 / 4 / n));  // fewer sources take as many small CTAs as fit in L2
 }
 
 cudaError_t launch_row_edges(int64_t m, const int32_t *ro, const int32_t *col, const void *w, void *edges,
@@ -418,7 +439,7 @@ cudaError_t init_sssp_row_kernels() {
 cudaError_t launch_sssp_rows(bool f32, const SsspArgs &a, int sm_count, cudaStream_t st) {
   if (a.sources <= 0 || a.slots <= 0) return cudaSuccess;
   if (!sssp_row_fits(a.n, 0) || !(a.delta > 0.0) || a.row_edges == nullptr) return cudaErrorInvalidValue;
-  const RowForm form = row_form(a.n, a.sources, sm_count);
+  const RowForm form = row_form(a.n, a.m, a.sources, sm_count);
   const bool pred = a.pred != nullptr;
   if (f32) return pred ? launch_rows_t<float, true>(a, form, st) : launch_rows_t<float, false>(a, form, st);
   return pred ? launch_rows_t<uint32_t, true>(a, form, st) : launch_rows_t<uint32_t, false>(a, form, st);

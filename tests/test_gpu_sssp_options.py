@@ -1,5 +1,5 @@
 """The boundary searches of one engine: options changed between solves, parts with
-few boundary vertices."""
+few boundary vertices, many sources on graphs of many edges."""
 import numpy as np
 import pytest
 import torch
@@ -85,3 +85,27 @@ def test_parts_with_few_boundary_vertices(gpu):
         eng.solve(e, q)
         torch.cuda.synchronize()
         assert torch.equal(d, e) and torch.equal(p, q)
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("n, degree, sources", [(52001, 5, 700), (52001, 5, 640), (52001, 4, 700), (49000, 6, 750),
+                                                (230001, 5, 155)])
+def test_wide_ctas_in_turns_match_batches(gpu, f32, n, degree, sources):
+    """Past four edges a vertex, shared memory's rows and L2's: sources in turns of
+    one an SM; on either side of each line the rows of the batched search."""
+    g = graphs.small_random_graph(n, degree * n + (degree == 5), True, True, seed=n, integer=not f32)
+    src = np.random.default_rng(n).permutation(n)[:sources].astype(np.int32)
+    L = gpu._lib
+    with gpu.Engine(n, g.row_offset, g.col_val, g.weight, 1, graph_id=np.ones(n, np.int32),
+                    dtype=gpu.DTYPE_F32 if f32 else gpu.DTYPE_I32) as eng:
+        out = []
+        for lanes in (0, 32, 0):
+            eng.set_option(L.OPT_SSSP_LANES, lanes)
+            d = torch.empty((sources, n), dtype=torch.float32 if f32 else torch.int32, device="cuda")
+            p = torch.empty((sources, n), dtype=torch.int32, device="cuda")
+            eng.sssp(src, d, p)
+            eng.sssp(src[:200], d[:200], p[:200])  # fewer, with what the scratch holds
+            torch.cuda.synchronize()
+            out.append((d, p))
+        for d, p in out[1:]:
+            assert torch.equal(d, out[0][0]) and torch.equal(p, out[0][1])
