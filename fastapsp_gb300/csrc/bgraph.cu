@@ -450,20 +450,25 @@ size_t bg_smem_bytes(bool wide, int nodes) {
 
 // The sources of a CTA: eight, whose relaxations of a node share its edges, or
 // four, which make twice the CTAs and half the table: where eight do not give
-// the GPU enough CTAs, and where their table leaves an SM one CTA (that of 8-byte
-// distances does as soon as they give it enough).  SSSP phase
-// with eight and four, ms: road-like graphs of 8,000 vertices 0.60 / 0.48, 20,000
-// 0.92 / 0.77, 40,000 1.65 / 1.40 (960 boundary vertices), 80,000 5.54 / 5.14 (table),
-// 114,599 10.97 / 9.81 (table); geometric 20,000 0.44 / 0.40, 65,536 (1,848
-// boundary vertices) 1.35 / 1.37; near the line, road-like graphs of 57,301 with
-// 1,408 3.44 / 3.20, with fewer 2.57 / 2.70.
+// every SM a CTA, and where their table leaves an SM one CTA.  SSSP phase with
+// eight and four, ms (parts of about 900 vertices):
+//   8-byte distances, road-like graphs, boundary vertices: 120 0.55 / 0.48; 754 1.68 /
+//   1.50; 1,036 2.82 / 2.39; 1,180 3.40 / 3.19; 1,228 2.97 / 3.08; 1,272 3.32 / 3.57;
+//   1,355 3.06 / 3.31; 1,471 4.00 / 4.21; 1,533 4.48 / 4.62; and past the table's
+//   line (1,600) 1,713 5.72 / 5.32; 2,397 9.59 / 8.94.
+//   4-byte, road-like with whole weights: 754 1.28 / 1.14; 1,180 2.52 / 2.31; 1,297
+//   2.77 / 3.01; 1,355 2.20 / 2.46; 1,533 3.08 / 3.22; 2,397 5.70 / 5.92; grids: 621
+//   0.98 / 0.73; 1,054 1.63 / 1.26; 1,537 2.63 / 2.76; geometric: 1,089 0.770 / 0.770;
+//   1,818 1.35 / 1.38.
+// (Of one road-like graph with 1,365: 4.11 / 3.69.)
 int bg_lanes(bool wide, int nodes, int sm_count) {
-  return wide || nodes <= 10 * sm_count || bg_smem_bytes(wide, nodes) > 113 * 1024 ? kBgLanes / 2 : kBgLanes;
+  return nodes <= kBgLanes * sm_count || bg_smem_bytes(wide, nodes) > 113 * 1024 ? kBgLanes / 2 : kBgLanes;
 }
 
 cudaError_t init_bg_kernels() {
   cudaError_t e;
   if ((e = set_bg_attrs<uint32_t, 8>()) != cudaSuccess || (e = set_bg_attrs<uint32_t, 4>()) != cudaSuccess ||
+      (e = set_bg_attrs<unsigned long long, 8>()) != cudaSuccess ||
       (e = set_bg_attrs<unsigned long long, 4>()) != cudaSuccess ||
       (e = set_rows_attr<unsigned long long, 16, true>()) != cudaSuccess ||
       (e = set_rows_attr<unsigned long long, 32, true>()) != cudaSuccess ||
@@ -480,6 +485,7 @@ cudaError_t launch_bg_local(bool wide, int lanes, const BgArgs &a, int njobs, in
   if (smem > kBgSmemMax) return cudaErrorInvalidValue;
   ++launch_count();
   if (wide && lanes == 4) bg_local_kernel<unsigned long long, 4><<<njobs, kBgThreads, smem, st>>>(a);
+  else if (wide && lanes == 8) bg_local_kernel<unsigned long long, 8><<<njobs, kBgThreads, smem, st>>>(a);
   else if (!wide && lanes == 4) bg_local_kernel<uint32_t, 4><<<njobs, kBgThreads, smem, st>>>(a);
   else if (!wide && lanes == 8) bg_local_kernel<uint32_t, 8><<<njobs, kBgThreads, smem, st>>>(a);
   else return cudaErrorInvalidValue;
@@ -492,6 +498,7 @@ cudaError_t launch_bg_boundary(bool wide, int lanes, const BgArgs &a, int njobs,
   if (smem > kBgSmemMax) return cudaErrorInvalidValue;
   ++launch_count();
   if (wide && lanes == 4) bg_boundary_kernel<unsigned long long, 4><<<njobs, kBgThreads, smem, st>>>(a);
+  else if (wide && lanes == 8) bg_boundary_kernel<unsigned long long, 8><<<njobs, kBgThreads, smem, st>>>(a);
   else if (!wide && lanes == 4) bg_boundary_kernel<uint32_t, 4><<<njobs, kBgThreads, smem, st>>>(a);
   else if (!wide && lanes == 8) bg_boundary_kernel<uint32_t, 8><<<njobs, kBgThreads, smem, st>>>(a);
   else return cudaErrorInvalidValue;
