@@ -54,16 +54,11 @@ struct MpSmem {
   int32_t Bp[2][kBK][kTile];
 };
 
-// Block index of list entry g of 0..nblocks-1 without block `skip` (and
-// `skip2`, when it is above `skip`), or of the one-block list `fix`; -1 past
-// the list.
-__device__ __forceinline__ int list_block(int g, int skip, int skip2, int fix, int nblocks) {
+// Block index of list entry g of 0..nblocks-1 without block `skip`, or of the
+// one-block list `fix`; -1 past the list.
+__device__ __forceinline__ int list_block(int g, int skip, int fix, int nblocks) {
   if (fix >= 0) return g == 0 ? fix : -1;
-  int b = g;
-  if (skip >= 0) {
-    if (b >= skip) b++;
-    if (skip2 > skip && b >= skip2) b++;
-  }
+  const int b = skip >= 0 && g >= skip ? g + 1 : g;
   return b < nblocks ? b : -1;
 }
 
@@ -147,8 +142,8 @@ __device__ __forceinline__ TileGeom tile_geom(const MpSegment &s, int tile) {
   const int nbr = (s.M + kBlk - 1) / kBlk, nbc = (s.N + kBlk - 1) / kBlk;
 #pragma unroll
   for (int i = 0; i < 2; i++) {
-    int rb = list_block(2 * tyt + i, s.row_skip, s.row_skip2, s.row_fix, nbr);
-    int cb = list_block(2 * txt + i, s.col_skip, s.col_skip2, s.col_fix, nbc);
+    int rb = list_block(2 * tyt + i, s.row_skip, s.row_fix, nbr);
+    int cb = list_block(2 * txt + i, s.col_skip, s.col_fix, nbc);
     g.rbase[i] = rb >= 0 ? rb * kBlk : -1;
     g.cbase[i] = cb >= 0 ? cb * kBlk : -1;
   }
@@ -355,13 +350,12 @@ __device__ __forceinline__ void strip_load_rows(unsigned *dst, const unsigned *s
 }
 
 // Sets the bits of kmask for the warp's rows of a B tile (two rows of 16
-// lanes for TN = 64, starting at lane 0's row kk, which is even; one row for
-// TN = 128) that have a finite entry: one ballot and one atomic per warp.
-template <int TN>
+// lanes, starting at lane 0's row kk, which is even) that have a finite entry:
+// one ballot and one atomic per warp.
 __device__ __forceinline__ void strip_mark_rows(unsigned *kmask, int kk, bool fin) {
   const unsigned bal = __ballot_sync(0xffffffffu, fin);
   if ((threadIdx.x & 31) == 0) {  // lane 0 holds the warp's first (even) row
-    const unsigned bits = TN == 64 ? ((bal & 0xffffu) ? 1u : 0u) | ((bal >> 16) ? 2u : 0u) : (bal ? 1u : 0u);
+    const unsigned bits = ((bal & 0xffffu) ? 1u : 0u) | ((bal >> 16) ? 2u : 0u);
     if (bits) atomicOr(&kmask[kk >> 5], bits << (kk & 31));
   }
 }
@@ -369,16 +363,16 @@ __device__ __forceinline__ void strip_mark_rows(unsigned *kmask, int kk, bool fi
 // Turns the B values this thread copied (same mapping as strip_load_rows)
 // into keys (d << 7) | (k + 1), and sets bit k of kmask (a 128-bit mask in
 // shared memory) for every row k that has a finite entry in the tile.
-// F32 (TN = 64): the values stay (FP32 bits, "unreached" = the bits of 1e8);
+// F32: the values stay (FP32 bits, "unreached" = the bits of 1e8);
 // the row bits are set and the values are also written to Bq, the tile's
 // copy by step group (word 4 (g TN + col) + q is step 4g + q of column col).
 // ks is a multiple of 4, so a warp's rows are all below ks or all at or past
 // it, and the warp's lanes run the loop together.
-template <int TN, bool F32 = false>
+template <bool F32>
 __device__ __forceinline__ void strip_keys_b(unsigned *Bs, int ks, unsigned *kmask,
-                                             unsigned *Bq = nullptr) {
-  static_assert(TN == 64 || TN == 128, "row marks assume 16 or 32 lanes a row");
-  constexpr int TPR = TN / 4;
+                                             unsigned *Bq) {
+  constexpr int TN = kStripCols, TPR = TN / 4;
+  static_assert(TPR == 16, "row marks assume 16 lanes a row");
   const int t = threadIdx.x;
   const int j = (t % TPR) * 4;
   for (int kk = t / TPR; kk < ks; kk += kThreads / TPR) {
@@ -386,7 +380,7 @@ __device__ __forceinline__ void strip_keys_b(unsigned *Bs, int ks, unsigned *kma
     const unsigned idx = (unsigned)(kk & kMaxPackedK) + 1u;
     uint4 v = *p;
     if (F32) {
-      strip_mark_rows<TN>(kmask, kk, min(min(v.x, v.y), min(v.z, v.w)) < __float_as_uint(Dist<float>::inf()));
+      strip_mark_rows(kmask, kk, min(min(v.x, v.y), min(v.z, v.w)) < __float_as_uint(Dist<float>::inf()));
       unsigned *q = Bq + ((kk >> 2) * TN + j) * 4 + (kk & 3);
       q[0] = v.x;
       q[4] = v.y;
@@ -400,7 +394,7 @@ __device__ __forceinline__ void strip_keys_b(unsigned *Bs, int ks, unsigned *kma
     v.z = (min(v.z, kPackH) << kIdxBits) | idx;
     v.w = (min(v.w, kPackH) << kIdxBits) | idx;
     *p = v;
-    strip_mark_rows<TN>(kmask, kk, fin);
+    strip_mark_rows(kmask, kk, fin);
   }
 }
 
@@ -632,7 +626,7 @@ __global__ void __launch_bounds__(kThreads, F32 ? 2 : 3)
         if (__any_sync(0xffffffffu, F32 ? v < INF : v < kPackH) && (threadIdx.x & 31) == 0)
           atomicOr(&s_amask[kk >> 5], 1u << (kk & 31));
       }
-    strip_keys_b<TN, F32>(Bcur, kseg, s_kmask[buf], Bq);
+    strip_keys_b<F32>(Bcur, kseg, s_kmask[buf], Bq);
     // List the tile's own columns (threads 0..TN-1 copied their column's
     // flags; slots are taken in any order through a counter).
     if (threadIdx.x == 0) s_own[buf ^ 1] = 0;  // used by the next tile
