@@ -29,7 +29,9 @@
 // vertices 23.9 -> 18.9 ms; 512 int32 matrices of 32 to 2,048 (a cluster of
 // four CTAs a matrix, walking its panel blocks) 58.2 -> 51.3 ms.  Of the chain
 // of one FP32 matrix (39 us at 2.07 GHz): loads 3, each 64^3 product 4 (32
-// add-mins a cycle on its one SM), the closure 9, its steps 2.6.
+// add-mins a cycle on its one SM), the closure 9, its steps 2.6.  At two CTAs an
+// SM the kernels have 64 registers a thread, and the FP32 ones with predecessors
+// spill (stores / loads: closing 56 / 80 bytes, panels 184 / 108).
 
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -476,15 +476,14 @@ __device__ __forceinline__ void addmin_groups_rows_f32(unsigned (&acc)[8][4], in
   }
 }
 
-// TN = 64 (the class K <= 48): 128x64 tiles, 8x4 outputs per thread, up to
-// three CTAs per SM.  TN = 128 (the class K <= 100): 128x128 tiles, 8x8
-// outputs per thread, up to two CTAs per SM.
-// F32: FP32 distances (any range).  The product keeps each output's value
-// bits and the step idx (k + 1, 0 = none) of its last strict improvement in
-// two registers: fl(a + b), then __vibmin_u32 for the minimum and whether the
-// current value was kept (non-negative floats order like their bits) -- the
-// reference's strict-<, ascending-k rule, as in the packed form.  Two
-// CTAs per SM.
+// 128x64 tiles, 8x4 outputs per thread; packed keys three CTAs per SM.
+// F32: FP32 distances (any range), two CTAs per SM.  The product keeps each
+// output's value bits (non-negative floats order like them) and which step
+// made its last strict improvement: in groups of four steps
+// (addmin_groups_rows_f32) where at least half of the tile's steps are active,
+// else step by step (fl(a + b), then __vibmin_u32 for the minimum and whether
+// the current value was kept).  Either is the reference's strict-<,
+// ascending-k rule, as the packed form's.
 template <bool PRED, bool F32>
 __global__ void __launch_bounds__(kThreads, F32 ? 2 : 3)
     mp_strip_kernel(const MpSegment *__restrict__ segs, int nseg, int ks, int per) {

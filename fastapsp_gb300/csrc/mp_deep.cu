@@ -5,10 +5,11 @@
 // MatrixMulCUDA6_path, fap/kernel/cuda/minplus.cu:32-189).
 //
 // C = A (x) B for the products that the strip kernel (minplus.cu) does not
-// take: more than 100 steps, leading dimensions of 2^24 and above, and int32
-// values outside the packed range.  Every add-min is an instruction on the
-// integer pipe, so that pipe bounds the kernel, and what counts is how few
-// other instructions it sees:
+// take: in a solve, parts of more than 48 boundary vertices (FP32 40); called
+// directly, more than 40 steps or fewer than 6 million outputs; and leading
+// dimensions of 2^24 and above, and int32 values outside the packed range.  Every
+// add-min is an instruction on the integer pipe, so that pipe bounds the kernel,
+// and what counts is how few other instructions it sees:
 //
 //  - Packed int32 (finite results below 2^24 - 1): one __viaddmin_u32 an
 //    add-min on keys (d << 7) | idx, where idx counts within a chunk of 64

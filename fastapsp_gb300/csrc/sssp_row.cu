@@ -46,8 +46,8 @@ namespace {
 // of rows at once), the batched search 220; wide CTAs, one an SM, one source after
 // the other, 139.  12 edges 229 / 134 / 75, 6 edges 112 / 84 / 41; nearest-neighbour
 // graphs of 65,536 with 8 edges 321 / 311 / 170.  So where the graph has more than
-// four edges a vertex, rows past shared memory and more of them at once than L2
-// holds, the wide ones go on.  Below, frontiers are narrow (roads; 114,599 vertices
+// four edges a vertex, rows do not fit in shared memory and those of the small
+// CTAs launched come to more than L2, the wide ones go on.  Below, frontiers are narrow (roads; 114,599 vertices
 // 18.7 ms against 24.4 in the wide form) or little is reached, and with shorter rows
 // small CTAs are as fast: 40,000 vertices of 24 edges 43.5 / 42.8, of 8 17.0 / 18.7.
 enum RowForm { kRowMany, kRowFew, kRowFewSmem };
