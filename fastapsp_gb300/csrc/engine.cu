@@ -283,11 +283,20 @@ bool sssp_row_form(const fap_engine *e) {
   return !(e->f32() && e->sssp_fp64) && e->sssp_lanes == 0 && fapk::sssp_row_fits(e->n, e->max_deg);
 }
 
-// Near-far step of that search in mean edge weights.  Measured on road graphs
-// of 4,801 to 114,599 vertices, a grid and a nearest-neighbour graph, with 16
-// to 2,448 sources: 64 is within 5 % of the best of 2 to 512 on each (8, the
-// batched search's, 5 to 30 % slower), so no trial runs choose it.
-constexpr double kRowDelta = 64.0;
+// Near-far step of that search in mean edge weights, by edges a vertex; no trial
+// runs choose it.  Up to 3.5 (road graphs of 4,801 to 114,599 vertices, grids, three
+// nearest neighbours, 16 to 2,448 sources) 64 is within 5 % of the best of 2 to 512
+// on each (8, the batched search's, 5 to 30 % slower).  The more edges, the more a
+// long step relaxes in vain.  Best steps, and ms there and at 64 (1,000 sources):
+// nearest-neighbour graphs of 65,536 vertices with 4 edges 4 to 8, 9.9 / 22.8; 5 edges
+// 6, 20.0 / 49.3; 8 edges 3, 21.7 / 120; 20 edges 0.5, 39.8 / 354; random graphs of
+// 100,000 with 6 edges 0.5 to 4, 16.0 to 17.8 / 29.0; 24 edges 0.5, 48.7 / 94.1; a full
+// grid of 40,000 (4 edges) 12 to 64, 2.73 / 2.71.  190 / edges^2, at least a half, is
+// within 15 % of the best on each.
+double row_delta(const fap_engine *e) {
+  const double edges = (double)e->m / std::max(e->n, 1);
+  return edges <= 3.5 ? 64.0 : std::max(0.5, 190.0 / (edges * edges));
+}
 
 // Near-far step of a search: with one CTA per source (row), or batched.
 double sssp_delta_of(const fap_engine *e, bool row) {
@@ -295,7 +304,7 @@ double sssp_delta_of(const fap_engine *e, bool row) {
   if (e->sssp_delta > 0) return e->sssp_delta;
   if (!row && e->sssp_delta_tuned > 0) return e->sssp_delta_tuned;
   // a few mean edge weights per near-far step (at least one unit for int32)
-  double d = (row ? kRowDelta : 8.0) * e->wmean;
+  double d = (row ? row_delta(e) : 8.0) * e->wmean;
   return e->f32() ? std::max(d, 1e-30) : std::max(1.0, std::floor(d));
 }
 

@@ -190,10 +190,11 @@ int fap_precondition(fap_engine *e);
  *                      Dijkstra.
  *   FAP_OPT_SSSP_DELTA near-far threshold step of the SSSP in distance units
  *                      (0 = automatic).  Changes speed only, never results.
- *                      Automatic is 64 x the mean weight where the search
- *                      runs one CTA per source (4-byte distances, automatic
- *                      batch width, no vertex of more than 64 edges), else
- *                      8 x, or what FAP_OPT_AUTOTUNE finds for it.
+ *                      Automatic is 64 x the mean weight (12 x to 0.5 x from
+ *                      3.5 edges a vertex on) where the search runs one CTA
+ *                      per source (4-byte distances, automatic batch width, no
+ *                      vertex of more than 64 edges), else 8 x, or what
+ *                      FAP_OPT_AUTOTUNE finds for it.
  *   FAP_OPT_AUTOTUNE   1 (default) = while the step is automatic, the first
  *                      run of a solve with the batched search times the SSSP
  *                      phase with a few steps (multiples of the mean edge

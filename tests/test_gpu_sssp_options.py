@@ -109,3 +109,27 @@ def test_wide_ctas_in_turns_match_batches(gpu, f32, n, degree, sources):
             out.append((d, p))
         for d, p in out[1:]:
             assert torch.equal(d, out[0][0]) and torch.equal(p, out[0][1])
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("degree, factor", [(3, 64.0), (4, 190 / 16), (8, 190 / 64), (24, 0.5)])
+def test_step_by_edges_a_vertex(gpu, f32, degree, factor):
+    """The automatic step of the search with one CTA per source shortens with the
+    edges a vertex has; the rows do not depend on it."""
+    n = 3001
+    g = graphs.small_random_graph(n, degree * n, True, True, seed=degree)
+    mean = float(np.mean(g.weight.astype(np.float64)))
+    want = factor * mean if f32 else max(1.0, np.floor(factor * mean))
+    src = np.arange(0, n, 7, dtype=np.int32)
+    with gpu.Engine(n, g.row_offset, g.col_val, g.weight, 1, graph_id=np.ones(n, np.int32),
+                    dtype=gpu.DTYPE_F32 if f32 else gpu.DTYPE_I32) as eng:
+        assert eng.get_option(gpu._lib.OPT_SSSP_DELTA) == pytest.approx(want)
+        out = []
+        for delta in (0.0, 64 * mean):
+            eng.set_option(gpu._lib.OPT_SSSP_DELTA, delta)
+            d = torch.empty((len(src), n), dtype=torch.float32 if f32 else torch.int32, device="cuda")
+            p = torch.empty((len(src), n), dtype=torch.int32, device="cuda")
+            eng.sssp(src, d, p)
+            torch.cuda.synchronize()
+            out.append((d, p))
+        assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
