@@ -41,15 +41,17 @@ namespace {
 // a CTA an SM); 2,448 of 114,599 104 -> 27.8 (38 with the edge records).
 // Four lanes a vertex instead of one: 0.72 -> 0.58 and 3.1 -> 2.5 for few
 // sources, 6.0 -> 9.4 for 1,200 of 57,301.
-// Small CTAs also need their rows in L2, where their frontiers hop: on random
-// graphs of 100,000 vertices 1,500 sources took 474 ms (24 edges a vertex, 243 MB
-// of rows at once), the batched search 220; wide CTAs, one an SM, one source after
-// the other, 139.  12 edges 229 / 134 / 75, 6 edges 112 / 84 / 41; nearest-neighbour
-// graphs of 65,536 with 8 edges 321 / 311 / 170.  So where the graph has more than
-// four edges a vertex, rows do not fit in shared memory and those of the small
-// CTAs launched come to more than L2, the wide ones go on.  Below, frontiers are narrow (roads; 114,599 vertices
-// 18.7 ms against 24.4 in the wide form) or little is reached, and with shorter rows
-// small CTAs are as fast: 40,000 vertices of 24 edges 43.5 / 42.8, of 8 17.0 / 18.7.
+// Small CTAs hold many rows at once, and frontiers that hop over a large graph read
+// them from device memory: 1,500 sources of random graphs of 100,000 vertices (608
+// CTAs, 243 MB of rows) with 24 edges a vertex took 232 ms, the batched search 220; wide
+// CTAs, one an SM, one source after the other, 70.  12 edges 131 / 134 / 44, 6 edges
+// 90 / 83 / 36; 200,000 vertices with 20 edges 244 / 415 / 174; nearest-neighbour graphs
+// of 200,000 with 8 edges 100 / 90 (small / wide).  So past four edges a vertex and 220 MB
+// of rows the wide ones go on.  Below, it is the graph that decides: nearest-neighbour ones of 52,000 with 8 edges (190 MB)
+// 18.7 / 25.7, 65,536 with 5 and 8 (199 MB) 25.3 / 28.1 and 35.1 / 30.4, 114,000 with 5 (208
+// MB) 39.9 / 45.1; random ones of 64,000 with 12 (195 MB) 37.5 / 27.0.  With fewer edges
+// frontiers are narrow (roads; 114,599 vertices 18.7 / 24.4; a full grid of 202,500 with
+// 608 sources 9.4 / 10.0) or little is reached.
 enum RowForm { kRowMany, kRowFew, kRowFewSmem };
 template <bool SMEM, bool WIDE>
 constexpr int kRowThreadsOf = SMEM ? 512 : WIDE ? 1024 : 256;
@@ -91,17 +93,16 @@ template <bool SMEM>
 __host__ __device__ inline size_t row_smem_bytes(int32_t n) {
   return (size_t)2 * kRowCap * sizeof(uint2) + (size_t)3 * row_words(n) * 4 + (SMEM ? (size_t)n * 4 : 0);
 }
-constexpr int64_t kRowL2 = (int64_t)128 << 20;
+constexpr int64_t kRowManyBytes = (int64_t)220 << 20;  // of the rows that small CTAs hold
 // CTAs of the form for many sources.
 inline int64_t many_ctas(int32_t n, int64_t sources, int sm_count) {
   const size_t smem = row_smem_bytes<false>(n) + 1024;
   return std::min<int64_t>(sources, (int64_t)std::min<size_t>(8, std::max<size_t>(1, (size_t)228 * 1024 / smem)) * sm_count);
 }
 inline RowForm row_form(int32_t n, int64_t m, int64_t sources, int sm_count) {
-  const bool fits = row_smem_bytes<true>(n) <= kRowSmem;
-  if (sources > sm_count && (fits || m <= 4 * (int64_t)n || many_ctas(n, sources, sm_count) * n * 4 <= kRowL2))
+  if (sources > sm_count && (m <= 4 * (int64_t)n || many_ctas(n, sources, sm_count) * n * 4 <= kRowManyBytes))
     return kRowMany;
-  return fits ? kRowFewSmem : kRowFew;
+  return row_smem_bytes<true>(n) <= kRowSmem ? kRowFewSmem : kRowFew;
 }
 
 __device__ __forceinline__ bool row_set_bit(unsigned *bits, int v) {
@@ -402,7 +403,7 @@ int sssp_row_ctas(int32_t n, int64_t m, int64_t sources, int sm_count) {
 int sssp_row_ctas_up_to(int32_t n, int64_t m, int64_t sources, int sm_count) {
   const int ctas = sssp_row_ctas(n, m, sources, sm_count);
   if (sources <= sm_count || row_form(n, m, sources, sm_count) == kRowMany) return ctas;
-  return std::max(ctas, (int)(kRowL2 / 4 / n));  // fewer sources take as many small CTAs as fit in L2
+  return std::max(ctas, (int)(kRowManyBytes / 4 / n));  // fewer sources take small CTAs up to the line
 }
 
 cudaError_t launch_row_edges(int64_t m, const int32_t *ro, const int32_t *col, const void *w, void *edges,

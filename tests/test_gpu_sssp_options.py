@@ -88,11 +88,11 @@ def test_parts_with_few_boundary_vertices(gpu):
 
 
 @pytest.mark.parametrize("f32", [False, True])
-@pytest.mark.parametrize("n, degree, sources", [(52001, 5, 700), (52001, 5, 640), (52001, 4, 700), (49000, 6, 750),
-                                                (230001, 5, 155)])
+@pytest.mark.parametrize("n, degree, sources", [(100001, 5, 580), (100001, 5, 570), (100001, 4, 580),
+                                                (230001, 5, 255)])
 def test_wide_ctas_in_turns_match_batches(gpu, f32, n, degree, sources):
-    """Past four edges a vertex, shared memory's rows and L2's: sources in turns of
-    one an SM; on either side of each line the rows of the batched search."""
+    """Past four edges a vertex and 220 MB of rows at once: sources in turns of one an
+    SM; on either side of each line the rows of the batched search."""
     g = graphs.small_random_graph(n, degree * n + (degree == 5), True, True, seed=n, integer=not f32)
     src = np.random.default_rng(n).permutation(n)[:sources].astype(np.int32)
     L = gpu._lib
