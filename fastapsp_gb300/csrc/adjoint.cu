@@ -16,6 +16,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "kernels.cuh"
 #include "launch.h"
 #include "path_walk.cuh"
@@ -137,7 +139,9 @@ __global__ void backward_dense_kernel(const DenseInst *__restrict__ inst, int32_
 
 }  // namespace
 
-bool pairs_by_row(int32_t n, int32_t walks) { return n <= kWalkMaxN && (int64_t)n * walks <= kWalkPairs; }
+bool pairs_by_row(int32_t n, int32_t walks) {
+  return walks_by_row(n, walks, std::min<int64_t>(12500, 8 * (int64_t)n), 100000000);
+}
 
 cudaError_t init_backward_kernels() {
   return cudaFuncSetAttribute(backward_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -2081,7 +2081,7 @@ int fap_query(fap_engine *e, const void *dist, const int32_t *pred, int32_t nq, 
   a.out_path = out_path;
   a.max_len = max_len;
   a.status = e->d_status;
-  a.nrest = fapk::queries_by_row(e->n, nq) ? walk_scratch(e, nq) : nullptr;
+  a.nrest = fapk::queries_by_row(e->n, nq, out_path != nullptr) ? walk_scratch(e, nq) : nullptr;
   a.rest = a.nrest ? a.nrest + 1 : nullptr;
   FAP_CUDA(fapk::launch_query(e->f32(), a, e->sm_count, st));
   FAP_CUDA(cudaStreamSynchronize(st));

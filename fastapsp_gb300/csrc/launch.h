@@ -203,7 +203,7 @@ struct QueryArgs {
   unsigned *status;
   int32_t *nrest, *rest;   // scratch: a counter and nq entries (null: queries_by_row() is false)
 };
-bool queries_by_row(int32_t n, int32_t walks);
+bool queries_by_row(int32_t n, int32_t walks, bool paths);
 cudaError_t init_query_kernels();
 cudaError_t launch_query(bool f32, const QueryArgs &a, int sm_count, cudaStream_t st);
 

@@ -8,14 +8,23 @@
 // vertices then runs over all of them at once.
 //
 // A row costs what it is long, and the chain does not care how many walk beside
-// it, so rows are for few walks or short rows: walks x vertices up to
-// kWalkQueries (a query in device memory walks twice) or kWalkPairs.  Walks of 100
-// to 222 hops on road graphs, by rows / in device memory, queries and pairs: 4,096
-// vertices 10,000 walks 111 / 529 us and 129 / 191 us, 200,000 walks 1,256 / 711 and
-// 1,419 / 491; 8,000 vertices 10,000 walks 191 / 960 and 240 / 415, 200,000 walks
-// 2,717 / 1,684 and 3,267 / 799; 24,575 vertices 200 walks 58 / 1,200 and 60 / 544,
-// 10,000 walks 753 / 2,778 and 937 / 1,014, 200,000 walks 13,219 / 4,252 us.  Short
-// walks (dense graphs) are finished by the thread that started them and never
+// it, so rows are for few walks and short rows (walks_by_row).  A query with its
+// path walks twice in device memory, without it once and without the look-up of an
+// edge.  By rows / in device memory, us, queries with paths | without | pairs of
+// road graphs (hops on average):
+//   500 vertices (35)      10,000 walks  65 / 85 | 63 / 43 | 82 / 76,   100,000  268 / 162 | 257 / 46 | 371 / 315
+//   1,000 (54)              3,000  58 / 185 | 55 / 52 | 69 / 95,   30,000  156 / 243 | 147 / 52 | 177 / 139
+//   4,096 (102)             1,000  51 / 527 | 50 / 70 | 59 / 187,   10,000  115 / 530 | 111 / 74 | 133 / 188
+//                          30,000  249 / 604 | 240 / 84 | 275 / 198,   100,000  665 / 660 | 643 / 97 | 749 / 337
+//   8,000 (132)             3,000  100 / 755 | 99 / 89 | 113 / 309,   30,000  474 / 1,429 | 463 / 193 | 558 / 438
+//   14,000 (177)            1,000  87 / 980 | 86 / 109 | 104 / 437,   10,000  426 / 1,932 | 423 / 261 | 520 / 715
+//   28,000 (242)            1,000  149 / 1,278 | 148 / 142 | 185 / 638,   10,000  864 / 3,161 | 856 / 361 | 1,117 / 1,008
+// and of grids, whose walks are shorter:
+//   1,024 (23)             10,000  59 / 70 | 57 / 40 | 76 / 65,   100,000  209 / 107 | 201 / 41 | 262 / 153
+//   10,000 (69)             3,000  89 / 244 | 87 / 61 | 107 / 203,   30,000  444 / 387 | 436 / 112 | 541 / 270
+//   22,500 (103)            3,000  191 / 394 | 190 / 75 | 248 / 318,   10,000  509 / 378 | 497 / 100 | 669 / 347
+// (The line for queries with paths is the roads': grids lose up to a third near it.)
+// Short walks (dense graphs) are finished by the thread that started them and never
 // read a row: 8 hops at most left half of a random graph's walks of 8 hops on
 // average to rows of 25,000 vertices (10,000 walks 190 us, 46 us without).  Rows of
 // more than kWalkMaxN vertices (two CTAs an SM) are walked in device memory.
@@ -29,7 +38,11 @@ namespace fapk {
 constexpr int kWalkThreads = 256;
 constexpr int kWalkHops = 16;
 constexpr int kWalkMaxN = 28000;
-constexpr int64_t kWalkQueries = 400000000, kWalkPairs = 100000000;
+
+// Whether `walks` walks go by row: at most `most` of them, and walks x vertices.
+inline bool walks_by_row(int n, int64_t walks, int64_t most, int64_t cells) {
+  return n <= kWalkMaxN && walks <= most && walks * n <= cells;
+}
 
 // Entries of a row in shared memory that are no vertex.
 constexpr unsigned kWalkNone = 0xffffu, kWalkBad = 0xfffeu;  // (negative; n or above)

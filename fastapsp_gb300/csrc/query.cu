@@ -100,7 +100,9 @@ cudaError_t init_query_kernels() {
                               (int)walk_smem(kWalkMaxN));
 }
 
-bool queries_by_row(int32_t n, int32_t walks) { return n <= kWalkMaxN && (int64_t)n * walks <= kWalkQueries; }
+bool queries_by_row(int32_t n, int32_t walks, bool paths) {
+  return paths ? walks_by_row(n, walks, 30000, 400000000) : walks_by_row(n, walks, 2000, 15000000);
+}
 
 cudaError_t launch_query(bool f32, const QueryArgs &a, int sm_count, cudaStream_t st) {
   if (a.nq <= 0) return cudaSuccess;
