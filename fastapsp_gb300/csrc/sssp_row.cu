@@ -171,6 +171,8 @@ __global__ void __launch_bounds__(kRowThreadsOf<SMEM, WIDE>, WIDE ? 1 : 4)
   unsigned *const s_dist = farbits + words;
   __shared__ int s_near[3], s_far[2];
   __shared__ unsigned s_minfar;
+  __shared__ int s_src;
+  __shared__ int64_t s_row;
   uint2 *const over =
       reinterpret_cast<uint2 *>(static_cast<unsigned char *>(a.scratch) + (size_t)blockIdx.x * row_scratch(n));
   int32_t *const farq = reinterpret_cast<int32_t *>(over + 2 * (size_t)n);
@@ -187,13 +189,17 @@ __global__ void __launch_bounds__(kRowThreadsOf<SMEM, WIDE>, WIDE ? 1 : 4)
   };
   unsigned long long st_steps = 0, st_splits = 0, st_relaxed = 0, st_scanned = 0, st_batches = 0;
   for (int64_t job = blockIdx.x; job < a.sources; job += gridDim.x) {
-    const SsspBatch &sb = a.batches[row_batch(a, job)];
-    const int slot = (int)(job - sb.first);
-    const int src = sb.src[slot];
-    unsigned *const row = static_cast<unsigned *>(a.dist) + sb.row_off[slot];
+    if (warp == 0) {
+      const SsspBatch &sb = a.batches[row_batch(a, job)];
+      if (lane == 0) s_src = sb.src[job - sb.first], s_row = sb.row_off[job - sb.first];
+    }
+    __syncthreads();
+    const int src = s_src;
+    unsigned *const row = static_cast<unsigned *>(a.dist) + s_row;
     unsigned *const d = SMEM ? s_dist : row;
     if (src < 0 || src >= n) {
       if (tid == 0) atomicOr(a.status, kErrBadInput);
+      __syncthreads();
       continue;
     }
     for (int i = tid; i < n; i += nthr) d[i] = INF;
