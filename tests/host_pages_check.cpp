@@ -19,7 +19,7 @@ size_t resident(unsigned char *p, size_t bytes) {
 }
 
 unsigned char *fresh(size_t bytes) {
-  void *p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+  void *p = mmap(nullptr, bytes, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
   return p == MAP_FAILED ? nullptr : static_cast<unsigned char *>(p);
 }
 
@@ -30,7 +30,7 @@ int main() {
   std::printf("OK (pages are left to the copy here)\n");
   return 0;
 #else
-  const size_t small = (size_t)64 << 20, large = (size_t)1 << 30;
+  const size_t small = (size_t)64 << 20, large = (size_t)4 << 30;
   unsigned char *a = fresh(small), *b = fresh(large);
   if (!a || !b) return 1;
   if (madvise(a, (size_t)sysconf(_SC_PAGESIZE), MADV_POPULATE_WRITE) != 0) {
